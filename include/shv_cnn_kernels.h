@@ -94,6 +94,47 @@ int shvk_cnn_pointwise_h(const float* A, const float* W, const float* b, const f
  * Replaces launch_pool (engine/cuda/cnn.cu:133-160,188-191). */
 int shvk_cnn_pool_tokens(const float* in, float* out, int F, void* stream);
 
+/* ---------------------------------------------------------------- fused encoder of the bf16 / fp16 modes
+ * The kernels above are one layer each, for any shape; these are the network's own layers fused (dtype: SHVK_BF16 or
+ * SHVK_F16, the type the operands of the 1x1 convolutions are rounded to; feature maps stay float32, roundings are those
+ * of shvk_cnn_pointwise_h between shvk_cnn_depthwise and shvk_cnn_se_gate).  Weights of 1x1 convolutions come as 16-bit
+ * fragments written once by shvk_cnn_pack_weights into `out` (host memory, shvk_cnn_packed_bytes bytes, then copied to
+ * the device): order 0 for blocks and the last convolution, 1 for shvk_cnn_rows_gate, 2 for shvk_cnn_token_proj.
+ * W [N][K] float32 in host memory. */
+size_t shvk_cnn_packed_bytes(int N, int K, int order);
+int shvk_cnn_pack_weights(const float* w, int N, int K, int order, int dtype, void* out);
+
+/* Stem (as shvk_cnn_stem) and block 1 (depthwise 3x3 + ReLU, 1x1 16 -> 16, + input): out [F][90][160][16].
+ * stem_w_host, stem_b_host: HOST pointers, [27][16] and [16] (they travel as kernel parameters).
+ * Replaces launch_stem, launch_dw and gemm of the first block (engine/cuda/engine.cu:343-395). */
+int shvk_cnn_stem_block(const uint8_t* frames, const float* lut, const float* stem_w_host, const float* stem_b_host, const float* wd,
+                        const float* bd, const void* wp, const float* bp, float* out, int F, int dtype, void* stream);
+
+/* Inverted-residual block 2 .. 15: 1x1 expand + activation, depthwise + activation, and, where the block has no
+ * squeeze-excite gate (2, 3, 7 .. 10), 1x1 project (+ x where shapes agree) -> out [F][h][w][C].  Where it has one, out is
+ * the depthwise map [F][h][w][expanded] and sums [F][tiles][expanded] its sums over the tiles of the map
+ * (shvk_cnn_block_tiles, 0 for blocks without a gate).  out must not be x.  Weights are packed with zero rows / columns up
+ * to shvk_cnn_block_padding: expand [columns][in], project [out][k].
+ * Replaces gemm, launch_dw, launch_se_pool and gemm of a block (engine/cuda/engine.cu:349-395). */
+int shvk_cnn_block_tiles(int block);
+void shvk_cnn_block_padding(int block, int* columns, int* k);
+int shvk_cnn_block(int block, const float* x, const void* we, const float* be, const float* wd, const float* bd, const void* wp,
+                   const float* bp, float* out, float* sums, int F, int dtype, void* stream);
+
+/* shvk_cnn_se_gate from the sums of shvk_cnn_block: mean over HW pixels, fc1 + ReLU, fc2 + Hardsigmoid -> gate [F][C]. */
+int shvk_cnn_se_gate_sums(const float* sums, const float* w1, const float* b1, const float* w2, const float* b2, float* gate, int F,
+                          int tiles, int HW, int C, int CS, void* stream);
+
+/* 1x1 projection behind a gate: out[m][n] = sum_k (A[m][k] gate[m / gate_rows][k]) W[n][k] + b[n] (+ R[m][n]); N 40, 112 or
+ * 160; R may alias out. */
+int shvk_cnn_rows_gate(const float* A, const void* W, const float* b, const float* gate, int gate_rows, const float* R, float* out,
+                       int M, int N, int K, int dtype, void* stream);
+
+/* Last 1x1 convolution 160 -> 960 + Hardswish + the pooling of shvk_cnn_pool_tokens: x [F][60][160] -> pooled [F][16][960]
+ * rounded to dtype, and the token projection of `rows` pooled rows: tokens [rows][384] float32. */
+int shvk_cnn_last_pool(const float* x, const void* w, const float* b, void* pooled, int F, int dtype, void* stream);
+int shvk_cnn_token_proj(const void* pooled, const void* W, float* tokens, int rows, int dtype, void* stream);
+
 #if defined(__GNUC__)
 #pragma GCC visibility pop
 #endif

@@ -176,6 +176,16 @@ def load_library(experimental: bool = True) -> C.CDLL:
         "shvk_cnn_pointwise_tf32": (i32, [vp, vp, vp, vp, i32, vp, vp, i32, i32, i32, i32, vp]),
         "shvk_cnn_pointwise_h": (i32, [vp, vp, vp, vp, i32, vp, vp, i32, i32, i32, i32, i32, vp]),
         "shvk_cnn_pool_tokens": (i32, [vp, vp, i32, vp]),
+        "shvk_cnn_packed_bytes": (sz, [i32, i32, i32]),
+        "shvk_cnn_pack_weights": (i32, [vp, i32, i32, i32, i32, vp]),
+        "shvk_cnn_stem_block": (i32, [vp] * 9 + [i32, i32, vp]),
+        "shvk_cnn_block_tiles": (i32, [i32]),
+        "shvk_cnn_block_padding": (None, [i32, C.POINTER(i32), C.POINTER(i32)]),
+        "shvk_cnn_block": (i32, [i32] + [vp] * 9 + [i32, i32, vp]),
+        "shvk_cnn_se_gate_sums": (i32, [vp] * 6 + [i32] * 5 + [vp]),
+        "shvk_cnn_rows_gate": (i32, [vp] * 4 + [i32, vp, vp] + [i32] * 4 + [vp]),
+        "shvk_cnn_last_pool": (i32, [vp] * 4 + [i32, i32, vp]),
+        "shvk_cnn_token_proj": (i32, [vp] * 3 + [i32, i32, vp]),
     }
     for name, (res, args) in sig.items():
         fn = getattr(L, name)

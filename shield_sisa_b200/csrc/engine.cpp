@@ -19,7 +19,10 @@
 // encode (F frames, reference run_encode engine/cuda/engine.cu:338-403): stem -> 15 inverted-residual blocks
 //   (expand 1x1 | depthwise | squeeze-excite gate | project 1x1 with the gate applied to its input rows, + residual)
 //   -> 1x1 160 -> 960 -> 4x4 pooling -> 960 -> 384 token projection into slot.d_tokens.  float32 NHWC storage in every
-//   mode; in the bf16 / fp16 modes the 1x1 convolutions round their operands to that type and multiply on the tensor cores.
+//   mode.  fp32 mode: a launch per layer (64).  bf16 / fp16 modes (33 launches): stem and block 1 in one kernel, expand +
+//   depthwise (+ project, where no gate stands between) of a block in one kernel, gate, project behind the gate, last
+//   convolution + pooling in one kernel; the 1x1 convolutions round their operands to the mode's type and multiply on the
+//   tensor cores.
 //
 // Storage policy (engine/cuda/engine.cu:150-164,213-219): h and the readout-row buffers are fp32 always; xn, on and the
 // all-row weights are the storage type of the mode.  Departures in the 16-bit modes, all inside the 2e-2 tolerance and
@@ -146,6 +149,8 @@ struct GdnDev {
 struct CnnBlockDev {
     const float *exp_w = nullptr, *exp_b = nullptr, *dw_w = nullptr, *dw_b = nullptr, *se_w1 = nullptr, *se_b1 = nullptr;
     const float *se_w2 = nullptr, *se_b2 = nullptr, *proj_w = nullptr, *proj_b = nullptr;
+    const void *exp_p = nullptr, *proj_p = nullptr;   // 16-bit modes: exp_w and proj_w as packed fragments
+    int tiles = 0;                                    // 16-bit modes: pooled sums per frame (squeeze-excite blocks)
 };
 
 // One all-row GEMM of the launch sequence: its argument block for the planned maximum row count and, in the 16-bit
@@ -228,6 +233,11 @@ public:
         return timed(s, [&] { run_encode(slot, F, s); });
     }
     int launches_per_encode() const override {
+        if (prec_ != Precision::FP32) {
+            int n = 1 + 2;                               // stem + block 1; last conv + pooling, token projection
+            for (int i = 1; i < 15; ++i) n += 1 + (cnn_.blocks[i].se ? 2 : 0);
+            return n;
+        }
         int n = 4;                                       // stem, last conv, pooling, token projection
         for (const CnnBlock& b : cnn_.blocks) n += 2 + (b.has_expand ? 1 : 0) + (b.se ? 2 : 0);
         return n;
@@ -259,6 +269,7 @@ private:
     CnnHost cnn_;
     const float *lut_ = nullptr, *stem_w_ = nullptr, *stem_b_ = nullptr, *last_w_ = nullptr, *last_b_ = nullptr, *tokproj_ = nullptr;
     CnnBlockDev blk_[15];
+    const void *last_p_ = nullptr, *tokproj_p_ = nullptr;
     float *cx_ = nullptr, *ce_ = nullptr, *cd_ = nullptr, *se_part_ = nullptr, *se_gate_ = nullptr, *pooled_ = nullptr;
     std::map<long long, cudaGraphExec_t> graphs_;
     cudaStream_t capture_ = nullptr;
@@ -401,12 +412,39 @@ private:
         for (int i = 0; i < 15; ++i) {
             const CnnBlock& b = cnn_.blocks[i];
             CnnBlockDev& d = blk_[i];
-            if (b.has_expand) { f32(&d.exp_w, b.exp_w); f32(&d.exp_b, b.exp_b); }
+            if (b.has_expand) {
+                if (prec_ == Precision::FP32) f32(&d.exp_w, b.exp_w);
+                f32(&d.exp_b, b.exp_b);
+            }
             f32(&d.dw_w, b.dw_w); f32(&d.dw_b, b.dw_b);
             if (b.se) { f32(&d.se_w1, b.se_w1); f32(&d.se_b1, b.se_b1); f32(&d.se_w2, b.se_w2); f32(&d.se_b2, b.se_b2); }
-            f32(&d.proj_w, b.proj_w); f32(&d.proj_b, b.proj_b);
+            if (prec_ == Precision::FP32) f32(&d.proj_w, b.proj_w);
+            f32(&d.proj_b, b.proj_b);
         }
-        f32(&last_w_, cnn_.last_w); f32(&last_b_, cnn_.last_b); f32(&tokproj_, hm.proj);
+        if (prec_ != Precision::FP32) {
+            // the 1x1 weights of the fused encoder: zero rows / columns up to the padding of the block's kernel, 16-bit fragments
+            auto packed = [&](const void** dst, const std::vector<float>& w, int n, int k, int n_pad, int k_pad, int order) {
+                std::vector<float> full(size_t(n_pad) * k_pad, 0.0f);
+                for (int r = 0; r < n; ++r) std::memcpy(&full[size_t(r) * k_pad], &w[size_t(r) * k], size_t(k) * sizeof(float));
+                std::vector<uint8_t> out(shvk_cnn_packed_bytes(n_pad, k_pad, order));
+                launch_ok(shvk_cnn_pack_weights(full.data(), n_pad, k_pad, order, dt_, out.data()), "weight packing");
+                put(dst, out.data(), out.size());
+            };
+            for (int i = 0; i < 15; ++i) {
+                const CnnBlock& b = cnn_.blocks[i];
+                CnnBlockDev& d = blk_[i];
+                int cols = b.exp, k = b.exp;
+                if (i > 0) shvk_cnn_block_padding(i + 1, &cols, &k);
+                d.tiles = shvk_cnn_block_tiles(i + 1);
+                if ((d.tiles > 0) != b.se || cols < b.exp || k < b.exp) throw std::runtime_error("fused encoder: block table mismatch");
+                if (b.has_expand) packed(&d.exp_p, b.exp_w, b.exp, b.in, cols, b.in, 0);
+                packed(&d.proj_p, b.proj_w, b.out, b.exp, b.out, k, b.se ? 1 : 0);
+            }
+            packed(&last_p_, cnn_.last_w, CNN_OUT, 160, CNN_OUT, 160, 0);
+            packed(&tokproj_p_, hm.proj, D, CNN_OUT, D, CNN_OUT, 2);
+        }
+        f32(&last_w_, cnn_.last_w); f32(&last_b_, cnn_.last_b);
+        if (prec_ == Precision::FP32) f32(&tokproj_, hm.proj);
         wts_.commit("weight upload");
         cuda_ok(cudaMemcpy(wts_.at<void>(0), host.data(), host.size(), cudaMemcpyHostToDevice), "weight upload");
         for (const Fix& f : fixes) *f.dst = wts_.at<uint8_t>(f.off);
@@ -430,6 +468,17 @@ private:
             if (b.has_expand) e_fl = std::max(e_fl, size_t(b.h_in) * b.w_in * b.exp);
             d_fl = std::max(d_fl, size_t(b.h_out) * b.w_out * b.exp);
             if (b.se) part_fl = std::max(part_fl, shvk_cnn_se_partial_floats(1, b.h_out * b.w_out, b.exp));
+        }
+        if (prec_ != Precision::FP32) {
+            // the fused kernels keep expanded maps on the SM: E is the other one of two block outputs, Dd the gated maps only
+            e_fl = x_fl;
+            d_fl = 0;
+            for (int i = 0; i < 15; ++i)
+                if (cnn_.blocks[i].se) {
+                    const CnnBlock& b = cnn_.blocks[i];
+                    d_fl = std::max(d_fl, size_t(b.h_out) * b.w_out * b.exp);
+                    part_fl = std::max(part_fl, size_t(blk_[i].tiles) * b.exp);
+                }
         }
         const size_t o_cx = acts_.reserve(Fm * x_fl * 4), o_ce = acts_.reserve(Fm * e_fl * 4), o_cd = acts_.reserve(Fm * d_fl * 4);
         const size_t o_sp = acts_.reserve(Fm * part_fl * 4), o_sg = acts_.reserve(Fm * CNN_OUT * 4);
@@ -565,15 +614,8 @@ private:
 
     // ---------------------------------------------------------------- frame encoder
     void run_encode(int slot, int F, cudaStream_t s) {
+        if (prec_ != Precision::FP32) { run_encode_fused(slot, F, s); return; }
         const Slot& sl = slots_[size_t(slot)];
-        // 1x1 convolutions: exact fma chains in fp32 mode, tensor-core products of operands rounded to the mode's 16-bit
-        // type in the bf16 / fp16 modes
-        const int ab = dt_;
-        auto pointwise = [&](const float* A, const float* W, const float* b, const float* gate, int gate_rows, const float* R,
-                             float* out, int M, int N, int K, int act, void* st) {
-            if (prec_ == Precision::FP32) return shvk_cnn_pointwise(A, W, b, gate, gate_rows, R, out, M, N, K, act, st);
-            return shvk_cnn_pointwise_h(A, W, b, gate, gate_rows, R, out, M, N, K, act, ab, st);
-        };
         launch_ok(shvk_cnn_stem(sl.d_frames, lut_, stem_w_, stem_b_, cx_, F, s), "stem");
         mark("cnn.stem", s);
         dump("cnn_stem_f0", cx_, size_t(16) * 90 * 160, SHVK_F32, s);
@@ -583,7 +625,7 @@ private:
             const int hw_in = b.h_in * b.w_in, hw_out = b.h_out * b.w_out;
             const float* dw_in = cx_;
             if (b.has_expand) {
-                launch_ok(pointwise(cx_, d.exp_w, d.exp_b, nullptr, 1, nullptr, ce_, F * hw_in, b.exp, b.in, b.act, s),
+                launch_ok(shvk_cnn_pointwise(cx_, d.exp_w, d.exp_b, nullptr, 1, nullptr, ce_, F * hw_in, b.exp, b.in, b.act, s),
                           "expand");
                 mark("cnn.expand", s);
                 dw_in = ce_;
@@ -598,7 +640,7 @@ private:
                 mark("cnn.se_gate", s);
                 gate = se_gate_;
             }
-            launch_ok(pointwise(cd_, d.proj_w, d.proj_b, gate, hw_out, b.residual ? cx_ : nullptr, cx_, F * hw_out, b.out,
+            launch_ok(shvk_cnn_pointwise(cd_, d.proj_w, d.proj_b, gate, hw_out, b.residual ? cx_ : nullptr, cx_, F * hw_out, b.out,
                                          b.exp, SHVK_ACT_NONE, s), "project");
             mark("cnn.project", s);
             if (!dump_dir_.empty()) {
@@ -607,21 +649,62 @@ private:
                 dump(name, cx_, size_t(b.out) * hw_out, SHVK_F32, s);
             }
         }
-        launch_ok(pointwise(cx_, last_w_, last_b_, nullptr, 1, nullptr, ce_, F * 60, CNN_OUT, 160, SHVK_ACT_HSWISH, s),
+        launch_ok(shvk_cnn_pointwise(cx_, last_w_, last_b_, nullptr, 1, nullptr, ce_, F * 60, CNN_OUT, 160, SHVK_ACT_HSWISH, s),
                   "last conv");
         mark("cnn.last", s);
         dump("cnn_map_f0", ce_, size_t(60) * CNN_OUT, SHVK_F32, s);
         launch_ok(shvk_cnn_pool_tokens(ce_, pooled_, F, s), "pool");
         mark("cnn.pool", s);
-        if (prec_ == Precision::FP32) {
-            shvk_gemm_args a{};
-            a.M = F * 16; a.N = D; a.K = CNN_OUT; a.A = pooled_; a.lda = CNN_OUT; a.W = tokproj_; a.ldw = CNN_OUT;
-            a.C = sl.d_tokens; a.ldc = D; a.c_dtype = SHVK_F32; a.r_div = 1.0f;
-            launch_ok(shvk_gemm_f32(&a, s), "token projection");
-        } else {
-            launch_ok(pointwise(pooled_, tokproj_, nullptr, nullptr, 1, nullptr, sl.d_tokens, F * 16, D, CNN_OUT, SHVK_ACT_NONE, s),
-                      "token projection");
+        shvk_gemm_args a{};
+        a.M = F * 16; a.N = D; a.K = CNN_OUT; a.A = pooled_; a.lda = CNN_OUT; a.W = tokproj_; a.ldw = CNN_OUT;
+        a.C = sl.d_tokens; a.ldc = D; a.c_dtype = SHVK_F32; a.r_div = 1.0f;
+        launch_ok(shvk_gemm_f32(&a, s), "token projection");
+        mark("cnn.token_proj", s);
+        dump("tokens", sl.d_tokens, size_t(16) * D, SHVK_F32, s);
+    }
+    // bf16 / fp16 modes: block outputs alternate between X and E (a block's tiles read each other's halos, so it cannot run
+    // in place); the projection behind a gate writes where its residual is
+    void run_encode_fused(int slot, int F, cudaStream_t s) {
+        const Slot& sl = slots_[size_t(slot)];
+        const CnnBlockDev& d0 = blk_[0];
+        launch_ok(shvk_cnn_stem_block(sl.d_frames, lut_, cnn_.stem_w.data(), cnn_.stem_b.data(), d0.dw_w, d0.dw_b, d0.proj_p, d0.proj_b, cx_,
+                                      F, dt_, s), "stem and block 1");
+        mark("cnn.stem_block", s);
+        if (!dump_dir_.empty()) {                        // the stem's own map, which the fused kernel keeps to itself
+            launch_ok(shvk_cnn_stem(sl.d_frames, lut_, stem_w_, stem_b_, ce_, 1, s), "stem");
+            dump("cnn_stem_f0", ce_, size_t(16) * 90 * 160, SHVK_F32, s);
+            dump("cnn_block01_f0", cx_, size_t(16) * 90 * 160, SHVK_F32, s);
         }
+        float *x = cx_, *y = ce_;
+        for (int i = 1; i < 15; ++i) {
+            const CnnBlock& b = cnn_.blocks[i];
+            const CnnBlockDev& d = blk_[i];
+            const int hw = b.h_out * b.w_out;
+            launch_ok(shvk_cnn_block(i + 1, x, d.exp_p, d.exp_b, d.dw_w, d.dw_b, d.proj_p, d.proj_b, b.se ? cd_ : y, se_part_, F, dt_, s),
+                      "encoder block");
+            mark(b.se ? "cnn.expand_dw" : "cnn.block", s);
+            if (b.se) {
+                launch_ok(shvk_cnn_se_gate_sums(se_part_, d.se_w1, d.se_b1, d.se_w2, d.se_b2, se_gate_, F, d.tiles, hw, b.exp, b.cs, s),
+                          "squeeze-excite");
+                mark("cnn.se_gate", s);
+                launch_ok(shvk_cnn_rows_gate(cd_, d.proj_p, d.proj_b, se_gate_, hw, b.residual ? x : nullptr, y, F * hw, b.out, b.exp, dt_, s),
+                          "project");
+                mark("cnn.project", s);
+            }
+            std::swap(x, y);
+            if (!dump_dir_.empty()) {
+                char name[32];
+                std::snprintf(name, sizeof name, "cnn_block%02d_f0", i + 1);
+                dump(name, x, size_t(b.out) * hw, SHVK_F32, s);
+            }
+        }
+        if (!dump_dir_.empty()) {
+            launch_ok(shvk_cnn_pointwise_h(x, last_w_, last_b_, nullptr, 1, nullptr, y, 60, CNN_OUT, 160, SHVK_ACT_HSWISH, dt_, s), "last conv");
+            dump("cnn_map_f0", y, size_t(60) * CNN_OUT, SHVK_F32, s);
+        }
+        launch_ok(shvk_cnn_last_pool(x, last_p_, last_b_, pooled_, F, dt_, s), "last conv and pool");
+        mark("cnn.last_pool", s);
+        launch_ok(shvk_cnn_token_proj(pooled_, tokproj_p_, sl.d_tokens, F * 16, dt_, s), "token projection");
         mark("cnn.token_proj", s);
         dump("tokens", sl.d_tokens, size_t(16) * D, SHVK_F32, s);
     }

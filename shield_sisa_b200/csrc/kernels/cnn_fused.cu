@@ -1,0 +1,907 @@
+// Fused frame-encoder kernels of the bf16 / fp16 modes (MobileNetV3-Large blocks on 320x180 crops; layer by layer the
+// same network is cnn.cu).  The reference's CUDA engine runs every layer as a launch of its own (engine/cuda/engine.cu:338-403).
+//
+// What bounded the layered form (640 crops, 11.2 ms): every expanded map crossed HBM twice (two thirds of 46 MB per
+// crop), and the 1x1 kernels spent three quarters of their time fetching, converting and parking operand slabs.  Here an
+// expanded map never leaves the SM: a block of threads takes a spatial tile, rounds its input pixels (with the halo the
+// depthwise filter needs) to the mode's 16-bit type once, and walks the expanded channels in chunks,
+//     expand (mma.sync m16n8k16 -> fp32 in shared memory) | depthwise (fp32 FMA out of shared memory)
+// and either rounds the chunk into the A operand of the projection, whose accumulators stay in registers over all chunks,
+// or, where a squeeze-excite gate stands between (it needs the whole map), writes the fp32 map and its pooled sums.
+// Roundings are those of the layered form: 1x1 operands in the mode's 16-bit type, everything else float32.
+//
+// mma.sync and not tcgen05: the products are 16 to 160 deep and 8 to 160 wide on tiles whose rows are gathered pixels;
+// they are a third of these kernels' instructions, the depthwise filter and the activations are the rest.
+//
+// Weights of the 1x1 convolutions arrive as 16-bit fragments (shvk_cnn_pack_weights): a lane's values for an mma are
+// contiguous, a warp's load is one coalesced row, and no shared memory or conversion is spent on them.
+#include "device_utils.cuh"
+#include "shv_cnn_kernels.h"
+
+namespace sb {
+namespace {
+
+// x * relu6(x + 3) / 6 as x * clamp(x / 6 + 1/2): one saturating FMA and a product
+__device__ __forceinline__ float hswish(float x) { return x * __saturatef(fmaf(x, 1.0f / 6.0f, 0.5f)); }
+template <bool HS> __device__ __forceinline__ float act(float x) { return HS ? hswish(x) : fmaxf(x, 0.0f); }
+
+// two float32 FMAs in one instruction (each rounded as fmaf rounds)
+__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
+    float2 d;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;"
+        : "=l"(reinterpret_cast<unsigned long long&>(d))
+        : "l"(reinterpret_cast<unsigned long long&>(a)), "l"(reinterpret_cast<unsigned long long&>(b)),
+          "l"(reinterpret_cast<unsigned long long&>(c)));
+    return d;
+}
+
+template <typename HT> struct Half;
+template <> struct Half<__nv_bfloat16> {
+    static __device__ __forceinline__ uint32_t pack(float lo, float hi) {
+        __nv_bfloat162 v = __floats2bfloat162_rn(lo, hi);
+        return *reinterpret_cast<uint32_t*>(&v);
+    }
+    static __device__ __forceinline__ void mma(float (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
+        asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
+                     : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
+                     : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+    }
+};
+template <> struct Half<__half> {
+    static __device__ __forceinline__ uint32_t pack(float lo, float hi) {
+        __half2 v = __floats2half2_rn(lo, hi);
+        return *reinterpret_cast<uint32_t*>(&v);
+    }
+    static __device__ __forceinline__ void mma(float (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
+        asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
+                     : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
+                     : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+    }
+};
+
+__device__ __forceinline__ void ldmatrix_x4(uint32_t (&r)[4], uint32_t addr) {
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0, %1, %2, %3}, [%4];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr));
+}
+__device__ __forceinline__ uint32_t smem_addr(const void* p) { return uint32_t(__cvta_generic_to_shared(p)); }
+
+__host__ __device__ constexpr int up(int a, int b) { return (a + b - 1) / b * b; }
+__host__ __device__ constexpr int cmax(int a, int b) { return a > b ? a : b; }
+
+// ---------------------------------------------------------------------------------------------------- depthwise
+// One thread's share of a depthwise filter: two channels, PX adjacent output pixels of SR rows.  e points at the tile's
+// float32 map (pitch P floats per pixel, IWA pixels per row) at the thread's first input pixel and channel pair; every
+// input pixel is read once and used by all outputs it belongs to.  Per output the taps are visited row by row.
+template <int KS, int S, int PX, int SR, int P, int IWA>
+__device__ __forceinline__ void depthwise_pair(const float* e, const float2 (&w)[KS * KS], float2 (&acc)[SR][PX]) {
+    constexpr int NIN = (PX - 1) * S + KS;
+#pragma unroll
+    for (int r = 0; r < SR; ++r)
+#pragma unroll
+        for (int p = 0; p < PX; ++p) acc[r][p] = make_float2(0.0f, 0.0f);
+#pragma unroll
+    for (int iy = 0; iy < (SR - 1) * S + KS; ++iy) {
+        float2 x[NIN];
+#pragma unroll
+        for (int j = 0; j < NIN; ++j) x[j] = *reinterpret_cast<const float2*>(e + (iy * IWA + j) * P);
+#pragma unroll
+        for (int r = 0; r < SR; ++r) {
+            const int ky = iy - r * S;
+            if (ky < 0 || ky >= KS) continue;
+#pragma unroll
+            for (int kx = 0; kx < KS; ++kx)
+#pragma unroll
+                for (int p = 0; p < PX; ++p) acc[r][p] = fma2(w[ky * KS + kx], x[p * S + kx], acc[r][p]);
+        }
+    }
+}
+
+// ---------------------------------------------------------------------------------------------------- inverted residual
+// CIN -> CEXP (1x1, activation) -> depthwise KS x KS, stride S, activation -> COUT (1x1, + residual); COUT = 0: stop after
+// the depthwise map (squeeze-excite blocks).  TH x TW output pixels per block of 256 threads, CE expanded channels at a time.
+template <int CIN_, int CEXP_, int COUT_, int KS_, int S_, int HI_, int WI_, int TH_, int TW_, int CE_, int PX_, int SR_, int NSPLIT_,
+          bool HS_, bool RES_, int MINB_>
+struct Block {
+    static constexpr int CIN = CIN_, CEXP = CEXP_, COUT = COUT_, KS = KS_, S = S_, HI = HI_, WI = WI_, TH = TH_, TW = TW_, CE = CE_;
+    static constexpr int PX = PX_, SR = SR_, NSPLIT = NSPLIT_, MINB = MINB_;
+    static constexpr bool HS = HS_, RES = RES_, SE = COUT_ == 0;
+    static constexpr int PAD = (KS - 1) / 2, HO = (HI + 2 * PAD - KS) / S + 1, WO = (WI + 2 * PAD - KS) / S + 1;
+    static constexpr int TY = (HO + TH - 1) / TH, TX = (WO + TW - 1) / TW, TILES = TY * TX;
+    static constexpr int IH = (TH - 1) * S + KS, IW = (TW - 1) * S + KS;
+    static constexpr int VH = IH < HI ? IH : HI, VW = IW < WI ? IW : WI;     // most input pixels of a tile that lie in the image
+    static constexpr int VPX = VH * VW, MROWS = up(VPX, 16);
+    static constexpr int KP = up(CIN, 16), KT = KP / 16, XP = KP + 8;        // 16-bit input tile: XP halves per pixel
+    static constexpr int NT = CE / 8, NW = NT / NSPLIT;
+    static constexpr int P = CE % 16 == 8 ? CE : CE + 8;                     // fp32 pitch = 8 mod 16 words: expand's stores miss each other's banks
+    static constexpr int CHUNKS = (CEXP + CE - 1) / CE;
+    static constexpr int OPX = TH * TW, OMT = (OPX + 15) / 16, ONT = cmax(COUT / 8, 1), CK = up(CE, 16), DP = CK + 8;
+    static constexpr int KFILL = cmax((CK - CE) / 2, 1);                       // k padding of a chunk, in pairs
+    static constexpr int UNITS = OMT * ONT, UPW = SE ? 1 : (UNITS + 7) / 8;
+    static constexpr int STRIPS = TH / SR, GX = TW / PX, ITEMS = CE / 2 * GX * STRIPS;
+    static constexpr int E_BYTES = up(IH * IW * P * 4, 16), X_BYTES = up(MROWS * XP * 2, 16), T_BYTES = up(MROWS * 2, 16);
+    static constexpr int D_BYTES = SE ? up(GX * STRIPS * CE * 4, 16) : up(OMT * 16 * DP * 2, 16);
+    static constexpr int SMEM = E_BYTES + X_BYTES + T_BYTES + D_BYTES;
+    static_assert(CE % 8 == 0 && NT % NSPLIT == 0 && 8 % NSPLIT == 0 && TW % PX == 0 && TH % SR == 0, "tile shape");
+    static_assert(SE ? CEXP % CE == 0 : CK == CE || CHUNKS == 1, "channel chunks");
+    static_assert(SE || COUT % 8 == 0, "output channels");
+};
+
+struct BlockArgs {
+    const float* x;            // [F][HI][WI][CIN]
+    const uint2* we;           // expand weights, fragments [n tile][k tile][lane]
+    const float* be;
+    const float* wd;           // depthwise filter [KS * KS][CEXP]
+    const float* bd;
+    const uint2* wp;           // projection weights, fragments [n tile][k tile][lane]
+    const float* bp;
+    float* out;                // [F][HO][WO][COUT], or the depthwise map [F][HO][WO][CEXP]
+    float* sums;               // squeeze-excite: [F][TILES][CEXP] sums of the map over a tile's pixels
+    int chunks_per_group;      // squeeze-excite: chunks a block takes (gridDim.y groups)
+};
+
+template <class C, typename HT>
+__global__ void __launch_bounds__(256, C::MINB) block_kernel(const BlockArgs a) {
+    extern __shared__ __align__(16) uint8_t smem[];
+    float* const E = reinterpret_cast<float*>(smem);
+    uint16_t* const X = reinterpret_cast<uint16_t*>(smem + C::E_BYTES);
+    uint16_t* const pos = reinterpret_cast<uint16_t*>(smem + C::E_BYTES + C::X_BYTES);   // E pixel of every input row of X
+    uint8_t* const D = smem + C::E_BYTES + C::X_BYTES + C::T_BYTES;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, t = lane & 3;
+    const int f = blockIdx.x / C::TILES, tile = blockIdx.x % C::TILES;
+    const int oy0 = tile / C::TX * C::TH, ox0 = tile % C::TX * C::TW;
+    const int iy0 = oy0 * C::S - C::PAD, ix0 = ox0 * C::S - C::PAD;
+    const int vy0 = max(iy0, 0), vy1 = min(iy0 + C::IH, C::HI), vx0 = max(ix0, 0), vx1 = min(ix0 + C::IW, C::WI);
+    const int vw = vx1 - vx0, nv = (vy1 - vy0) * vw;
+    const float* const img = a.x + (long long)f * (C::HI * C::WI * C::CIN);
+    const int first = C::SE ? blockIdx.y * a.chunks_per_group : 0;
+    const int last = C::SE ? min(first + a.chunks_per_group, C::CHUNKS) : C::CHUNKS;
+
+    // input pixels of the tile, rounded to 16 bits; channels past CIN and the halo outside the image are zero
+    constexpr int Q4 = C::KP / 4;
+    for (int i = tid; i < nv * Q4; i += 256) {
+        const int r = i / Q4, q = i % Q4, vy = r / vw, vx = r - vy * vw;
+        uint2 v = make_uint2(0u, 0u);
+        if (C::CIN % 16 == 0 || q * 4 < C::CIN) {
+            const float4 p = *reinterpret_cast<const float4*>(img + ((vy0 + vy) * C::WI + vx0 + vx) * C::CIN + q * 4);
+            v = make_uint2(Half<HT>::pack(p.x, p.y), Half<HT>::pack(p.z, p.w));
+        }
+        *reinterpret_cast<uint2*>(X + r * C::XP + q * 4) = v;
+        if (q == 0) pos[r] = uint16_t((vy0 - iy0 + vy) * C::IW + (vx0 - ix0 + vx));
+    }
+    if (nv < C::IH * C::IW)
+        for (int i = tid; i < C::E_BYTES / 16; i += 256) reinterpret_cast<uint4*>(E)[i] = make_uint4(0u, 0u, 0u, 0u);
+    if (!C::SE && C::CK != C::CE)                    // projection k padding of a single chunk
+        for (int i = tid; i < C::OMT * 16 * C::KFILL; i += 256)
+            reinterpret_cast<uint32_t*>(D)[i / C::KFILL * (C::DP / 2) + C::CE / 2 + i % C::KFILL] = 0u;
+    float pacc[C::UPW][4];
+#pragma unroll
+    for (int u = 0; u < C::UPW; ++u)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) pacc[u][e] = 0.0f;
+    __syncthreads();
+
+    const int ns = warp % C::NSPLIT, mtiles = (nv + 15) >> 4;
+    const uint32_t xrow = smem_addr(X) + uint32_t(((lane & 15) * C::XP + (lane >> 4) * 8) * 2);
+    for (int ch = first; ch < last; ++ch) {
+        // ---- expand: this warp's n tiles of the chunk for every (8 / NSPLIT)-th group of 16 input pixels
+        {
+            uint2 b[C::NW][C::KT];
+            float2 bias[C::NW];
+#pragma unroll
+            for (int n = 0; n < C::NW; ++n) {
+                const int nt = ch * C::NT + ns * C::NW + n, col = nt * 8 + 2 * t;
+#pragma unroll
+                for (int k = 0; k < C::KT; ++k) b[n][k] = __ldg(a.we + (nt * C::KT + k) * 32 + lane);
+                bias[n] = C::CEXP % C::CE == 0 || col < C::CEXP ? __ldg(reinterpret_cast<const float2*>(a.be + col)) : make_float2(0.0f, 0.0f);
+            }
+            for (int mt = warp / C::NSPLIT; mt < mtiles; mt += 8 / C::NSPLIT) {
+                float c[C::NW][4];
+#pragma unroll
+                for (int n = 0; n < C::NW; ++n)
+#pragma unroll
+                    for (int e = 0; e < 4; ++e) c[n][e] = 0.0f;
+#pragma unroll
+                for (int k = 0; k < C::KT; ++k) {
+                    uint32_t af[4];
+                    ldmatrix_x4(af, xrow + uint32_t((mt * 16 * C::XP + k * 16) * 2));
+#pragma unroll
+                    for (int n = 0; n < C::NW; ++n) Half<HT>::mma(c[n], af, b[n][k].x, b[n][k].y);
+                }
+#pragma unroll
+                for (int h = 0; h < 2; ++h) {
+                    const int r = mt * 16 + g + h * 8;
+                    if (r >= nv) continue;
+                    float* const er = E + pos[r] * C::P + ns * C::NW * 8 + 2 * t;
+#pragma unroll
+                    for (int n = 0; n < C::NW; ++n)
+                        *reinterpret_cast<float2*>(er + n * 8) =
+                            make_float2(act<C::HS>(c[n][2 * h] + bias[n].x), act<C::HS>(c[n][2 * h + 1] + bias[n].y));
+                }
+            }
+        }
+        __syncthreads();
+        // ---- depthwise
+        for (int i = tid; i < C::ITEMS; i += 256) {
+            const int cp = i % (C::CE / 2), gx = i / (C::CE / 2) % C::GX, st = i / (C::CE / 2 * C::GX);
+            const int col = ch * C::CE + cp * 2;
+            const bool live = C::CEXP % C::CE == 0 || col < C::CEXP;
+            float2 w[C::KS * C::KS], acc[C::SR][C::PX];
+#pragma unroll
+            for (int k = 0; k < C::KS * C::KS; ++k)
+                w[k] = live ? __ldg(reinterpret_cast<const float2*>(a.wd + k * C::CEXP + col)) : make_float2(0.0f, 0.0f);
+            const float2 bias = live ? __ldg(reinterpret_cast<const float2*>(a.bd + col)) : make_float2(0.0f, 0.0f);
+            const int oy = st * C::SR, ox = gx * C::PX;
+            depthwise_pair<C::KS, C::S, C::PX, C::SR, C::P, C::IW>(E + (oy * C::S * C::IW + ox * C::S) * C::P + cp * 2, w, acc);
+            float2 sum = make_float2(0.0f, 0.0f);
+#pragma unroll
+            for (int r = 0; r < C::SR; ++r) {
+#pragma unroll
+                for (int p = 0; p < C::PX; ++p) {
+                    const float2 v = make_float2(act<C::HS>(acc[r][p].x + bias.x), act<C::HS>(acc[r][p].y + bias.y));
+                    if (C::SE) {
+                        if ((C::HO % C::TH == 0 || oy0 + oy + r < C::HO) && (C::WO % C::TW == 0 || ox0 + ox + p < C::WO)) {
+                            *reinterpret_cast<float2*>(a.out + ((long long)(f * C::HO + oy0 + oy + r) * C::WO + ox0 + ox + p) * C::CEXP + col) = v;
+                            sum.x += v.x;
+                            sum.y += v.y;
+                        }
+                    } else {
+                        reinterpret_cast<uint32_t*>(D)[((oy + r) * C::TW + ox + p) * (C::DP / 2) + cp] = Half<HT>::pack(v.x, v.y);
+                    }
+                }
+            }
+            if (C::SE) *reinterpret_cast<float2*>(D + ((st * C::GX + gx) * C::CE + cp * 2) * 4) = sum;
+        }
+        __syncthreads();
+        if constexpr (C::SE) {
+            // the tile's sums, thread groups in a fixed order
+            if (tid < C::CE) {
+                float s = 0.0f;
+#pragma unroll 4
+                for (int i = 0; i < C::GX * C::STRIPS; ++i) s += reinterpret_cast<const float*>(D)[i * C::CE + tid];
+                a.sums[((long long)f * C::TILES + tile) * C::CEXP + ch * C::CE + tid] = s;
+            }
+        } else {
+            // ---- projection: this chunk's k range into the accumulators of the warp's (pixel group, n tile) units
+            const uint32_t drow = smem_addr(D) + uint32_t(((lane & 15) * C::DP + (lane >> 4) * 8) * 2);
+            constexpr int KC = C::CK / 16, KALL = C::CHUNKS * KC;
+#pragma unroll
+            for (int k = 0; k < KC; ++k)
+#pragma unroll
+                for (int u = 0; u < C::UPW; ++u) {
+                    const int unit = warp + u * 8;
+                    if (C::UNITS % 8 != 0 && unit >= C::UNITS) break;
+                    uint32_t af[4];
+                    ldmatrix_x4(af, drow + uint32_t(((unit % C::OMT) * 16 * C::DP + k * 16) * 2));
+                    const uint2 b = __ldg(a.wp + ((unit / C::OMT) * KALL + ch * KC + k) * 32 + lane);
+                    Half<HT>::mma(pacc[u], af, b.x, b.y);
+                }
+        }
+    }
+    if constexpr (C::SE) return;
+#pragma unroll
+    for (int u = 0; u < C::UPW; ++u) {
+        const int unit = warp + u * 8;
+        if (C::UNITS % 8 != 0 && unit >= C::UNITS) break;
+        const int n = unit / C::OMT * 8 + 2 * t;
+        const float2 bias = __ldg(reinterpret_cast<const float2*>(a.bp + n));
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            const int p = unit % C::OMT * 16 + g + h * 8, oy = oy0 + p / C::TW, ox = ox0 + p % C::TW;
+            if (p >= C::OPX || oy >= C::HO || ox >= C::WO) continue;
+            float2 v = make_float2(pacc[u][2 * h] + bias.x, pacc[u][2 * h + 1] + bias.y);
+            const long long at = ((long long)(f * C::HO + oy) * C::WO + ox) * C::COUT + n;
+            if (C::RES) {
+                const float2 r = *reinterpret_cast<const float2*>(a.x + at);
+                v.x += r.x;
+                v.y += r.y;
+            }
+            *reinterpret_cast<float2*>(a.out + at) = v;
+        }
+    }
+}
+
+// ---------------------------------------------------------------------------------------------------- stem + first block
+// uint8 crop -> normalisation -> 3x3/2 convolution 3 -> 16, Hardswish -> depthwise 3x3, ReLU -> 1x1 16 -> 16, + the stem's
+// output.  A block takes 10 x 32 output pixels: the 25 x 69 input pixels are looked up once into float32, the stem runs one
+// thread per pixel with its filter as kernel parameters (an FMA takes one operand from the constant bank, so a tap costs no
+// load), and its map stays in shared memory.
+struct StemParams {
+    float w[27 * 16];          // ((ky * 3 + kx) * 3 + ci) * 16 + co
+    float b[16];
+};
+struct Stem {
+    static constexpr int H = 90, W = 160, IMH = 180, IMW = 320, TH = 10, TW = 32, TILES = (H / TH) * (W / TW);
+    static constexpr int SH = TH + 2, SW = TW + 2, UH = 2 * SH + 1, UW = 2 * SW + 1, UP = UW * 3 + 1;   // stem map and input tile
+    static constexpr int P = 20, DP = 24, PX = 2, SR = 5;
+    static constexpr int OMT = TH * TW / 16;
+    static constexpr int S_BYTES = SH * SW * P * 4, U_BYTES = up(UH * UP * 4, 16), D_BYTES = TH * TW * DP * 2;
+    static constexpr int SMEM = S_BYTES + cmax(U_BYTES, D_BYTES) + 768 * 4;
+};
+
+template <typename HT>
+__global__ void __launch_bounds__(256, 3)
+stem_block_kernel(const uint8_t* __restrict__ frames, const float* __restrict__ lut, const __grid_constant__ StemParams sp,
+                  const float* __restrict__ wd, const float* __restrict__ bd, const uint2* __restrict__ wp,
+                  const float* __restrict__ bp, float* __restrict__ out) {
+    extern __shared__ __align__(16) uint8_t smem[];
+    float* const M = reinterpret_cast<float*>(smem);                          // stem map, pitch P
+    float* const U = reinterpret_cast<float*>(smem + Stem::S_BYTES);          // normalised input; D reuses it
+    uint32_t* const D = reinterpret_cast<uint32_t*>(smem + Stem::S_BYTES);
+    float* const L = reinterpret_cast<float*>(smem + Stem::S_BYTES + cmax(Stem::U_BYTES, Stem::D_BYTES));
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, t = lane & 3;
+    const int f = blockIdx.x / Stem::TILES, tile = blockIdx.x % Stem::TILES;
+    const int oy0 = tile / (Stem::W / Stem::TW) * Stem::TH, ox0 = tile % (Stem::W / Stem::TW) * Stem::TW;
+    const uint8_t* const img = frames + (long long)f * (Stem::IMH * Stem::IMW * 3);
+    for (int i = tid; i < 768; i += 256) L[i] = lut[i];
+    __syncthreads();
+    // stem pixel (sy, sx) of the tile is map pixel (oy0 - 1 + sy, ox0 - 1 + sx); its taps start at crop pixel 2 (.) - 1
+    const int uy0 = 2 * (oy0 - 1) - 1, ux0 = 2 * (ox0 - 1) - 1;
+    for (int i = tid; i < Stem::UH * Stem::UW * 3; i += 256) {
+        const int r = i / (Stem::UW * 3), c = i % (Stem::UW * 3), y = uy0 + r, x3 = ux0 * 3 + c;
+        float v = 0.0f;
+        if (y >= 0 && y < Stem::IMH && x3 >= 0 && x3 < Stem::IMW * 3) v = L[(c % 3) * 256 + img[y * (Stem::IMW * 3) + x3]];
+        U[r * Stem::UP + c] = v;
+    }
+    __syncthreads();
+    for (int i = tid; i < Stem::SH * Stem::SW; i += 256) {
+        const int sy = i / Stem::SW, sx = i % Stem::SW, y = oy0 - 1 + sy, x = ox0 - 1 + sx;
+        float acc[16];
+#pragma unroll
+        for (int c = 0; c < 16; ++c) acc[c] = 0.0f;
+        const float* const u = U + 2 * sy * Stem::UP + 6 * sx;
+#pragma unroll
+        for (int k = 0; k < 27; ++k) {
+            const float v = u[(k / 9) * Stem::UP + k % 9];
+#pragma unroll
+            for (int c = 0; c < 16; ++c) acc[c] = fmaf(sp.w[k * 16 + c], v, acc[c]);
+        }
+        const bool in = y >= 0 && y < Stem::H && x >= 0 && x < Stem::W;       // the depthwise filter sees zeros outside the map
+#pragma unroll
+        for (int q = 0; q < 4; ++q)
+            *reinterpret_cast<float4*>(M + i * Stem::P + q * 4) =
+                in ? make_float4(hswish(acc[4 * q] + sp.b[4 * q]), hswish(acc[4 * q + 1] + sp.b[4 * q + 1]),
+                                 hswish(acc[4 * q + 2] + sp.b[4 * q + 2]), hswish(acc[4 * q + 3] + sp.b[4 * q + 3]))
+                   : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    }
+    __syncthreads();
+    {
+        constexpr int GX = Stem::TW / Stem::PX;
+        const int cp = tid % 8, gx = tid / 8 % GX, st = tid / (8 * GX);
+        static_assert(8 * GX * (Stem::TH / Stem::SR) == 256, "one depthwise item per thread");
+        float2 w[9], acc[Stem::SR][Stem::PX];
+#pragma unroll
+        for (int k = 0; k < 9; ++k) w[k] = __ldg(reinterpret_cast<const float2*>(wd + k * 16 + cp * 2));
+        const float2 bias = __ldg(reinterpret_cast<const float2*>(bd + cp * 2));
+        depthwise_pair<3, 1, Stem::PX, Stem::SR, Stem::P, Stem::SW>(M + (st * Stem::SR * Stem::SW + gx * Stem::PX) * Stem::P + cp * 2, w, acc);
+#pragma unroll
+        for (int r = 0; r < Stem::SR; ++r)
+#pragma unroll
+            for (int p = 0; p < Stem::PX; ++p)
+                D[((st * Stem::SR + r) * Stem::TW + gx * Stem::PX + p) * (Stem::DP / 2) + cp] =
+                    Half<HT>::pack(fmaxf(acc[r][p].x + bias.x, 0.0f), fmaxf(acc[r][p].y + bias.y, 0.0f));
+    }
+    __syncthreads();
+    const uint32_t drow = smem_addr(D) + uint32_t(((lane & 15) * Stem::DP + (lane >> 4) * 8) * 2);
+    const uint2 b0 = __ldg(wp + lane), b1 = __ldg(wp + 32 + lane);
+#pragma unroll
+    for (int u = 0; u < (Stem::OMT + 7) / 8; ++u) {
+        const int mt = warp + u * 8;
+        if (mt >= Stem::OMT) break;
+        uint32_t af[4];
+        ldmatrix_x4(af, drow + uint32_t(mt * 16 * Stem::DP * 2));
+#pragma unroll
+        for (int nt = 0; nt < 2; ++nt) {
+            float c[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+            Half<HT>::mma(c, af, nt ? b1.x : b0.x, nt ? b1.y : b0.y);
+            const int n = nt * 8 + 2 * t;
+            const float2 bias = __ldg(reinterpret_cast<const float2*>(bp + n));
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                const int p = mt * 16 + g + h * 8, y = p / Stem::TW, x = p % Stem::TW;
+                const float2 r = *reinterpret_cast<const float2*>(M + ((y + 1) * Stem::SW + x + 1) * Stem::P + n);
+                *reinterpret_cast<float2*>(out + (((long long)f * Stem::H + oy0 + y) * Stem::W + ox0 + x) * 16 + n) =
+                    make_float2(c[2 * h] + bias.x + r.x, c[2 * h + 1] + bias.y + r.y);
+            }
+        }
+    }
+}
+
+// ---------------------------------------------------------------------------------------------------- squeeze-excite gate
+// A cluster of eight blocks takes G frames.  Every block reduces the frames' pooled sums, computes an eighth of the hidden
+// layer (a warp per unit, lanes over the channels, a weight row read once for all G frames), hands it to the other seven
+// through distributed shared memory, and computes an eighth of the gates.  One block per frame read all 1.8 MB of the
+// widest layer's weights through one SM: 52 us however few the frames, 210 us at 640.
+__device__ __forceinline__ void cluster_sync() {
+    asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+template <int G>
+__global__ void __cluster_dims__(8, 1, 1) __launch_bounds__(256)
+se_gate_cluster_kernel(const float* __restrict__ sums, const float* __restrict__ w1, const float* __restrict__ b1,
+                       const float* __restrict__ w2, const float* __restrict__ b2, float* __restrict__ gate, int F, int tiles, float hw,
+                       int C, int CS) {
+    extern __shared__ __align__(16) uint8_t smem[];
+    float* const pooled = reinterpret_cast<float*>(smem);           // [G][C]
+    float* const hid = pooled + G * C;                               // [G][CS]
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, rank = blockIdx.x & 7;
+    const int f0 = int(blockIdx.x >> 3) * G, nf = min(G, F - f0);
+    for (int i = tid; i < G * C; i += 256) {
+        const int fr = i / C, c = i - fr * C;
+        float s = 0.0f;
+        if (fr < nf)
+            for (int k = 0; k < tiles; ++k) s += sums[((long long)(f0 + fr) * tiles + k) * C + c];
+        pooled[i] = s / hw;
+    }
+    cluster_sync();                                                  // pooled is complete, and every block of the cluster runs
+    for (int j = rank * 8 + warp; j < CS; j += 64) {
+        float acc[G];
+#pragma unroll
+        for (int fr = 0; fr < G; ++fr) acc[fr] = 0.0f;
+#pragma unroll 4
+        for (int c = lane * 4; c < C; c += 128) {
+            const float4 w = __ldg(reinterpret_cast<const float4*>(w1 + (long long)j * C + c));
+#pragma unroll
+            for (int fr = 0; fr < G; ++fr) {
+                const float4 p = *reinterpret_cast<const float4*>(pooled + fr * C + c);
+                acc[fr] = fmaf(w.x, p.x, fmaf(w.y, p.y, fmaf(w.z, p.z, fmaf(w.w, p.w, acc[fr]))));
+            }
+        }
+        const float bj = b1[j];
+#pragma unroll
+        for (int fr = 0; fr < G; ++fr) {
+            const float v = fmaxf(warp_sum(acc[fr]) + bj, 0.0f);
+            if (lane < 8) {                                          // lane r stores into block r of the cluster
+                const uint32_t local = smem_addr(hid + fr * CS + j);
+                uint32_t remote;
+                asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote) : "r"(local), "r"(lane));
+                asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(remote), "f"(v) : "memory");
+            }
+        }
+    }
+    cluster_sync();
+    for (int c = rank * 8 + warp; c < C; c += 64) {
+        float acc[G];
+#pragma unroll
+        for (int fr = 0; fr < G; ++fr) acc[fr] = 0.0f;
+#pragma unroll 2
+        for (int j = lane * 4; j < CS; j += 128) {
+            const float4 w = __ldg(reinterpret_cast<const float4*>(w2 + (long long)c * CS + j));
+#pragma unroll
+            for (int fr = 0; fr < G; ++fr) {
+                const float4 p = *reinterpret_cast<const float4*>(hid + fr * CS + j);
+                acc[fr] = fmaf(w.x, p.x, fmaf(w.y, p.y, fmaf(w.z, p.z, fmaf(w.w, p.w, acc[fr]))));
+            }
+        }
+#pragma unroll
+        for (int fr = 0; fr < G; ++fr) acc[fr] = warp_sum(acc[fr]);
+        if (lane == 0)
+#pragma unroll
+            for (int fr = 0; fr < G; ++fr)
+                if (fr < nf) gate[(long long)(f0 + fr) * C + c] = __saturatef((acc[fr] + b2[c] + 3.0f) * (1.0f / 6.0f));
+    }
+}
+
+// ---------------------------------------------------------------------------------------------------- 1x1 on rows
+// out[m][n] = sum_k A[m][k] W[n][k] + b[n] (+ R[m][n]), A float32 scaled by a squeeze-excite gate per group of gate_rows
+// rows, rounded to 16 bits, or already 16-bit.  A warp owns 16 rows and NT n tiles and is on its own: its A fragments come
+// straight from memory into registers (the k order inside an mma is permuted so that a lane's values are one 16-byte load;
+// the packed weights carry the same order), no shared memory, no barrier, STEP loads in flight.
+template <int NT, typename HT>
+__global__ void __launch_bounds__(128, NT > 14 ? 3 : 4)
+rows_gate_kernel(const float* __restrict__ A, const uint4* __restrict__ W, const float* __restrict__ bias, const float* __restrict__ gate,
+                 int gate_rows, const float* R, float* out, int M, int N, int K) {
+    constexpr int NP = (NT + 1) / 2;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, t = lane & 3;
+    const int m0 = (blockIdx.x * 4 + warp) * 16;
+    if (m0 >= M) return;
+    const int ra = min(m0 + g, M - 1), rb = min(m0 + g + 8, M - 1);
+    const float* const pa = A + (long long)ra * K + t * 4;
+    const float* const pb = A + (long long)rb * K + t * 4;
+    const float* const ga = gate + (long long)(ra / gate_rows) * K + t * 4;
+    const float* const gb = gate + (long long)(rb / gate_rows) * K + t * 4;
+    const int np0 = blockIdx.y * NP, npall = gridDim.y * NP;
+    float acc[NT][4];
+#pragma unroll
+    for (int n = 0; n < NT; ++n)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) acc[n][e] = 0.0f;
+    const float4 zero = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    const int kt = (K + 15) / 16;
+    auto load = [&](float4 (&v)[4], int k) {
+        const bool in = k < kt && k * 16 + t * 4 < K;
+        v[0] = in ? __ldg(reinterpret_cast<const float4*>(pa + k * 16)) : zero;
+        v[1] = in ? __ldg(reinterpret_cast<const float4*>(pb + k * 16)) : zero;
+        v[2] = in ? __ldg(reinterpret_cast<const float4*>(ga + k * 16)) : zero;
+        v[3] = in ? __ldg(reinterpret_cast<const float4*>(gb + k * 16)) : zero;
+    };
+    auto step = [&](const float4 (&v)[4], int k) {
+        uint32_t af[4];
+        af[0] = Half<HT>::pack(v[0].x * v[2].x, v[0].y * v[2].y);
+        af[1] = Half<HT>::pack(v[1].x * v[3].x, v[1].y * v[3].y);
+        af[2] = Half<HT>::pack(v[0].z * v[2].z, v[0].w * v[2].w);
+        af[3] = Half<HT>::pack(v[1].z * v[3].z, v[1].w * v[3].w);
+        const uint4* w = W + ((long long)k * npall + np0) * 32 + lane;
+#pragma unroll
+        for (int n = 0; n < NP; ++n) {
+            const uint4 b = __ldg(w + n * 32);
+            Half<HT>::mma(acc[2 * n], af, b.x, b.y);
+            if (2 * n + 1 < NT) Half<HT>::mma(acc[2 * n + 1 < NT ? 2 * n + 1 : 0], af, b.z, b.w);
+        }
+    };
+    float4 v0[4], v1[4];
+    load(v0, 0);
+    for (int k = 0; k < kt; k += 2) {
+        load(v1, k + 1);
+        step(v0, k);
+        load(v0, k + 2);
+        if (k + 1 < kt) step(v1, k + 1);
+    }
+#pragma unroll
+    for (int n = 0; n < NT; ++n) {
+        const int col = blockIdx.y * (NP * 16) + n * 8 + 2 * t;
+        const float2 bv = __ldg(reinterpret_cast<const float2*>(bias + col));
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            const int m = m0 + g + h * 8;
+            if (m >= M) continue;
+            float2 v = make_float2(acc[n][2 * h] + bv.x, acc[n][2 * h + 1] + bv.y);
+            const long long at = (long long)m * N + col;
+            if (R) {
+                const float2 r = *reinterpret_cast<const float2*>(R + at);
+                v.x += r.x;
+                v.y += r.y;
+            }
+            *reinterpret_cast<float2*>(out + at) = v;
+        }
+    }
+}
+
+// the same with A already in the mode's 16-bit type [M][K], K a multiple of 32, no bias (the token projection)
+template <int NT, typename HT>
+__global__ void __launch_bounds__(128)
+rows_h_kernel(const uint16_t* __restrict__ A, const uint4* __restrict__ W, float* __restrict__ out, int M, int N, int K) {
+    constexpr int NP = NT / 2;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, t = lane & 3;
+    const int m0 = (blockIdx.x * 4 + warp) * 16;
+    if (m0 >= M) return;
+    const uint16_t* const pa = A + (long long)min(m0 + g, M - 1) * K + t * 8;
+    const uint16_t* const pb = A + (long long)min(m0 + g + 8, M - 1) * K + t * 8;
+    const int np0 = blockIdx.y * NP, npall = gridDim.y * NP;
+    float acc[NT][4];
+#pragma unroll
+    for (int n = 0; n < NT; ++n)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) acc[n][e] = 0.0f;
+    const int ks = K / 32;
+    uint4 va = __ldg(reinterpret_cast<const uint4*>(pa)), vb = __ldg(reinterpret_cast<const uint4*>(pb));
+#pragma unroll 2
+    for (int k = 0; k < ks; ++k) {
+        const int kn = k + 1 < ks ? k + 1 : k;
+        const uint4 na = __ldg(reinterpret_cast<const uint4*>(pa + kn * 32)), nb = __ldg(reinterpret_cast<const uint4*>(pb + kn * 32));
+        const uint4* w = W + ((long long)k * 2 * npall + np0) * 32 + lane;
+        const uint32_t a0[4] = {va.x, vb.x, va.y, vb.y}, a1[4] = {va.z, vb.z, va.w, vb.w};
+#pragma unroll
+        for (int n = 0; n < NP; ++n) {
+            const uint4 b = __ldg(w + n * 32);
+            Half<HT>::mma(acc[2 * n], a0, b.x, b.y);
+            Half<HT>::mma(acc[2 * n + 1], a0, b.z, b.w);
+        }
+#pragma unroll
+        for (int n = 0; n < NP; ++n) {
+            const uint4 b = __ldg(w + (npall + n) * 32);
+            Half<HT>::mma(acc[2 * n], a1, b.x, b.y);
+            Half<HT>::mma(acc[2 * n + 1], a1, b.z, b.w);
+        }
+        va = na;
+        vb = nb;
+    }
+#pragma unroll
+    for (int n = 0; n < NT; ++n) {
+        const int col = (np0 * 2 + n) * 8 + 2 * t;
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            const int m = m0 + g + h * 8;
+            if (m < M) *reinterpret_cast<float2*>(out + (long long)m * N + col) = make_float2(acc[n][2 * h], acc[n][2 * h + 1]);
+        }
+    }
+}
+
+// ---------------------------------------------------------------------------------------------------- last convolution + pooling
+// 1x1 160 -> 960, Hardswish, adaptive 4x4 average pooling of the 6 x 10 map, rounded to the 16-bit type the token projection
+// reads it in.  A block takes a frame and 96 output channels; the map stays in shared memory.
+struct Last {
+    static constexpr int K = 160, KT = 10, XP = K + 8, N = 960, CE = 96, NT = CE / 8, P = CE + 8, PXS = 60;
+    static constexpr int X_BYTES = 64 * XP * 2, SMEM = X_BYTES + PXS * P * 4;
+};
+template <typename HT>
+__global__ void __launch_bounds__(256, 3)
+last_pool_kernel(const float* __restrict__ x, const uint2* __restrict__ w, const float* __restrict__ b, uint16_t* __restrict__ pooled) {
+    extern __shared__ __align__(16) uint8_t smem[];
+    uint16_t* const X = reinterpret_cast<uint16_t*>(smem);
+    float* const E = reinterpret_cast<float*>(smem + Last::X_BYTES);
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, t = lane & 3, f = blockIdx.x;
+    const float* const img = x + (long long)f * (Last::PXS * Last::K);
+    for (int i = tid; i < Last::PXS * Last::K / 4; i += 256) {
+        const float4 p = *reinterpret_cast<const float4*>(img + i * 4);
+        *reinterpret_cast<uint2*>(X + i / 40 * Last::XP + i % 40 * 4) = make_uint2(Half<HT>::pack(p.x, p.y), Half<HT>::pack(p.z, p.w));
+    }
+    // warp: one half of the n tiles, one of the four pixel groups
+    const int mt = warp & 3, nt0 = (warp >> 2) * (Last::NT / 2);
+    float c[Last::NT / 2][4];
+#pragma unroll
+    for (int n = 0; n < Last::NT / 2; ++n)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) c[n][e] = 0.0f;
+    __syncthreads();
+    const uint32_t xrow = smem_addr(X) + uint32_t(((mt * 16 + (lane & 15)) * Last::XP + (lane >> 4) * 8) * 2);
+    const uint2* const wf = w + ((blockIdx.y * Last::NT + nt0) * Last::KT) * 32 + lane;
+#pragma unroll 2
+    for (int k = 0; k < Last::KT; ++k) {
+        uint32_t af[4];
+        ldmatrix_x4(af, xrow + uint32_t(k * 32));
+#pragma unroll
+        for (int n = 0; n < Last::NT / 2; ++n) {
+            const uint2 bf = __ldg(wf + (n * Last::KT + k) * 32);
+            Half<HT>::mma(c[n], af, bf.x, bf.y);
+        }
+    }
+#pragma unroll
+    for (int n = 0; n < Last::NT / 2; ++n) {
+        const int col = (nt0 + n) * 8 + 2 * t;
+        const float2 bv = __ldg(reinterpret_cast<const float2*>(b + blockIdx.y * Last::CE + col));
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            const int r = mt * 16 + g + h * 8;
+            if (r < Last::PXS) *reinterpret_cast<float2*>(E + r * Last::P + col) = make_float2(hswish(c[n][2 * h] + bv.x), hswish(c[n][2 * h + 1] + bv.y));
+        }
+    }
+    __syncthreads();
+    for (int i = tid; i < 16 * Last::CE / 2; i += 256) {
+        const int cp = i % (Last::CE / 2), tok = i / (Last::CE / 2), r = tok >> 2, q = tok & 3;
+        const int y0 = (r * 6) / 4, y1 = ((r + 1) * 6 + 3) / 4, x0 = (q * 10) / 4, x1 = ((q + 1) * 10 + 3) / 4;
+        float2 s = make_float2(0.0f, 0.0f);
+        for (int y = y0; y < y1; ++y)
+            for (int xx = x0; xx < x1; ++xx) {
+                const float2 v = *reinterpret_cast<const float2*>(E + (y * 10 + xx) * Last::P + cp * 2);
+                s.x += v.x;
+                s.y += v.y;
+            }
+        const float cnt = float((y1 - y0) * (x1 - x0));
+        *reinterpret_cast<uint32_t*>(pooled + ((long long)f * 16 + tok) * Last::N + blockIdx.y * Last::CE + cp * 2) = Half<HT>::pack(s.x / cnt, s.y / cnt);
+    }
+}
+
+//                CIN CEXP COUT K  S  HI  WI  TH  TW  CE PX SR NS  HS     RES   blocks/SM
+using B2 = Block<16, 64, 24, 3, 2, 90, 160, 9, 8, 32, 2, 3, 1, false, false, 3>;
+using B3 = Block<24, 72, 24, 3, 1, 45, 80, 9, 16, 72, 4, 3, 1, false, true, 2>;
+using B4 = Block<24, 72, 0, 5, 2, 45, 80, 12, 10, 24, 2, 3, 1, false, false, 2>;
+using B5 = Block<40, 120, 0, 5, 1, 23, 40, 12, 20, 40, 4, 4, 1, false, false, 2>;
+using B7 = Block<40, 240, 80, 3, 2, 23, 40, 6, 10, 48, 2, 3, 1, true, false, 2>;
+using B8 = Block<80, 200, 80, 3, 1, 12, 20, 6, 20, 32, 4, 3, 2, true, true, 2>;
+using B9 = Block<80, 184, 80, 3, 1, 12, 20, 6, 20, 32, 4, 3, 2, true, true, 2>;
+using B11 = Block<80, 480, 0, 3, 1, 12, 20, 12, 20, 32, 4, 3, 2, true, false, 2>;
+using B12 = Block<112, 672, 0, 3, 1, 12, 20, 12, 20, 32, 4, 3, 2, true, false, 2>;
+using B13 = Block<112, 672, 0, 5, 2, 12, 20, 6, 10, 32, 2, 2, 2, true, false, 2>;
+using B14 = Block<160, 960, 0, 5, 1, 6, 10, 6, 10, 64, 2, 3, 4, true, false, 2>;
+
+inline unsigned blocks_of(long long n, int per) { return unsigned((n + per - 1) / per); }
+inline bool unaligned(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) != 0; }
+
+template <class C, typename HT>
+int launch_block(const BlockArgs& args, int F, cudaStream_t s) {
+    static_assert(C::SMEM <= 227 * 1024, "shared memory");
+    cudaError_t e = cudaFuncSetAttribute(block_kernel<C, HT>, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM);
+    if (e != cudaSuccess) return int(e);
+    BlockArgs a = args;
+    dim3 grid(unsigned(F) * C::TILES, 1);
+    if (C::SE) {
+        // a block redoes the tile's input for its share of the channels: as few shares as give the GPU four blocks per SM
+        const int want = int((4LL * 148 + grid.x - 1) / grid.x);
+        const int groups = want < 1 ? 1 : want > C::CHUNKS ? C::CHUNKS : want;
+        a.chunks_per_group = (C::CHUNKS + groups - 1) / groups;
+        grid.y = unsigned((C::CHUNKS + a.chunks_per_group - 1) / a.chunks_per_group);
+    }
+    block_kernel<C, HT><<<grid, 256, C::SMEM, s>>>(a);
+    return int(cudaGetLastError());
+}
+
+template <typename HT>
+int dispatch_block(int block, const BlockArgs& a, int F, cudaStream_t s) {
+    switch (block) {
+    case 2: return launch_block<B2, HT>(a, F, s);
+    case 3: return launch_block<B3, HT>(a, F, s);
+    case 4: return launch_block<B4, HT>(a, F, s);
+    case 5: case 6: return launch_block<B5, HT>(a, F, s);
+    case 7: return launch_block<B7, HT>(a, F, s);
+    case 8: return launch_block<B8, HT>(a, F, s);
+    case 9: case 10: return launch_block<B9, HT>(a, F, s);
+    case 11: return launch_block<B11, HT>(a, F, s);
+    case 12: return launch_block<B12, HT>(a, F, s);
+    case 13: return launch_block<B13, HT>(a, F, s);
+    case 14: case 15: return launch_block<B14, HT>(a, F, s);
+    default: return int(cudaErrorInvalidValue);
+    }
+}
+int block_tiles(int block) {
+    switch (block) {
+    case 4: return B4::TILES;
+    case 5: case 6: return B5::TILES;
+    case 11: return B11::TILES;
+    case 12: return B12::TILES;
+    case 13: return B13::TILES;
+    case 14: case 15: return B14::TILES;
+    default: return 0;
+    }
+}
+// expanded channels a block walks (a multiple of its chunk), and the k range of its projection
+void block_padding(int block, int* cols, int* k) {
+#define SB_PAD(B) do { *cols = B::CHUNKS * B::CE; *k = B::SE ? B::CEXP : B::CHUNKS * B::CK; } while (0)
+    *cols = *k = 0;
+    switch (block) {
+    case 2: SB_PAD(B2); break;
+    case 3: SB_PAD(B3); break;
+    case 4: SB_PAD(B4); break;
+    case 5: case 6: SB_PAD(B5); break;
+    case 7: SB_PAD(B7); break;
+    case 8: SB_PAD(B8); break;
+    case 9: case 10: SB_PAD(B9); break;
+    case 11: SB_PAD(B11); break;
+    case 12: SB_PAD(B12); break;
+    case 13: SB_PAD(B13); break;
+    case 14: case 15: SB_PAD(B14); break;
+    default: break;
+    }
+#undef SB_PAD
+}
+
+}  // namespace
+}  // namespace sb
+
+// Host side: W [N][K] float32 -> 16-bit mma fragments.  order 0: fragments [n tile][k tile][lane] of 4 values, k as the
+// instruction numbers it; order 1 / 2: [k tile][pair of n tiles][lane] of 8 values, k permuted so that a lane's operand A is
+// four (1) or, over two k tiles, eight (2) consecutive values of a row.
+extern "C" size_t shvk_cnn_packed_bytes(int N, int K, int order) {
+    if (N <= 0 || K <= 0 || order < 0 || order > 2) return 0;
+    const size_t kt = size_t(order == 2 ? (K + 31) / 32 * 2 : (K + 15) / 16);
+    return order == 0 ? size_t((N + 7) / 8) * kt * 32 * 8 : kt * size_t((N + 15) / 16) * 32 * 16;
+}
+extern "C" int shvk_cnn_pack_weights(const float* w, int N, int K, int order, int dtype, void* out) {
+    if (!w || !out || !shvk_cnn_packed_bytes(N, K, order) || (dtype != sb::DT_BF16 && dtype != sb::DT_F16)) return int(cudaErrorInvalidValue);
+    uint16_t* o = static_cast<uint16_t*>(out);
+    auto put = [&](int n, int k) {
+        const float v = n < N && k < K ? w[size_t(n) * K + k] : 0.0f;
+        if (dtype == sb::DT_BF16) {
+            const __nv_bfloat16 h = __float2bfloat16_rn(v);
+            *o++ = *reinterpret_cast<const uint16_t*>(&h);
+        } else {
+            const __half h = __float2half_rn(v);
+            *o++ = *reinterpret_cast<const uint16_t*>(&h);
+        }
+    };
+    if (order == 0) {
+        for (int nt = 0; nt < (N + 7) / 8; ++nt)
+            for (int kt = 0; kt < (K + 15) / 16; ++kt)
+                for (int lane = 0; lane < 32; ++lane)
+                    for (int e = 0; e < 4; ++e) put(nt * 8 + lane / 4, kt * 16 + (e / 2) * 8 + (lane % 4) * 2 + e % 2);
+    } else {
+        const int kts = order == 2 ? (K + 31) / 32 * 2 : (K + 15) / 16;
+        for (int kt = 0; kt < kts; ++kt)
+            for (int np = 0; np < (N + 15) / 16; ++np)
+                for (int lane = 0; lane < 32; ++lane)
+                    for (int e = 0; e < 8; ++e) {
+                        const int n = np * 16 + (e / 4) * 8 + lane / 4;
+                        const int k = order == 1 ? kt * 16 + (lane % 4) * 4 + e % 4 : (kt / 2) * 32 + (lane % 4) * 8 + (kt % 2) * 4 + e % 4;
+                        put(n, k);
+                    }
+    }
+    return 0;
+}
+
+extern "C" int shvk_cnn_block_tiles(int block) { return sb::block_tiles(block); }
+extern "C" void shvk_cnn_block_padding(int block, int* columns, int* k) { sb::block_padding(block, columns, k); }
+
+extern "C" int shvk_cnn_block(int block, const float* x, const void* we, const float* be, const float* wd, const float* bd,
+                              const void* wp, const float* bp, float* out, float* sums, int F, int dtype, void* stream) {
+    if (F <= 0) return 0;
+    const bool se = sb::block_tiles(block) > 0;
+    if (!x || !we || !be || !wd || !bd || !out || (se ? !sums : !wp || !bp) || out == x || sb::unaligned(x) || sb::unaligned(out) ||
+        sb::unaligned(we) || (wp && sb::unaligned(wp)) || sb::unaligned(be) || sb::unaligned(wd) || sb::unaligned(bd) || (bp && sb::unaligned(bp)))
+        return int(cudaErrorInvalidValue);
+    const sb::BlockArgs a{x, static_cast<const uint2*>(we), be, wd, bd, static_cast<const uint2*>(wp), bp, out, sums, 0};
+    if (dtype == sb::DT_BF16) return sb::dispatch_block<__nv_bfloat16>(block, a, F, cudaStream_t(stream));
+    if (dtype == sb::DT_F16) return sb::dispatch_block<__half>(block, a, F, cudaStream_t(stream));
+    return int(cudaErrorInvalidValue);
+}
+
+extern "C" int shvk_cnn_stem_block(const uint8_t* frames, const float* lut, const float* stem_w_host, const float* stem_b_host,
+                                   const float* wd, const float* bd, const void* wp, const float* bp, float* out, int F, int dtype,
+                                   void* stream) {
+    if (F <= 0) return 0;
+    if (!frames || !lut || !stem_w_host || !stem_b_host || !wd || !bd || !wp || !bp || !out || sb::unaligned(out) || sb::unaligned(wp) ||
+        sb::unaligned(wd) || sb::unaligned(bd) || sb::unaligned(bp) || (dtype != sb::DT_BF16 && dtype != sb::DT_F16))
+        return int(cudaErrorInvalidValue);
+    sb::StemParams sp;
+    for (int i = 0; i < 27 * 16; ++i) sp.w[i] = stem_w_host[i];
+    for (int i = 0; i < 16; ++i) sp.b[i] = stem_b_host[i];
+    const unsigned grid = unsigned(F) * sb::Stem::TILES;
+    auto go = [&](auto kernel) {
+        const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, sb::Stem::SMEM);
+        if (e != cudaSuccess) return int(e);
+        kernel<<<grid, 256, sb::Stem::SMEM, cudaStream_t(stream)>>>(frames, lut, sp, wd, bd, static_cast<const uint2*>(wp), bp, out);
+        return int(cudaGetLastError());
+    };
+    return dtype == sb::DT_BF16 ? go(sb::stem_block_kernel<__nv_bfloat16>) : go(sb::stem_block_kernel<__half>);
+}
+
+extern "C" int shvk_cnn_se_gate_sums(const float* sums, const float* w1, const float* b1, const float* w2, const float* b2, float* gate,
+                                     int F, int tiles, int HW, int C, int CS, void* stream) {
+    if (F <= 0) return 0;
+    if (!sums || tiles <= 0 || HW <= 0 || C <= 0 || CS <= 0 || (C & 3) || (CS & 3) || sb::unaligned(w1) || sb::unaligned(w2))
+        return int(cudaErrorInvalidValue);
+    // frames per cluster: one while that leaves the GPU a wave of blocks or less, else four (a weight row serves four frames)
+    const int G = F <= 37 ? 1 : 4;
+    const size_t smem = size_t(G) * size_t(C + CS) * sizeof(float);
+    if (smem > 48 * 1024) return int(cudaErrorInvalidValue);
+    const unsigned grid = sb::blocks_of(F, G) * 8;
+    cudaStream_t s = cudaStream_t(stream);
+    if (G == 1) sb::se_gate_cluster_kernel<1><<<grid, 256, smem, s>>>(sums, w1, b1, w2, b2, gate, F, tiles, float(HW), C, CS);
+    else sb::se_gate_cluster_kernel<4><<<grid, 256, smem, s>>>(sums, w1, b1, w2, b2, gate, F, tiles, float(HW), C, CS);
+    return int(cudaGetLastError());
+}
+
+namespace sb {
+namespace {
+template <typename HT>
+int launch_rows_gate(const float* A, const uint4* W, const float* b, const float* gate, int gate_rows, const float* R, float* out, int M,
+                     int N, int K, cudaStream_t s) {
+    const unsigned gx = blocks_of(M, 64);
+    switch (N) {
+    case 40: rows_gate_kernel<5, HT><<<gx, 128, 0, s>>>(A, W, b, gate, gate_rows, R, out, M, N, K); break;
+    case 112: rows_gate_kernel<14, HT><<<gx, 128, 0, s>>>(A, W, b, gate, gate_rows, R, out, M, N, K); break;
+    case 160: rows_gate_kernel<20, HT><<<gx, 128, 0, s>>>(A, W, b, gate, gate_rows, R, out, M, N, K); break;
+    default: return int(cudaErrorInvalidValue);
+    }
+    return int(cudaGetLastError());
+}
+}  // namespace
+}  // namespace sb
+
+extern "C" int shvk_cnn_rows_gate(const float* A, const void* W, const float* b, const float* gate, int gate_rows, const float* R,
+                                  float* out, int M, int N, int K, int dtype, void* stream) {
+    if (M <= 0) return 0;
+    if (!A || !W || !b || !gate || gate_rows <= 0 || !out || K <= 0 || (K & 3) || sb::unaligned(A) || sb::unaligned(W) || sb::unaligned(b) ||
+        sb::unaligned(gate) || (R && sb::unaligned(R)) || sb::unaligned(out))
+        return int(cudaErrorInvalidValue);
+    const uint4* w = static_cast<const uint4*>(W);
+    if (dtype == sb::DT_BF16) return sb::launch_rows_gate<__nv_bfloat16>(A, w, b, gate, gate_rows, R, out, M, N, K, cudaStream_t(stream));
+    if (dtype == sb::DT_F16) return sb::launch_rows_gate<__half>(A, w, b, gate, gate_rows, R, out, M, N, K, cudaStream_t(stream));
+    return int(cudaErrorInvalidValue);
+}
+
+extern "C" int shvk_cnn_last_pool(const float* x, const void* w, const float* b, void* pooled, int F, int dtype, void* stream) {
+    if (F <= 0) return 0;
+    if (!x || !w || !b || !pooled || sb::unaligned(x) || sb::unaligned(w) || sb::unaligned(b) || sb::unaligned(pooled))
+        return int(cudaErrorInvalidValue);
+    auto go = [&](auto kernel) {
+        const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, sb::Last::SMEM);
+        if (e != cudaSuccess) return int(e);
+        kernel<<<dim3(unsigned(F), sb::Last::N / sb::Last::CE), 256, sb::Last::SMEM, cudaStream_t(stream)>>>(x, static_cast<const uint2*>(w), b,
+                                                                                                     static_cast<uint16_t*>(pooled));
+        return int(cudaGetLastError());
+    };
+    if (dtype == sb::DT_BF16) return go(sb::last_pool_kernel<__nv_bfloat16>);
+    if (dtype == sb::DT_F16) return go(sb::last_pool_kernel<__half>);
+    return int(cudaErrorInvalidValue);
+}
+
+extern "C" int shvk_cnn_token_proj(const void* pooled, const void* W, float* tokens, int rows, int dtype, void* stream) {
+    if (rows <= 0) return 0;
+    if (!pooled || !W || !tokens || sb::unaligned(pooled) || sb::unaligned(W) || sb::unaligned(tokens)) return int(cudaErrorInvalidValue);
+    const uint16_t* A = static_cast<const uint16_t*>(pooled);
+    const uint4* w = static_cast<const uint4*>(W);
+    cudaStream_t s = cudaStream_t(stream);
+    const dim3 grid(sb::blocks_of(rows, 64), 384 / 64);
+    if (dtype == sb::DT_BF16) sb::rows_h_kernel<8, __nv_bfloat16><<<grid, 128, 0, s>>>(A, w, tokens, rows, 384, 960);
+    else if (dtype == sb::DT_F16) sb::rows_h_kernel<8, __half><<<grid, 128, 0, s>>>(A, w, tokens, rows, 384, 960);
+    else return int(cudaErrorInvalidValue);
+    return int(cudaGetLastError());
+}

@@ -303,3 +303,134 @@ def test_encode_frame_independence_and_graphs(weight_files):
     assert eager.encode_launches() == 4 + sum(2 + (1 if e != i else 0) + (2 if se else 0) for (i, _k, e, _o, se, _a, _s) in BLOCKS)
     eager.close()
     graph.close()
+
+
+# ---------------------------------------------------------------------------------------------- fused kernels (16-bit modes)
+def _pack(L, w, order, dtype, n_pad=None, k_pad=None):
+    import torch
+    n, k = w.shape
+    full = np.zeros((n_pad or n, k_pad or k), np.float32)
+    full[:n, :k] = w
+    out = np.zeros(L.shvk_cnn_packed_bytes(*full.shape, order), np.uint8)
+    assert L.shvk_cnn_pack_weights(full.ctypes.data, *full.shape, order, dtype, out.ctypes.data) == 0
+    return torch.from_numpy(out).cuda()
+
+
+_BLOCKS = [(16, 3, 16, 16, False, 1), (16, 3, 64, 24, False, 2), (24, 3, 72, 24, False, 1), (24, 5, 72, 40, True, 2),
+           (40, 5, 120, 40, True, 1), (40, 5, 120, 40, True, 1), (40, 3, 240, 80, False, 2), (80, 3, 200, 80, False, 1),
+           (80, 3, 184, 80, False, 1), (80, 3, 184, 80, False, 1), (80, 3, 480, 112, True, 1), (112, 3, 672, 112, True, 1),
+           (112, 5, 672, 160, True, 2), (160, 5, 960, 160, True, 1), (160, 5, 960, 160, True, 1)]
+
+
+@pytest.mark.parametrize("dtype", [1, 2])
+@pytest.mark.parametrize("block", [2, 3, 4, 5, 7, 8, 9, 11, 12, 13, 14])
+def test_fused_block_matches_layers(L, block, dtype):
+    """One fused block (expand + depthwise + project or pooled sums, gate, gated project) against the layer kernels on the same
+    input.  Both round the 1x1 operands to the same type; the fused Hardswish differs in the last bit of a float32, so an operand
+    can round the other way: an ulp of the 16-bit type (at most 2^-7 or 2^-10 relative) on isolated terms of a K-term sum."""
+    import torch
+    cin, k, cexp, cout, se, stride = _BLOCKS[block - 1]
+    H, W = 90, 160
+    for _cin, kk, *_r, st in _BLOCKS[:block - 1]:
+        H, W = (H + 2 * ((kk - 1) // 2) - kk) // st + 1, (W + 2 * ((kk - 1) // 2) - kk) // st + 1
+    pad = (k - 1) // 2
+    Ho, Wo = (H + 2 * pad - k) // stride + 1, (W + 2 * pad - k) // stride + 1
+    act = 1 if block < 7 else 2
+    rng = np.random.default_rng(block)
+    F = 3
+    f32 = lambda *s: rng.standard_normal(s).astype(np.float32)  # noqa: E731
+    x, we, be = dev(f32(F, H, W, cin)), f32(cexp, cin) / np.float32(np.sqrt(cin)), dev(f32(cexp))
+    wd, bd = dev(f32(k * k, cexp) / np.float32(k)), dev(f32(cexp))
+    wp, bp = f32(cout, cexp) / np.float32(np.sqrt(cexp)), dev(f32(cout))
+    zeros = lambda *s: torch.zeros(s, device="cuda")  # noqa: E731
+    # layer by layer
+    E, Dm, Y = zeros(F, H, W, cexp), zeros(F, Ho, Wo, cexp), zeros(F, Ho, Wo, cout)
+    d_we, d_wp = dev(we), dev(wp)
+    assert L.shvk_cnn_pointwise_h(_ptr(x), _ptr(d_we), _ptr(be), None, 1, None, _ptr(E), F * H * W, cexp, cin, act, dtype, stream_ptr()) == 0
+    assert L.shvk_cnn_depthwise(_ptr(E), _ptr(wd), _ptr(bd), _ptr(Dm), F, H, W, cexp, k, stride, Ho, Wo, act, stream_ptr()) == 0
+    res = x if stride == 1 and cin == cout else None
+    gate = zeros(F, cexp)
+    if se:
+        cs = {72: 24, 120: 32, 480: 120, 672: 168, 960: 240}[cexp]
+        w1, b1, w2, b2 = dev(f32(cs, cexp) / np.float32(np.sqrt(cexp))), dev(f32(cs)), dev(f32(cexp, cs) / np.float32(np.sqrt(cs))), dev(f32(cexp))
+        part = zeros(L.shvk_cnn_se_partial_floats(F, Ho * Wo, cexp))
+        assert L.shvk_cnn_se_gate(_ptr(Dm), _ptr(part), _ptr(w1), _ptr(b1), _ptr(w2), _ptr(b2), _ptr(gate), F, Ho * Wo, cexp, cs, stream_ptr()) == 0
+    assert L.shvk_cnn_pointwise_h(_ptr(Dm), _ptr(d_wp), _ptr(bp), _ptr(gate) if se else None, Ho * Wo, _ptr(res) if res is not None else None,
+                                  _ptr(Y), F * Ho * Wo, cout, cexp, 0, dtype, stream_ptr()) == 0
+    # fused
+    cols, kp = C.c_int(), C.c_int()
+    L.shvk_cnn_block_padding(block, C.byref(cols), C.byref(kp))
+    tiles = L.shvk_cnn_block_tiles(block)
+    assert (tiles > 0) == se and cols.value >= cexp and kp.value >= cexp
+    p_we = _pack(L, we, 0, dtype, cols.value)
+    p_wp = _pack(L, wp, 1 if se else 0, dtype, None, kp.value)
+    out = zeros(F, Ho, Wo, cexp if se else cout)
+    sums = torch.full((F, max(tiles, 1), cexp), float("nan"), device="cuda")
+    args = [block, _ptr(x), _ptr(p_we), _ptr(be), _ptr(wd), _ptr(bd), None if se else _ptr(p_wp), None if se else _ptr(bp)]
+    assert L.shvk_cnn_block(*args, _ptr(out), _ptr(sums), F, dtype, stream_ptr()) == 0
+    assert L.shvk_cnn_block(*args, _ptr(x), _ptr(sums), F, dtype, stream_ptr()) != 0        # in place is refused
+    if se:
+        sync()
+        assert rel_err(out.cpu().numpy(), Dm.cpu().numpy()) < 2e-6                            # float32 arithmetic on the same mma sums
+        assert rel_err(sums.sum(1).cpu().numpy(), Dm.sum((1, 2)).cpu().numpy()) < 1e-5
+        g2, y2 = zeros(F, cexp), zeros(F, Ho, Wo, cout)
+        assert L.shvk_cnn_se_gate_sums(_ptr(sums), _ptr(w1), _ptr(b1), _ptr(w2), _ptr(b2), _ptr(g2), F, tiles, Ho * Wo, cexp, cs, stream_ptr()) == 0
+        assert L.shvk_cnn_rows_gate(_ptr(out), _ptr(p_wp), _ptr(bp), _ptr(g2), Ho * Wo, _ptr(res) if res is not None else None, _ptr(y2),
+                                    F * Ho * Wo, cout, cexp, dtype, stream_ptr()) == 0
+        sync()
+        assert np.abs((g2 - gate).cpu().numpy()).max() < 1e-5
+        out = y2
+    sync()
+    got, ref = out.cpu().numpy(), Y.cpu().numpy()
+    unit = 2.0 ** -8 if dtype == 1 else 2.0 ** -11
+    assert np.abs(got - ref).max() < 4 * unit * float(Dm.abs().max()) * np.abs(wp).max()   # two operands rounded the other way, an ulp each
+    assert np.sqrt(((got - ref) ** 2).mean() / (ref ** 2).mean()) < unit / 16
+    # a frame's result does not depend on the batch it is in
+    one, s1 = zeros(1, *[int(v) for v in (Ho, Wo, cexp if se else cout)]), zeros(1, max(tiles, 1), cexp)
+    x1 = x[2:3].contiguous()
+    assert L.shvk_cnn_block(block, _ptr(x1), *args[2:], _ptr(one), _ptr(s1), 1, dtype, stream_ptr()) == 0
+    sync()
+    if se:
+        assert torch.equal(s1[0], sums[2])
+    else:
+        assert torch.equal(one[0], out[2])
+
+
+@pytest.mark.parametrize("dtype", [1, 2])
+def test_fused_ends_of_the_encoder(L, dtype):
+    """Stem + block 1 and last convolution + pooling + token projection against the layer kernels."""
+    import torch
+    from oracle import cnn_oracle as CO
+    rng = np.random.default_rng(9)
+    F = 3
+    f32 = lambda *s: rng.standard_normal(s).astype(np.float32)  # noqa: E731
+    zeros = lambda *s: torch.zeros(s, device="cuda")  # noqa: E731
+    unit = 2.0 ** -8 if dtype == 1 else 2.0 ** -11
+    frames = dev(rng.integers(0, 256, size=(F, 180, 320, 3), dtype=np.uint8))
+    lut = np.stack([((np.arange(256, dtype=np.float32) / np.float32(255)) - CO.MEAN[c]) / CO.STD[c] for c in range(3)]).astype(np.float32)
+    ws, bs, wd, bd, wp, bp = f32(27, 16) * np.float32(0.3), f32(16), dev(f32(9, 16) / 3), dev(f32(16)), f32(16, 16) / 4, dev(f32(16))
+    d_lut, d_ws, d_bs, d_wp = dev(lut), dev(ws), dev(bs), dev(wp)
+    S, Dm, Y, out = zeros(F, 90, 160, 16), zeros(F, 90, 160, 16), zeros(F, 90, 160, 16), zeros(F, 90, 160, 16)
+    assert L.shvk_cnn_stem(_ptr(frames), _ptr(d_lut), _ptr(d_ws), _ptr(d_bs), _ptr(S), F, stream_ptr()) == 0
+    assert L.shvk_cnn_depthwise(_ptr(S), _ptr(wd), _ptr(bd), _ptr(Dm), F, 90, 160, 16, 3, 1, 90, 160, 1, stream_ptr()) == 0
+    assert L.shvk_cnn_pointwise_h(_ptr(Dm), _ptr(d_wp), _ptr(bp), None, 1, _ptr(S), _ptr(Y), F * 14400, 16, 16, 0, dtype, stream_ptr()) == 0
+    p_wp = _pack(L, wp, 0, dtype)
+    assert L.shvk_cnn_stem_block(_ptr(frames), _ptr(d_lut), ws.ctypes.data, bs.ctypes.data, _ptr(wd), _ptr(bd), _ptr(p_wp), _ptr(bp),
+                                 _ptr(out), F, dtype, stream_ptr()) == 0
+    sync()
+    assert float((out - Y).abs().max()) < 2 * unit * float(Dm.abs().max()) * np.abs(wp).max()   # one operand rounded the other way: one ulp
+    assert float(((out - Y) ** 2).mean().sqrt() / (Y ** 2).mean().sqrt()) < unit / 64
+    x, wl, bl, wt = dev(f32(F, 60, 160)), f32(960, 160) / np.float32(np.sqrt(160)), dev(f32(960)), f32(384, 960) / np.float32(np.sqrt(960))
+    fmap, pooled, tok = zeros(F, 60, 960), zeros(F, 16, 960), zeros(F * 16, 384)
+    d_wl, d_wt = dev(wl), dev(wt)
+    assert L.shvk_cnn_pointwise_h(_ptr(x), _ptr(d_wl), _ptr(bl), None, 1, None, _ptr(fmap), F * 60, 960, 160, 2, dtype, stream_ptr()) == 0
+    assert L.shvk_cnn_pool_tokens(_ptr(fmap), _ptr(pooled), F, stream_ptr()) == 0
+    assert L.shvk_cnn_pointwise_h(_ptr(pooled), _ptr(d_wt), None, None, 1, None, _ptr(tok), F * 16, 384, 960, 0, dtype, stream_ptr()) == 0
+    p_wl, p_wt = _pack(L, wl, 0, dtype), _pack(L, wt, 2, dtype)
+    low = torch.zeros((F, 16, 960), device="cuda", dtype=torch.bfloat16 if dtype == 1 else torch.float16)
+    tok2 = zeros(F * 16, 384)
+    assert L.shvk_cnn_last_pool(_ptr(x), _ptr(p_wl), _ptr(bl), _ptr(low), F, dtype, stream_ptr()) == 0
+    assert L.shvk_cnn_token_proj(_ptr(low), _ptr(p_wt), _ptr(tok2), F * 16, dtype, stream_ptr()) == 0
+    sync()
+    assert rel_err(low.float().cpu().numpy(), pooled.cpu().numpy()) < unit
+    assert rel_err(tok2.cpu().numpy(), tok.cpu().numpy()) < unit
