@@ -14,9 +14,10 @@
 // shvk_gdn_inproj_row_order): tile 3h = [q_h | k_h], 3h + 1 = v_h, 3h + 2 = gate_h for head h; tile 18 = [a | b | 0].
 // Token tiles per clip: tokens 0..175 and tokens 160..335 (176 columns each; the second tile computes tokens 160..175
 // again only as the convolution's history and writes chunks 11..20; token slots 321.. are written as zeros).
-// One work item = (clip, token tile) = all 19 channel tiles: the item's xn rows (176 x 384, 132 KB) are brought into
+// One work item = (clip, token tile) = all 19 channel tiles, or, where whole items would leave SMs idle, a share of them
+// (rule at the launch): the item's xn rows (176 x 384, 132 KB) are brought into
 // shared memory ONCE and stay there while the 19 weight tiles stream past them through a five-stage ring, so the
-// operand traffic out of L2 is 4.0 MB per clip instead of 8.6 MB with both operands streamed (which alone took
+// operand traffic out of L2 is 4.0 MB per clip (whole items) instead of 8.6 MB with both operands streamed (which alone took
 // 2.0 ms per launch at 4096 clips, more than the products).  Neighbouring CTAs take the two tiles of one clip.
 //
 // Roles (352 threads): warp 0 streams W' tiles (TMA, 128-byte swizzle, no multicast), warp 2 loads the xn tile of the
@@ -67,6 +68,7 @@ struct InprojParams {
     const float *conv_w, *conv_b, *a_log, *dt_bias;
     uint8_t* pt;
     uint32_t spin_limit;
+    int whole;       // work split of the launch: whole items, or shares of channel tiles
     int starve;      // test launch only: the producer withholds the first weight tile of its first work item
     int qk_f16;      // q^T / k^T tiles in fp16 (fp16 mode) instead of bf16
     int probe;       // timing probes of a development build (-DSHVK_DEV_PROBES, SHVK_INPROJ_PROBE): 1 no global stores,
@@ -327,7 +329,19 @@ gdn_inproj_kernel(const __grid_constant__ InprojMaps maps, const InprojParams p,
     const uint32_t tmem_base = tmem_base_slot;
     volatile int* abortp = &abort_flag;
     [[maybe_unused]] const long long tk0 = PROF_T();
-    const long long items = 2ll * p.B;                           // item = 2 * clip + token tile
+    // item = 2 * clip + token tile.  Either whole items, one every gridDim.x (p.whole), or a contiguous share of the units
+    // (item, channel tile), walked in segments: channel tiles m0 .. m1 - 1 of one item.
+    const long long units = 2ll * p.B * M_TILES;
+    const long long u0 = p.whole ? (long long)blockIdx.x * M_TILES : units * blockIdx.x / gridDim.x;
+    const long long u1 = p.whole ? units : units * (blockIdx.x + 1ll) / gridDim.x;
+    const long long hop = p.whole ? (long long)(gridDim.x - 1) * M_TILES : 0;      // from the end of a segment to the next one
+    auto segment = [&](long long u, long long& item, int& m0, int& m1) {
+        item = u / M_TILES;
+        m0 = int(u - item * M_TILES);
+        m1 = int(min((long long)M_TILES, m0 + (u1 - u)));
+    };
+    long long item;
+    int m0, m1;
 
     if (warp == 0) {
         if (lane == 0) {                                         // ---- W' tiles: 19 x 6 k-blocks per item through the ring
@@ -335,13 +349,14 @@ gdn_inproj_kernel(const __grid_constant__ InprojMaps maps, const InprojParams p,
             uint32_t phase = 0;
             bool ok = true;
             const uint64_t pol_w = policy_evict_last();
-            for (long long item = blockIdx.x; ok && item < items; item += gridDim.x) {
-                for (int m = 0; ok && m < M_TILES; ++m) {
+            for (long long u = u0; ok && u < u1; u += m1 - m0 + hop) {
+                segment(u, item, m0, m1);
+                for (int m = m0; ok && m < m1; ++m) {
                     for (int kb = 0; kb < KBLOCKS; ++kb) {
                         [[maybe_unused]] const long long tw0 = PROF_T();
                         if (!mbar_wait(wempty_bar(stage), phase ^ 1u, abortp, p.spin_limit)) { ok = false; break; }
                         PROF_ADD(0, PROF_T() - tw0);
-                        if (p.starve && item == (long long)blockIdx.x && m == 0 && kb == 0) {   // test launch: this stage never fills
+                        if (p.starve && u == u0 && m == m0 && kb == 0) {   // test launch: this stage never fills
                             if (++stage == W_STAGES) { stage = 0; phase ^= 1u; }
                             continue;
                         }
@@ -357,7 +372,8 @@ gdn_inproj_kernel(const __grid_constant__ InprojMaps maps, const InprojParams p,
         if (lane == 0) {                                         // ---- the item's xn rows, once per item
             uint32_t n = 0;
             bool ok = true;
-            for (long long item = blockIdx.x; ok && item < items; item += gridDim.x, ++n) {
+            for (long long u = u0; u < u1; u += m1 - m0 + hop, ++n) {
+                segment(u, item, m0, m1);
                 const int row0 = int(item >> 1) * kTok + int(item & 1) * TT_STRIDE;
                 if (!mbar_wait(xempty_bar, (n & 1u) ^ 1u, abortp, p.spin_limit)) { ok = false; break; }
                 mbar_expect_tx(xfull_bar, uint32_t(XN_BYTES));
@@ -371,11 +387,12 @@ gdn_inproj_kernel(const __grid_constant__ InprojMaps maps, const InprojParams p,
             uint32_t phase = 0, acc_phase = 0, n = 0;
             bool ok = true;
             [[maybe_unused]] const int probe_bits = p.probe;
-            for (long long item = blockIdx.x; ok && item < items; item += gridDim.x, ++n) {
+            for (long long u = u0; ok && u < u1; u += m1 - m0 + hop, ++n) {
+                segment(u, item, m0, m1);
                 { [[maybe_unused]] const long long tm2 = PROF_T();
                   if (!mbar_wait(xfull_bar, n & 1u, abortp, p.spin_limit)) { ok = false; break; }
                   PROF_ADD(2, PROF_T() - tm2); }
-                for (int m = 0; ok && m < M_TILES; ++m) {
+                for (int m = m0; ok && m < m1; ++m) {
                     [[maybe_unused]] const long long tm0 = PROF_T();
                     if (!mbar_wait(acce_bar(acc), acc_phase ^ 1u, abortp, p.spin_limit)) { ok = false; break; }
                     PROF_ADD(0, PROF_T() - tm0);
@@ -409,7 +426,8 @@ gdn_inproj_kernel(const __grid_constant__ InprojMaps maps, const InprojParams p,
         int acc = 0;
         uint32_t acc_phase = 0;
         bool ok = true;
-        for (long long item = blockIdx.x; ok && item < items; item += gridDim.x) {
+        for (long long u = u0; ok && u < u1; u += m1 - m0 + hop) {
+            segment(u, item, m0, m1);
             const int clip = int(item >> 1), tt = int(item & 1);
             // this warp's columns of the accumulator: [col0, col0 + ncols), written from chunk `chunk0` on; its three
             // history tokens are the columns just before col0 (none at the start of the clip)
@@ -417,9 +435,9 @@ gdn_inproj_kernel(const __grid_constant__ InprojMaps maps, const InprojParams p,
             const int ncols = half ? 80 : (tt ? 80 : 96);
             const int tok0 = tt * TT_STRIDE + col0, chunk0 = tok0 >> 4;
             const bool has_hist = col0 > 0;
-            ChanSite cur = chan_site(p, 0, r);
-            for (int m = 0; m < M_TILES; ++m) {
-                const ChanSite nxt = chan_site(p, m + 1 < M_TILES ? m + 1 : m, r);   // its loads fly during this tile's work
+            ChanSite cur = chan_site(p, m0, r);
+            for (int m = m0; m < m1; ++m) {
+                const ChanSite nxt = chan_site(p, m + 1 < m1 ? m + 1 : m, r);   // its loads fly during this tile's work
                 [[maybe_unused]] const long long tp0 = PROF_T();
                 if (!mbar_wait(accf_bar(acc), acc_phase, abortp, p.spin_limit)) { ok = false; break; }
                 [[maybe_unused]] const long long tp1 = PROF_T();
@@ -555,8 +573,15 @@ static int inproj_launch(const void* host_plan, int B, void* stream, int starve,
     p.B = B;
     p.starve = starve;
     p.spin_limit = spin_limit;
-    const long long items = 2ll * B;
-    const unsigned grid = unsigned(items < sms ? items : sms);
+    // Whole items cost rounds x (19 channel tiles + one token tile load), a round being an item on every SM; shares cost
+    // their tiles and a load per item touched.  A load with its bubble is worth about two channel tiles, and a tile of a
+    // share about 1.07 of a whole item's (the SMs are then at different channel tiles, and each weight tile is fetched for
+    // fewer of them at a time).  us per launch, whole / shares: 1 window 48 / 14, 20 53 / 27, 45 57 / 43, 64 59 / 60,
+    // 80 99 / 64, 96 101 / 73, 160 146 / 111, 224 192 / 150, 4096 2852 / 3004.
+    const long long items = 2ll * B, units = items * M_TILES, rounds = (items + sms - 1) / sms, share = (units + sms - 1) / sms;
+    p.whole = 100 * rounds * (M_TILES + 2) <= 107 * share + 200 * (share / M_TILES + 2);
+    const long long blocks = p.whole ? items : units;
+    const unsigned grid = unsigned(blocks < sms ? blocks : sms);
 #ifdef SHVK_DEV_PROBES
     {
         const char* e = getenv("SHVK_INPROJ_PROBE");

@@ -629,6 +629,23 @@ def test_gdn_inproj_scan_clips_are_independent(L, weight_files):
     assert torch.isfinite(outs[0][1].float()).all()
 
 
+@pytest.mark.parametrize("B", [2, 4, 45, 75, 97, 150])
+def test_gdn_inproj_work_splits_give_the_same_tiles(L, weight_files, B):
+    """Few clips are split over the SMs by channel tile, in shares that start and end inside a token tile (one tile a share up
+    to 3 clips, shares across two or three items above), more go out as whole items: the blocks of every clip are, bit for
+    bit, those of the clip alone."""
+    import torch
+    _, w0 = weight_files("W3", 1)
+    w = rounded_mixer_weights(w0, "gdn_b")
+    distinct = bf16_round(np.random.default_rng(43).standard_normal((2, 321, 384)))
+    alone = [run_inproj(L, w, "gdn_b", distinct[i:i + 1], 1, prep=False)[0].clone() for i in range(2)]
+    pt, keep = run_inproj(L, w, "gdn_b", distinct[np.arange(B) % 2], B, prep=False)
+    pt = pt.reshape(B, -1)
+    assert tc_status(L) == 0
+    for i in range(2):
+        assert (pt[i::2] == alone[i].reshape(1, -1)).all()
+
+
 def test_starved_launches_give_up_and_the_status_clears(L, weight_files):
     """A bounded wait that runs out: the tensor-core GEMM, the scan, the fused in-projection and the fused feed-forward
     block are each launched once with their input withheld.
