@@ -174,6 +174,9 @@ public:
         fbuckets_ = size_classes(cfg_.max_frames);
         wbuckets_ = size_classes(cfg_.max_windows);
         dt_ = dtype_code(p);
+        int dev = 0;
+        cuda_ok(cudaGetDevice(&dev), "device");
+        cuda_ok(cudaDeviceGetAttribute(&sms_, cudaDevAttrMultiProcessorCount, dev), "device");
         cnn_ = fold_cnn(hm);
         upload(hm);
         allocate();
@@ -219,7 +222,7 @@ public:
         starve_kind_ = kind;
         starve_batches_ = batches > 0 ? batches : 0;
     }
-    // 16-bit modes: 24 kernels.  Exact tier: 23 (its feed-forward blocks are two GEMMs each) + a launch that splits the
+    // 16-bit modes: 24 kernels (26 in a batch whose feed-forward blocks are two GEMMs each).  Exact tier: 23 (its feed-forward blocks are two GEMMs each) + a launch that splits the
     // A operand of the five GEMMs that do not read a normalised row (three o-projections, two FFN down projections)
     int launches_per_classify() const override { return prec_ == Precision::FP32 ? 28 : 24; }
 
@@ -258,6 +261,20 @@ private:
     float *h_ = nullptr, *P_ = nullptr;
     void *xn_ = nullptr, *on_ = nullptr, *hid_ = nullptr;
     float* a2_ = nullptr;
+    // 16-bit modes: whether the feed-forward blocks run as two GEMMs.  The fused kernel gives every 128 rows one SM, which takes
+    // 42 us for them however few there are; the two GEMMs spread a row block's columns over the SMs (the same sums in the
+    // same order) but move the hidden layer through L2: 12 us + 0.32 us per row block.  us per block, fused / two GEMMs: 1
+    // window 41 / 14, 8 42 / 19, 20 42 / 26, 40 44 / 42, 48 44 / 43, 56 44 / 46, 64 82 / 57, 80 83 / 69, 96 85 / 86,
+    // 112 85 / 98, 128 129 / 114.  Beyond FFN_TWO_ROWS the hidden layer would not stay in L2.
+    static constexpr int FFN_TWO_ROWS = 128 * NTOK;
+    bool two_launch_ffn(int rows) const {
+        if (size_t(rows) > hid_rows_) return false;
+        if (prec_ == Precision::FP32) return true;
+        const int blocks = (rows + 127) / 128;
+        return 12 + 0.32 * blocks < 42.0 * ((blocks + sms_ - 1) / sms_);
+    }
+    int sms_ = 148;
+    size_t hid_rows_ = 0;                               // rows hid_ holds
     static constexpr int SB_COLS = 960, SG_LD = 112;    // SISA rows of the 16-bit modes: [K | V | B] fp16, [theta | alpha | forget | pad] fp32
     float *s16_ = nullptr, *sg_ = nullptr;
     float *qc_ = nullptr, *y_ = nullptr, *x2_ = nullptr;
@@ -455,8 +472,10 @@ private:
     void allocate() {
         const size_t Bm = size_t(cfg_.max_windows), Mm = Bm * NTOK, Fm = size_t(cfg_.max_frames), ts = dtype_bytes(prec_);
         const size_t o_h = acts_.reserve(Mm * D * 4), o_p = acts_.reserve(Mm * GLD * 4), o_xn = acts_.reserve(prec_ == Precision::FP32 ? 256 : Mm * D * ts);   // exact tier: the norm kernels write into a2_
-        // the hidden layer of the feed-forward blocks exists in memory only in the exact tier (the 16-bit modes keep it on the SM)
-        const size_t o_on = acts_.reserve(Mm * VD * ts), o_hid = acts_.reserve(prec_ == Precision::FP32 ? Mm * DFF * ts : 0);
+        // the hidden layer of the feed-forward blocks exists in memory for every row in the exact tier; the 16-bit modes keep it
+        // on the SM, except in small batches (two_launch_ffn)
+        hid_rows_ = prec_ == Precision::FP32 ? Mm : std::min(Mm, size_t(FFN_TWO_ROWS));
+        const size_t o_on = acts_.reserve(Mm * VD * ts), o_hid = acts_.reserve(hid_rows_ * DFF * ts);
         const size_t o_qc = acts_.reserve(Bm * SQN * 4), o_y = acts_.reserve(Bm * D * 4), o_x2 = acts_.reserve(Bm * D * 4);
         // exact tier: the split A operand [lo | hi] of the GEMM about to run (widest: the FFN hidden layer)
         const size_t o_a2 = acts_.reserve(prec_ == Precision::FP32 ? Mm * 2 * DFF * 4 : 0);
@@ -488,7 +507,7 @@ private:
         se_part_ = acts_.at<float>(o_sp); se_gate_ = acts_.at<float>(o_sg); pooled_ = acts_.at<float>(o_po);
         h_ = acts_.at<float>(o_h); P_ = acts_.at<float>(o_p);
         xn_ = acts_.at<void>(o_xn); on_ = acts_.at<void>(o_on);
-        hid_ = prec_ == Precision::FP32 ? acts_.at<void>(o_hid) : nullptr;
+        hid_ = acts_.at<void>(o_hid);
         qc_ = acts_.at<float>(o_qc); y_ = acts_.at<float>(o_y); x2_ = acts_.at<float>(o_x2);
         a2_ = prec_ == Precision::FP32 ? acts_.at<float>(o_a2) : nullptr;
         act_bytes_ = acts_.size();
@@ -534,24 +553,19 @@ private:
             if (prec_ == Precision::FP32) make_site(in_[i], GN, D, xn_, g.in_w, P_, GLD, SHVK_F32);
             make_site(oproj_[i], D, VD, on_, g.o_proj, h_, D, SHVK_F32);
             oproj_[i].args.R = h_; oproj_[i].args.ldr = D; oproj_[i].args.r_div = inv_div[i];
-            if (prec_ == Precision::FP32) {
-                make_site(up_[i], 2 * DFF, D, xn_, g.ffn_up, hid_, DFF, dt_);
-                up_[i].args.swiglu = 1;
-                make_site(down_[i], D, DFF, hid_, g.ffn_down, h_, D, SHVK_F32);
-                down_[i].args.R = h_; down_[i].args.ldr = D;
-            }
+            make_site(up_[i], 2 * DFF, D, xn_, g.ffn_up, hid_, DFF, dt_);
+            up_[i].args.swiglu = 1;
+            make_site(down_[i], D, DFF, hid_, g.ffn_down, h_, D, SHVK_F32);
+            down_[i].args.R = h_; down_[i].args.ldr = D;
+            up_[i].args.M = down_[i].args.M = int(hid_rows_);
         }
         make_site(sisa_in_, SN, D, xn_, s_w_all_, P_, SLD, SHVK_F32);
         sisa_in_.args.bias = s_b_all_;
-        for (Site* st : {&oproj_[0], &oproj_[1]}) {
+        for (Site* st : {&oproj_[0], &oproj_[1], &up_[0], &up_[1], &down_[0], &down_[1]}) {
             launch_ok(shvk_gemm_tc_plan(&st->args, dt_, st->plan), "tensor-core GEMM plan");
             st->planned = true;
         }
         if (prec_ == Precision::FP32) {
-            for (Site* st : {&up_[0], &up_[1], &down_[0], &down_[1]}) {
-                launch_ok(shvk_gemm_tc_plan(&st->args, dt_, st->plan), "tensor-core GEMM plan");
-                st->planned = true;
-            }
             launch_ok(shvk_gemm_tc_plan(&sisa_in_.args, dt_, sisa_in_.plan), "tensor-core GEMM plan");
         } else {
             // 16-bit modes: K | V | B of the SISA projection leave as fp16 rows (S16), theta | alpha | forget as fp32 rows
@@ -751,7 +765,7 @@ private:
                 launch_ok(shvk_rmsnorm(h_, D, next_norm, xn_out, xn_code, xn_ld, M, s), "rmsnorm");
                 mark("rmsnorm", s);
             }
-            if (prec_ == Precision::FP32) {
+            if (two_launch_ffn(M)) {
                 rows_gemm(up_[st], M, s);
                 mark("gemm.ffn_up", s);
                 rows_gemm(down_[st], M, s);

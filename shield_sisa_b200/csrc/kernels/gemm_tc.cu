@@ -457,6 +457,7 @@ struct HostPlan {
     void* C; long long ldc; int c_dtype;
     const float* R; long long ldr;
     void* C16; long long ldc16;     // EPI_SPLIT16: the fp16 output
+    const void* W; long long ldw;
     int epi, ab_dtype, valid;
 };
 static_assert(sizeof(HostPlan) <= 512, "plan must fit the caller's 512-byte buffer");
@@ -476,8 +477,34 @@ int choose_bn(int n) {
     return best;
 }
 
+int device_sms() {
+    int dev = 0, sms = 148;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    return sms;
+}
+
+// Accumulator width of one launch.  With tiles for every SM many times over it is the plan's: what counts is the time of a
+// row block.  While the plan's width gives no more than two tiles per SM, what counts is the longest chain of one SM: tiles
+// per SM times (k steps, and filling the ring and draining the last accumulator: about 600 + 8 bn cycles), and a narrower
+// tile spreads a short problem over more SMs.  o-projection (N 384, K 768), us per launch at the plan's width / this one: 1
+// window 25 / 17, 8 26 / 17, 32 34 / 29, from 64 on the same.
+// A column's sum does not depend on the width of its tile.  EPI_SPLIT16 needs multiples of 32.
+int launch_bn(const TcParams& p, int epi, int sms) {
+    if ((long long)p.m_tiles * p.n_tiles > 2ll * sms) return p.BN;
+    const int step = epi == EPI_SPLIT16 ? 32 : 16, nk = p.K / p.tile_k;
+    int best = p.BN;
+    long long best_cost = -1;
+    for (int bn = p.BN; bn >= 64; bn -= step) {
+        const long long tiles = (long long)p.m_tiles * ((p.N + bn - 1) / bn), waves = (tiles + sms - 1) / sms;
+        const long long cost = waves * (nk * (2 * bn > 128 + bn ? 2 * bn : 128 + bn) + 600 + 8 * bn);
+        if (best_cost < 0 || cost < best_cost) { best_cost = cost; best = bn; }
+    }
+    return best;
+}
+
 template <typename T, int EPI, typename SH> int launch_tc(const TcMaps& maps, const TcParams& p, cudaStream_t s) {
-    int dev = 0, sms = 0;
+    int dev = 0;
     cudaGetDevice(&dev);
     // one bit per device ordinal: the dynamic shared memory opt-in is per device.  Engines of several devices launch
     // from their own threads, hence the atomic; setting the attribute twice is harmless.
@@ -487,7 +514,7 @@ template <typename T, int EPI, typename SH> int launch_tc(const TcMaps& maps, co
         if (e != cudaSuccess) return int(e);
         if (dev < 64) attr_done.fetch_or(1ull << dev, std::memory_order_release);
     }
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    const int sms = device_sms();
     const long long total = (long long)p.m_tiles * p.n_tiles;
     const unsigned grid = unsigned(total < sms ? total : sms);
     TcParams q = p;
@@ -568,6 +595,7 @@ static int plan_impl(const shvk_gemm_args* g, int ab_dtype, void* host_plan, int
     hp->C = g->C; hp->ldc = g->ldc; hp->c_dtype = g->c_dtype;
     hp->R = g->R; hp->ldr = g->ldr;
     hp->C16 = C16; hp->ldc16 = ldc16;
+    hp->W = g->W; hp->ldw = g->ldw;
     p.split_n = split_col;
     if (split_col && (bn & 31)) return int(cudaErrorInvalidValue);      // a 32-column block must not straddle the split
     hp->epi = epi;
@@ -593,6 +621,13 @@ int launch_rows(const void* host_plan, int rows, void* stream, int starve, uint3
     maps.a = hp->map_a;
     maps.w = hp->map_w;
     bool ok;
+    const int bn = launch_bn(p, hp->epi, device_sms());
+    if (bn != p.BN) {
+        p.BN = bn;
+        p.n_tiles = (p.N + bn - 1) / bn;
+        p.idesc = (p.idesc & ~(0x3fu << 17)) | (uint32_t(bn >> 3) << 17);
+        if (!make_map(&maps.w, hp->W, p.tf32 ? 4 : 2, p.N, p.K, hp->ldw, bn, p.tile_k, true)) return int(cudaErrorNotSupported);
+    }
     if (hp->epi == EPI_SWIGLU) {
         const int cb = hp->c_dtype == DT_F32 ? 4 : 2;
         ok = make_map(&maps.c_full, hp->C, cb, rows, p.N / 2, hp->ldc, 32, 16, false) &&

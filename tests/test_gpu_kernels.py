@@ -198,6 +198,38 @@ def test_gemm_tc_rows_do_not_depend_on_the_batch(L):
     assert torch.equal(big[515], one[0])
 
 
+@pytest.mark.parametrize("rows", [1, 128, 129, 321, 1900, 5000, 9473])
+def test_gemm_tc_rows_do_not_depend_on_the_tile_width(L, rows):
+    """A launch of few rows takes narrower column tiles than its plan: the rows are bitwise those of a full launch, in every
+    epilogue, and nothing past them is written."""
+    import torch
+    rng = np.random.default_rng(19)
+    M, K = 128 * 300, 768                                 # 600 tiles of 192 columns: the plan's own width
+    a = dev(rng.standard_normal((M, K)).astype(np.float32), torch.bfloat16)
+    wo, wu = (dev((rng.standard_normal((n, K)) / 25).astype(np.float32), torch.bfloat16) for n in (384, 1920))
+    ws = dev((rng.standard_normal((1068, K)) / 25).astype(np.float32), torch.bfloat16)
+    bias = dev(rng.standard_normal(1068).astype(np.float32))
+    r0 = dev(rng.standard_normal((M, 384)).astype(np.float32))
+    outs = []
+    for m in (M, rows):
+        H, U = r0.clone(), torch.full((M, 960), 9.0, device="cuda", dtype=torch.bfloat16)
+        S16, SG = torch.full((M, 960), 9.0, device="cuda", dtype=torch.float16), torch.full((M, 112), 9.0, device="cuda")
+        plans = [tc_plan(L, gemm_args(M, 384, K, a, wo, H, 384, R=H, ldr=384), 1),
+                 tc_plan(L, gemm_args(M, 1920, K, a, wu, U, 960, c_dtype=1, swiglu=1), 1)]
+        buf = (C.c_char * 1024)()
+        split = (C.addressof(buf) + 63) & ~63
+        g = gemm_args(M, 1068, K, a, ws, SG, 112, bias=bias)
+        ok(L.shvk_gemm_tc_plan_split16(g, 1, 960, S16.data_ptr(), 960, split))
+        for p in (plans[0][1], plans[1][1], split):
+            ok(L.shvk_gemm_tc_rows(p, m, stream_ptr()))
+        sync()
+        assert tc_status(L) == 0
+        outs.append((H, U, S16, SG[:, :108]))            # the four padding columns are written or not
+    for full, part, rest in zip(outs[0], outs[1], (r0, None, None, None)):
+        assert torch.equal(part[:rows], full[:rows])
+        assert torch.equal(part[rows:], rest[rows:]) if rest is not None else (part[rows:] == 9.0).all()
+
+
 # ---------------------------------------------------------------------------------------------- fused feed-forward block
 @pytest.mark.parametrize("dtype", ["bf16", "fp16"])
 def test_ffn_fused_equals_the_two_gemm_path(L, dtype):
