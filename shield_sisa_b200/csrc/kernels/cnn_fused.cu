@@ -411,9 +411,6 @@ stem_block_kernel(const uint8_t* __restrict__ frames, const float* __restrict__ 
 // layer (a warp per unit, lanes over the channels, a weight row read once for all G frames), hands it to the other seven
 // through distributed shared memory, and computes an eighth of the gates.  One block per frame read all 1.8 MB of the
 // widest layer's weights through one SM: 52 us however few the frames, 210 us at 640.
-__device__ __forceinline__ void cluster_sync() {
-    asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
 template <int G>
 __global__ void __cluster_dims__(8, 1, 1) __launch_bounds__(256)
 se_gate_cluster_kernel(const float* __restrict__ sums, const float* __restrict__ w1, const float* __restrict__ b1,

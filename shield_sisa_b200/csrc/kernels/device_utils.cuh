@@ -36,6 +36,12 @@ __device__ __forceinline__ float warp_max(float v) {
     return v;
 }
 
+// Barrier over the blocks of a cluster; shared-memory writes before it, remote ones included, are visible behind it.
+__device__ __forceinline__ void cluster_sync() {
+    __syncwarp();                                            // the aligned forms want whole warps
+    asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+
 // Four consecutive outputs in storage type T (16, 8 or 8 bytes, address aligned accordingly).
 template <typename T> __device__ __forceinline__ void store_quad(T* p, float a, float b, float c, float d);
 template <> __device__ __forceinline__ void store_quad<float>(float* p, float a, float b, float c, float d) {

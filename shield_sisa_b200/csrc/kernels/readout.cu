@@ -7,7 +7,7 @@
 //
 // Only row 320 leaves the SISA block, so this work is B rows, not 321 B (engine/cuda/engine.cu:451-469;
 // engine/model/isa_impl.hpp:1092-1133).  A CTA takes TB clips (16 when the batch is large enough to give every SM a
-// CTA that way, else 4, 2 or 1) and walks the small matrix products one after the other with all activations of its
+// CTA that way, else 4, 2 or 1; up to about 120 clips eight CTAs share a batch's clips, see below) and walks the small matrix products one after the other with all activations of its
 // clips in shared memory: a thread owns one or two output columns for all TB clips (TB or 2 TB accumulators), reads its
 // weights coalesced from a [K][N] (transposed) copy that stays in L2, several steps of k in flight at a time, and the
 // activations as 128-bit broadcast loads.  Every output is one fp32 FMA chain over k in ascending order, whatever the
@@ -17,8 +17,6 @@
 // (engine/cuda/engine.cu:451-469, engine/cuda/seq.cu:309-336).
 #include "device_utils.cuh"
 #include "shv_seq_kernels.h"
-
-#include <stdlib.h>
 
 namespace sb {
 namespace {
@@ -195,41 +193,272 @@ readout_tail_kernel(const float* __restrict__ Y, const float* __restrict__ h_las
     }
 }
 
+// ---------------------------------------------------------------------------------------------------- small batches
+// The two kernels above keep a clip's whole row on one SM, which then reads all 5.2 MB (0.9 MB) of the matrices, and with one
+// clip per SM waits for most of those loads: 81 us (23 us) whether the batch has 45 clips or 128.  Here eight SMs share TB
+// clips: each takes an eighth of the columns of every product for all of them.  Its slices of the matrices stream through
+// a ring of shared-memory chunks (cp.async, up to three chunks of 23 to 30 KB ahead, across the products: nothing of them
+// depends on the data), and the eight hand each other their outputs through distributed shared memory, a buffer per
+// hand-over, so that a cluster barrier between products is all they need.  An output is the same FMA chain over k.
+constexpr int CL = 8, NTC = 256, RING = 4, CHUNK_BYTES = 30720;
+constexpr int WO_C = kD / CL, UP_C = 2 * kDFF / CL, HEAD_C = 128 / CL, QC_C = kSQN / CL;         // columns of one SM: 48, 240, 16, 72
+constexpr int WO_K = 128, UP_K = 32, DN_K = 120, HEAD_K = kD, QC_K = 96;                           // k rows of a chunk
+constexpr int G_UP = kD / WO_K, G_DN = G_UP + kD / UP_K, G_HEAD = G_DN + kDFF / DN_K, G_END = G_HEAD + 1;   // first chunk of a product
+static_assert(WO_K * WO_C * 4 <= CHUNK_BYTES && UP_K * UP_C * 4 <= CHUNK_BYTES && DN_K * WO_C * 4 <= CHUNK_BYTES &&
+              HEAD_K * HEAD_C * 4 <= CHUNK_BYTES && QC_K * QC_C * 4 <= CHUNK_BYTES, "chunks");
+static_assert(kD % WO_K == 0 && kD % UP_K == 0 && kDFF % DN_K == 0 && kD % QC_K == 0, "chunks");
+
+__device__ __forceinline__ uint32_t smem_of(const void* p) { return uint32_t(__cvta_generic_to_shared(p)); }
+__device__ __forceinline__ void cp16(uint32_t dst, const float* src) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
+}
+__device__ __forceinline__ void cp_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int N> __device__ __forceinline__ void cp_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
+// a float (pair) into the same place of every block of the cluster
+__device__ __forceinline__ uint32_t peer_of(uint32_t local, int rank) {
+    uint32_t remote;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote) : "r"(local), "r"(rank));
+    return remote;
+}
+__device__ __forceinline__ void share2(float* p, float a, float b) {
+#pragma unroll
+    for (int r = 0; r < CL; ++r)
+        asm volatile("st.shared::cluster.v2.f32 [%0], {%1, %2};" ::"r"(peer_of(smem_of(p), r)), "f"(a), "f"(b) : "memory");
+}
+__device__ __forceinline__ void share1(float* p, float a) {
+#pragma unroll
+    for (int r = 0; r < CL; ++r) asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(peer_of(smem_of(p), r)), "f"(a) : "memory");
+}
+
+// rows [KC][COLS] of a [K][ldw] matrix into a chunk
+template <int COLS, int KC> __device__ __forceinline__ void fetch_chunk(uint32_t dst, const float* src, int ldw, int tid) {
+    constexpr int V = COLS / 4;
+    for (int i = tid; i < KC * V; i += NTC) cp16(dst + uint32_t(i) * 16u, src + (long long)(i / V) * ldw + i % V * 4);
+}
+// One product's share of a thread: TPC clips of a column pair.  A block's pairs are dealt to the threads first, the clips to
+// as many groups of threads as there are.
+template <int COLS, int TB> struct Share {
+    static constexpr int PAIRS = COLS / 2, MAXG = NTC / PAIRS, GROUPS = TB <= 4 && TB < MAXG ? TB : MAXG >= 4 ? 4 : MAXG >= 2 ? 2 : 1;
+    static constexpr int TPC = TB / GROUPS;
+    static_assert(TB % GROUPS == 0 && PAIRS * GROUPS <= NTC, "clips per thread");
+    int pair, clip;
+    bool active;
+    __device__ explicit Share(int tid) : pair(tid % PAIRS), clip(tid / PAIRS * TPC), active(tid < PAIRS * GROUPS) {}
+};
+// acc[c][e] += sum over a chunk's k of X[c][k] W[k][pair]; k ascending
+template <int COLS, int KC, int TPC>
+__device__ __forceinline__ void chunk_product(const float* w, const float* x, int xp, float (&acc)[TPC][2]) {
+#pragma unroll 4
+    for (int k = 0; k < KC; k += 4) {
+        float2 v[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) v[i] = *reinterpret_cast<const float2*>(w + (k + i) * COLS);
+#pragma unroll
+        for (int c = 0; c < TPC; ++c) {
+            const float4 q = *reinterpret_cast<const float4*>(x + c * xp + k);
+            acc[c][0] = fmaf(q.x, v[0].x, acc[c][0]); acc[c][1] = fmaf(q.x, v[0].y, acc[c][1]);
+            acc[c][0] = fmaf(q.y, v[1].x, acc[c][0]); acc[c][1] = fmaf(q.y, v[1].y, acc[c][1]);
+            acc[c][0] = fmaf(q.z, v[2].x, acc[c][0]); acc[c][1] = fmaf(q.z, v[2].y, acc[c][1]);
+            acc[c][0] = fmaf(q.w, v[3].x, acc[c][0]); acc[c][1] = fmaf(q.w, v[3].y, acc[c][1]);
+        }
+    }
+}
+template <int K, int COLS, int KC, int TB, typename Fetch>
+__device__ __forceinline__ void stream_product(const Share<COLS, TB>& sh, int g0, const Fetch& fetch, const float* ring, const float* x, int xp,
+                                               float (&acc)[Share<COLS, TB>::TPC][2]) {
+    constexpr int TPC = Share<COLS, TB>::TPC;
+#pragma unroll
+    for (int c = 0; c < TPC; ++c) { acc[c][0] = 0.0f; acc[c][1] = 0.0f; }
+    for (int c = 0; c < K / KC; ++c) {
+        const int g = g0 + c;
+        cp_wait<RING - 2>();                              // this thread's part of chunk g has landed
+        __syncthreads();                                  // everyone's has, and chunk g - 1 is consumed
+        fetch(g + RING - 1);
+        if (sh.active) chunk_product<COLS, KC, TPC>(ring + (g % RING) * (CHUNK_BYTES / 4) + 2 * sh.pair, x + sh.clip * xp + c * KC, xp, acc);
+    }
+}
+
+template <int TB>
+__global__ void __launch_bounds__(NTC, 1)
+readout_qc_split_kernel(const float* __restrict__ h_last, long long ldh, const float* __restrict__ norm_w, const float* __restrict__ wqc_t,
+                        float* __restrict__ QC, int B) {
+    extern __shared__ __align__(16) float split_smem[];
+    float* ring = split_smem;
+    float* xs = ring + RING * CHUNK_BYTES / 4;                // [TB][XP]
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, rank = blockIdx.x % CL;
+    const int clip0 = int(blockIdx.x / CL) * TB;
+    auto fetch = [&](int g) {
+        if (g < kD / QC_K)
+            fetch_chunk<QC_C, QC_K>(smem_of(ring) + uint32_t(g % RING) * CHUNK_BYTES, wqc_t + (long long)g * QC_K * kSQN + rank * QC_C, kSQN, tid);
+        cp_commit();
+    };
+    for (int g = 0; g < RING - 1; ++g) fetch(g);
+    for (int i = tid; i < TB * kD; i += NTC) {
+        const int c = i / kD, k = i - c * kD;
+        xs[c * XP + k] = clip0 + c < B ? h_last[(long long)(clip0 + c) * ldh + k] : 0.0f;
+    }
+    __syncthreads();
+    norm_rows<TB, NTC>(xs, xs, norm_w, warp, lane);
+    const Share<QC_C, TB> sh(tid);
+    float acc[Share<QC_C, TB>::TPC][2];
+    stream_product<kD, QC_C, QC_K, TB>(sh, 0, fetch, ring, xs, XP, acc);
+    if (sh.active)
+#pragma unroll
+        for (int c = 0; c < Share<QC_C, TB>::TPC; ++c)
+            if (clip0 + sh.clip + c < B)
+                *reinterpret_cast<float2*>(QC + (long long)(clip0 + sh.clip + c) * kSQN + rank * QC_C + 2 * sh.pair) = make_float2(acc[c][0], acc[c][1]);
+}
+
+template <int TB>
+__global__ void __cluster_dims__(CL, 1, 1) __launch_bounds__(NTC, 1)
+readout_tail_split_kernel(const float* __restrict__ Y, const float* __restrict__ h_last, long long ldh, const TailWeights tw,
+                          float* __restrict__ x2_out, float* __restrict__ logits, int B) {
+    extern __shared__ __align__(16) float split_smem[];
+    float* ring = split_smem;
+    float* ya = ring + RING * CHUNK_BYTES / 4;                // [TB][XP]  attention output
+    float* xb = ya + TB * XP;                                 // [TB][XP]  x1, then normalised
+    float* xc = xb + TB * XP;                                 // [TB][XP]  x2, then normalised
+    float* hid = xc + TB * XP;                                // [TB][HP]  SwiGLU product
+    float* hh = hid + TB * HP;                                // [TB][128] head's hidden layer (block 0 of the cluster)
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, rank = blockIdx.x % CL;
+    const int clip0 = int(blockIdx.x / CL) * TB;
+    auto fetch = [&](int g) {
+        const uint32_t dst = smem_of(ring) + uint32_t(g % RING) * CHUNK_BYTES;
+        if (g < G_UP) fetch_chunk<WO_C, WO_K>(dst, tw.wo_t + (long long)g * WO_K * kD + rank * WO_C, kD, tid);
+        else if (g < G_DN) fetch_chunk<UP_C, UP_K>(dst, tw.up_t + (long long)(g - G_UP) * UP_K * (2 * kDFF) + rank * UP_C, 2 * kDFF, tid);
+        else if (g < G_HEAD) fetch_chunk<WO_C, DN_K>(dst, tw.down_t + (long long)(g - G_DN) * DN_K * kD + rank * WO_C, kD, tid);
+        else if (g < G_END) fetch_chunk<HEAD_C, HEAD_K>(dst, tw.head_w0_t + rank * HEAD_C, 128, tid);
+        cp_commit();
+    };
+    for (int g = 0; g < RING - 1; ++g) fetch(g);
+    for (int i = tid; i < TB * kD; i += NTC) {
+        const int c = i / kD, k = i - c * kD;
+        ya[c * XP + k] = clip0 + c < B ? Y[(long long)(clip0 + c) * kD + k] : 0.0f;
+    }
+    const Share<WO_C, TB> so(tid);
+    float x1[Share<WO_C, TB>::TPC][2], acc[Share<WO_C, TB>::TPC][2];   // this thread's columns of the residual row
+#pragma unroll
+    for (int c = 0; c < Share<WO_C, TB>::TPC; ++c) {
+        const int clip = clip0 + so.clip + c;
+        const float2 r = so.active && clip < B ? *reinterpret_cast<const float2*>(h_last + (long long)clip * ldh + rank * WO_C + 2 * so.pair)
+                                               : make_float2(0.0f, 0.0f);
+        x1[c][0] = r.x; x1[c][1] = r.y;
+    }
+    cluster_sync();                                           // every block of the cluster runs: its shared memory may be written
+    // x1 = h + Y . W_O^T
+    stream_product<kD, WO_C, WO_K, TB>(so, 0, fetch, ring, ya, XP, acc);
+    if (so.active)
+#pragma unroll
+        for (int c = 0; c < Share<WO_C, TB>::TPC; ++c) {
+            x1[c][0] += acc[c][0]; x1[c][1] += acc[c][1];
+            share2(xb + (so.clip + c) * XP + rank * WO_C + 2 * so.pair, x1[c][0], x1[c][1]);
+        }
+    cluster_sync();
+    norm_rows<TB, NTC>(xb, xb, tw.ffn_norm_w, warp, lane);
+    // hid[j] = silu(gate_j) * up_j  (the product's first barrier orders it behind the norm)
+    {
+        const Share<UP_C, TB> su(tid);
+        float u[Share<UP_C, TB>::TPC][2];
+        stream_product<kD, UP_C, UP_K, TB>(su, G_UP, fetch, ring, xb, XP, u);
+        if (su.active)
+#pragma unroll
+            for (int c = 0; c < Share<UP_C, TB>::TPC; ++c) share1(hid + (su.clip + c) * HP + rank * (UP_C / 2) + su.pair, silu_f(u[c][0]) * u[c][1]);
+    }
+    cluster_sync();
+    // x2 = x1 + hid . W_down^T
+    stream_product<kDFF, WO_C, DN_K, TB>(so, G_DN, fetch, ring, hid, HP, acc);
+    if (so.active)
+#pragma unroll
+        for (int c = 0; c < Share<WO_C, TB>::TPC; ++c) {
+            const float a = x1[c][0] + acc[c][0], b = x1[c][1] + acc[c][1];
+            share2(xc + (so.clip + c) * XP + rank * WO_C + 2 * so.pair, a, b);
+            const int clip = clip0 + so.clip + c;
+            if (x2_out && clip < B) *reinterpret_cast<float2*>(x2_out + (long long)clip * kD + rank * WO_C + 2 * so.pair) = make_float2(a, b);
+        }
+    cluster_sync();
+    norm_rows<TB, NTC>(xc, xc, tw.final_norm_w, warp, lane);
+    // head: 128 hidden units, then their weighted sum per clip on the cluster's first block
+    {
+        const Share<HEAD_C, TB> sh(tid);
+        float u[Share<HEAD_C, TB>::TPC][2];
+        stream_product<kD, HEAD_C, HEAD_K, TB>(sh, G_HEAD, fetch, ring, xc, XP, u);
+        const int o = rank * HEAD_C + 2 * sh.pair;
+        if (sh.active)
+#pragma unroll
+            for (int c = 0; c < Share<HEAD_C, TB>::TPC; ++c) {
+                const float a = __ldg(tw.head_w2 + o) * silu_f(u[c][0] + __ldg(tw.head_b0 + o));
+                const float b = __ldg(tw.head_w2 + o + 1) * silu_f(u[c][1] + __ldg(tw.head_b0 + o + 1));
+                asm volatile("st.shared::cluster.v2.f32 [%0], {%1, %2};"
+                             ::"r"(peer_of(smem_of(hh + (sh.clip + c) * 128 + o), 0)), "f"(a), "f"(b) : "memory");
+            }
+    }
+    cluster_sync();
+    if (rank == 0)
+        for (int c = warp; c < TB; c += NTC / 32) {
+            const float s = warp_sum((hh[c * 128 + lane] + hh[c * 128 + lane + 32]) + (hh[c * 128 + lane + 64] + hh[c * 128 + lane + 96]));
+            if (lane == 0 && clip0 + c < B) logits[clip0 + c] = s + __ldg(tw.head_b2);
+        }
+}
+constexpr int qc_split_smem(int tb) { return RING * CHUNK_BYTES + tb * XP * 4; }
+constexpr int tail_split_smem(int tb) { return RING * CHUNK_BYTES + tb * (3 * XP + HP + 128) * 4; }
+static_assert(tail_split_smem(8) <= 232448, "shared memory");
+
 constexpr int tail_smem_bytes(int tb) { return (2 * tb * XP + tb * HP) * int(sizeof(float)); }
 
-// Clips and threads per CTA for a batch of B: 16 clips once that still gives every SM a CTA, else 4, 2 (the few hundred
-// clips of a pipeline batch: at B = 512 two clips per CTA 0.087 ms for the tail kernel, one 0.144, four 0.108; two or four
-// clips with 512 threads 0.121 / 0.089, four with 1024 0.122), else 1.  The arithmetic of an output does not depend on
-// the choice (one FMA chain over k ascending in every form).
-struct ReadoutShape { int tb, nt; };
+// How the clips of a batch of B are dealt out: `tb` to a cluster of eight blocks (split) or to one block.  As long as one
+// wave of clusters holds the batch (about 15 of them on a B200: 120 clips) it is split, with as few clips to a cluster as that
+// allows; tail kernel in us, split / one block: 1 clip 28 / 43, 45 clips 36 / 82, 96 clips 43 / 82, but 128 clips (two
+// waves) 83 / 81.  Above, a block takes 16 clips once that still gives every SM one, else 4, 2 (the few hundred clips of a
+// pipeline batch: at 512 two clips per block 87 us, one 144, four 108) or 1.
+struct ReadoutShape { int tb; bool split; };
 ReadoutShape readout_shape(int B) {
-    int dev = 0, sms = 148;
+    int dev = 0, sms = 148, clusters = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    ReadoutShape r = B >= 16 * sms ? ReadoutShape{16, 256} : B >= 4 * sms ? ReadoutShape{4, 256} : B >= 2 * sms ? ReadoutShape{2, 256} : ReadoutShape{1, 256};
-#ifdef SHVK_DEV_PROBES
-    if (const char* e = getenv("SHVK_READOUT_TB")) { r.tb = atoi(e); r.nt = 256; }
-    if (const char* e = getenv("SHVK_READOUT_NT")) r.nt = atoi(e);
-#endif
-    return r;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(unsigned(sms / CL) * CL);
+    cfg.blockDim = dim3(NTC);
+    cfg.dynamicSmemBytes = tail_split_smem(8);
+    if (cudaFuncSetAttribute(readout_tail_split_kernel<8>, cudaFuncAttributeMaxDynamicSharedMemorySize, tail_split_smem(8)) != cudaSuccess ||
+        cudaOccupancyMaxActiveClusters(&clusters, readout_tail_split_kernel<8>, &cfg) != cudaSuccess) {
+        cudaGetLastError();
+        clusters = 0;
+    }
+    for (int tb = 1; tb <= 8; tb *= 2)
+        if ((B + tb - 1) / tb <= clusters) return {tb, true};
+    return {B >= 16 * sms ? 16 : B >= 4 * sms ? 4 : B >= 2 * sms ? 2 : 1, false};
 }
 
-template <int TB, int NT>
+template <int TB, bool SPLIT>
 int launch_qc(const float* h_last, long long ldh, const float* norm_w, const float* wqc_t, float* QC, int B, cudaStream_t s) {
-    readout_qc_kernel<TB, NT><<<unsigned((B + TB - 1) / TB), NT, 0, s>>>(h_last, ldh, norm_w, wqc_t, QC, B);
+    const unsigned groups = unsigned((B + TB - 1) / TB);
+    if constexpr (SPLIT) {
+        const cudaError_t e = cudaFuncSetAttribute(readout_qc_split_kernel<TB>, cudaFuncAttributeMaxDynamicSharedMemorySize, qc_split_smem(TB));
+        if (e != cudaSuccess) return int(e);
+        readout_qc_split_kernel<TB><<<groups * CL, NTC, qc_split_smem(TB), s>>>(h_last, ldh, norm_w, wqc_t, QC, B);
+    } else {
+        readout_qc_kernel<TB, 256><<<groups, 256, 0, s>>>(h_last, ldh, norm_w, wqc_t, QC, B);
+    }
     return int(cudaGetLastError());
 }
-template <int TB, int NT>
+template <int TB, bool SPLIT>
 int launch_tail(const float* Y, const float* h_last, long long ldh, const TailWeights& tw, float* x2_out, float* logits, int B,
                 cudaStream_t s) {
-    const cudaError_t e = cudaFuncSetAttribute(readout_tail_kernel<TB, NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, tail_smem_bytes(TB));
-    if (e != cudaSuccess) return int(e);
-    readout_tail_kernel<TB, NT><<<unsigned((B + TB - 1) / TB), NT, tail_smem_bytes(TB), s>>>(Y, h_last, ldh, tw, x2_out, logits, B);
+    const unsigned groups = unsigned((B + TB - 1) / TB);
+    if constexpr (SPLIT) {
+        const cudaError_t e = cudaFuncSetAttribute(readout_tail_split_kernel<TB>, cudaFuncAttributeMaxDynamicSharedMemorySize, tail_split_smem(TB));
+        if (e != cudaSuccess) return int(e);
+        readout_tail_split_kernel<TB><<<groups * CL, NTC, tail_split_smem(TB), s>>>(Y, h_last, ldh, tw, x2_out, logits, B);
+    } else {
+        const cudaError_t e = cudaFuncSetAttribute(readout_tail_kernel<TB, 256>, cudaFuncAttributeMaxDynamicSharedMemorySize, tail_smem_bytes(TB));
+        if (e != cudaSuccess) return int(e);
+        readout_tail_kernel<TB, 256><<<groups, 256, tail_smem_bytes(TB), s>>>(Y, h_last, ldh, tw, x2_out, logits, B);
+    }
     return int(cudaGetLastError());
 }
 
-// the shapes that are compiled: clips per CTA * 10000 + threads
-#define SHVK_READOUT_SHAPES(X) X(16, 256) X(8, 256) X(4, 256) X(2, 256) X(1, 256)
+// the shapes that are compiled
+#define SHVK_READOUT_SHAPES(X) X(16, false) X(4, false) X(2, false) X(1, false) X(8, true) X(4, true) X(2, true) X(1, true)
 
 }  // namespace
 }  // namespace sb
@@ -240,8 +469,8 @@ extern "C" int shvk_readout_qc(const float* h_last, long long ldh, const float* 
     if (!h_last || !norm_w || !wqc_t || !QC) return int(cudaErrorInvalidValue);
     cudaStream_t s = cudaStream_t(stream);
     const sb::ReadoutShape sh = sb::readout_shape(B);
-    switch (sh.tb * 10000 + sh.nt) {
-#define X(TB, NT) case TB * 10000 + NT: return sb::launch_qc<TB, NT>(h_last, ldh, norm_w, wqc_t, QC, B, s);
+    switch (2 * sh.tb + sh.split) {
+#define X(TB, SPLIT) case 2 * TB + SPLIT: return sb::launch_qc<TB, SPLIT>(h_last, ldh, norm_w, wqc_t, QC, B, s);
         SHVK_READOUT_SHAPES(X)
 #undef X
         default: return int(cudaErrorInvalidValue);
@@ -255,8 +484,8 @@ extern "C" int shvk_readout_tail(const float* Y, const float* h_last, long long 
     const sb::TailWeights tw{w->wo_t, w->ffn_norm_w, w->up_t, w->down_t, w->final_norm_w, w->head_w0_t, w->head_b0, w->head_w2, w->head_b2};
     cudaStream_t s = cudaStream_t(stream);
     const sb::ReadoutShape sh = sb::readout_shape(B);
-    switch (sh.tb * 10000 + sh.nt) {
-#define X(TB, NT) case TB * 10000 + NT: return sb::launch_tail<TB, NT>(Y, h_last, ldh, tw, x2_out, logits, B, s);
+    switch (2 * sh.tb + sh.split) {
+#define X(TB, SPLIT) case 2 * TB + SPLIT: return sb::launch_tail<TB, SPLIT>(Y, h_last, ldh, tw, x2_out, logits, B, s);
         SHVK_READOUT_SHAPES(X)
 #undef X
         default: return int(cudaErrorInvalidValue);

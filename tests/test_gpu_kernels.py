@@ -906,6 +906,30 @@ def test_readout_row_kernels_match_oracle(L, weight_files):
     assert np.abs(outs[Bbig][0] - ref).max() < 2e-5
 
 
+@pytest.mark.parametrize("n", [1, 2, 14, 15, 27, 29, 45, 57, 96, 112, 113, 121])
+def test_readout_row_split_over_eight_blocks(L, n):
+    """Batches up to about 120 clips share eight blocks among 1, 2, 4 or 8 clips: bitwise the one-block form of larger
+    batches, and nothing is written past the batch."""
+    import torch
+    rng = np.random.default_rng(8)
+    shapes = {"wo_t": (384, 384), "ffn_norm_w": 384, "up_t": (384, 1920), "down_t": (960, 384), "final_norm_w": 384,
+              "head_w0_t": (384, 128), "head_b0": 128, "head_w2": 128, "head_b2": 1}
+    keep = {k: dev((rng.standard_normal(v) / 20).astype(np.float32)) for k, v in shapes.items()}
+    rw = binding.ReadoutWeights(**{k: v.data_ptr() for k, v in keep.items()})
+    nw, wqc = dev(rng.standard_normal(384).astype(np.float32)), dev((rng.standard_normal((384, 576)) / 20).astype(np.float32))
+    big = 1025
+    H, Y = dev(rng.standard_normal((big, 384)).astype(np.float32)), dev(rng.standard_normal((big, 384)).astype(np.float32))
+    outs = []
+    for b in (big, n):
+        lg, x2, q = (torch.full(sh, 9.0, device="cuda") for sh in ((big,), (big, 384), (big, 576)))
+        ok(L.shvk_readout_qc(H.data_ptr(), 384, nw.data_ptr(), wqc.data_ptr(), q.data_ptr(), b, stream_ptr()))
+        ok(L.shvk_readout_tail(Y.data_ptr(), H.data_ptr(), 384, C.byref(rw), x2.data_ptr(), lg.data_ptr(), b, stream_ptr()))
+        sync()
+        outs.append((lg, x2, q))
+    for whole, part in zip(*outs):
+        assert torch.equal(part[:n], whole[:n]) and (part[n:] == 9.0).all()
+
+
 def test_store_tokens(L):
     import torch
     blocks = torch.arange(4 * 6144, device="cuda", dtype=torch.float32).reshape(4, 6144)
