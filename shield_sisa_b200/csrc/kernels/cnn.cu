@@ -213,92 +213,111 @@ se_gate_kernel(const float* __restrict__ partial, const float* __restrict__ w1, 
 }
 
 // ---------------------------------------------------------------------------------------------------- 1x1 convolution
-// Row GEMM on CUDA cores, 256 threads, k in slabs of 8, next slab fetched into registers while the current one is
-// consumed.  One fma chain over k per output, so a pixel's result does not depend on the tile shape's row count.
+// Row GEMM on CUDA cores, k in slabs, next slab fetched into registers while the current one is consumed; two output
+// channels to a packed FMA (fma.rn.f32x2: the same roundings, half the issue slots, of which the loads from shared memory
+// and the copies need the rest: 18,000 pixels, 112 -> 672 channels 97 -> 91 us, of the 37 the FMAs take).  The gate
+// multiplies on the way into shared memory, so that no load is waited for while the previous slab is summed (480 -> 112
+// channels 78 -> 63 us).  One fma chain over k per output, so a pixel's result does not depend on the tile shape's row count.
 // Tile shapes (pixels x output channels, per-thread outputs): 256 x 16 and 128 x 32 and 64 x 64 with 4 x 4 for the narrow
-// layers (every thread has live columns), 128 x 128 with 8 x 8 for the wide ones (half the shared-memory reads per fma).
-constexpr int PW_K = 8;
-template <int BM, int BN, int TM, int TN>
-__global__ void __launch_bounds__(256)
+// layers (every thread has live columns), 128 x 128 with 8 x 8 for the wide ones (half the shared-memory reads per fma), a
+// whole row of 24 to 80 channels with 8 x 4; rules and slab depths (deep ones where K is long: a slab of a small tile is
+// summed faster than the next one arrives) at the launch.
+constexpr int PW_K = 8;                          // K is a multiple of this; slabs are KS deep, the last one may be shorter
+__host__ __device__ constexpr int pw_threads(int bm, int bn, int tm, int tn) { return bm / tm * (bn / tn); }
+template <int BM, int BN, int TM, int TN, int KS, bool GATE, bool PACK>
+__global__ void __launch_bounds__(pw_threads(BM, BN, TM, TN), TM * TN == 64 && KS == PW_K ? 2 : 0)
 pointwise_kernel(const float* __restrict__ A, const float* __restrict__ W, const float* __restrict__ bias,
                  const float* __restrict__ gate, int gate_rows, const float* R, float* out, int M, int N, int K, int act, int col_tiles) {
-    static_assert((BM / TM) * (BN / TN) == 256, "256 threads");
-    constexpr int NX = BN / TN, PA = BM + 4, PB = BN + 4, SLOTS = (BM + BN) * 2, PER = (SLOTS + 255) / 256;
-    __shared__ __align__(16) float sa[2][PW_K][PA];
-    __shared__ __align__(16) float sw[2][PW_K][PB];
+    constexpr int NT = pw_threads(BM, BN, TM, TN);
+    static_assert(NT % 32 == 0 && KS % PW_K == 0 && TM % 4 == 0 && TN % 4 == 0, "whole warps, 128-bit reads");
+    constexpr int NX = BN / TN, PA = BM + 4, PB = BN + 4, ROWS = BM + BN, SLOTS = ROWS * (KS / 4), PER = (SLOTS + NT - 1) / NT;
+    __shared__ __align__(16) float sa[2][KS][PA];
+    __shared__ __align__(16) float sw[2][KS][PB];
     const int tid = threadIdx.x, tx = tid % NX, ty = tid / NX;
     const long long m0 = (long long)(blockIdx.x / col_tiles) * BM;   // column tiles of a row tile are neighbours
     const int n0 = int(blockIdx.x % col_tiles) * BN;
-    // loader slots: slot i covers row i / 2 (A rows first, then W rows), k quad i % 2
+    // loader slots: slot i covers row (i / 2) % ROWS (A rows first, then W rows), k quad i % 2 of the i / (2 ROWS)-th eight
+    auto slot_row = [&](int r) { return ((tid + r * NT) >> 1) % ROWS; };
+    auto slot_k = [&](int r) { return ((tid + r * NT) >> 1) / ROWS * 8 + (tid & 1) * 4; };
     const float* src[PER];
-    const float* gsrc[PER];
-    float4 reg[PER];
+    const float* gsrc[GATE ? PER : 1];
+    float4 reg[PER], greg[GATE ? PER : 1];
 #pragma unroll
     for (int r = 0; r < PER; ++r) {
-        const int i = tid + r * 256, row = i >> 1;
+        const int row = slot_row(r);
         src[r] = nullptr;
-        gsrc[r] = nullptr;
-        if (i < SLOTS) {
+        if (GATE) gsrc[r] = nullptr;
+        if (tid + r * NT < SLOTS) {
             if (row < BM) {
                 const long long m = m0 + row;
                 if (m < M) {
-                    src[r] = A + m * K + (i & 1) * 4;
-                    if (gate) gsrc[r] = gate + (m / gate_rows) * K + (i & 1) * 4;
+                    src[r] = A + m * K + slot_k(r);
+                    if (GATE) gsrc[r] = gate + (m / gate_rows) * K + slot_k(r);
                 }
             } else if (n0 + row - BM < N) {
-                src[r] = W + (long long)(n0 + row - BM) * K + (i & 1) * 4;
+                src[r] = W + (long long)(n0 + row - BM) * K + slot_k(r);
             }
         }
     }
+    // the loads of the next slab stay untouched until it is stored (the gate is applied there): they fly during this slab's sums
     auto fetch = [&](int k0) {
 #pragma unroll
         for (int r = 0; r < PER; ++r) {
-            reg[r] = src[r] ? *reinterpret_cast<const float4*>(src[r] + k0) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-            if (gsrc[r]) {
-                const float4 g = *reinterpret_cast<const float4*>(gsrc[r] + k0);
-                reg[r].x *= g.x; reg[r].y *= g.y; reg[r].z *= g.z; reg[r].w *= g.w;
-            }
+            const bool in = src[r] && (KS == PW_K || k0 + slot_k(r) < K);
+            reg[r] = in ? *reinterpret_cast<const float4*>(src[r] + k0) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+            if constexpr (GATE)
+                greg[r] = in && gsrc[r] ? *reinterpret_cast<const float4*>(gsrc[r] + k0) : make_float4(1.0f, 1.0f, 1.0f, 1.0f);
         }
     };
     auto stash = [&](int buf) {
 #pragma unroll
         for (int r = 0; r < PER; ++r) {
-            const int i = tid + r * 256, row = i >> 1, kq = (i & 1) * 4;
-            if (i >= SLOTS) continue;
+            const int row = slot_row(r), kq = slot_k(r);
+            if (tid + r * NT >= SLOTS) continue;
+            float4 v = reg[r];
+            if constexpr (GATE) { v.x *= greg[r].x; v.y *= greg[r].y; v.z *= greg[r].z; v.w *= greg[r].w; }
             float* dst = row < BM ? &sa[buf][kq][row] : &sw[buf][kq][row - BM];
             const int pitch = row < BM ? PA : PB;
-            dst[0] = reg[r].x; dst[pitch] = reg[r].y; dst[2 * pitch] = reg[r].z; dst[3 * pitch] = reg[r].w;
+            dst[0] = v.x; dst[pitch] = v.y; dst[2 * pitch] = v.z; dst[3 * pitch] = v.w;
         }
     };
-    float acc[TM][TN];
+    float2 acc[TM][TN / 2];                      // pairs of adjacent output channels
 #pragma unroll
     for (int i = 0; i < TM; ++i)
 #pragma unroll
-        for (int j = 0; j < TN; ++j) acc[i][j] = 0.0f;
-    const int nk = K / PW_K;
+        for (int j = 0; j < TN / 2; ++j) acc[i][j] = make_float2(0.0f, 0.0f);
+    const int nk = (K + KS - 1) / KS;
     fetch(0);
     stash(0);
     __syncthreads();
     for (int kb = 0; kb < nk; ++kb) {
         const int buf = kb & 1;
-        if (kb + 1 < nk) fetch((kb + 1) * PW_K);
+        if (kb + 1 < nk) fetch((kb + 1) * KS);
 #pragma unroll
-        for (int k = 0; k < PW_K; ++k) {
-            float av[TM], wv[TN];
+        for (int ke = 0; ke < KS; ke += PW_K) {
+            if (KS != PW_K && kb * KS + ke >= K) break;
 #pragma unroll
-            for (int h = 0; h < TM / 4; ++h) {       // row groups of four, BM / 2 apart when there are two
-                const float4 a = *reinterpret_cast<const float4*>(&sa[buf][k][h * (BM / 2) + ty * 4]);
-                av[4 * h] = a.x; av[4 * h + 1] = a.y; av[4 * h + 2] = a.z; av[4 * h + 3] = a.w;
+            for (int k = ke; k < ke + PW_K; ++k) {
+                float av[TM];
+                float2 wv[TN / 2];
+#pragma unroll
+                for (int h = 0; h < TM / 4; ++h) {       // row groups of four, BM / 2 apart when there are two
+                    const float4 a = *reinterpret_cast<const float4*>(&sa[buf][k][h * (BM / 2) + ty * 4]);
+                    av[4 * h] = a.x; av[4 * h + 1] = a.y; av[4 * h + 2] = a.z; av[4 * h + 3] = a.w;
+                }
+#pragma unroll
+                for (int h = 0; h < TN / 4; ++h) {
+                    const float4 w = *reinterpret_cast<const float4*>(&sw[buf][k][h * (BN / 2) + tx * 4]);
+                    wv[2 * h] = make_float2(w.x, w.y); wv[2 * h + 1] = make_float2(w.z, w.w);
+                }
+#pragma unroll
+                for (int i = 0; i < TM; ++i)
+#pragma unroll
+                    for (int j = 0; j < TN / 2; ++j) {
+                        if constexpr (PACK) acc[i][j] = fma2(make_float2(av[i], av[i]), wv[j], acc[i][j]);
+                        else acc[i][j] = make_float2(fmaf(av[i], wv[j].x, acc[i][j].x), fmaf(av[i], wv[j].y, acc[i][j].y));
+                    }
             }
-#pragma unroll
-            for (int h = 0; h < TN / 4; ++h) {
-                const float4 w = *reinterpret_cast<const float4*>(&sw[buf][k][h * (BN / 2) + tx * 4]);
-                wv[4 * h] = w.x; wv[4 * h + 1] = w.y; wv[4 * h + 2] = w.z; wv[4 * h + 3] = w.w;
-            }
-#pragma unroll
-            for (int i = 0; i < TM; ++i)
-#pragma unroll
-                for (int j = 0; j < TN; ++j) acc[i][j] = fmaf(av[i], wv[j], acc[i][j]);
         }
         if (kb + 1 < nk) {
             stash(buf ^ 1);
@@ -314,8 +333,8 @@ pointwise_kernel(const float* __restrict__ A, const float* __restrict__ W, const
         for (int i = 0; i < TM; ++i) {
             const long long m = m0 + (i / 4) * (BM / 2) + ty * 4 + (i & 3);
             if (m >= M) continue;
-            float4 v = make_float4(activate(acc[i][4 * hj] + bv.x, act), activate(acc[i][4 * hj + 1] + bv.y, act),
-                                   activate(acc[i][4 * hj + 2] + bv.z, act), activate(acc[i][4 * hj + 3] + bv.w, act));
+            const float2 lo = acc[i][2 * hj], hi = acc[i][2 * hj + 1];
+            float4 v = make_float4(activate(lo.x + bv.x, act), activate(lo.y + bv.y, act), activate(hi.x + bv.z, act), activate(hi.y + bv.w, act));
             if (R) {
                 const float4 r = *reinterpret_cast<const float4*>(R + m * N + n);
                 v.x += r.x; v.y += r.y; v.z += r.z; v.w += r.w;
@@ -653,6 +672,11 @@ extern "C" int shvk_cnn_se_gate(const float* x, float* partial, const float* w1,
     if (e != cudaSuccess) return int(e);
     const size_t smem = size_t(C + CS) * sizeof(float);
     if (smem > 48 * 1024) return int(cudaErrorInvalidValue);
+    // the gate itself on clusters of eight blocks (cnn_fused.cu: a weight row is read once for four frames, and an eighth of
+    // them by a block) where its 128-bit loads and its shared memory allow: both launches, 960 channels, one block a frame /
+    // clusters: 4 frames 52 / 30 us, 75 frames 91 / 58, 300 frames (4 to a cluster) 83
+    if ((CS & 3) == 0 && !sb::misaligned(w1) && !sb::misaligned(w2) && 4 * smem <= 48 * 1024)
+        return shvk_cnn_se_gate_sums(partial, w1, b1, w2, b2, gate, F, S, HW, C, CS, stream);
     sb::se_gate_kernel<<<unsigned(F), 1024, smem, s>>>(partial, w1, b1, w2, b2, gate, HW, C, CS, S);
     return int(cudaGetLastError());
 }
@@ -713,16 +737,35 @@ extern "C" int shvk_cnn_pointwise(const float* A, const float* W, const float* b
     if (M <= 0 || N <= 0) return 0;
     if (sb::pointwise_args_bad(A, W, b, gate, gate_rows, R, out, N, K)) return int(cudaErrorInvalidValue);
     cudaStream_t s = cudaStream_t(stream);
-    const int bn = sb::pointwise_tile_width(N);
+    // Layers of 24, 40, 72 or 80 output channels: one tile spans the row, so a pixel is read once instead of for every 16 or 32
+    // columns (75 frames: 24 -> 72 channels 55 -> 44 us; 40 channels 51 -> 35, 80 channels 36 -> 33), as long as that leaves
+    // about a block per SM (20 frames, 80 channels: 37 against 24 us).  Wide layers: 128 columns do more per shared-memory
+    // read, but a block alone on its SM waits for its loads; up to three 64 x 64 tiles per SM are faster (75 frames, 160 channels
+    // of 960: 123 -> 85 us; token projection 109 -> 49; 112 channels, 564 tiles: 85 against 64).
+    int bn = sb::pointwise_tile_width(N);
+    if ((N == 24 || N == 40 || N == 72 || N == 80) && sb::blocks_for(M, 128) >= 100) bn = N;
+    else if (bn == 128 && (long long)sb::blocks_for(M, 64) * ((N + 63) / 64) <= 3 * 148) bn = 64;
     const unsigned gy = unsigned((N + bn - 1) / bn);
-    if (bn == 128)
-        sb::pointwise_kernel<128, 128, 8, 8><<<sb::blocks_for(M, 128) * gy, 256, 0, s>>>(A, W, b, gate, gate_rows, R, out, M, N, K, act, int(gy));
-    else if (bn == 64)
-        sb::pointwise_kernel<64, 64, 4, 4><<<sb::blocks_for(M, 64) * gy, 256, 0, s>>>(A, W, b, gate, gate_rows, R, out, M, N, K, act, int(gy));
-    else if (bn == 32)
-        sb::pointwise_kernel<128, 32, 4, 4><<<sb::blocks_for(M, 128) * gy, 256, 0, s>>>(A, W, b, gate, gate_rows, R, out, M, N, K, act, int(gy));
-    else
-        sb::pointwise_kernel<256, 16, 4, 4><<<sb::blocks_for(M, 256) * gy, 256, 0, s>>>(A, W, b, gate, gate_rows, R, out, M, N, K, act, int(gy));
+    const bool deep = K >= 256;
+#define SHVK_POINTWISE(BM_, BN_, TM_, TN_, KS_, PACK_)                                                                           \
+    do {                                                                                                                        \
+        const unsigned blocks = sb::blocks_for(M, BM_) * gy, threads = sb::pw_threads(BM_, BN_, TM_, TN_);                       \
+        if (gate)                                                                                                               \
+            sb::pointwise_kernel<BM_, BN_, TM_, TN_, KS_, true, PACK_><<<blocks, threads, 0, s>>>(A, W, b, gate, gate_rows, R, out, M, N, K, act, int(gy)); \
+        else                                                                                                                    \
+            sb::pointwise_kernel<BM_, BN_, TM_, TN_, KS_, false, PACK_><<<blocks, threads, 0, s>>>(A, W, b, gate, gate_rows, R, out, M, N, K, act, int(gy)); \
+    } while (0)
+    if (bn == 128 && deep && !gate) SHVK_POINTWISE(128, 128, 8, 8, 16, true);
+    else if (bn == 128) SHVK_POINTWISE(128, 128, 8, 8, 8, true);
+    else if (bn == 64 && deep) SHVK_POINTWISE(64, 64, 4, 4, 32, true);
+    else if (bn == 64) SHVK_POINTWISE(64, 64, 4, 4, 8, true);
+    else if (bn == 24) SHVK_POINTWISE(256, 24, 8, 4, 8, true);
+    else if (bn == 40) SHVK_POINTWISE(128, 40, 8, 4, 8, true);
+    else if (bn == 72) SHVK_POINTWISE(128, 72, 8, 4, 8, true);
+    else if (bn == 80) SHVK_POINTWISE(128, 80, 8, 4, 8, true);
+    else if (bn == 32) SHVK_POINTWISE(128, 32, 4, 4, 8, false);
+    else SHVK_POINTWISE(256, 16, 4, 4, 8, false);
+#undef SHVK_POINTWISE
     return int(cudaGetLastError());
 }
 

@@ -25,16 +25,6 @@ namespace {
 __device__ __forceinline__ float hswish(float x) { return x * __saturatef(fmaf(x, 1.0f / 6.0f, 0.5f)); }
 template <bool HS> __device__ __forceinline__ float act(float x) { return HS ? hswish(x) : fmaxf(x, 0.0f); }
 
-// two float32 FMAs in one instruction (each rounded as fmaf rounds)
-__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
-    float2 d;
-    asm("fma.rn.f32x2 %0, %1, %2, %3;"
-        : "=l"(reinterpret_cast<unsigned long long&>(d))
-        : "l"(reinterpret_cast<unsigned long long&>(a)), "l"(reinterpret_cast<unsigned long long&>(b)),
-          "l"(reinterpret_cast<unsigned long long&>(c)));
-    return d;
-}
-
 template <typename HT> struct Half;
 template <> struct Half<__nv_bfloat16> {
     static __device__ __forceinline__ uint32_t pack(float lo, float hi) {

@@ -36,6 +36,16 @@ __device__ __forceinline__ float warp_max(float v) {
     return v;
 }
 
+// Two float32 FMAs in one instruction (each rounded as fmaf rounds).
+__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
+    float2 d;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;"
+        : "=l"(reinterpret_cast<unsigned long long&>(d))
+        : "l"(reinterpret_cast<unsigned long long&>(a)), "l"(reinterpret_cast<unsigned long long&>(b)),
+          "l"(reinterpret_cast<unsigned long long&>(c)));
+    return d;
+}
+
 // Barrier over the blocks of a cluster; shared-memory writes before it, remote ones included, are visible behind it.
 __device__ __forceinline__ void cluster_sync() {
     __syncwarp();                                            // the aligned forms want whole warps

@@ -305,6 +305,38 @@ def test_encode_frame_independence_and_graphs(weight_files):
     graph.close()
 
 
+@pytest.mark.parametrize("N,K,gated", [(16, 16, False), (24, 64, False), (24, 72, True), (40, 120, True), (72, 24, False), (80, 184, False),
+                                       (80, 200, True), (64, 16, False), (112, 480, True), (160, 264, True), (384, 960, False), (672, 112, False)])
+def test_pointwise_tiles_give_the_same_rows(L, N, K, gated):
+    """The fp32 1x1 convolution picks its tile from the row count (one tile a row, 64 or 128 columns, slabs of 8, 16 or 32 channels
+    whose last one may be short): rows are the same bits whatever the tile, and near float64 (K products in float32: the error of
+    a sum is below (K + 4) 2^-24 times the sum of magnitudes, first order)."""
+    import torch
+    rng = np.random.default_rng(N * K)
+    big, rows_per_gate = 13001, 240
+    a = rng.standard_normal((big, K)).astype(np.float32)
+    w, b = (rng.standard_normal((N, K)) / 8).astype(np.float32), rng.standard_normal(N).astype(np.float32)
+    g = rng.random(((big + rows_per_gate - 1) // rows_per_gate, K)).astype(np.float32)
+    r = rng.standard_normal((big, N)).astype(np.float32)
+    A, Wt, Bt, G, R = (torch.from_numpy(x).cuda() for x in (a, w, b, g, r))
+    outs = []
+    for m in (big, 3333, 65, 1):
+        out = torch.full((big, N), 9.0, device="cuda")
+        rc = L.shvk_cnn_pointwise(A.data_ptr(), Wt.data_ptr(), Bt.data_ptr(), G.data_ptr() if gated else None, rows_per_gate, R.data_ptr(),
+                                  out.data_ptr(), m, N, K, 0, torch.cuda.current_stream().cuda_stream)
+        assert rc == 0
+        torch.cuda.synchronize()
+        assert (out[m:] == 9.0).all()
+        outs.append(out[:m])
+    for o in outs[1:]:
+        assert torch.equal(o, outs[0][:len(o)])
+    rows = np.r_[0:200, big - 200:big]
+    x = a[rows].astype(np.float64) * (g[rows // rows_per_gate].astype(np.float64) if gated else 1.0)
+    want = x @ w.T.astype(np.float64) + b + r[rows]
+    bound = (K + 4) * 2.0 ** -24 * (np.abs(x) @ np.abs(w.T).astype(np.float64) + np.abs(b) + np.abs(r[rows]))
+    assert (np.abs(outs[0][torch.from_numpy(rows).cuda()].cpu().numpy() - want) <= bound).all()
+
+
 # ---------------------------------------------------------------------------------------------- fused kernels (16-bit modes)
 def _pack(L, w, order, dtype, n_pad=None, k_pad=None):
     import torch
