@@ -11,11 +11,11 @@
 // T2 and M do not depend on the state, only R, U, O and S' do.  Two kernels, chunk-parallel where the algebra allows:
 //
 //   prep   one warp per block, all B x H x T/16 blocks at once: the two Gram products on mma.sync, the decay masks, the
-//          16 x 16 triangular inverse (forward substitution over 16 lanes), T2 and M as bf16 tiles and the cumulative
-//          decays into a workspace of 1,152 bytes per block
-//   scan   one CTA per (batch, head) walks the blocks with the state resident: per block only the chain R -> U -> O and
+//          16 x 16 triangular inverse (forward substitution over 16 lanes), T2 and M as bf16 tiles and the decays'
+//          exponentials into a workspace of 1,152 bytes per block
+//   scan   one CTA per (batch, head), or two or four with a share of the value columns each, walks the blocks with the state resident: per block only the chain R -> U -> O and
 //          the state update remain, every operand fragment read straight out of the staged K, Q, V, T2, M tiles with
-//          ldmatrix (tiles arrive by cp.async into a three-slot ring, XOR-swizzled so the fragment reads are
+//          ldmatrix (tiles arrive by cp.async into a ring of three or four slots, XOR-swizzled so the fragment reads are
 //          conflict-free), one CTA barrier per block, the previous block's output rows written while the next block's
 //          products run
 //
@@ -37,7 +37,8 @@ namespace {
 
 constexpr int CB = 16;                       // tokens per block
 constexpr int CDV = 128;
-constexpr int WS_T2 = 0, WS_M = 512, WS_CUM = 1024, WS_BLOCK = 1152;   // workspace block: T2 | M (bf16 16 x 16) | c (fp32 16) | pad
+// workspace block: T2 | M (bf16 16 x 16) | exp(c_i) | exp(c_16 - c_i) (fp32 16 each)
+constexpr int WS_T2 = 0, WS_M = 512, WS_EG = 1024, WS_DJ = 1088, WS_BLOCK = 1152;
 constexpr int OT_PITCH = CDV + 4;            // floats per token row of the o tile (fragment stores fall into 32 banks)
 
 __device__ __forceinline__ uint32_t cpack(float lo, float hi) {
@@ -50,6 +51,13 @@ __device__ __forceinline__ void cmma(float (&d)[4], const uint32_t (&a)[4], uint
     asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
                  : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
                  : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+}
+__device__ __forceinline__ float2 mul2(float2 a, float2 b) {
+    float2 d;
+    asm("mul.rn.f32x2 %0, %1, %2;"
+        : "=l"(reinterpret_cast<unsigned long long&>(d))
+        : "l"(reinterpret_cast<unsigned long long&>(a)), "l"(reinterpret_cast<unsigned long long&>(b)));
+    return d;
 }
 __device__ __forceinline__ void ldsm4(uint32_t addr, uint32_t (&r)[4]) {
     asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0, %1, %2, %3}, [%4];"
@@ -74,122 +82,153 @@ template <int ROWB> __device__ __forceinline__ uint32_t tile_off(int row, int ch
 }
 
 // ---------------------------------------------------------------------------------------------------- prep kernel
+// A warp takes two blocks: their Gram products and masks one after the other on all 32 lanes (the second block's rows are
+// fetched meanwhile), then both triangular inverses at once, a half-warp each, rows of L read 128 bits at a time.  The
+// kernel is bound by issue and shared-memory latency, not by its 250 MB (64 x 2,048 tokens, 6 heads); with one block a warp
+// everywhere both kernels take 259 us there against 248.
 // (declared with a minimum of CTAs per SM: without one the assembler keeps the kernel at 40-48 registers by moving loads
 // next to their uses)
+constexpr int LF_PITCH = CB + 4, LF_SLOT = CB * LF_PITCH + 16;    // floats; the two slots start 16 banks apart
+template <int DK> struct PrepWarp {
+    __align__(16) uint8_t k[CB * DK * 2], q[CB * DK * 2];
+    __align__(16) float lf[2 * LF_SLOT];
+    float cum[CB], beta[2][CB];
+    __align__(16) uint8_t out[2][WS_BLOCK];
+};
 template <int DK>
 __global__ void __launch_bounds__(128, 4)
 gdn_chunked_prep_kernel(const __nv_bfloat16* __restrict__ Q, const __nv_bfloat16* __restrict__ K, const float* __restrict__ G,
                         const float* __restrict__ Beta, uint8_t* __restrict__ ws, int T, int H, int NB, long long blocks,
-                        float scale) {
-    constexpr int ROWB = DK * 2, VPR = DK / 8, KSTEP = DK / 16;          // bytes and 16-byte vectors per tile row
-    struct WarpSmem {
-        __align__(16) uint8_t k[CB * ROWB], q[CB * ROWB];
-        float lf[CB][CB + 1];
-        float cum[CB], beta[CB];
-        __align__(16) uint8_t out[WS_BLOCK];
-    };
+                        int per, float scale) {
+    constexpr int ROWB = DK * 2, VPR = DK / 8, KSTEP = DK / 16, VEC = CB * VPR / 32;     // bytes and 16-byte vectors per tile row
     extern __shared__ __align__(16) uint8_t prep_smem_raw[];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    WarpSmem& sm = reinterpret_cast<WarpSmem*>(prep_smem_raw)[warp];
-    const long long blk = (long long)blockIdx.x * 4 + warp;
-    if (blk >= blocks) return;
-    const long long bh = blk / NB;
-    const int c = int(blk - bh * NB), t0 = c * CB;
-    const int bidx = int(bh / H), head = int(bh - (long long)bidx * H);
+    PrepWarp<DK>& sm = reinterpret_cast<PrepWarp<DK>*>(prep_smem_raw)[warp];
+    const long long blk0 = ((long long)blockIdx.x * 4 + warp) * per;
+    if (blk0 >= blocks) return;
+    const int nslot = blk0 + per <= blocks ? per : 1;
     const int g = lane >> 2, t = lane & 3, lm = lane >> 3, lr = lane & 7;
     const long long tok_stride = (long long)H * DK;
-    const __nv_bfloat16* Ks = K + ((long long)bidx * T * H + head) * DK;
-    const __nv_bfloat16* Qs = Q + ((long long)bidx * T * H + head) * DK;
 
-    // K and Q rows of the block, 16-byte vectors, eight (DK = 64) or sixteen lanes per 128 / 256-byte row
-#pragma unroll
-    for (int i = 0; i < CB * VPR / 32; ++i) {
-        const int v = lane + 32 * i, row = v / VPR, c8 = v % VPR;
-        const bool ok = t0 + row < T;
+    // K and Q rows of a block, 16-byte vectors, eight (DK = 64) or sixteen lanes per 128 / 256-byte row; decay and beta of
+    // its tokens; tokens past T are inert
+    uint4 kv[VEC], qv[VEC];
+    float dec, bt;
+    auto fetch = [&](long long blk) {
+        const long long bh = blk / NB;
+        const int t0 = int(blk - bh * NB) * CB, bidx = int(bh / H), head = int(bh - (long long)bidx * H);
+        const __nv_bfloat16* Ks = K + ((long long)bidx * T * H + head) * DK;
+        const __nv_bfloat16* Qs = Q + ((long long)bidx * T * H + head) * DK;
         const uint4 z = make_uint4(0, 0, 0, 0);
-        const uint4 kv = ok ? *reinterpret_cast<const uint4*>(Ks + (long long)(t0 + row) * tok_stride + c8 * 8) : z;
-        const uint4 qv = ok ? *reinterpret_cast<const uint4*>(Qs + (long long)(t0 + row) * tok_stride + c8 * 8) : z;
-        *reinterpret_cast<uint4*>(sm.k + tile_off<ROWB>(row, c8)) = kv;
-        *reinterpret_cast<uint4*>(sm.q + tile_off<ROWB>(row, c8)) = qv;
-    }
-    // decays: inclusive prefix sum over the 16 tokens (both half-warps compute it); tokens past T are inert
-    {
+#pragma unroll
+        for (int i = 0; i < VEC; ++i) {
+            const int v = lane + 32 * i, row = v / VPR, c8 = v % VPR;
+            const bool ok = t0 + row < T;
+            kv[i] = ok ? *reinterpret_cast<const uint4*>(Ks + (long long)(t0 + row) * tok_stride + c8 * 8) : z;
+            qv[i] = ok ? *reinterpret_cast<const uint4*>(Qs + (long long)(t0 + row) * tok_stride + c8 * 8) : z;
+        }
         const int tok = lane & (CB - 1);
         const bool ok = t0 + tok < T;
-        float cs = ok ? G[((long long)bidx * T + t0 + tok) * H + head] : 0.0f;
-        const float bt = ok ? Beta[((long long)bidx * T + t0 + tok) * H + head] : 0.0f;
+        dec = ok ? G[((long long)bidx * T + t0 + tok) * H + head] : 0.0f;
+        bt = ok ? Beta[((long long)bidx * T + t0 + tok) * H + head] : 0.0f;
+    };
+    auto land = [&](int slot) {
+#pragma unroll
+        for (int i = 0; i < VEC; ++i) {
+            const int v = lane + 32 * i, row = v / VPR, c8 = v % VPR;
+            *reinterpret_cast<uint4*>(sm.k + tile_off<ROWB>(row, c8)) = kv[i];
+            *reinterpret_cast<uint4*>(sm.q + tile_off<ROWB>(row, c8)) = qv[i];
+        }
+        // inclusive prefix sum of the decays over the 16 tokens (both half-warps compute it)
+        float cs = dec;
 #pragma unroll
         for (int o = 1; o < CB; o <<= 1) {
             const float up = __shfl_up_sync(0xffffffffu, cs, o);
-            if (tok >= o) cs += up;
+            if ((lane & (CB - 1)) >= o) cs += up;
         }
-        if (lane < CB) { sm.cum[lane] = cs; sm.beta[lane] = bt; }
-    }
-    __syncwarp();
-    // Gram products over the keys: A = K K^T, Bm = Q K^T (16 x 16 each)
-    float acc[2][4], accq[2][4];
+        const float last = __shfl_sync(0xffffffffu, cs, CB - 1);
+        if (lane < CB) {
+            sm.cum[lane] = cs;
+            sm.beta[slot][lane] = bt;
+            reinterpret_cast<float*>(sm.out[slot] + WS_EG)[lane] = __expf(cs);
+            reinterpret_cast<float*>(sm.out[slot] + WS_DJ)[lane] = __expf(last - cs);
+        }
+        __syncwarp();
+    };
+    fetch(blk0);
+#pragma unroll 1
+    for (int slot = 0; slot < nslot; ++slot) {
+        land(slot);
+        if (slot + 1 < nslot) fetch(blk0 + 1);
+        // Gram products over the keys: A = K K^T, Bm = Q K^T (16 x 16 each)
+        float acc[2][4], accq[2][4];
 #pragma unroll
-    for (int ni = 0; ni < 2; ++ni)
+        for (int ni = 0; ni < 2; ++ni)
 #pragma unroll
-        for (int e = 0; e < 4; ++e) { acc[ni][e] = 0.0f; accq[ni][e] = 0.0f; }
-    const uint32_t k_s = smem_u32(sm.k), q_s = smem_u32(sm.q);
+            for (int e = 0; e < 4; ++e) { acc[ni][e] = 0.0f; accq[ni][e] = 0.0f; }
+        const uint32_t k_s = smem_u32(sm.k), q_s = smem_u32(sm.q);
 #pragma unroll
-    for (int p = 0; p < KSTEP; ++p) {
-        // matrices (tokens 0-7, keys lo), (tokens 8-15, keys lo), (tokens 0-7, keys hi), (tokens 8-15, keys hi) of k-step p:
-        // the A fragment of [token][key]; as B fragments of the transposed product: (r[ni], r[ni + 2])
-        const uint32_t off = tile_off<ROWB>((lm & 1) * 8 + lr, 2 * p + (lm >> 1));
-        uint32_t kf[4], qf[4];
-        ldsm4(k_s + off, kf);
-        ldsm4(q_s + off, qf);
+        for (int p = 0; p < KSTEP; ++p) {
+            // matrices (tokens 0-7, keys lo), (tokens 8-15, keys lo), (tokens 0-7, keys hi), (tokens 8-15, keys hi) of k-step
+            // p: the A fragment of [token][key]; as B fragments of the transposed product: (r[ni], r[ni + 2])
+            const uint32_t off = tile_off<ROWB>((lm & 1) * 8 + lr, 2 * p + (lm >> 1));
+            uint32_t kf[4], qf[4];
+            ldsm4(k_s + off, kf);
+            ldsm4(q_s + off, qf);
+#pragma unroll
+            for (int ni = 0; ni < 2; ++ni) {
+                cmma(acc[ni], kf, kf[ni], kf[ni + 2]);
+                cmma(accq[ni], qf, kf[ni], kf[ni + 2]);
+            }
+        }
+        // acc[ni][0,1]: row i = g, columns j = 8 ni + 2t, + 1;  acc[ni][2,3]: row i = g + 8
+        uint32_t* mw = reinterpret_cast<uint32_t*>(sm.out[slot] + WS_M);           // 8 words per row
+        float* lf = sm.lf + slot * LF_SLOT;
 #pragma unroll
         for (int ni = 0; ni < 2; ++ni) {
-            cmma(acc[ni], kf, kf[ni], kf[ni + 2]);
-            cmma(accq[ni], qf, kf[ni], kf[ni + 2]);
-        }
-    }
-    // acc[ni][0,1]: row i = g, columns j = 8 ni + 2t, + 1;  acc[ni][2,3]: row i = g + 8
-    uint32_t* mw = reinterpret_cast<uint32_t*>(sm.out + WS_M);                 // 8 words per row
+            float l[4], m[4];
 #pragma unroll
-    for (int ni = 0; ni < 2; ++ni) {
-        float m[4];
-#pragma unroll
-        for (int e = 0; e < 4; ++e) {
-            const int i = g + (e >> 1) * 8, j = 8 * ni + 2 * t + (e & 1);
-            const float dec = __expf(j <= i ? sm.cum[i] - sm.cum[j] : 0.0f);
-            sm.lf[i][j] = j < i ? sm.beta[i] * dec * acc[ni][e] : 0.0f;
-            m[e] = j <= i ? scale * dec * accq[ni][e] : 0.0f;
+            for (int e = 0; e < 4; ++e) {
+                const int i = g + (e >> 1) * 8, j = 8 * ni + 2 * t + (e & 1);
+                const float dcy = __expf(j <= i ? sm.cum[i] - sm.cum[j] : 0.0f);
+                l[e] = j < i ? sm.beta[slot][i] * dcy * acc[ni][e] : 0.0f;
+                m[e] = j <= i ? scale * dcy * accq[ni][e] : 0.0f;
+            }
+            *reinterpret_cast<float2*>(lf + g * LF_PITCH + 8 * ni + 2 * t) = make_float2(l[0], l[1]);
+            *reinterpret_cast<float2*>(lf + (g + 8) * LF_PITCH + 8 * ni + 2 * t) = make_float2(l[2], l[3]);
+            mw[g * 8 + 4 * ni + t] = cpack(m[0], m[1]);
+            mw[(g + 8) * 8 + 4 * ni + t] = cpack(m[2], m[3]);
         }
-        mw[g * 8 + 4 * ni + t] = cpack(m[0], m[1]);
-        mw[(g + 8) * 8 + 4 * ni + t] = cpack(m[2], m[3]);
+        __syncwarp();                                     // L is complete; the tiles and cum may be overwritten
     }
-    __syncwarp();
-    if (lane < CB) {                                      // column `lane` of (I + L)^-1 by forward substitution
+    {                                                     // column `col` of (I + L)^-1 of the half-warp's block by forward substitution
+        const int half = lane >> 4, col = lane & (CB - 1), slot = half < nslot ? half : 0;
+        const float* lf = sm.lf + slot * LF_SLOT;
         float x[CB];
 #pragma unroll
         for (int i = 0; i < CB; ++i) {
             // four partial sums: the dependent chain per row is i / 4 long instead of i
-            float s0 = i == lane ? 1.0f : 0.0f, s1 = 0.0f, s2 = 0.0f, s3 = 0.0f;
+            float s0 = i == col ? 1.0f : 0.0f, s1 = 0.0f, s2 = 0.0f, s3 = 0.0f;
 #pragma unroll
-            for (int j = 0; j < i; ++j) {
-                const float l = sm.lf[i][j];
-                if ((j & 3) == 0) s0 = fmaf(-l, x[j], s0);
-                else if ((j & 3) == 1) s1 = fmaf(-l, x[j], s1);
-                else if ((j & 3) == 2) s2 = fmaf(-l, x[j], s2);
-                else s3 = fmaf(-l, x[j], s3);
+            for (int j = 0; j < i; j += 4) {
+                const float4 l = *reinterpret_cast<const float4*>(lf + i * LF_PITCH + j);
+                s0 = fmaf(-l.x, x[j], s0);
+                if (j + 1 < i) s1 = fmaf(-l.y, x[j + 1], s1);
+                if (j + 2 < i) s2 = fmaf(-l.z, x[j + 2], s2);
+                if (j + 3 < i) s3 = fmaf(-l.w, x[j + 3], s3);
             }
             x[i] = (s0 + s1) + (s2 + s3);
         }
-        const float bc = sm.beta[lane];
-        __nv_bfloat16* t2 = reinterpret_cast<__nv_bfloat16*>(sm.out + WS_T2);
+        const float bc = sm.beta[slot][col];
+        __nv_bfloat16* t2 = reinterpret_cast<__nv_bfloat16*>(sm.out[slot] + WS_T2);
+        if (half < nslot)
 #pragma unroll
-        for (int i = 0; i < CB; ++i) t2[i * CB + lane] = __float2bfloat16_rn(x[i] * bc);
-        reinterpret_cast<float*>(sm.out + WS_CUM)[lane] = sm.cum[lane];
-        reinterpret_cast<float*>(sm.out + WS_CUM)[CB + lane] = 0.0f;
+            for (int i = 0; i < CB; ++i) t2[i * CB + col] = __float2bfloat16_rn(x[i] * bc);
     }
     __syncwarp();
-    uint4* dst = reinterpret_cast<uint4*>(ws + blk * WS_BLOCK);
-    const uint4* src = reinterpret_cast<const uint4*>(sm.out);
-    for (int i = lane; i < WS_BLOCK / 16; i += 32) dst[i] = src[i];
+    uint4* dst = reinterpret_cast<uint4*>(ws + blk0 * WS_BLOCK);
+    const uint4* src = reinterpret_cast<const uint4*>(sm.out[0]);
+    for (int i = lane; i < nslot * (WS_BLOCK / 16); i += 32) dst[i] = src[i];
 }
 
 // ---------------------------------------------------------------------------------------------------- scan kernel
@@ -199,13 +238,14 @@ template <int DK> struct ScanStage {                      // one block's operand
     __align__(16) uint8_t w[WS_BLOCK];                     // T2 | M | c of the block
 };
 
-// DK = 64: MI = 2 row tiles per warp, 4 warps;  DK = 128: MI = 1, 8 warps.
-template <int DK, typename TO>
-__global__ void __launch_bounds__(DK == 64 ? 128 : 256)
+// MI row tiles of 16 values per warp, NWARP warps: NWARP * 16 * MI values per CTA, blockIdx.y says which of the 128.
+template <int DK, typename TO, int MI, int NWARP, int NSLOT>
+__global__ void __launch_bounds__(NWARP * 32, NWARP * MI < 8 ? 0 : DK == 64 ? 3 : 2)
 gdn_chunked_scan_kernel(const __nv_bfloat16* __restrict__ Q, const __nv_bfloat16* __restrict__ K, const __nv_bfloat16* __restrict__ V,
                         const uint8_t* __restrict__ ws, TO* __restrict__ O, int T, int H, int NB, float scale) {
-    constexpr int MI = DK == 64 ? 2 : 1, NWARP = DK == 64 ? 4 : 8, NTHR = NWARP * 32;
-    constexpr int KSTEP = DK / 16, NJ = DK / 8, ROWB = DK * 2, VPR = DK / 8, NSLOT = 3;
+    constexpr int NTHR = NWARP * 32, V8 = NWARP * 2 * MI;                  // V8: 16-byte vectors of a token's values here
+    constexpr int KSTEP = DK / 16, NJ = DK / 8, ROWB = DK * 2, VPR = DK / 8, KI = CB * VPR / NTHR, VI = CB * V8 / NTHR;
+    static_assert(CB * VPR % NTHR == 0 && CB * V8 % NTHR == 0, "whole rounds of copies");
     struct Smem {
         ScanStage<DK> st[NSLOT];
         float ot[2][CB][OT_PITCH];
@@ -215,7 +255,7 @@ gdn_chunked_scan_kernel(const __nv_bfloat16* __restrict__ Q, const __nv_bfloat16
     const int bh = blockIdx.x, bidx = bh / H, head = bh % H;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int g = lane >> 2, t = lane & 3, lm = lane >> 3, lr = lane & 7;
-    const int dvb = warp * 16 * MI;
+    const int v0 = blockIdx.y * V8, dvb = v0 * 8 + warp * 16 * MI;
     const long long tok_stride_k = (long long)H * DK, tok_stride_v = (long long)H * CDV;
     const __nv_bfloat16* Qs = Q + ((long long)bidx * T * H + head) * DK;
     const __nv_bfloat16* Ks = K + ((long long)bidx * T * H + head) * DK;
@@ -231,53 +271,74 @@ gdn_chunked_scan_kernel(const __nv_bfloat16* __restrict__ Q, const __nv_bfloat16
 #pragma unroll
             for (int e = 0; e < 4; ++e) S[mi][nj][e] = 0.0f;
 
-    // asynchronous copies of block `c` into ring slot c % 3; every thread issues its share and commits one group
+    // asynchronous copies of block `c` into ring slot c % NSLOT; every thread issues its share and commits one group
+    // the thread's first element of the next block to fetch, and of the next block of output rows; its i-th copy is KROWS (VROWS)
+    // token rows further on
+    constexpr int KROWS = NTHR / VPR, VROWS = NTHR / V8;
+    const __nv_bfloat16* kp = Ks + (tid / VPR) * tok_stride_k + tid % VPR * 8;
+    const __nv_bfloat16* qp = Qs + (tid / VPR) * tok_stride_k + tid % VPR * 8;
+    const __nv_bfloat16* vp = Vs + (tid / V8) * tok_stride_v + (v0 + tid % V8) * 8;
+    TO* op = Os + (tid / V8) * tok_stride_v + (v0 + tid % V8) * 8;
+    const uint8_t* wp = Ws;
     auto issue = [&](int c) {
         if (c < NB) {
             ScanStage<DK>& st = sm.st[c % NSLOT];
-            const int t0 = c * CB;
-            for (int v = tid; v < CB * VPR; v += NTHR) {
-                const int row = v / VPR, c8 = v % VPR;
-                const int ok = t0 + row < T ? 16 : 0;
-                const long long src = (long long)(ok ? t0 + row : 0) * tok_stride_k + c8 * 8;
-                cp_async16(smem_u32(st.k) + tile_off<ROWB>(row, c8), Ks + src, ok);
-                cp_async16(smem_u32(st.q) + tile_off<ROWB>(row, c8), Qs + src, ok);
+            const int left = T - c * CB;                  // tokens from this block on: rows past them are filled with zeros
+            const uint32_t sk = smem_u32(st.k), sq = smem_u32(st.q), sv = smem_u32(st.v[0]);
+#pragma unroll
+            for (int i = 0; i < KI; ++i) {
+                const int row = tid / VPR + i * KROWS, n = row < left ? 16 : 0;
+                const uint32_t dst = tile_off<ROWB>(row, tid % VPR);
+                cp_async16(sk + dst, n ? static_cast<const void*>(kp + i * KROWS * tok_stride_k) : wp, n);
+                cp_async16(sq + dst, n ? static_cast<const void*>(qp + i * KROWS * tok_stride_k) : wp, n);
             }
-            for (int v = tid; v < CB * 16; v += NTHR) {
-                const int row = v >> 4, c16 = v & 15;
-                const int ok = t0 + row < T ? 16 : 0;
-                cp_async16(smem_u32(st.v[c16 >> 3]) + tile_off<128>(row, c16 & 7), Vs + (long long)(ok ? t0 + row : 0) * tok_stride_v + c16 * 8, ok);
+#pragma unroll
+            for (int i = 0; i < VI; ++i) {
+                const int row = tid / V8 + i * VROWS, n = row < left ? 16 : 0, c16 = v0 + tid % V8;
+                cp_async16(sv + uint32_t(c16 >> 3) * (CB * 128) + tile_off<128>(row, c16 & 7),
+                           n ? static_cast<const void*>(vp + i * VROWS * tok_stride_v) : wp, n);
             }
-            for (int v = tid; v < WS_BLOCK / 16; v += NTHR) cp_async16(smem_u32(st.w) + v * 16, Ws + (long long)c * WS_BLOCK + v * 16, 16);
+            for (int v = tid; v < WS_BLOCK / 16; v += NTHR) cp_async16(smem_u32(st.w) + v * 16, wp + v * 16, 16);
+            kp += CB * tok_stride_k;
+            qp += CB * tok_stride_k;
+            vp += CB * tok_stride_v;
+            wp += WS_BLOCK;
         }
         cp_commit();                                      // an empty group past the end keeps the group count in step
     };
-    // rows of a finished block from its o tile to global memory: 16 tokens x 128 values, eight values per thread and pass
+    // rows of a finished block from its o tile to global memory: 16 tokens, eight values per thread and pass
     auto store_rows = [&](int c) {
         const float* ot = &sm.ot[c & 1][0][0];
-        const int t0 = c * CB;
-        for (int idx = tid; idx < CB * CDV / 8; idx += NTHR) {
-            const int row = idx >> 4, c8 = idx & 15;
-            if (t0 + row < T) {
+        const int left = T - c * CB;
+#pragma unroll
+        for (int i = 0; i < VI; ++i) {
+            const int row = tid / V8 + i * VROWS, c8 = v0 + tid % V8;
+            if (row < left) {
                 const float4 a = *reinterpret_cast<const float4*>(ot + row * OT_PITCH + c8 * 8);
                 const float4 b = *reinterpret_cast<const float4*>(ot + row * OT_PITCH + c8 * 8 + 4);
-                TO* dst = Os + (long long)(t0 + row) * tok_stride_v + c8 * 8;
-                store_quad<TO>(dst, a.x, a.y, a.z, a.w);
-                store_quad<TO>(dst + 4, b.x, b.y, b.z, b.w);
+                TO* dst = op + i * VROWS * tok_stride_v;
+                if constexpr (sizeof(TO) == 2) {
+                    *reinterpret_cast<uint4*>(dst) = make_uint4(cpack(a.x, a.y), cpack(a.z, a.w), cpack(b.x, b.y), cpack(b.z, b.w));
+                } else {
+                    store_quad<TO>(dst, a.x, a.y, a.z, a.w);
+                    store_quad<TO>(dst + 4, b.x, b.y, b.z, b.w);
+                }
             }
         }
+        op += CB * tok_stride_v;
     };
 
-    issue(0);
-    issue(1);
+#pragma unroll
+    for (int c = 0; c < NSLOT - 1; ++c) issue(c);
     for (int c = 0; c < NB; ++c) {
-        cp_wait<1>();                                     // this thread's copies of block c have landed (block c + 1 may still fly)
-        __syncthreads();                                  // everyone's have; the o tile of block c - 1 is complete; slot (c + 2) % 3 is free
-        issue(c + 2);
+        cp_wait<NSLOT - 2>();                             // this thread's copies of block c have landed (later ones may still fly)
+        __syncthreads();                                  // everyone's have; the o tile of block c - 1 is complete; the slot of block c - 1 is free
+        issue(c + NSLOT - 1);
         if (c > 0) store_rows(c - 1);
         ScanStage<DK>& st = sm.st[c % NSLOT];
         const uint32_t k_s = smem_u32(st.k), q_s = smem_u32(st.q);
-        const float* cum = reinterpret_cast<const float*>(st.w + WS_CUM);
+        const float* eg = reinterpret_cast<const float*>(st.w + WS_EG);
+        const float* dj = reinterpret_cast<const float*>(st.w + WS_DJ);
         // ---------------------------------------------------------------- R^T = S0^T K^T and (Q S0)^T
         float R[MI][2][4], QS[MI][2][4];
 #pragma unroll
@@ -306,17 +367,14 @@ gdn_chunked_scan_kernel(const __nv_bfloat16* __restrict__ Q, const __nv_bfloat16
             }
         }
         // per-token scalars of this lane's tokens 8 ni + 2t, + 1
-        float er[2][2], eq[2][2], dj[2][2];
-        const float clast = cum[CB - 1];
+        float2 ner[2], eq[2], dj2[2];
 #pragma unroll
-        for (int ni = 0; ni < 2; ++ni)
-#pragma unroll
-            for (int e = 0; e < 2; ++e) {
-                const float cv = cum[8 * ni + 2 * t + e];
-                er[ni][e] = __expf(cv);
-                eq[ni][e] = er[ni][e] * scale;
-                dj[ni][e] = __expf(clast - cv);
-            }
+        for (int ni = 0; ni < 2; ++ni) {
+            const float2 e = *reinterpret_cast<const float2*>(eg + 8 * ni + 2 * t);
+            ner[ni] = make_float2(-e.x, -e.y);
+            eq[ni] = make_float2(e.x * scale, e.y * scale);
+            dj2[ni] = *reinterpret_cast<const float2*>(dj + 8 * ni + 2 * t);
+        }
         // B fragments of T2 and M (row-major 16 x 16, 32-byte rows): matrices (rows 0-7, cols lo), (rows 0-7, cols hi),
         // (rows 8-15, cols lo), (rows 8-15, cols hi)
         uint32_t bt[4], bm[4];
@@ -326,9 +384,11 @@ gdn_chunked_scan_kernel(const __nv_bfloat16* __restrict__ Q, const __nv_bfloat16
             ldsm4(smem_u32(st.w + WS_M) + off, bm);
         }
         // K^T fragments of the state update, B[token][key]: transposed reads; kf[q][2 h + c]: keys 16 q + 8 h + g, tokens 8 c + 2t, + 1
+        // (eight warps of the wider keys have no registers to hold them that early)
+        constexpr bool LATE_K = DK == 128 && NWARP == 8;
         uint32_t kf[KSTEP][4];
 #pragma unroll
-        for (int q = 0; q < KSTEP; ++q) ldsm4t(k_s + tile_off<ROWB>((lm & 1) * 8 + lr, 2 * q + (lm >> 1)), kf[q]);
+        for (int q = 0; q < KSTEP && !LATE_K; ++q) ldsm4t(k_s + tile_off<ROWB>((lm & 1) * 8 + lr, 2 * q + (lm >> 1)), kf[q]);
         float* otile = &sm.ot[c & 1][0][0];
         uint32_t da[MI][4];
 #pragma unroll
@@ -343,10 +403,12 @@ gdn_chunked_scan_kernel(const __nv_bfloat16* __restrict__ Q, const __nv_bfloat16
             }
             // vv[0]: value g, tokens 2t, +1 | vv[1]: value g + 8, same tokens | vv[2]: value g, tokens 8 + 2t | vv[3]: value g + 8
             uint32_t va[4];
-            va[0] = cpack(bf_lo(vv[0]) - er[0][0] * R[mi][0][0], bf_hi(vv[0]) - er[0][1] * R[mi][0][1]);
-            va[1] = cpack(bf_lo(vv[1]) - er[0][0] * R[mi][0][2], bf_hi(vv[1]) - er[0][1] * R[mi][0][3]);
-            va[2] = cpack(bf_lo(vv[2]) - er[1][0] * R[mi][1][0], bf_hi(vv[2]) - er[1][1] * R[mi][1][1]);
-            va[3] = cpack(bf_lo(vv[3]) - er[1][0] * R[mi][1][2], bf_hi(vv[3]) - er[1][1] * R[mi][1][3]);
+#pragma unroll
+            for (int h = 0; h < 4; ++h) {                 // tokens 8 (h / 2) + 2t, + 1 of value row g + 8 (h % 2)
+                const float2 r = make_float2(R[mi][h >> 1][2 * (h & 1)], R[mi][h >> 1][2 * (h & 1) + 1]);
+                const float2 d = fma2(ner[h >> 1], r, make_float2(bf_lo(vv[h]), bf_hi(vv[h])));
+                va[h] = cpack(d.x, d.y);
+            }
             float U[2][4];
 #pragma unroll
             for (int ni = 0; ni < 2; ++ni) {
@@ -359,30 +421,37 @@ gdn_chunked_scan_kernel(const __nv_bfloat16* __restrict__ Q, const __nv_bfloat16
             for (int ni = 0; ni < 2; ++ni) {
                 ua[2 * ni] = cpack(U[ni][0], U[ni][1]);
                 ua[2 * ni + 1] = cpack(U[ni][2], U[ni][3]);
-                da[mi][2 * ni] = cpack(U[ni][0] * dj[ni][0], U[ni][1] * dj[ni][1]);
-                da[mi][2 * ni + 1] = cpack(U[ni][2] * dj[ni][0], U[ni][3] * dj[ni][1]);
+                const float2 d0 = mul2(make_float2(U[ni][0], U[ni][1]), dj2[ni]), d1 = mul2(make_float2(U[ni][2], U[ni][3]), dj2[ni]);
+                da[mi][2 * ni] = cpack(d0.x, d0.y);
+                da[mi][2 * ni + 1] = cpack(d1.x, d1.y);
             }
 #pragma unroll
             for (int ni = 0; ni < 2; ++ni) {
                 float Oa[4] = {0.0f, 0.0f, 0.0f, 0.0f};
                 cmma(Oa, ua, bm[2 * ni], bm[2 * ni + 1]);
                 const int tok = 8 * ni + 2 * t;
-                otile[tok * OT_PITCH + r0] = Oa[0] + eq[ni][0] * QS[mi][ni][0];
-                otile[(tok + 1) * OT_PITCH + r0] = Oa[1] + eq[ni][1] * QS[mi][ni][1];
-                otile[tok * OT_PITCH + r1] = Oa[2] + eq[ni][0] * QS[mi][ni][2];
-                otile[(tok + 1) * OT_PITCH + r1] = Oa[3] + eq[ni][1] * QS[mi][ni][3];
+                const float2 o0 = fma2(eq[ni], make_float2(QS[mi][ni][0], QS[mi][ni][1]), make_float2(Oa[0], Oa[1]));
+                const float2 o1 = fma2(eq[ni], make_float2(QS[mi][ni][2], QS[mi][ni][3]), make_float2(Oa[2], Oa[3]));
+                otile[tok * OT_PITCH + r0] = o0.x;
+                otile[(tok + 1) * OT_PITCH + r0] = o0.y;
+                otile[tok * OT_PITCH + r1] = o1.x;
+                otile[(tok + 1) * OT_PITCH + r1] = o1.y;
             }
         }
         // ---------------------------------------------------------------- S^T <- e_last S^T + (diag(d) U)^T K
         {
-            const float elast = __expf(clast);
+            const float2 elast = make_float2(eg[CB - 1], eg[CB - 1]);
 #pragma unroll
             for (int nj = 0; nj < NJ; ++nj) {
+                if (LATE_K && nj % 2 == 0) ldsm4t(k_s + tile_off<ROWB>((lm & 1) * 8 + lr, nj + (lm >> 1)), kf[nj >> 1]);
                 const uint32_t b0 = kf[nj >> 1][2 * (nj & 1)], b1 = kf[nj >> 1][2 * (nj & 1) + 1];
 #pragma unroll
                 for (int mi = 0; mi < MI; ++mi) {
 #pragma unroll
-                    for (int e = 0; e < 4; ++e) S[mi][nj][e] *= elast;
+                    for (int e = 0; e < 4; e += 2) {
+                        const float2 v = mul2(make_float2(S[mi][nj][e], S[mi][nj][e + 1]), elast);
+                        S[mi][nj][e] = v.x; S[mi][nj][e + 1] = v.y;
+                    }
                     cmma(S[mi][nj], da[mi], b0, b1);
                 }
             }
@@ -393,28 +462,41 @@ gdn_chunked_scan_kernel(const __nv_bfloat16* __restrict__ Q, const __nv_bfloat16
     store_rows(NB - 1);
 }
 
-constexpr int prep_smem_bytes(int dk) { return 4 * (2 * CB * dk * 2 + CB * (CB + 1) * 4 + 2 * CB * 4 + WS_BLOCK + 64); }
+template <int DK, typename TO, int MI, int NWARP, int NSLOT>
+int launch_scan(const void* q, const void* k, const void* v, const void* ws, void* o, int B, int T, int H, int NB, float scale, cudaStream_t s) {
+    const int smem = NSLOT * int(sizeof(ScanStage<DK>)) + 2 * CB * OT_PITCH * 4 + 128;
+    const cudaError_t e = cudaFuncSetAttribute(gdn_chunked_scan_kernel<DK, TO, MI, NWARP, NSLOT>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    if (e != cudaSuccess) return int(e);
+    gdn_chunked_scan_kernel<DK, TO, MI, NWARP, NSLOT><<<dim3(unsigned(B) * unsigned(H), CDV / (16 * MI * NWARP)), NWARP * 32, smem, s>>>(
+        static_cast<const __nv_bfloat16*>(q), static_cast<const __nv_bfloat16*>(k), static_cast<const __nv_bfloat16*>(v),
+        static_cast<const uint8_t*>(ws), static_cast<TO*>(o), T, H, NB, scale);
+    return int(cudaGetLastError());
+}
 
 template <int DK, typename TO>
 int launch_chunked(const void* q, const void* k, const void* v, const float* g, const float* beta, void* o, void* ws, int B, int T,
                    int H, float scale, cudaStream_t s) {
     const int NB = (T + CB - 1) / CB;
-    const long long blocks = (long long)B * H * NB;
-    // the struct sizes the kernels use (kept in one place: the kernels take their layout from the same templates)
-    const int prep_smem = prep_smem_bytes(DK);
+    const long long blocks = (long long)B * H * NB, seqs = (long long)B * H;
+    const int prep_smem = 4 * int(sizeof(PrepWarp<DK>));
     cudaError_t e = cudaFuncSetAttribute(gdn_chunked_prep_kernel<DK>, cudaFuncAttributeMaxDynamicSharedMemorySize, prep_smem);
     if (e != cudaSuccess) return int(e);
-    gdn_chunked_prep_kernel<DK><<<unsigned((blocks + 3) / 4), 128, prep_smem, s>>>(
-        static_cast<const __nv_bfloat16*>(q), static_cast<const __nv_bfloat16*>(k), g, beta, static_cast<uint8_t*>(ws), T, H, NB, blocks, scale);
+    int dev = 0, sms = 148;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    // one block a warp while that is a single wave of warps (576 blocks of the wider keys: 9.4 us for both kernels against 11.0)
+    const int per = blocks <= 16ll * sms ? 1 : 2;
+    gdn_chunked_prep_kernel<DK><<<unsigned((blocks + 4 * per - 1) / (4 * per)), 128, prep_smem, s>>>(
+        static_cast<const __nv_bfloat16*>(q), static_cast<const __nv_bfloat16*>(k), g, beta, static_cast<uint8_t*>(ws), T, H, NB, blocks, per, scale);
     e = cudaGetLastError();
     if (e != cudaSuccess) return int(e);
-    const int scan_smem = 3 * int(sizeof(ScanStage<DK>)) + 2 * CB * OT_PITCH * 4 + 128;
-    e = cudaFuncSetAttribute(gdn_chunked_scan_kernel<DK, TO>, cudaFuncAttributeMaxDynamicSharedMemorySize, scan_smem);
-    if (e != cudaSuccess) return int(e);
-    gdn_chunked_scan_kernel<DK, TO><<<unsigned(B) * unsigned(H), DK == 64 ? 128 : 256, scan_smem, s>>>(
-        static_cast<const __nv_bfloat16*>(q), static_cast<const __nv_bfloat16*>(k), static_cast<const __nv_bfloat16*>(v),
-        static_cast<const uint8_t*>(ws), static_cast<TO*>(o), T, H, NB, scale);
-    return int(cudaGetLastError());
+    // The value columns of a sequence are independent: while sequences are too few to give every SM one, a sequence's columns
+    // are split over two CTAs or, with the wider keys, four, whose warps then have a scheduler each to themselves.  Both kernels, us,
+    // whole / 2 / 4: DK 64, 1,024 tokens: 72 sequences 59 / 39 / 43, 144 66 / 58 / 63; 18 sequences of 1,021 56 / 35 / 38; DK 128:
+    // 18 sequences of 1,021 84 / 52 / 47; of 1,024: 36 85 / 54 / 48, 72 89 / 58 / 56, 144 106 / 90 / 113; 288 of 2,048 343 / 348 / 395.
+    if (DK == 128 && 2 * seqs <= sms) return launch_scan<DK, TO, 1, 2, 4>(q, k, v, ws, o, B, T, H, NB, scale, s);
+    if (seqs <= sms) return launch_scan<DK, TO, 1, 4, 4>(q, k, v, ws, o, B, T, H, NB, scale, s);
+    return launch_scan<DK, TO, DK == 64 ? 2 : 1, DK == 64 ? 4 : 8, 3>(q, k, v, ws, o, B, T, H, NB, scale, s);
 }
 
 }  // namespace

@@ -69,6 +69,20 @@ def test_long_sequence_stress_shape(L, dk):
     assert rel_err(low, ref) < TOL
 
 
+@pytest.mark.parametrize("dk,out_bf16", [(64, False), (64, True), (128, False), (128, True)])
+def test_sequences_are_bitwise_the_same_however_they_are_split(L, dk, out_bf16):
+    """Few sequences are split over two or four CTAs each and prepared one block a warp, many run whole with two blocks a warp (an
+    odd number of blocks here): a sequence gives the same bits in all of them, and alone."""
+    t = 16 * 32 + 1                                            # 33 blocks, the last with one token
+    q, k, v, gg, beta = delta_inputs(3, t, 1, dk, 128, seed=5)
+    alone = [run_chunked(L, *(x[i:i + 1] for x in (q, k, v, gg, beta)), out_bf16=out_bf16)[0][0] for i in range(3)]
+    for n in (74, 75, 148, 149):
+        idx = np.arange(n) % 3
+        got, _ = run_chunked(L, *(x[idx] for x in (q, k, v, gg, beta)), out_bf16=out_bf16)
+        for i in range(n):
+            np.testing.assert_array_equal(got[i], alone[i % 3])
+
+
 def test_rejects_unsupported_shapes(L):
     import torch
     x = torch.zeros(4096, device="cuda")
