@@ -280,6 +280,21 @@ gdn_chunked_scan_kernel(const __nv_bfloat16* __restrict__ Q, const __nv_bfloat16
     const __nv_bfloat16* vp = Vs + (tid / V8) * tok_stride_v + (v0 + tid % V8) * 8;
     TO* op = Os + (tid / V8) * tok_stride_v + (v0 + tid % V8) * 8;
     const uint8_t* wp = Ws;
+    // a split sequence has registers to keep its destinations; a whole one computes them again
+    constexpr bool KEEP = NWARP * MI < 8;
+    auto k_dst = [&](int i) { return tile_off<ROWB>(tid / VPR + i * KROWS, tid % VPR); };
+    auto v_dst = [&](int i) {
+        const int c16 = v0 + tid % V8;
+        return uint32_t(c16 >> 3) * (CB * 128) + tile_off<128>(tid / V8 + i * VROWS, c16 & 7);
+    };
+    uint32_t kdst[KEEP ? KI : 1], vdst[KEEP ? VI : 1];
+    if constexpr (KEEP) {
+#pragma unroll
+        for (int i = 0; i < KI; ++i) { kdst[i] = k_dst(i); asm volatile("" : "+r"(kdst[i])); }
+#pragma unroll
+        for (int i = 0; i < VI; ++i) { vdst[i] = v_dst(i); asm volatile("" : "+r"(vdst[i])); }
+    }
+    const long long kstep = KROWS * tok_stride_k;
     auto issue = [&](int c) {
         if (c < NB) {
             ScanStage<DK>& st = sm.st[c % NSLOT];
@@ -288,15 +303,14 @@ gdn_chunked_scan_kernel(const __nv_bfloat16* __restrict__ Q, const __nv_bfloat16
 #pragma unroll
             for (int i = 0; i < KI; ++i) {
                 const int row = tid / VPR + i * KROWS, n = row < left ? 16 : 0;
-                const uint32_t dst = tile_off<ROWB>(row, tid % VPR);
-                cp_async16(sk + dst, n ? static_cast<const void*>(kp + i * KROWS * tok_stride_k) : wp, n);
-                cp_async16(sq + dst, n ? static_cast<const void*>(qp + i * KROWS * tok_stride_k) : wp, n);
+                const uint32_t dst = KEEP ? kdst[KEEP ? i : 0] : k_dst(i);
+                cp_async16(sk + dst, n ? static_cast<const void*>(kp + i * kstep) : wp, n);
+                cp_async16(sq + dst, n ? static_cast<const void*>(qp + i * kstep) : wp, n);
             }
 #pragma unroll
             for (int i = 0; i < VI; ++i) {
-                const int row = tid / V8 + i * VROWS, n = row < left ? 16 : 0, c16 = v0 + tid % V8;
-                cp_async16(sv + uint32_t(c16 >> 3) * (CB * 128) + tile_off<128>(row, c16 & 7),
-                           n ? static_cast<const void*>(vp + i * VROWS * tok_stride_v) : wp, n);
+                const int row = tid / V8 + i * VROWS, n = row < left ? 16 : 0;
+                cp_async16(sv + (KEEP ? vdst[KEEP ? i : 0] : v_dst(i)), n ? static_cast<const void*>(vp + i * VROWS * tok_stride_v) : wp, n);
             }
             for (int v = tid; v < WS_BLOCK / 16; v += NTHR) cp_async16(smem_u32(st.w) + v * 16, wp + v * 16, 16);
             kp += CB * tok_stride_k;
