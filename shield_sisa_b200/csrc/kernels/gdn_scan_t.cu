@@ -348,8 +348,11 @@ gdn_scan_t_kernel(const uint8_t* __restrict__ ptb, const float* __restrict__ o_n
             const float4 o = *reinterpret_cast<const float4*>(op + k * OT_PITCH);
             const float4 pp = *reinterpret_cast<const float4*>(sp + 4 * k);   // the four warps' partial sums of o^2
             const float rstd = rsqrtf(((pp.x + pp.y) + (pp.z + pp.w)) * (1.0f / float(kDV)) + 1e-6f);
+            const float2 r2 = make_float2(rstd, rstd);
+            const float2 lo = mul2(mul2(make_float2(o.x, o.y), r2), make_float2(onw.x, onw.y));
+            const float2 hi = mul2(mul2(make_float2(o.z, o.w), r2), make_float2(onw.z, onw.w));
             if (first + k < pnt)
-                store_quad<T>(dst + k * kVD, (o.x * rstd) * onw.x, (o.y * rstd) * onw.y, (o.z * rstd) * onw.z, (o.w * rstd) * onw.w);
+                store_quad<T>(dst + k * kVD, lo.x, lo.y, hi.x, hi.y);
         }
     };
 
@@ -410,25 +413,24 @@ gdn_scan_t_kernel(const uint8_t* __restrict__ ptb, const float* __restrict__ o_n
         const uint32_t* mqw = reinterpret_cast<const uint32_t*>(&x.mq[0][0]);
         // per-token scalars of this lane's tokens 8 ni + 2t, + 1, with the norms folded in:
         //   er = exp(c) / |k|  (R = K S0),  eq = exp(c) * 0.125 / |q|  (Q S0),  dj2 = exp(c_last - c) / |k|  (state update)
-        float er[2][2], eq[2][2], dj2[2][2], ikt[2][2];
+        // (pairs of tokens, two to an instruction from here on; the first one negated)
+        float2 ner[2], eq[2], dj2[2], ikt[2];
 #pragma unroll
-        for (int ni = 0; ni < 2; ++ni)
-#pragma unroll
-            for (int e = 0; e < 2; ++e) {
-                const int tok = 8 * ni + 2 * t + e;
-                const float egv = x.eg[tok], ikv = x.ik[tok];
-                er[ni][e] = egv * ikv;
-                eq[ni][e] = egv * x.iq[tok];
-                dj2[ni][e] = x.dj[tok] * ikv;
-                ikt[ni][e] = ikv;
-            }
+        for (int ni = 0; ni < 2; ++ni) {
+            const int tok = 8 * ni + 2 * t;
+            const float2 egv = *reinterpret_cast<const float2*>(&x.eg[tok]);
+            ikt[ni] = *reinterpret_cast<const float2*>(&x.ik[tok]);
+            ner[ni] = mul2(make_float2(-egv.x, -egv.y), ikt[ni]);
+            eq[ni] = mul2(egv, *reinterpret_cast<const float2*>(&x.iq[tok]));
+            dj2[ni] = mul2(*reinterpret_cast<const float2*>(&x.dj[tok]), ikt[ni]);
+        }
         uint32_t bt[2][2], bm[2][2];
 #pragma unroll
         for (int ni = 0; ni < 2; ++ni) {
             bt[ni][0] = t2w[(8 * ni + g) * 8 + t]; bt[ni][1] = t2w[(8 * ni + g) * 8 + t + 4];
             bm[ni][0] = mqw[(8 * ni + g) * 8 + t]; bm[ni][1] = mqw[(8 * ni + g) * 8 + t + 4];
         }
-        float sq[2][2] = {{0.0f, 0.0f}, {0.0f, 0.0f}};    // sum of o^2 over this thread's value rows, per token 8 ni + 2t + e
+        float2 sq[2] = {make_float2(0.0f, 0.0f), make_float2(0.0f, 0.0f)};   // sum of o^2 over this thread's value rows, tokens 8 ni + 2t, + 1
         uint32_t da[2][4];                                // decay-scaled U^T as A fragments, for the state update
         // every shared-memory load of this phase is issued before its first o-tile store (a store would hold back the
         // loads behind it): V^T and gate^T for both row halves and the K^T fragments of the state update
@@ -451,8 +453,9 @@ gdn_scan_t_kernel(const uint8_t* __restrict__ ptb, const float* __restrict__ o_n
 #pragma unroll
             for (int ni = 0; ni < 2; ++ni) {
                 const float2 v0 = h2_floats(vv[mi][ni]), v1 = h2_floats(vv[mi][ni + 2]);
-                va[2 * ni] = pack_op<T>(v0.x - er[ni][0] * R[mi][ni][0], v0.y - er[ni][1] * R[mi][ni][1]);
-                va[2 * ni + 1] = pack_op<T>(v1.x - er[ni][0] * R[mi][ni][2], v1.y - er[ni][1] * R[mi][ni][3]);
+                const float2 d0 = fma2(ner[ni], make_float2(R[mi][ni][0], R[mi][ni][1]), v0), d1 = fma2(ner[ni], make_float2(R[mi][ni][2], R[mi][ni][3]), v1);
+                va[2 * ni] = pack_op<T>(d0.x, d0.y);
+                va[2 * ni + 1] = pack_op<T>(d1.x, d1.y);
             }
             float U[2][4];
 #pragma unroll
@@ -464,10 +467,13 @@ gdn_scan_t_kernel(const uint8_t* __restrict__ ptb, const float* __restrict__ o_n
             uint32_t ua[4];
 #pragma unroll
             for (int ni = 0; ni < 2; ++ni) {
-                ua[2 * ni] = pack_op<T>(U[ni][0] * ikt[ni][0], U[ni][1] * ikt[ni][1]);      // U / |k| for the O product
-                ua[2 * ni + 1] = pack_op<T>(U[ni][2] * ikt[ni][0], U[ni][3] * ikt[ni][1]);
-                da[mi][2 * ni] = pack_op<T>(U[ni][0] * dj2[ni][0], U[ni][1] * dj2[ni][1]);
-                da[mi][2 * ni + 1] = pack_op<T>(U[ni][2] * dj2[ni][0], U[ni][3] * dj2[ni][1]);
+                const float2 u0 = make_float2(U[ni][0], U[ni][1]), u1 = make_float2(U[ni][2], U[ni][3]);
+                const float2 a0 = mul2(u0, ikt[ni]), a1 = mul2(u1, ikt[ni]);                // U / |k| for the O product
+                const float2 b0 = mul2(u0, dj2[ni]), b1 = mul2(u1, dj2[ni]);
+                ua[2 * ni] = pack_op<T>(a0.x, a0.y);
+                ua[2 * ni + 1] = pack_op<T>(a1.x, a1.y);
+                da[mi][2 * ni] = pack_op<T>(b0.x, b0.y);
+                da[mi][2 * ni + 1] = pack_op<T>(b1.x, b1.y);
             }
             // O^T = U^T M^T + diag(e) (Q S0)^T, stored times the output gate; sum(o^2) is taken before the gate
 #pragma unroll
@@ -475,21 +481,20 @@ gdn_scan_t_kernel(const uint8_t* __restrict__ ptb, const float* __restrict__ o_n
                 float O[4] = {0.0f, 0.0f, 0.0f, 0.0f};
                 mma16816<T>(O, ua, bm[ni][0], bm[ni][1]);
                 const int tok = 8 * ni + 2 * t;
-                const float o00 = O[0] + eq[ni][0] * QS[mi][ni][0], o01 = O[1] + eq[ni][1] * QS[mi][ni][1];
-                const float o10 = O[2] + eq[ni][0] * QS[mi][ni][2], o11 = O[3] + eq[ni][1] * QS[mi][ni][3];
-                const float2 g0 = h2_floats(gg[mi][ni]), g1 = h2_floats(gg[mi][ni + 2]);
-                otile[tok * OT_PITCH + r0] = o00 * g0.x;
-                otile[(tok + 1) * OT_PITCH + r0] = o01 * g0.y;
-                otile[tok * OT_PITCH + r1] = o10 * g1.x;
-                otile[(tok + 1) * OT_PITCH + r1] = o11 * g1.y;
-                sq[ni][0] = fmaf(o00, o00, fmaf(o10, o10, sq[ni][0]));
-                sq[ni][1] = fmaf(o01, o01, fmaf(o11, o11, sq[ni][1]));
+                const float2 o0 = fma2(eq[ni], make_float2(QS[mi][ni][0], QS[mi][ni][1]), make_float2(O[0], O[1]));
+                const float2 o1 = fma2(eq[ni], make_float2(QS[mi][ni][2], QS[mi][ni][3]), make_float2(O[2], O[3]));
+                const float2 y0 = mul2(o0, h2_floats(gg[mi][ni])), y1 = mul2(o1, h2_floats(gg[mi][ni + 2]));
+                otile[tok * OT_PITCH + r0] = y0.x;
+                otile[(tok + 1) * OT_PITCH + r0] = y0.y;
+                otile[tok * OT_PITCH + r1] = y1.x;
+                otile[(tok + 1) * OT_PITCH + r1] = y1.y;
+                sq[ni] = fma2(o0, o0, fma2(o1, o1, sq[ni]));
             }
         }
         SCAN_TICK(3);
         // ---------------------------------------------------------------- S^T <- e_last S^T + (diag(d) U)^T K
         {
-            const float elast = x.eg[TC - 1];
+            const float2 elast = make_float2(x.eg[TC - 1], x.eg[TC - 1]);
 #pragma unroll
             for (int nj = 0; nj < 8; ++nj) {
                 // keys 8 nj + g: fragment kf[nj / 2], row half nj % 2; tokens 2t, + 1 (b0) and 8 + 2t, + 1 (b1)
@@ -497,7 +502,10 @@ gdn_scan_t_kernel(const uint8_t* __restrict__ ptb, const float* __restrict__ o_n
 #pragma unroll
                 for (int mi = 0; mi < 2; ++mi) {
 #pragma unroll
-                    for (int e = 0; e < 4; ++e) S[mi][nj][e] *= elast;
+                    for (int e = 0; e < 4; e += 2) {
+                        const float2 v = mul2(make_float2(S[mi][nj][e], S[mi][nj][e + 1]), elast);
+                        S[mi][nj][e] = v.x; S[mi][nj][e + 1] = v.y;
+                    }
                     mma16816<T>(S[mi][nj], da[mi], b0, b1);
                 }
             }
@@ -508,7 +516,7 @@ gdn_scan_t_kernel(const uint8_t* __restrict__ ptb, const float* __restrict__ o_n
         for (int ni = 0; ni < 2; ++ni)
 #pragma unroll
             for (int e = 0; e < 2; ++e) {
-                float v = sq[ni][e];
+                float v = e ? sq[ni].y : sq[ni].x;
                 v += __shfl_xor_sync(0xffffffffu, v, 4);
                 v += __shfl_xor_sync(0xffffffffu, v, 8);
                 v += __shfl_xor_sync(0xffffffffu, v, 16);
