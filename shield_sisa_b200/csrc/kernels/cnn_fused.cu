@@ -472,8 +472,11 @@ se_gate_cluster_kernel(const float* __restrict__ sums, const float* __restrict__
 // rows, rounded to 16 bits, or already 16-bit.  A warp owns 16 rows and NT n tiles and is on its own: its A fragments come
 // straight from memory into registers (the k order inside an mma is permuted so that a lane's values are one 16-byte load;
 // the packed weights carry the same order), no shared memory, no barrier, STEP loads in flight.
-template <int NT, typename HT>
-__global__ void __launch_bounds__(128, NT > 14 ? 3 : 4)
+// AHEAD = 0: a warp takes all n tiles of its rows, their weights come as they are used.  AHEAD > 0, for few rows: the n tiles are
+// split over gridDim.y, and everything of a k step, weights included, is loaded AHEAD steps before it is used; the order of a
+// sum is the same.
+template <int NT, int AHEAD, typename HT>
+__global__ void __launch_bounds__(128, AHEAD > 0 ? 2 : NT > 14 ? 3 : 4)
 rows_gate_kernel(const float* __restrict__ A, const uint4* __restrict__ W, const float* __restrict__ bias, const float* __restrict__ gate,
                  int gate_rows, const float* R, float* out, int M, int N, int K) {
     constexpr int NP = (NT + 1) / 2;
@@ -500,27 +503,46 @@ rows_gate_kernel(const float* __restrict__ A, const uint4* __restrict__ W, const
         v[2] = in ? __ldg(reinterpret_cast<const float4*>(ga + k * 16)) : zero;
         v[3] = in ? __ldg(reinterpret_cast<const float4*>(gb + k * 16)) : zero;
     };
-    auto step = [&](const float4 (&v)[4], int k) {
+    auto weight = [&](int k, int n) { return __ldg(W + ((long long)k * npall + np0 + n) * 32 + lane); };
+    auto step = [&](const float4 (&v)[4], auto b_of) {
         uint32_t af[4];
         af[0] = Half<HT>::pack(v[0].x * v[2].x, v[0].y * v[2].y);
         af[1] = Half<HT>::pack(v[1].x * v[3].x, v[1].y * v[3].y);
         af[2] = Half<HT>::pack(v[0].z * v[2].z, v[0].w * v[2].w);
         af[3] = Half<HT>::pack(v[1].z * v[3].z, v[1].w * v[3].w);
-        const uint4* w = W + ((long long)k * npall + np0) * 32 + lane;
 #pragma unroll
         for (int n = 0; n < NP; ++n) {
-            const uint4 b = __ldg(w + n * 32);
+            const uint4 b = b_of(n);
             Half<HT>::mma(acc[2 * n], af, b.x, b.y);
             if (2 * n + 1 < NT) Half<HT>::mma(acc[2 * n + 1 < NT ? 2 * n + 1 : 0], af, b.z, b.w);
         }
     };
-    float4 v0[4], v1[4];
-    load(v0, 0);
-    for (int k = 0; k < kt; k += 2) {
-        load(v1, k + 1);
-        step(v0, k);
-        load(v0, k + 2);
-        if (k + 1 < kt) step(v1, k + 1);
+    if constexpr (AHEAD == 0) {
+        float4 v0[4], v1[4];
+        load(v0, 0);
+        for (int k = 0; k < kt; k += 2) {
+            load(v1, k + 1);
+            step(v0, [&](int n) { return weight(k, n); });
+            load(v0, k + 2);
+            if (k + 1 < kt) step(v1, [&](int n) { return weight(k + 1, n); });
+        }
+    } else {
+        float4 v[AHEAD > 0 ? AHEAD : 1][4];
+        uint4 w[AHEAD > 0 ? AHEAD : 1][NP];
+        auto fetch = [&](int d, int k) {
+            load(v[d], k);
+#pragma unroll
+            for (int n = 0; n < NP; ++n) w[d][n] = k < kt ? weight(k, n) : make_uint4(0u, 0u, 0u, 0u);
+        };
+#pragma unroll
+        for (int d = 0; d < AHEAD; ++d) fetch(d, d);
+        for (int k0 = 0; k0 < kt; k0 += AHEAD)
+#pragma unroll
+            for (int d = 0; d < AHEAD; ++d) {
+                if (k0 + d >= kt) break;
+                step(v[d], [&](int n) { return w[d][n]; });
+                fetch(d, k0 + d + AHEAD);
+            }
     }
 #pragma unroll
     for (int n = 0; n < NT; ++n) {
@@ -543,7 +565,7 @@ rows_gate_kernel(const float* __restrict__ A, const uint4* __restrict__ W, const
 }
 
 // the same with A already in the mode's 16-bit type [M][K], K a multiple of 32, no bias (the token projection)
-template <int NT, typename HT>
+template <int NT, int AHEAD, typename HT>
 __global__ void __launch_bounds__(128)
 rows_h_kernel(const uint16_t* __restrict__ A, const uint4* __restrict__ W, float* __restrict__ out, int M, int N, int K) {
     constexpr int NP = NT / 2;
@@ -559,27 +581,52 @@ rows_h_kernel(const uint16_t* __restrict__ A, const uint4* __restrict__ W, float
 #pragma unroll
         for (int e = 0; e < 4; ++e) acc[n][e] = 0.0f;
     const int ks = K / 32;
-    uint4 va = __ldg(reinterpret_cast<const uint4*>(pa)), vb = __ldg(reinterpret_cast<const uint4*>(pb));
-#pragma unroll 2
-    for (int k = 0; k < ks; ++k) {
-        const int kn = k + 1 < ks ? k + 1 : k;
-        const uint4 na = __ldg(reinterpret_cast<const uint4*>(pa + kn * 32)), nb = __ldg(reinterpret_cast<const uint4*>(pb + kn * 32));
-        const uint4* w = W + ((long long)k * 2 * npall + np0) * 32 + lane;
+    auto weight = [&](int k, int h, int n) { return __ldg(W + ((long long)(2 * k + h) * npall + np0 + n) * 32 + lane); };
+    auto step = [&](const uint4& va, const uint4& vb, auto b_of) {
         const uint32_t a0[4] = {va.x, vb.x, va.y, vb.y}, a1[4] = {va.z, vb.z, va.w, vb.w};
 #pragma unroll
         for (int n = 0; n < NP; ++n) {
-            const uint4 b = __ldg(w + n * 32);
+            const uint4 b = b_of(0, n);
             Half<HT>::mma(acc[2 * n], a0, b.x, b.y);
             Half<HT>::mma(acc[2 * n + 1], a0, b.z, b.w);
         }
 #pragma unroll
         for (int n = 0; n < NP; ++n) {
-            const uint4 b = __ldg(w + (npall + n) * 32);
+            const uint4 b = b_of(1, n);
             Half<HT>::mma(acc[2 * n], a1, b.x, b.y);
             Half<HT>::mma(acc[2 * n + 1], a1, b.z, b.w);
         }
-        va = na;
-        vb = nb;
+    };
+    if constexpr (AHEAD == 0) {
+        uint4 va = __ldg(reinterpret_cast<const uint4*>(pa)), vb = __ldg(reinterpret_cast<const uint4*>(pb));
+#pragma unroll 2
+        for (int k = 0; k < ks; ++k) {
+            const int kn = k + 1 < ks ? k + 1 : k;
+            const uint4 na = __ldg(reinterpret_cast<const uint4*>(pa + kn * 32)), nb = __ldg(reinterpret_cast<const uint4*>(pb + kn * 32));
+            step(va, vb, [&](int h, int n) { return weight(k, h, n); });
+            va = na;
+            vb = nb;
+        }
+    } else {
+        uint4 va[AHEAD > 0 ? AHEAD : 1], vb[AHEAD > 0 ? AHEAD : 1], w[AHEAD > 0 ? AHEAD : 1][2][NP];
+        auto fetch = [&](int d, int k) {
+            const int kc = min(k, ks - 1);
+            va[d] = __ldg(reinterpret_cast<const uint4*>(pa + kc * 32));
+            vb[d] = __ldg(reinterpret_cast<const uint4*>(pb + kc * 32));
+#pragma unroll
+            for (int h = 0; h < 2; ++h)
+#pragma unroll
+                for (int n = 0; n < NP; ++n) w[d][h][n] = weight(kc, h, n);
+        };
+#pragma unroll
+        for (int d = 0; d < AHEAD; ++d) fetch(d, d);
+        for (int k0 = 0; k0 < ks; k0 += AHEAD)
+#pragma unroll
+            for (int d = 0; d < AHEAD; ++d) {
+                if (k0 + d >= ks) break;
+                step(va[d], vb[d], [&](int h, int n) { return w[d][h][n]; });
+                fetch(d, k0 + d + AHEAD);
+            }
     }
 #pragma unroll
     for (int n = 0; n < NT; ++n) {
@@ -841,13 +888,20 @@ template <typename HT>
 int launch_rows_gate(const float* A, const uint4* W, const float* b, const float* gate, int gate_rows, const float* R, float* out, int M,
                      int N, int K, cudaStream_t s) {
     const unsigned gx = blocks_of(M, 64);
+    // Few rows: a warp's chain of k steps is all the time there is, so its loads run ahead and the n tiles go to other blocks.  us,
+    // whole / split: 160 channels of 960: 4 frames 41 / 15, 40 frames 64 / 18, 160 frames 64 / 43, 320 frames 75 / 87; 112 channels
+    // of 480: 4 frames 23 / 10, 40 frames 33 / 24, 80 frames 33 / 39 (300 row blocks).
+    const bool few = gx <= 160;
+    auto go = [&](auto kernel, unsigned gy) {
+        kernel<<<dim3(gx, gy), 128, 0, s>>>(A, W, b, gate, gate_rows, R, out, M, N, K);
+        return int(cudaGetLastError());
+    };
     switch (N) {
-    case 40: rows_gate_kernel<5, HT><<<gx, 128, 0, s>>>(A, W, b, gate, gate_rows, R, out, M, N, K); break;
-    case 112: rows_gate_kernel<14, HT><<<gx, 128, 0, s>>>(A, W, b, gate, gate_rows, R, out, M, N, K); break;
-    case 160: rows_gate_kernel<20, HT><<<gx, 128, 0, s>>>(A, W, b, gate, gate_rows, R, out, M, N, K); break;
+    case 40: return few ? go(rows_gate_kernel<5, 4, HT>, 1) : go(rows_gate_kernel<5, 0, HT>, 1);
+    case 112: return few ? go(rows_gate_kernel<2, 6, HT>, 7) : go(rows_gate_kernel<14, 0, HT>, 1);
+    case 160: return few ? go(rows_gate_kernel<4, 6, HT>, 5) : go(rows_gate_kernel<20, 0, HT>, 1);
     default: return int(cudaErrorInvalidValue);
     }
-    return int(cudaGetLastError());
 }
 }  // namespace
 }  // namespace sb
@@ -886,9 +940,13 @@ extern "C" int shvk_cnn_token_proj(const void* pooled, const void* W, float* tok
     const uint16_t* A = static_cast<const uint16_t*>(pooled);
     const uint4* w = static_cast<const uint4*>(W);
     cudaStream_t s = cudaStream_t(stream);
-    const dim3 grid(sb::blocks_of(rows, 64), 384 / 64);
-    if (dtype == sb::DT_BF16) sb::rows_h_kernel<8, __nv_bfloat16><<<grid, 128, 0, s>>>(A, w, tokens, rows, 384, 960);
-    else if (dtype == sb::DT_F16) sb::rows_h_kernel<8, __half><<<grid, 128, 0, s>>>(A, w, tokens, rows, 384, 960);
-    else return int(cudaErrorInvalidValue);
-    return int(cudaGetLastError());
+    const unsigned gx = sb::blocks_of(rows, 64);
+    const bool few = gx <= 80;          // as in launch_rows_gate: 4 frames 26 / 9 us, 40 frames 55 / 12, 320 frames 51 / 37
+    auto go = [&](auto kernel, unsigned gy) {
+        kernel<<<dim3(gx, gy), 128, 0, s>>>(A, w, tokens, rows, 384, 960);
+        return int(cudaGetLastError());
+    };
+    if (dtype == sb::DT_BF16) return few ? go(sb::rows_h_kernel<2, 8, __nv_bfloat16>, 24) : go(sb::rows_h_kernel<8, 0, __nv_bfloat16>, 6);
+    if (dtype == sb::DT_F16) return few ? go(sb::rows_h_kernel<2, 8, __half>, 24) : go(sb::rows_h_kernel<8, 0, __half>, 6);
+    return int(cudaErrorInvalidValue);
 }

@@ -355,6 +355,38 @@ _BLOCKS = [(16, 3, 16, 16, False, 1), (16, 3, 64, 24, False, 2), (24, 3, 72, 24,
 
 
 @pytest.mark.parametrize("dtype", [1, 2])
+@pytest.mark.parametrize("N,K", [(40, 72), (40, 120), (112, 480), (112, 672), (160, 672), (160, 960), (384, 960)])
+def test_row_kernels_split_by_channels_give_the_same_rows(L, N, K, dtype):
+    """The gated projection and (N = 384) the token projection split few rows by output channels and load ahead: the same bits as
+    the unsplit form of many rows, nothing written past the rows."""
+    import torch
+    rng = np.random.default_rng(N + K)
+    tdt = torch.bfloat16 if dtype == 1 else torch.float16
+    st = torch.cuda.current_stream().cuda_stream
+    big = 64 * 161 + 5
+    w = (rng.standard_normal((N, K)) / 16).astype(np.float32)
+    a = rng.standard_normal((big, K)).astype(np.float32)
+    outs = []
+    if N == 384:
+        A, P = torch.from_numpy(a).cuda().to(tdt), _pack(L, w, 2, dtype)
+    else:
+        A, P = torch.from_numpy(a).cuda(), _pack(L, w, 1, dtype, k_pad=(K + 15) // 16 * 16)
+        G = torch.rand((big + 59) // 60, K, device="cuda")
+        R, b = torch.randn(big, N, device="cuda"), torch.randn(N, device="cuda")
+    for m in (big, 5000, 77, 1):
+        out = torch.full((big, N), 9.0, device="cuda")
+        if N == 384:
+            assert L.shvk_cnn_token_proj(A.data_ptr(), P.data_ptr(), out.data_ptr(), m, dtype, st) == 0
+        else:
+            assert L.shvk_cnn_rows_gate(A.data_ptr(), P.data_ptr(), b.data_ptr(), G.data_ptr(), 60, R.data_ptr(), out.data_ptr(), m, N, K, dtype, st) == 0
+        torch.cuda.synchronize()
+        assert (out[m:] == 9.0).all()
+        outs.append(out[:m])
+    for o in outs[1:]:
+        assert torch.equal(o, outs[0][:len(o)])
+
+
+@pytest.mark.parametrize("dtype", [1, 2])
 @pytest.mark.parametrize("block", [2, 3, 4, 5, 7, 8, 9, 11, 12, 13, 14])
 def test_fused_block_matches_layers(L, block, dtype):
     """One fused block (expand + depthwise + project or pooled sums, gate, gated project) against the layer kernels on the same
