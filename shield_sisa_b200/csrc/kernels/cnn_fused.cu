@@ -401,7 +401,7 @@ stem_block_kernel(const uint8_t* __restrict__ frames, const float* __restrict__ 
 // layer (a warp per unit, lanes over the channels, a weight row read once for all G frames), hands it to the other seven
 // through distributed shared memory, and computes an eighth of the gates.  One block per frame read all 1.8 MB of the
 // widest layer's weights through one SM: 52 us however few the frames, 210 us at 640.
-template <int G>
+template <int G, int UNITS>
 __global__ void __cluster_dims__(8, 1, 1) __launch_bounds__(256)
 se_gate_cluster_kernel(const float* __restrict__ sums, const float* __restrict__ w1, const float* __restrict__ b1,
                        const float* __restrict__ w2, const float* __restrict__ b2, float* __restrict__ gate, int F, int tiles, float hw,
@@ -419,51 +419,73 @@ se_gate_cluster_kernel(const float* __restrict__ sums, const float* __restrict__
         pooled[i] = s / hw;
     }
     cluster_sync();                                                  // pooled is complete, and every block of the cluster runs
-    for (int j = rank * 8 + warp; j < CS; j += 64) {
-        float acc[G];
+    // UNITS outputs of a warp at a time, so that their weight loads fly together: with one, an output costs a round trip to L2
+    constexpr int UNROLL = UNITS == 1 ? 4 : 2;
+    for (int j0 = rank * 8 + warp; j0 < CS; j0 += 64 * UNITS) {
+        float acc[UNITS][G];
 #pragma unroll
-        for (int fr = 0; fr < G; ++fr) acc[fr] = 0.0f;
-#pragma unroll 4
+        for (int u = 0; u < UNITS; ++u)
+#pragma unroll
+            for (int fr = 0; fr < G; ++fr) acc[u][fr] = 0.0f;
+#pragma unroll UNROLL
         for (int c = lane * 4; c < C; c += 128) {
-            const float4 w = __ldg(reinterpret_cast<const float4*>(w1 + (long long)j * C + c));
+            float4 w[UNITS];
+#pragma unroll
+            for (int u = 0; u < UNITS; ++u) w[u] = __ldg(reinterpret_cast<const float4*>(w1 + (long long)min(j0 + 64 * u, CS - 1) * C + c));
 #pragma unroll
             for (int fr = 0; fr < G; ++fr) {
                 const float4 p = *reinterpret_cast<const float4*>(pooled + fr * C + c);
-                acc[fr] = fmaf(w.x, p.x, fmaf(w.y, p.y, fmaf(w.z, p.z, fmaf(w.w, p.w, acc[fr]))));
+#pragma unroll
+                for (int u = 0; u < UNITS; ++u) acc[u][fr] = fmaf(w[u].x, p.x, fmaf(w[u].y, p.y, fmaf(w[u].z, p.z, fmaf(w[u].w, p.w, acc[u][fr]))));
             }
         }
-        const float bj = b1[j];
 #pragma unroll
-        for (int fr = 0; fr < G; ++fr) {
-            const float v = fmaxf(warp_sum(acc[fr]) + bj, 0.0f);
-            if (lane < 8) {                                          // lane r stores into block r of the cluster
-                const uint32_t local = smem_addr(hid + fr * CS + j);
-                uint32_t remote;
-                asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote) : "r"(local), "r"(lane));
-                asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(remote), "f"(v) : "memory");
+        for (int u = 0; u < UNITS; ++u) {
+            const int j = j0 + 64 * u;
+            if (j >= CS) break;
+            const float bj = b1[j];
+#pragma unroll
+            for (int fr = 0; fr < G; ++fr) {
+                const float v = fmaxf(warp_sum(acc[u][fr]) + bj, 0.0f);
+                if (lane < 8) {                                      // lane r stores into block r of the cluster
+                    const uint32_t local = smem_addr(hid + fr * CS + j);
+                    uint32_t remote;
+                    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote) : "r"(local), "r"(lane));
+                    asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(remote), "f"(v) : "memory");
+                }
             }
         }
     }
     cluster_sync();
-    for (int c = rank * 8 + warp; c < C; c += 64) {
-        float acc[G];
+    for (int c0 = rank * 8 + warp; c0 < C; c0 += 64 * UNITS) {
+        float acc[UNITS][G];
 #pragma unroll
-        for (int fr = 0; fr < G; ++fr) acc[fr] = 0.0f;
+        for (int u = 0; u < UNITS; ++u)
+#pragma unroll
+            for (int fr = 0; fr < G; ++fr) acc[u][fr] = 0.0f;
 #pragma unroll 2
         for (int j = lane * 4; j < CS; j += 128) {
-            const float4 w = __ldg(reinterpret_cast<const float4*>(w2 + (long long)c * CS + j));
+            float4 w[UNITS];
+#pragma unroll
+            for (int u = 0; u < UNITS; ++u) w[u] = __ldg(reinterpret_cast<const float4*>(w2 + (long long)min(c0 + 64 * u, C - 1) * CS + j));
 #pragma unroll
             for (int fr = 0; fr < G; ++fr) {
                 const float4 p = *reinterpret_cast<const float4*>(hid + fr * CS + j);
-                acc[fr] = fmaf(w.x, p.x, fmaf(w.y, p.y, fmaf(w.z, p.z, fmaf(w.w, p.w, acc[fr]))));
+#pragma unroll
+                for (int u = 0; u < UNITS; ++u) acc[u][fr] = fmaf(w[u].x, p.x, fmaf(w[u].y, p.y, fmaf(w[u].z, p.z, fmaf(w[u].w, p.w, acc[u][fr]))));
             }
         }
 #pragma unroll
-        for (int fr = 0; fr < G; ++fr) acc[fr] = warp_sum(acc[fr]);
-        if (lane == 0)
+        for (int u = 0; u < UNITS; ++u) {
+            const int c = c0 + 64 * u;
+            if (c >= C) break;
 #pragma unroll
-            for (int fr = 0; fr < G; ++fr)
-                if (fr < nf) gate[(long long)(f0 + fr) * C + c] = __saturatef((acc[fr] + b2[c] + 3.0f) * (1.0f / 6.0f));
+            for (int fr = 0; fr < G; ++fr) acc[u][fr] = warp_sum(acc[u][fr]);
+            if (lane == 0)
+#pragma unroll
+                for (int fr = 0; fr < G; ++fr)
+                    if (fr < nf) gate[(long long)(f0 + fr) * C + c] = __saturatef((acc[u][fr] + b2[c] + 3.0f) * (1.0f / 6.0f));
+        }
     }
 }
 
@@ -877,9 +899,14 @@ extern "C" int shvk_cnn_se_gate_sums(const float* sums, const float* w1, const f
     if (smem > 48 * 1024) return int(cudaErrorInvalidValue);
     const unsigned grid = sb::blocks_of(F, G) * 8;
     cudaStream_t s = cudaStream_t(stream);
-    if (G == 1) sb::se_gate_cluster_kernel<1><<<grid, 256, smem, s>>>(sums, w1, b1, w2, b2, gate, F, tiles, float(HW), C, CS);
-    else sb::se_gate_cluster_kernel<4><<<grid, 256, smem, s>>>(sums, w1, b1, w2, b2, gate, F, tiles, float(HW), C, CS);
-    return int(cudaGetLastError());
+    // four outputs of a warp at a time while about two waves of clusters hold the frames (960 channels: 4 frames 26 -> 20 us, 40
+    // frames 51 -> 33, 100 frames 53 -> 34); beyond, other clusters hide the loads and the registers cost more than they bring (640 frames 133 against 161)
+    auto go = [&](auto kernel) {
+        kernel<<<grid, 256, smem, s>>>(sums, w1, b1, w2, b2, gate, F, tiles, float(HW), C, CS);
+        return int(cudaGetLastError());
+    };
+    if (G == 1) return go(sb::se_gate_cluster_kernel<1, 4>);
+    return grid <= 28 * 8 ? go(sb::se_gate_cluster_kernel<4, 4>) : go(sb::se_gate_cluster_kernel<4, 1>);
 }
 
 namespace sb {
