@@ -900,7 +900,8 @@ extern "C" int shvk_cnn_se_gate_sums(const float* sums, const float* w1, const f
     const unsigned grid = sb::blocks_of(F, G) * 8;
     cudaStream_t s = cudaStream_t(stream);
     // four outputs of a warp at a time while about two waves of clusters hold the frames (960 channels: 4 frames 26 -> 20 us, 40
-    // frames 51 -> 33, 100 frames 53 -> 34); beyond, other clusters hide the loads and the registers cost more than they bring (640 frames 133 against 161)
+    // frames 51 -> 33, 100 frames 53 -> 34); beyond, other clusters hide the loads and the registers cost more than they
+    // bring (640 frames 133 against 161)
     auto go = [&](auto kernel) {
         kernel<<<grid, 256, smem, s>>>(sums, w1, b1, w2, b2, gate, F, tiles, float(HW), C, CS);
         return int(cudaGetLastError());
