@@ -503,7 +503,8 @@ int launch_chunked(const void* q, const void* k, const void* v, const float* g, 
     // 18 sequences of 1,021 84 / 52 / 47; of 1,024: 36 85 / 54 / 48, 72 89 / 58 / 56, 144 106 / 90 / 113; 288 of 2,048 343 / 348 / 395.
     if (DK == 128 && 2 * seqs <= sms) return launch_scan<DK, TO, 1, 2, 4>(q, k, v, ws, o, B, T, H, NB, scale, s);
     if (seqs <= sms) return launch_scan<DK, TO, 1, 4, 4>(q, k, v, ws, o, B, T, H, NB, scale, s);
-    return launch_scan<DK, TO, DK == 64 ? 2 : 1, DK == 64 ? 4 : 8, 3>(q, k, v, ws, o, B, T, H, NB, scale, s);
+    // ring slots of a whole sequence, 3 / 4: 64 x 2,048, DK 64 248 / 254 us; 48 x 2,048, DK 128 314 / 309
+    return launch_scan<DK, TO, DK == 64 ? 2 : 1, DK == 64 ? 4 : 8, DK == 64 ? 3 : 4>(q, k, v, ws, o, B, T, H, NB, scale, s);
 }
 
 }  // namespace
