@@ -36,7 +36,7 @@ __device__ __forceinline__ float warp_max(float v) {
     return v;
 }
 
-// Two float32 FMAs / products in one instruction (each rounded as its scalar form rounds).
+// Two float32 FMAs / products / sums in one instruction (each rounded as its scalar form rounds).
 __device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
     float2 d;
     asm("fma.rn.f32x2 %0, %1, %2, %3;"
@@ -48,6 +48,13 @@ __device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
 __device__ __forceinline__ float2 mul2(float2 a, float2 b) {
     float2 d;
     asm("mul.rn.f32x2 %0, %1, %2;"
+        : "=l"(reinterpret_cast<unsigned long long&>(d))
+        : "l"(reinterpret_cast<unsigned long long&>(a)), "l"(reinterpret_cast<unsigned long long&>(b)));
+    return d;
+}
+__device__ __forceinline__ float2 add2(float2 a, float2 b) {
+    float2 d;
+    asm("add.rn.f32x2 %0, %1, %2;"
         : "=l"(reinterpret_cast<unsigned long long&>(d))
         : "l"(reinterpret_cast<unsigned long long&>(a)), "l"(reinterpret_cast<unsigned long long&>(b)));
     return d;

@@ -498,3 +498,92 @@ def test_fused_ends_of_the_encoder(L, dtype):
     sync()
     assert rel_err(low.float().cpu().numpy(), pooled.cpu().numpy()) < unit
     assert rel_err(tok2.cpu().numpy(), tok.cpu().numpy()) < unit
+
+
+def _block_both_ways(L, block, dtype, F, seed=0):
+    """Block `block` of the network on F frames of random maps, by the layer kernels and by the fused ones.  Returns (layers, fused),
+    each a dict of out (the block's map, or behind a gate the depthwise map) and, where the block has a gate, sums, gate and y (the
+    gated projection)."""
+    import torch
+    cin, k, cexp, cout, se, stride = _BLOCKS[block - 1]
+    H, W = 90, 160
+    for _cin, kk, *_r, st in _BLOCKS[:block - 1]:
+        H, W = (H + 2 * ((kk - 1) // 2) - kk) // st + 1, (W + 2 * ((kk - 1) // 2) - kk) // st + 1
+    pad = (k - 1) // 2
+    Ho, Wo = (H + 2 * pad - k) // stride + 1, (W + 2 * pad - k) // stride + 1
+    act = 1 if block < 7 else 2
+    gen = torch.Generator(device="cuda").manual_seed(100 * block + seed)
+    rn = lambda *s: torch.randn(*s, device="cuda", generator=gen)  # noqa: E731
+    zeros = lambda *s: torch.zeros(s, device="cuda")  # noqa: E731
+    x, we, be = 2 * rn(F, H, W, cin), rn(cexp, cin) / cin ** 0.5, rn(cexp)
+    wd, bd, wp, bp = rn(k * k, cexp) / k, rn(cexp), rn(cout, cexp) / cexp ** 0.5, rn(cout)
+    res = x if stride == 1 and cin == cout else None
+    E, a, f = zeros(F, H, W, cexp), {}, {}
+    dw = zeros(F, Ho, Wo, cexp)
+    assert L.shvk_cnn_pointwise_h(_ptr(x), _ptr(we), _ptr(be), None, 1, None, _ptr(E), F * H * W, cexp, cin, act, dtype, stream_ptr()) == 0
+    assert L.shvk_cnn_depthwise(_ptr(E), _ptr(wd), _ptr(bd), _ptr(dw), F, H, W, cexp, k, stride, Ho, Wo, act, stream_ptr()) == 0
+    if se:
+        cs = {72: 24, 120: 32, 480: 120, 672: 168, 960: 240}[cexp]
+        w1, b1, w2, b2 = rn(cs, cexp) / cexp ** 0.5, rn(cs), rn(cexp, cs) / cs ** 0.5, rn(cexp)
+        a["sums"] = zeros(F, L.shvk_cnn_se_partial_floats(1, Ho * Wo, cexp) // cexp, cexp)
+        a["gate"] = zeros(F, cexp)
+        assert L.shvk_cnn_se_gate(_ptr(dw), _ptr(a["sums"]), _ptr(w1), _ptr(b1), _ptr(w2), _ptr(b2), _ptr(a["gate"]), F, Ho * Wo, cexp, cs,
+                                  stream_ptr()) == 0
+    y = zeros(F, Ho, Wo, cout)
+    assert L.shvk_cnn_pointwise_h(_ptr(dw), _ptr(wp), _ptr(bp), _ptr(a["gate"]) if se else None, Ho * Wo, _ptr(res) if res is not None else None,
+                                  _ptr(y), F * Ho * Wo, cout, cexp, 0, dtype, stream_ptr()) == 0
+    a["out"] = dw if se else y
+    cols, kp = C.c_int(), C.c_int()
+    L.shvk_cnn_block_padding(block, C.byref(cols), C.byref(kp))
+    p_we, p_wp = _pack(L, we.cpu().numpy(), 0, dtype, cols.value), _pack(L, wp.cpu().numpy(), 1 if se else 0, dtype, None, kp.value)
+    tiles = L.shvk_cnn_block_tiles(block)
+    f["out"], f["sums"] = zeros(F, Ho, Wo, cexp if se else cout), torch.full((F, max(tiles, 1), cexp), float("nan"), device="cuda")
+    assert L.shvk_cnn_block(block, _ptr(x), _ptr(p_we), _ptr(be), _ptr(wd), _ptr(bd), None if se else _ptr(p_wp), None if se else _ptr(bp),
+                            _ptr(f["out"]), _ptr(f["sums"]), F, dtype, stream_ptr()) == 0
+    if se:
+        a["y"], f["y"], f["gate"] = y, zeros(F, Ho, Wo, cout), zeros(F, cexp)
+        assert L.shvk_cnn_se_gate_sums(_ptr(f["sums"]), _ptr(w1), _ptr(b1), _ptr(w2), _ptr(b2), _ptr(f["gate"]), F, tiles, Ho * Wo, cexp, cs,
+                                       stream_ptr()) == 0
+        assert L.shvk_cnn_rows_gate(_ptr(f["out"]), _ptr(p_wp), _ptr(bp), _ptr(f["gate"]), Ho * Wo, _ptr(res) if res is not None else None,
+                                    _ptr(f["y"]), F * Ho * Wo, cout, cexp, dtype, stream_ptr()) == 0
+    sync()
+    return a, f
+
+
+@pytest.mark.parametrize("dtype", [1, 2])
+@pytest.mark.parametrize("block", [2, 3, 4, 5, 7, 8, 9, 11, 12, 13, 14])
+def test_fused_block_gives_the_bits_of_the_layers(L, block, dtype):
+    """Expand, depthwise and (no gate between) projection in one kernel: every step rounds as the layer kernels round it, so the maps
+    are the same bits."""
+    import torch
+    a, f = _block_both_ways(L, block, dtype, 3)
+    assert torch.equal(f["out"], a["out"])
+
+
+@pytest.mark.parametrize("dtype", [1, 2])
+def test_fused_ends_give_the_bits_of_the_layers(L, dtype):
+    """Stem + block 1, and last convolution + pooling (rounded to the 16-bit type, as the token projection rounds its operand)."""
+    import torch
+    gen = torch.Generator(device="cuda").manual_seed(5)
+    rn = lambda *s: torch.randn(*s, device="cuda", generator=gen)  # noqa: E731
+    zeros = lambda *s: torch.zeros(s, device="cuda")  # noqa: E731
+    F, tdt = 3, torch.bfloat16 if dtype == 1 else torch.float16
+    frames = torch.randint(0, 256, (F, 180, 320, 3), device="cuda", generator=gen, dtype=torch.uint8)
+    lut, ws, bs, wd, bd, wp, bp = 1.3 * rn(3, 256), 0.3 * rn(27, 16), rn(16), rn(9, 16) / 3, rn(16), rn(16, 16) / 4, rn(16)
+    s, dw, y, out = zeros(F, 90, 160, 16), zeros(F, 90, 160, 16), zeros(F, 90, 160, 16), zeros(F, 90, 160, 16)
+    assert L.shvk_cnn_stem(_ptr(frames), _ptr(lut), _ptr(ws), _ptr(bs), _ptr(s), F, stream_ptr()) == 0
+    assert L.shvk_cnn_depthwise(_ptr(s), _ptr(wd), _ptr(bd), _ptr(dw), F, 90, 160, 16, 3, 1, 90, 160, 1, stream_ptr()) == 0
+    assert L.shvk_cnn_pointwise_h(_ptr(dw), _ptr(wp), _ptr(bp), None, 1, _ptr(s), _ptr(y), F * 14400, 16, 16, 0, dtype, stream_ptr()) == 0
+    p_wp, h_ws, h_bs = _pack(L, wp.cpu().numpy(), 0, dtype), ws.cpu().numpy(), bs.cpu().numpy()
+    assert L.shvk_cnn_stem_block(_ptr(frames), _ptr(lut), h_ws.ctypes.data, h_bs.ctypes.data, _ptr(wd), _ptr(bd), _ptr(p_wp), _ptr(bp),
+                                 _ptr(out), F, dtype, stream_ptr()) == 0
+    sync()
+    assert torch.equal(out, y)
+    x, wl, bl = 2 * rn(F, 60, 160), rn(960, 160) / 160 ** 0.5, rn(960)
+    fmap, pooled, low = zeros(F, 60, 960), zeros(F, 16, 960), torch.zeros((F, 16, 960), device="cuda", dtype=tdt)
+    assert L.shvk_cnn_pointwise_h(_ptr(x), _ptr(wl), _ptr(bl), None, 1, None, _ptr(fmap), F * 60, 960, 160, 2, dtype, stream_ptr()) == 0
+    assert L.shvk_cnn_pool_tokens(_ptr(fmap), _ptr(pooled), F, stream_ptr()) == 0
+    p_wl = _pack(L, wl.cpu().numpy(), 0, dtype)
+    assert L.shvk_cnn_last_pool(_ptr(x), _ptr(p_wl), _ptr(bl), _ptr(low), F, dtype, stream_ptr()) == 0
+    sync()
+    assert torch.equal(low, pooled.to(tdt))
