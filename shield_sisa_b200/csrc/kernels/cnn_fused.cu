@@ -594,7 +594,11 @@ rows_gate_kernel(const float* __restrict__ A, const uint4* __restrict__ W, const
     }
 }
 
-// the same with A already in the mode's 16-bit type [M][K], K a multiple of 32, no bias (the token projection)
+// The same with A already in the mode's 16-bit type [M][K], K a multiple of 32, no bias (the token projection).  A lane loads 16
+// bytes, eight values of k; the first of two mma must have the lower sixteen of their 32 k, as in the layer kernel (which k share an
+// mma shows in the rounding, their order in it does not), so lanes t and t + 2 exchange 8 bytes: 4 frames
+// 5.1 us, 80 frames 12.8, 320 frames 35.7, 640 frames 41.9 (k permuted over both mma instead 4.6, 11.4, 31.6, 45.9; 8-byte loads 5.5,
+// 16.1, 47.9, 50.7).
 template <int NT, int AHEAD, typename HT>
 __global__ void __launch_bounds__(128)
 rows_h_kernel(const uint16_t* __restrict__ A, const uint4* __restrict__ W, float* __restrict__ out, int M, int N, int K) {
@@ -612,7 +616,14 @@ rows_h_kernel(const uint16_t* __restrict__ A, const uint4* __restrict__ W, float
         for (int e = 0; e < 4; ++e) acc[n][e] = 0.0f;
     const int ks = K / 32;
     auto weight = [&](int k, int h, int n) { return __ldg(W + ((long long)(2 * k + h) * npall + np0 + n) * 32 + lane); };
-    auto step = [&](const uint4& va, const uint4& vb, auto b_of) {
+    const bool upper = (t & 2) != 0;
+    // .x, .y: the lane's operand of the first mma, .z, .w: of the second
+    auto exchange = [&](const uint4& v) {
+        const uint32_t r0 = __shfl_xor_sync(0xffffffffu, upper ? v.x : v.z, 2), r1 = __shfl_xor_sync(0xffffffffu, upper ? v.y : v.w, 2);
+        return upper ? make_uint4(r0, r1, v.z, v.w) : make_uint4(v.x, v.y, r0, r1);
+    };
+    auto step = [&](const uint4& ra, const uint4& rb, auto b_of) {
+        const uint4 va = exchange(ra), vb = exchange(rb);
         const uint32_t a0[4] = {va.x, vb.x, va.y, vb.y}, a1[4] = {va.z, vb.z, va.w, vb.w};
 #pragma unroll
         for (int n = 0; n < NP; ++n) {
@@ -821,8 +832,9 @@ void block_padding(int block, int* cols, int* k) {
 }  // namespace sb
 
 // Host side: W [N][K] float32 -> 16-bit mma fragments.  order 0: fragments [n tile][k tile][lane] of 4 values, k as the
-// instruction numbers it; order 1 / 2: [k tile][pair of n tiles][lane] of 8 values, k permuted so that a lane's operand A is
-// four (1) or, over two k tiles, eight (2) consecutive values of a row.
+// instruction numbers it; order 1 / 2: [k tile][pair of n tiles][lane] of 8 values, k permuted inside a k tile so that a lane's
+// operand A is four consecutive values of a row (1), or what it has of a tile after the exchange of rows_h_kernel (2: an even
+// number of k tiles).
 extern "C" size_t shvk_cnn_packed_bytes(int N, int K, int order) {
     if (N <= 0 || K <= 0 || order < 0 || order > 2) return 0;
     const size_t kt = size_t(order == 2 ? (K + 31) / 32 * 2 : (K + 15) / 16);
@@ -853,8 +865,8 @@ extern "C" int shvk_cnn_pack_weights(const float* w, int N, int K, int order, in
                 for (int lane = 0; lane < 32; ++lane)
                     for (int e = 0; e < 8; ++e) {
                         const int n = np * 16 + (e / 4) * 8 + lane / 4;
-                        const int k = order == 1 ? kt * 16 + (lane % 4) * 4 + e % 4 : (kt / 2) * 32 + (lane % 4) * 8 + (kt % 2) * 4 + e % 4;
-                        put(n, k);
+                        const int t = lane % 4, quad = order == 1 ? t : (t & 1) * 2 + (t >> 1);
+                        put(n, kt * 16 + quad * 4 + e % 4);
                     }
     }
     return 0;

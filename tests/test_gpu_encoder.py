@@ -587,3 +587,20 @@ def test_fused_ends_give_the_bits_of_the_layers(L, dtype):
     assert L.shvk_cnn_last_pool(_ptr(x), _ptr(p_wl), _ptr(bl), _ptr(low), F, dtype, stream_ptr()) == 0
     sync()
     assert torch.equal(low, pooled.to(tdt))
+
+
+@pytest.mark.parametrize("dtype", [1, 2])
+@pytest.mark.parametrize("rows", [16, 80, 77, 5136])
+def test_token_projection_gives_the_bits_of_the_layer(L, rows, dtype):
+    """The token projection sums 16 values of k to an mma in ascending order, in both its forms (rows up to 5,120 split by channels), as the
+    16-bit 1x1 layer does."""
+    import torch
+    tdt = torch.bfloat16 if dtype == 1 else torch.float16
+    gen = torch.Generator(device="cuda").manual_seed(rows)
+    a, w = (torch.randn(n, 960, device="cuda", generator=gen) for n in (rows, 384))
+    low, got, want = a.to(tdt), torch.zeros(rows, 384, device="cuda"), torch.zeros(rows, 384, device="cuda")
+    p_w = _pack(L, w.cpu().numpy(), 2, dtype)
+    assert L.shvk_cnn_token_proj(_ptr(low), _ptr(p_w), _ptr(got), rows, dtype, stream_ptr()) == 0
+    assert L.shvk_cnn_pointwise_h(_ptr(a), _ptr(w), None, None, 1, None, _ptr(want), rows, 384, 960, 0, dtype, stream_ptr()) == 0
+    sync()
+    assert torch.equal(got, want)
