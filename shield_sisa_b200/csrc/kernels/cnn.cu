@@ -11,6 +11,7 @@
 #include <string>
 
 namespace sb {
+size_t se_gate_frame_bytes(int C, int CS);       // cnn_fused.cu
 namespace {
 
 constexpr int kImgH = 180, kImgW = 320, kStemH = 90, kStemW = 160, kStemC = 16, kMapH = 6, kMapW = 10, kMapC = 960;
@@ -673,9 +674,9 @@ extern "C" int shvk_cnn_se_gate(const float* x, float* partial, const float* w1,
     const size_t smem = size_t(C + CS) * sizeof(float);
     if (smem > 48 * 1024) return int(cudaErrorInvalidValue);
     // the gate itself on clusters of eight blocks (cnn_fused.cu: a weight row is read once for four frames, and an eighth of
-    // them by a block) where its 128-bit loads and its shared memory allow: both launches, 960 channels, one block a frame /
-    // clusters: 4 frames 52 / 30 us, 75 frames 91 / 58, 300 frames (4 to a cluster) 83
-    if ((CS & 3) == 0 && !sb::misaligned(w1) && !sb::misaligned(w2) && 4 * smem <= 48 * 1024)
+    // them by a block; the same bits) where four frames fit its shared memory: both launches, 960 channels, one block a frame /
+    // clusters: 4 frames 52 / 16 us, 75 frames 91 / 34, 300 frames (4 to a cluster) 71
+    if (4 * sb::se_gate_frame_bytes(C, CS) <= 48 * 1024)
         return shvk_cnn_se_gate_sums(partial, w1, b1, w2, b2, gate, F, S, HW, C, CS, stream);
     sb::se_gate_kernel<<<unsigned(F), 1024, smem, s>>>(partial, w1, b1, w2, b2, gate, HW, C, CS, S);
     return int(cudaGetLastError());

@@ -19,6 +19,7 @@
 #include "shv_cnn_kernels.h"
 
 namespace sb {
+size_t se_gate_frame_bytes(int C, int CS);       // shared memory of a frame in the gate's cluster form (asked by cnn.cu too)
 namespace {
 
 // x * relu6(x + 3) / 6 of a pair, each step rounded as cnn.cu rounds it.  The quotient is a product and an FMA with 1/6 in two
@@ -408,15 +409,61 @@ stem_block_kernel(const uint8_t* __restrict__ frames, const float* __restrict__ 
 // A cluster of eight blocks takes G frames.  Every block reduces the frames' pooled sums, computes an eighth of the hidden
 // layer (a warp per unit, lanes over the channels, a weight row read once for all G frames), hands it to the other seven
 // through distributed shared memory, and computes an eighth of the gates.  One block per frame read all 1.8 MB of the
-// widest layer's weights through one SM: 52 us however few the frames, 210 us at 640.
+// widest layer's weights through one SM: 52 us however few the frames, 210 us at 640; now 13 us and 109.
+//
+// Sums and roundings are those of se_gate_kernel: an output is a warp's, lane l sums the inputs l, l + 32, ... in order, then the
+// lanes are added.  So weights come as coalesced 4-byte loads; the frames of a cluster lie next to each other in shared memory,
+// one 128-bit read for all four.
+template <int G> __device__ __forceinline__ void load_frames(const float* p, float (&v)[G]) {
+    if constexpr (G == 4) {
+        const float4 q = *reinterpret_cast<const float4*>(p);
+        v[0] = q.x; v[1] = q.y; v[2] = q.z; v[3] = q.w;
+    } else {
+#pragma unroll
+        for (int i = 0; i < G; ++i) v[i] = p[i];
+    }
+}
+// acc[u][fr] = sum over k of W[rows u][k] x[k][fr], each lane its share of k.  x has zeros up to a multiple of 32 GATE_BATCH, so that
+// every batch is whole: the weights of GATE_BATCH steps are loaded before the first is used (an output is a chain of round trips
+// to L2), and nothing is asked between the sums.
+constexpr int GATE_BATCH = 8;
+__host__ __device__ constexpr int gate_rows_padded(int k) { return up(k, 32 * GATE_BATCH); }
+template <int G, int UNITS>
+__device__ __forceinline__ void lane_sums(const float* __restrict__ W, int K, const int (&row)[UNITS], const float* x, int lane, float (&acc)[UNITS][G]) {
+    const float* w[UNITS];
+#pragma unroll
+    for (int u = 0; u < UNITS; ++u) {
+        w[u] = W + (long long)row[u] * K;
+#pragma unroll
+        for (int fr = 0; fr < G; ++fr) acc[u][fr] = 0.0f;
+    }
+#pragma unroll 1
+    for (int k0 = lane; k0 < gate_rows_padded(K); k0 += 32 * GATE_BATCH) {
+        float wv[GATE_BATCH][UNITS];
+#pragma unroll
+        for (int d = 0; d < GATE_BATCH; ++d)
+#pragma unroll
+            for (int u = 0; u < UNITS; ++u) wv[d][u] = k0 + 32 * d < K ? __ldg(w[u] + k0 + 32 * d) : 0.0f;
+#pragma unroll
+        for (int d = 0; d < GATE_BATCH; ++d) {
+            float p[G];
+            load_frames<G>(x + (k0 + 32 * d) * G, p);
+#pragma unroll
+            for (int u = 0; u < UNITS; ++u)
+#pragma unroll
+                for (int fr = 0; fr < G; ++fr) acc[u][fr] = fmaf(wv[d][u], p[fr], acc[u][fr]);
+        }
+    }
+}
 template <int G, int UNITS>
 __global__ void __cluster_dims__(8, 1, 1) __launch_bounds__(256)
 se_gate_cluster_kernel(const float* __restrict__ sums, const float* __restrict__ w1, const float* __restrict__ b1,
                        const float* __restrict__ w2, const float* __restrict__ b2, float* __restrict__ gate, int F, int tiles, float hw,
                        int C, int CS) {
     extern __shared__ __align__(16) uint8_t smem[];
-    float* const pooled = reinterpret_cast<float*>(smem);           // [G][C]
-    float* const hid = pooled + G * C;                               // [G][CS]
+    const int CP = gate_rows_padded(C), CSP = gate_rows_padded(CS);
+    float* const pooled = reinterpret_cast<float*>(smem);           // [CP][G]
+    float* const hid = pooled + G * CP;                              // [CSP][G]
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, rank = blockIdx.x & 7;
     const int f0 = int(blockIdx.x >> 3) * G, nf = min(G, F - f0);
     for (int i = tid; i < G * C; i += 256) {
@@ -424,29 +471,18 @@ se_gate_cluster_kernel(const float* __restrict__ sums, const float* __restrict__
         float s = 0.0f;
         if (fr < nf)
             for (int k = 0; k < tiles; ++k) s += sums[((long long)(f0 + fr) * tiles + k) * C + c];
-        pooled[i] = s / hw;
+        pooled[c * G + fr] = s / hw;
     }
+    for (int i = G * C + tid; i < G * CP; i += 256) pooled[i] = 0.0f;
+    for (int i = G * CS + tid; i < G * CSP; i += 256) hid[i] = 0.0f;
     cluster_sync();                                                  // pooled is complete, and every block of the cluster runs
     // UNITS outputs of a warp at a time, so that their weight loads fly together: with one, an output costs a round trip to L2
-    constexpr int UNROLL = UNITS == 1 ? 4 : 2;
     for (int j0 = rank * 8 + warp; j0 < CS; j0 += 64 * UNITS) {
+        int row[UNITS];
         float acc[UNITS][G];
 #pragma unroll
-        for (int u = 0; u < UNITS; ++u)
-#pragma unroll
-            for (int fr = 0; fr < G; ++fr) acc[u][fr] = 0.0f;
-#pragma unroll UNROLL
-        for (int c = lane * 4; c < C; c += 128) {
-            float4 w[UNITS];
-#pragma unroll
-            for (int u = 0; u < UNITS; ++u) w[u] = __ldg(reinterpret_cast<const float4*>(w1 + (long long)min(j0 + 64 * u, CS - 1) * C + c));
-#pragma unroll
-            for (int fr = 0; fr < G; ++fr) {
-                const float4 p = *reinterpret_cast<const float4*>(pooled + fr * C + c);
-#pragma unroll
-                for (int u = 0; u < UNITS; ++u) acc[u][fr] = fmaf(w[u].x, p.x, fmaf(w[u].y, p.y, fmaf(w[u].z, p.z, fmaf(w[u].w, p.w, acc[u][fr]))));
-            }
-        }
+        for (int u = 0; u < UNITS; ++u) row[u] = min(j0 + 64 * u, CS - 1);
+        lane_sums<G, UNITS>(w1, C, row, pooled, lane, acc);
 #pragma unroll
         for (int u = 0; u < UNITS; ++u) {
             const int j = j0 + 64 * u;
@@ -456,7 +492,7 @@ se_gate_cluster_kernel(const float* __restrict__ sums, const float* __restrict__
             for (int fr = 0; fr < G; ++fr) {
                 const float v = fmaxf(warp_sum(acc[u][fr]) + bj, 0.0f);
                 if (lane < 8) {                                      // lane r stores into block r of the cluster
-                    const uint32_t local = smem_addr(hid + fr * CS + j);
+                    const uint32_t local = smem_addr(hid + j * G + fr);
                     uint32_t remote;
                     asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote) : "r"(local), "r"(lane));
                     asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(remote), "f"(v) : "memory");
@@ -466,23 +502,11 @@ se_gate_cluster_kernel(const float* __restrict__ sums, const float* __restrict__
     }
     cluster_sync();
     for (int c0 = rank * 8 + warp; c0 < C; c0 += 64 * UNITS) {
+        int row[UNITS];
         float acc[UNITS][G];
 #pragma unroll
-        for (int u = 0; u < UNITS; ++u)
-#pragma unroll
-            for (int fr = 0; fr < G; ++fr) acc[u][fr] = 0.0f;
-#pragma unroll 2
-        for (int j = lane * 4; j < CS; j += 128) {
-            float4 w[UNITS];
-#pragma unroll
-            for (int u = 0; u < UNITS; ++u) w[u] = __ldg(reinterpret_cast<const float4*>(w2 + (long long)min(c0 + 64 * u, C - 1) * CS + j));
-#pragma unroll
-            for (int fr = 0; fr < G; ++fr) {
-                const float4 p = *reinterpret_cast<const float4*>(hid + fr * CS + j);
-#pragma unroll
-                for (int u = 0; u < UNITS; ++u) acc[u][fr] = fmaf(w[u].x, p.x, fmaf(w[u].y, p.y, fmaf(w[u].z, p.z, fmaf(w[u].w, p.w, acc[u][fr]))));
-            }
-        }
+        for (int u = 0; u < UNITS; ++u) row[u] = min(c0 + 64 * u, C - 1);
+        lane_sums<G, UNITS>(w2, CS, row, hid, lane, acc);
 #pragma unroll
         for (int u = 0; u < UNITS; ++u) {
             const int c = c0 + 64 * u;
@@ -492,7 +516,7 @@ se_gate_cluster_kernel(const float* __restrict__ sums, const float* __restrict__
             if (lane == 0)
 #pragma unroll
                 for (int fr = 0; fr < G; ++fr)
-                    if (fr < nf) gate[(long long)(f0 + fr) * C + c] = __saturatef((acc[u][fr] + b2[c] + 3.0f) * (1.0f / 6.0f));
+                    if (fr < nf) gate[(long long)(f0 + fr) * C + c] = fminf(fmaxf(acc[u][fr] + b2[c] + 3.0f, 0.0f), 6.0f) / 6.0f;
         }
     }
 }
@@ -908,26 +932,27 @@ extern "C" int shvk_cnn_stem_block(const uint8_t* frames, const float* lut, cons
     return dtype == sb::DT_BF16 ? go(sb::stem_block_kernel<__nv_bfloat16>) : go(sb::stem_block_kernel<__half>);
 }
 
+size_t sb::se_gate_frame_bytes(int C, int CS) { return size_t(gate_rows_padded(C) + gate_rows_padded(CS)) * sizeof(float); }
+
 extern "C" int shvk_cnn_se_gate_sums(const float* sums, const float* w1, const float* b1, const float* w2, const float* b2, float* gate,
                                      int F, int tiles, int HW, int C, int CS, void* stream) {
     if (F <= 0) return 0;
-    if (!sums || tiles <= 0 || HW <= 0 || C <= 0 || CS <= 0 || (C & 3) || (CS & 3) || sb::unaligned(w1) || sb::unaligned(w2))
-        return int(cudaErrorInvalidValue);
-    // frames per cluster: one while that leaves the GPU a wave of blocks or less, else four (a weight row serves four frames)
-    const int G = F <= 37 ? 1 : 4;
-    const size_t smem = size_t(G) * size_t(C + CS) * sizeof(float);
+    if (!sums || tiles <= 0 || HW <= 0 || C <= 0 || CS <= 0 || (C & 3)) return int(cudaErrorInvalidValue);
+    // Frames per cluster: one while that gives an SM three blocks or fewer (960 channels, one / four: 56 frames 18.7 / 27 us, 75 frames
+    // 29.8 / 29.8, 112 frames 33 / 30), else four (a weight row serves four frames)
+    const int sms = sb::device_sms(), G = 8LL * F <= 3 * sms ? 1 : 4;
+    const size_t smem = size_t(G) * sb::se_gate_frame_bytes(C, CS);
     if (smem > 48 * 1024) return int(cudaErrorInvalidValue);
     const unsigned grid = sb::blocks_of(F, G) * 8;
     cudaStream_t s = cudaStream_t(stream);
-    // four outputs of a warp at a time while about two waves of clusters hold the frames (960 channels: 4 frames 26 -> 20 us, 40
-    // frames 51 -> 33, 100 frames 53 -> 34); beyond, other clusters hide the loads and the registers cost more than they
-    // bring (640 frames 133 against 161)
+    // Four outputs of a warp at a time up to two blocks an SM (960 channels, four / one: 75 frames 29.7 / 33.6 us, 130 frames 31.7 / 36.6);
+    // beyond, other clusters hide the loads and the narrow maps pay for the registers (120 channels, 300 frames 14.1 / 11.4)
     auto go = [&](auto kernel) {
         kernel<<<grid, 256, smem, s>>>(sums, w1, b1, w2, b2, gate, F, tiles, float(HW), C, CS);
         return int(cudaGetLastError());
     };
     if (G == 1) return go(sb::se_gate_cluster_kernel<1, 4>);
-    return grid <= 28 * 8 ? go(sb::se_gate_cluster_kernel<4, 4>) : go(sb::se_gate_cluster_kernel<4, 1>);
+    return grid <= 2u * sms ? go(sb::se_gate_cluster_kernel<4, 4>) : go(sb::se_gate_cluster_kernel<4, 1>);
 }
 
 namespace sb {

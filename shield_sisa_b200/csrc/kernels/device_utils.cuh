@@ -36,6 +36,14 @@ __device__ __forceinline__ float warp_max(float v) {
     return v;
 }
 
+// SMs of the current device (host code: launch rules are stated in blocks per SM)
+inline int device_sms() {
+    int dev = 0, sms = 148;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    return sms;
+}
+
 // Two float32 FMAs / products / sums in one instruction (each rounded as its scalar form rounds).
 __device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
     float2 d;

@@ -477,13 +477,6 @@ int choose_bn(int n) {
     return best;
 }
 
-int device_sms() {
-    int dev = 0, sms = 148;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    return sms;
-}
-
 // Accumulator width of one launch.  With tiles for every SM many times over it is the plan's: what counts is the time of a
 // row block.  While the plan's width gives no more than two tiles per SM, what counts is the longest chain of one SM: tiles
 // per SM times (k steps, and filling the ring and draining the last accumulator: about 600 + 8 bn cycles), and a narrower

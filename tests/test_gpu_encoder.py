@@ -604,3 +604,34 @@ def test_token_projection_gives_the_bits_of_the_layer(L, rows, dtype):
     assert L.shvk_cnn_pointwise_h(_ptr(a), _ptr(w), None, None, 1, None, _ptr(want), rows, 384, 960, 0, dtype, stream_ptr()) == 0
     sync()
     assert torch.equal(got, want)
+
+
+@pytest.mark.parametrize("Cn,CS", [(72, 24), (120, 32), (480, 120), (672, 168), (960, 240), (64, 18)])
+def test_se_gate_forms_give_the_same_bits(L, Cn, CS):
+    """A gate comes from a cluster of blocks while four frames fit its shared memory (below 3,072 channels in both layers), else from one block.
+    Channels of zeros take the same layer to the second form: the same bits.  Frame counts: one and four frames a cluster, the last
+    one partly filled, one and four outputs of a warp at a time."""
+    import torch
+    HW, wide, Fmax = 60, 3072, 151
+    gen = torch.Generator(device="cuda").manual_seed(Cn)
+    rn = lambda *s: torch.randn(*s, device="cuda", generator=gen)  # noqa: E731
+    x, w1, b1, w2, b2 = rn(Fmax, HW, Cn), rn(CS, Cn) / Cn ** 0.5, rn(CS), rn(Cn, CS) / CS ** 0.5, rn(Cn)
+
+    def pad(t, *shape):
+        out = torch.zeros(shape, device="cuda")
+        out[tuple(slice(0, n) for n in t.shape)] = t
+        return out
+
+    big = (pad(x, Fmax, HW, wide), pad(w1, CS, wide), b1, pad(w2, wide, CS), pad(b2, wide))
+
+    def gate(args, F, ch):
+        x_, w1_, b1_, w2_, b2_ = args
+        part, out = torch.zeros(L.shvk_cnn_se_partial_floats(F, HW, ch), device="cuda"), torch.full((Fmax, ch), 9.0, device="cuda")
+        assert L.shvk_cnn_se_gate(_ptr(x_), _ptr(part), _ptr(w1_), _ptr(b1_), _ptr(w2_), _ptr(b2_), _ptr(out), F, HW, ch, CS, stream_ptr()) == 0
+        sync()
+        assert (out[F:] == 9.0).all()
+        return out[:F, :Cn]
+
+    want = gate(big, Fmax, wide)
+    for F in (1, 3, 55, 57, 75, 148, Fmax):
+        assert torch.equal(gate((x, w1, b1, w2, b2), F, Cn), want[:F])
