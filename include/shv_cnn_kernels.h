@@ -112,11 +112,12 @@ int shvk_cnn_stem_block(const uint8_t* frames, const float* lut, const float* st
 
 /* Inverted-residual block 2 .. 15: 1x1 expand + activation, depthwise + activation, and, where the block has no
  * squeeze-excite gate (2, 3, 7 .. 10), 1x1 project (+ x where shapes agree) -> out [F][h][w][C].  Where it has one, out is
- * the depthwise map [F][h][w][expanded] and sums [F][tiles][expanded] its sums over the tiles of the map
- * (shvk_cnn_block_tiles, 0 for blocks without a gate).  out must not be x.  Weights are packed with zero rows / columns up
+ * the depthwise map [F][h][w][expanded] and sums [F][tiles][expanded] its sums over groups of 64 pixels in row
+ * order, the partial sums of shvk_cnn_se_gate (shvk_cnn_block_tiles groups, 0 for blocks without a gate).  out must not be x.  Weights are packed with zero rows / columns up
  * to shvk_cnn_block_padding: expand [columns][in], project [out][k].
  * Replaces gemm, launch_dw, launch_se_pool and gemm of a block (engine/cuda/engine.cu:349-395). */
 int shvk_cnn_block_tiles(int block);
+int shvk_cnn_block_launches(int block);      /* kernels per call */
 void shvk_cnn_block_padding(int block, int* columns, int* k);
 int shvk_cnn_block(int block, const float* x, const void* we, const float* be, const float* wd, const float* bd, const void* wp,
                    const float* bp, float* out, float* sums, int F, int dtype, void* stream);

@@ -180,6 +180,7 @@ def load_library(experimental: bool = True) -> C.CDLL:
         "shvk_cnn_pack_weights": (i32, [vp, i32, i32, i32, i32, vp]),
         "shvk_cnn_stem_block": (i32, [vp] * 9 + [i32, i32, vp]),
         "shvk_cnn_block_tiles": (i32, [i32]),
+        "shvk_cnn_block_launches": (i32, [i32]),
         "shvk_cnn_block_padding": (None, [i32, C.POINTER(i32), C.POINTER(i32)]),
         "shvk_cnn_block": (i32, [i32] + [vp] * 9 + [i32, i32, vp]),
         "shvk_cnn_se_gate_sums": (i32, [vp] * 6 + [i32] * 5 + [vp]),

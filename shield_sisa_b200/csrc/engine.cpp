@@ -238,7 +238,7 @@ public:
     int launches_per_encode() const override {
         if (prec_ != Precision::FP32) {
             int n = 1 + 2;                               // stem + block 1; last conv + pooling, token projection
-            for (int i = 1; i < 15; ++i) n += 1 + (cnn_.blocks[i].se ? 2 : 0);
+            for (int i = 1; i < 15; ++i) n += shvk_cnn_block_launches(i + 1) + (cnn_.blocks[i].se ? 2 : 0);
             return n;
         }
         int n = 4;                                       // stem, last conv, pooling, token projection

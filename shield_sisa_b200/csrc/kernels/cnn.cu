@@ -12,6 +12,7 @@
 
 namespace sb {
 size_t se_gate_frame_bytes(int C, int CS);       // cnn_fused.cu
+int se_partial_sums(const float* x, float* partial, int F, int HW, int C, cudaStream_t s);
 namespace {
 
 constexpr int kImgH = 180, kImgW = 320, kStemH = 90, kStemW = 160, kStemC = 16, kMapH = 6, kMapW = 10, kMapC = 960;
@@ -655,6 +656,12 @@ extern "C" int shvk_cnn_depthwise(const float* in, const float* w, const float* 
     return int(cudaGetLastError());
 }
 
+int sb::se_partial_sums(const float* x, float* partial, int F, int HW, int C, cudaStream_t s) {
+    const int S = (HW + kSeGroup - 1) / kSeGroup;
+    se_partial_kernel<<<dim3(unsigned(F), unsigned(S), unsigned((C + 127) / 128)), 256, 0, s>>>(x, partial, HW, C, S);
+    return int(cudaGetLastError());
+}
+
 extern "C" size_t shvk_cnn_se_partial_floats(int F, int HW, int C) {
     if (F <= 0 || HW <= 0 || C <= 0) return 0;
     return size_t(F) * size_t((HW + sb::kSeGroup - 1) / sb::kSeGroup) * size_t(C);
@@ -668,9 +675,8 @@ extern "C" int shvk_cnn_se_gate(const float* x, float* partial, const float* w1,
     const int S = (HW + sb::kSeGroup - 1) / sb::kSeGroup;
     if (S > 65535) return int(cudaErrorInvalidValue);
     cudaStream_t s = cudaStream_t(stream);
-    sb::se_partial_kernel<<<dim3(unsigned(F), unsigned(S), unsigned((C + 127) / 128)), 256, 0, s>>>(x, partial, HW, C, S);
-    cudaError_t e = cudaGetLastError();
-    if (e != cudaSuccess) return int(e);
+    const int e = sb::se_partial_sums(x, partial, F, HW, C, s);
+    if (e != 0) return e;
     const size_t smem = size_t(C + CS) * sizeof(float);
     if (smem > 48 * 1024) return int(cudaErrorInvalidValue);
     // the gate itself on clusters of eight blocks (cnn_fused.cu: a weight row is read once for four frames, and an eighth of

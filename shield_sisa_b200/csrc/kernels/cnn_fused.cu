@@ -8,7 +8,8 @@
 //     expand (mma.sync m16n8k16 -> fp32 in shared memory) | depthwise (fp32 FMA out of shared memory)
 // and either rounds the chunk into the A operand of the projection, whose accumulators stay in registers over all chunks,
 // or, where a squeeze-excite gate stands between (it needs the whole map), writes the fp32 map and its pooled sums.
-// Roundings are those of the layered form: 1x1 operands in the mode's 16-bit type, everything else float32.
+// Every step rounds and sums as the layer kernels of cnn.cu do: 1x1 operands in the mode's 16-bit type, everything else
+// float32, activations operation by operation, pooled sums over the same groups of pixels.  The maps are the same bits.
 //
 // mma.sync and not tcgen05: the products are 16 to 160 deep and 8 to 160 wide on tiles whose rows are gathered pixels;
 // they are a third of these kernels' instructions, the depthwise filter and the activations are the rest.
@@ -20,6 +21,7 @@
 
 namespace sb {
 size_t se_gate_frame_bytes(int C, int CS);       // shared memory of a frame in the gate's cluster form (asked by cnn.cu too)
+int se_partial_sums(const float* x, float* partial, int F, int HW, int C, cudaStream_t s);   // cnn.cu
 namespace {
 
 // x * relu6(x + 3) / 6 of a pair, each step rounded as cnn.cu rounds it.  The quotient is a product and an FMA with 1/6 in two
@@ -118,12 +120,19 @@ struct Block {
     static constexpr int KFILL = cmax((CK - CE) / 2, 1);                       // k padding of a chunk, in pairs
     static constexpr int UNITS = OMT * ONT, UPW = SE ? 1 : (UNITS + 7) / 8;
     static constexpr int STRIPS = TH / SR, GX = TW / PX, ITEMS = CE / 2 * GX * STRIPS;
+    // squeeze-excite: the pooled sums are taken over groups of 64 pixels in row order, as se_partial_kernel takes them.  A tile that
+    // consists of whole groups sums them itself (POOL)
+    static constexpr int GROUP = 64, GROUPS = (HO * WO + GROUP - 1) / GROUP, TGROUPS = (TH * TW + GROUP - 1) / GROUP;
+    static constexpr bool POOL = SE && TW == WO && (TILES == 1 || (S == 1 && TH * TW % GROUP == 0));
+    static constexpr int RUN = TW % 8 == 0 ? 8 : TW % 4 == 0 ? 4 : 2;        // pixels of a row that are together in a group
     static constexpr int E_BYTES = up(IH * IW * P * 4, 16), X_BYTES = up(MROWS * XP * 2, 16), T_BYTES = up(MROWS * 2, 16);
-    static constexpr int D_BYTES = SE ? up(GX * STRIPS * CE * 4, 16) : up(OMT * 16 * DP * 2, 16);
+    static constexpr int D_BYTES = SE ? 0 : up(OMT * 16 * DP * 2, 16);
     static constexpr int SMEM = E_BYTES + X_BYTES + T_BYTES + D_BYTES;
     static_assert(CE % 8 == 0 && NT % NSPLIT == 0 && 8 % NSPLIT == 0 && TW % PX == 0 && TH % SR == 0, "tile shape");
     static_assert(SE ? CEXP % CE == 0 : CK == CE || CHUNKS == 1, "channel chunks");
     static_assert(SE || COUT % 8 == 0, "output channels");
+    static_assert(!SE || ITEMS <= 256, "a thread keeps its outputs until the tile's map is consumed");
+    static_assert(!POOL || (TW % RUN == 0 && GROUP % RUN == 0), "groups");
 };
 
 struct BlockArgs {
@@ -135,7 +144,7 @@ struct BlockArgs {
     const uint2* wp;           // projection weights, fragments [n tile][k tile][lane]
     const float* bp;
     float* out;                // [F][HO][WO][COUT], or the depthwise map [F][HO][WO][CEXP]
-    float* sums;               // squeeze-excite: [F][TILES][CEXP] sums of the map over a tile's pixels
+    float* sums;               // squeeze-excite: [F][GROUPS][CEXP] sums of the map over groups of pixels
     int chunks_per_group;      // squeeze-excite: chunks a block takes (gridDim.y groups)
 };
 
@@ -220,46 +229,82 @@ __global__ void __launch_bounds__(256, C::MINB) block_kernel(const BlockArgs a) 
         }
         __syncthreads();
         // ---- depthwise
-        for (int i = tid; i < C::ITEMS; i += 256) {
-            const int cp = i % (C::CE / 2), gx = i / (C::CE / 2) % C::GX, st = i / (C::CE / 2 * C::GX);
+        auto depthwise = [&](int i, float2 (&v)[C::SR][C::PX], int& oy, int& ox, int& cp) {
+            cp = i % (C::CE / 2);
+            ox = i / (C::CE / 2) % C::GX * C::PX;
+            oy = i / (C::CE / 2 * C::GX) * C::SR;
             const int col = ch * C::CE + cp * 2;
             const bool live = C::CEXP % C::CE == 0 || col < C::CEXP;
-            float2 w[C::KS * C::KS], acc[C::SR][C::PX];
+            float2 w[C::KS * C::KS];
 #pragma unroll
             for (int k = 0; k < C::KS * C::KS; ++k)
                 w[k] = live ? __ldg(reinterpret_cast<const float2*>(a.wd + k * C::CEXP + col)) : make_float2(0.0f, 0.0f);
             const float2 bias = live ? __ldg(reinterpret_cast<const float2*>(a.bd + col)) : make_float2(0.0f, 0.0f);
-            const int oy = st * C::SR, ox = gx * C::PX;
-            depthwise_pair<C::KS, C::S, C::PX, C::SR, C::P, C::IW>(E + (oy * C::S * C::IW + ox * C::S) * C::P + cp * 2, w, acc);
-            float2 sum = make_float2(0.0f, 0.0f);
+            depthwise_pair<C::KS, C::S, C::PX, C::SR, C::P, C::IW>(E + (oy * C::S * C::IW + ox * C::S) * C::P + cp * 2, w, v);
 #pragma unroll
-            for (int r = 0; r < C::SR; ++r) {
+            for (int r = 0; r < C::SR; ++r)
 #pragma unroll
-                for (int p = 0; p < C::PX; ++p) {
-                    const float2 v = act2<C::HS>(add2(acc[r][p], bias));
-                    if (C::SE) {
-                        if ((C::HO % C::TH == 0 || oy0 + oy + r < C::HO) && (C::WO % C::TW == 0 || ox0 + ox + p < C::WO)) {
-                            *reinterpret_cast<float2*>(a.out + ((long long)(f * C::HO + oy0 + oy + r) * C::WO + ox0 + ox + p) * C::CEXP + col) = v;
-                            sum.x += v.x;
-                            sum.y += v.y;
-                        }
-                    } else {
-                        reinterpret_cast<uint32_t*>(D)[((oy + r) * C::TW + ox + p) * (C::DP / 2) + cp] = Half<HT>::pack(v.x, v.y);
-                    }
-                }
-            }
-            if (C::SE) *reinterpret_cast<float2*>(D + ((st * C::GX + gx) * C::CE + cp * 2) * 4) = sum;
-        }
-        __syncthreads();
+                for (int p = 0; p < C::PX; ++p) v[r][p] = act2<C::HS>(add2(v[r][p], bias));
+        };
+        float2 v[C::SR][C::PX];
+        int oy, ox, cp;
         if constexpr (C::SE) {
-            // the tile's sums, thread groups in a fixed order
-            if (tid < C::CE) {
-                float s = 0.0f;
-#pragma unroll 4
-                for (int i = 0; i < C::GX * C::STRIPS; ++i) s += reinterpret_cast<const float*>(D)[i * C::CE + tid];
-                a.sums[((long long)f * C::TILES + tile) * C::CEXP + ch * C::CE + tid] = s;
+            const bool mine = C::ITEMS == 256 || tid < C::ITEMS;
+            auto inside = [&](int r, int p) { return (C::HO % C::TH == 0 || oy0 + oy + r < C::HO) && (C::WO % C::TW == 0 || ox0 + ox + p < C::WO); };
+            if (mine) {
+                depthwise(tid, v, oy, ox, cp);
+#pragma unroll
+                for (int r = 0; r < C::SR; ++r)
+#pragma unroll
+                    for (int p = 0; p < C::PX; ++p)
+                        if (inside(r, p))
+                            *reinterpret_cast<float2*>(a.out + ((long long)(f * C::HO + oy0 + oy + r) * C::WO + ox0 + ox + p) * C::CEXP + ch * C::CE + cp * 2) = v[r][p];
+            }
+            __syncthreads();                             // the expanded chunk is consumed
+            if constexpr (C::POOL) {
+                // the outputs take the places of expanded pixels of the image (the next chunk writes those again, the halo stays zero)
+                if (mine)
+#pragma unroll
+                    for (int r = 0; r < C::SR; ++r)
+#pragma unroll
+                        for (int p = 0; p < C::PX; ++p)
+                            if (inside(r, p)) *reinterpret_cast<float2*>(E + ((oy + r + C::PAD) * C::IW + ox + p + C::PAD) * C::P + cp * 2) = v[r][p];
+                __syncthreads();
+                // A group's sum: eight partial sums of every eighth pixel, then those in order.  640 frames, us per launch with the maps
+                // of blocks 5 / 11 / 12 / 13 / 14 summed here: 249 / 219 / 305 / 240 / 166; with sums per tile in the order of the
+                // threads, which rounds otherwise, 235 / 195 / 268 / 218 / 158; block 4, whose tiles cut the groups, is read again
+                // (332 -> 364).
+                const int n = C::HO % C::TH == 0 ? C::TH * C::TW : min(C::TH, C::HO - oy0) * C::TW;
+                for (int i = tid; i < C::CE * C::TGROUPS; i += 256) {
+                    const int c = i % C::CE, s = C::TGROUPS == 1 ? 0 : i / C::CE;
+                    float part[8];
+#pragma unroll
+                    for (int e = 0; e < 8; ++e) part[e] = 0.0f;
+#pragma unroll
+                    for (int q = 0; q < C::GROUP; q += C::RUN) {
+                        const int p = s * C::GROUP + q;
+                        const float* const row = E + ((p / C::TW + C::PAD) * C::IW + p % C::TW + C::PAD) * C::P + c;
+                        if (p < n)                       // n is a multiple of RUN
+#pragma unroll
+                            for (int e = 0; e < C::RUN; ++e) part[(q + e) & 7] += row[e * C::P];
+                    }
+                    float t = part[0];
+#pragma unroll
+                    for (int e = 1; e < 8; ++e) t += part[e];
+                    a.sums[((long long)f * C::GROUPS + tile * C::TGROUPS + s) * C::CEXP + ch * C::CE + c] = t;
+                }
+                __syncthreads();
             }
         } else {
+            for (int i = tid; i < C::ITEMS; i += 256) {
+                depthwise(i, v, oy, ox, cp);
+#pragma unroll
+                for (int r = 0; r < C::SR; ++r)
+#pragma unroll
+                    for (int p = 0; p < C::PX; ++p)
+                        reinterpret_cast<uint32_t*>(D)[((oy + r) * C::TW + ox + p) * (C::DP / 2) + cp] = Half<HT>::pack(v[r][p].x, v[r][p].y);
+            }
+            __syncthreads();
             // ---- projection: this chunk's k range into the accumulators of the warp's (pixel group, n tile) units
             const uint32_t drow = smem_addr(D) + uint32_t(((lane & 15) * C::DP + (lane >> 4) * 8) * 2);
             constexpr int KC = C::CK / 16, KALL = C::CHUNKS * KC;
@@ -773,14 +818,14 @@ last_pool_kernel(const float* __restrict__ x, const uint2* __restrict__ w, const
 using B2 = Block<16, 64, 24, 3, 2, 90, 160, 9, 8, 32, 2, 3, 1, false, false, 3>;
 using B3 = Block<24, 72, 24, 3, 1, 45, 80, 9, 16, 72, 4, 3, 1, false, true, 2>;
 using B4 = Block<24, 72, 0, 5, 2, 45, 80, 12, 10, 24, 2, 3, 1, false, false, 2>;
-using B5 = Block<40, 120, 0, 5, 1, 23, 40, 12, 20, 40, 4, 4, 1, false, false, 2>;
+using B5 = Block<40, 120, 0, 5, 1, 23, 40, 8, 40, 24, 4, 4, 1, false, false, 2>;
 using B7 = Block<40, 240, 80, 3, 2, 23, 40, 6, 10, 48, 2, 3, 1, true, false, 2>;
 using B8 = Block<80, 200, 80, 3, 1, 12, 20, 6, 20, 32, 4, 3, 2, true, true, 2>;
 using B9 = Block<80, 184, 80, 3, 1, 12, 20, 6, 20, 32, 4, 3, 2, true, true, 2>;
-using B11 = Block<80, 480, 0, 3, 1, 12, 20, 12, 20, 32, 4, 3, 2, true, false, 2>;
-using B12 = Block<112, 672, 0, 3, 1, 12, 20, 12, 20, 32, 4, 3, 2, true, false, 2>;
+using B11 = Block<80, 480, 0, 3, 1, 12, 20, 12, 20, 32, 4, 4, 2, true, false, 2>;
+using B12 = Block<112, 672, 0, 3, 1, 12, 20, 12, 20, 32, 4, 4, 2, true, false, 2>;
 using B13 = Block<112, 672, 0, 5, 2, 12, 20, 6, 10, 32, 2, 2, 2, true, false, 2>;
-using B14 = Block<160, 960, 0, 5, 1, 6, 10, 6, 10, 64, 2, 3, 4, true, false, 2>;
+using B14 = Block<160, 960, 0, 5, 1, 6, 10, 6, 10, 64, 5, 3, 4, true, false, 2>;
 
 inline unsigned blocks_of(long long n, int per) { return unsigned((n + per - 1) / per); }
 inline bool unaligned(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) != 0; }
@@ -800,7 +845,9 @@ int launch_block(const BlockArgs& args, int F, cudaStream_t s) {
         grid.y = unsigned((C::CHUNKS + a.chunks_per_group - 1) / a.chunks_per_group);
     }
     block_kernel<C, HT><<<grid, 256, C::SMEM, s>>>(a);
-    return int(cudaGetLastError());
+    e = cudaGetLastError();
+    if (e != cudaSuccess || !C::SE || C::POOL) return int(e);
+    return se_partial_sums(a.out, a.sums, F, C::HO * C::WO, C::CEXP, s);
 }
 
 template <typename HT>
@@ -820,14 +867,14 @@ int dispatch_block(int block, const BlockArgs& a, int F, cudaStream_t s) {
     default: return int(cudaErrorInvalidValue);
     }
 }
-int block_tiles(int block) {
+int block_groups(int block) {
     switch (block) {
-    case 4: return B4::TILES;
-    case 5: case 6: return B5::TILES;
-    case 11: return B11::TILES;
-    case 12: return B12::TILES;
-    case 13: return B13::TILES;
-    case 14: case 15: return B14::TILES;
+    case 4: return B4::GROUPS;
+    case 5: case 6: return B5::GROUPS;
+    case 11: return B11::GROUPS;
+    case 12: return B12::GROUPS;
+    case 13: return B13::GROUPS;
+    case 14: case 15: return B14::GROUPS;
     default: return 0;
     }
 }
@@ -896,13 +943,14 @@ extern "C" int shvk_cnn_pack_weights(const float* w, int N, int K, int order, in
     return 0;
 }
 
-extern "C" int shvk_cnn_block_tiles(int block) { return sb::block_tiles(block); }
+extern "C" int shvk_cnn_block_tiles(int block) { return sb::block_groups(block); }
+extern "C" int shvk_cnn_block_launches(int block) { return block == 4 && !sb::B4::POOL ? 2 : 1; }
 extern "C" void shvk_cnn_block_padding(int block, int* columns, int* k) { sb::block_padding(block, columns, k); }
 
 extern "C" int shvk_cnn_block(int block, const float* x, const void* we, const float* be, const float* wd, const float* bd,
                               const void* wp, const float* bp, float* out, float* sums, int F, int dtype, void* stream) {
     if (F <= 0) return 0;
-    const bool se = sb::block_tiles(block) > 0;
+    const bool se = sb::block_groups(block) > 0;
     if (!x || !we || !be || !wd || !bd || !out || (se ? !sums : !wp || !bp) || out == x || sb::unaligned(x) || sb::unaligned(out) ||
         sb::unaligned(we) || (wp && sb::unaligned(wp)) || sb::unaligned(be) || sb::unaligned(wd) || sb::unaligned(bd) || (bp && sb::unaligned(bp)))
         return int(cudaErrorInvalidValue);

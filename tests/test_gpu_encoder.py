@@ -635,3 +635,16 @@ def test_se_gate_forms_give_the_same_bits(L, Cn, CS):
     want = gate(big, Fmax, wide)
     for F in (1, 3, 55, 57, 75, 148, Fmax):
         assert torch.equal(gate((x, w1, b1, w2, b2), F, Cn), want[:F])
+
+
+@pytest.mark.parametrize("dtype", [1, 2])
+@pytest.mark.parametrize("block", [4, 5, 11, 12, 13, 14])
+def test_gated_block_gives_the_bits_of_the_layers(L, block, dtype):
+    """Behind a gate: the pooled sums (groups of 64 pixels, eight partial sums each), the gate and the gated projection are the bits of the
+    layer kernels, whatever share of the channels a thread block walks: one chunk (3 frames), several (38 to 150 frames, by block) or
+    all of them (600 frames); the gate's forms change in the same range."""
+    import torch
+    for F in (3, 38, 75, 150, 600):
+        a, f = _block_both_ways(L, block, dtype, F, seed=F)
+        for name in ("out", "sums", "gate", "y"):
+            assert torch.equal(f[name], a[name]), (F, name)
