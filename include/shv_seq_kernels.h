@@ -177,11 +177,14 @@ int shvk_sisa_attn_h16(const void* S16, const float* SG, const float* QC, const 
 
 /* Readout row (token 320) of the SISA block, fp32 in every mode, part 1: xl = rmsnorm(h_last) * norm_w, then
  * QC = xl * W_qc^T.  h_last: row 320 of clip c at h_last + c * ldh (elements); wqc_t: [384][576] = [W_Q | W_C]
- * transposed; QC: [B][576].  Replaces launch_rmsnorm + gemm<float> (engine/cuda/engine.cu:451-452). */
+ * transposed, 8-byte aligned (16 lets eight SMs share a small batch: same bits, faster); QC: [B][576], 8-byte aligned.
+ * Replaces launch_rmsnorm + gemm<float> (engine/cuda/engine.cu:451-452). */
 int shvk_readout_qc(const float* h_last, long long ldh, const float* norm_w, const float* wqc_t, float* QC, int B, void* stream);
 /* Part 2, after the attention: x1 = h_last + Y * W_O^T; x2 = x1 + down(silu(gate(n)) * up(n)) with n = rmsnorm(x1);
  * logit = head(rmsnorm(x2)).  All matrices transposed to [K][N] (fp32); up_t holds the (gate, up) output pairs of the
- * SwiGLU FFN in adjacent columns (2j, 2j + 1).  Y: [B][384]; x2_out: [B][384] or NULL; logits: [B].
+ * SwiGLU FFN in adjacent columns (2j, 2j + 1).  Y: [B][384]; x2_out: [B][384], 8-byte aligned, or NULL; logits: [B].
+ * wo_t, up_t and down_t are 8-byte aligned; with all four matrices aligned to 16, h_last to 8 and ldh even, eight SMs
+ * share a small batch (same bits, faster).
  * Replaces three gemm<float>, one launch_rmsnorm and launch_head (engine/cuda/engine.cu:455-469, seq.cu:309-336). */
 typedef struct shvk_readout_weights {
     const float* wo_t;          /* [384][384]  */

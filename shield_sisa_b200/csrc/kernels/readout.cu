@@ -410,8 +410,11 @@ constexpr int tail_smem_bytes(int tb) { return (2 * tb * XP + tb * HP) * int(siz
 // allows; tail kernel in us, split / one block: 1 clip 28 / 43, 45 clips 36 / 82, 96 clips 43 / 82, but 128 clips (two
 // waves) 83 / 81.  Above, a block takes 16 clips once that still gives every SM one, else 4, 2 (the few hundred clips of a
 // pipeline batch: at 512 two clips per block 87 us, one 144, four 108) or 1.
+// The split form copies the matrices 16 bytes at a time and reads the residual row in pairs (`may_split`: they are aligned for
+// that); the one-block form wants 8 bytes of the matrices and nothing of the row.  Both give the same bits.
 struct ReadoutShape { int tb; bool split; };
-ReadoutShape readout_shape(int B) {
+inline bool aligned_to(const void* p, uintptr_t bytes) { return (reinterpret_cast<uintptr_t>(p) & (bytes - 1)) == 0; }
+ReadoutShape readout_shape(int B, bool may_split) {
     int dev = 0, sms = 148, clusters = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
@@ -424,7 +427,7 @@ ReadoutShape readout_shape(int B) {
         cudaGetLastError();
         clusters = 0;
     }
-    for (int tb = 1; tb <= 8; tb *= 2)
+    for (int tb = 1; may_split && tb <= 8; tb *= 2)
         if ((B + tb - 1) / tb <= clusters) return {tb, true};
     return {B >= 16 * sms ? 16 : B >= 4 * sms ? 4 : B >= 2 * sms ? 2 : 1, false};
 }
@@ -468,7 +471,7 @@ extern "C" int shvk_readout_qc(const float* h_last, long long ldh, const float* 
     if (B <= 0) return 0;
     if (!h_last || !norm_w || !wqc_t || !QC) return int(cudaErrorInvalidValue);
     cudaStream_t s = cudaStream_t(stream);
-    const sb::ReadoutShape sh = sb::readout_shape(B);
+    const sb::ReadoutShape sh = sb::readout_shape(B, sb::aligned_to(wqc_t, 16));
     switch (2 * sh.tb + sh.split) {
 #define X(TB, SPLIT) case 2 * TB + SPLIT: return sb::launch_qc<TB, SPLIT>(h_last, ldh, norm_w, wqc_t, QC, B, s);
         SHVK_READOUT_SHAPES(X)
@@ -483,7 +486,9 @@ extern "C" int shvk_readout_tail(const float* Y, const float* h_last, long long 
     if (!Y || !h_last || !w || !logits) return int(cudaErrorInvalidValue);
     const sb::TailWeights tw{w->wo_t, w->ffn_norm_w, w->up_t, w->down_t, w->final_norm_w, w->head_w0_t, w->head_b0, w->head_w2, w->head_b2};
     cudaStream_t s = cudaStream_t(stream);
-    const sb::ReadoutShape sh = sb::readout_shape(B);
+    const bool may_split = sb::aligned_to(w->wo_t, 16) && sb::aligned_to(w->up_t, 16) && sb::aligned_to(w->down_t, 16) &&
+                           sb::aligned_to(w->head_w0_t, 16) && sb::aligned_to(h_last, 8) && (ldh & 1) == 0;
+    const sb::ReadoutShape sh = sb::readout_shape(B, may_split);
     switch (2 * sh.tb + sh.split) {
 #define X(TB, SPLIT) case 2 * TB + SPLIT: return sb::launch_tail<TB, SPLIT>(Y, h_last, ldh, tw, x2_out, logits, B, s);
         SHVK_READOUT_SHAPES(X)

@@ -930,6 +930,49 @@ def test_readout_row_split_over_eight_blocks(L, n):
         assert torch.equal(part[:n], whole[:n]) and (part[n:] == 9.0).all()
 
 
+@pytest.mark.parametrize("n", [1, 45, 120, 300])
+@pytest.mark.parametrize("what", ["rows", "odd_stride", "matrices", "head"])
+def test_readout_takes_what_only_the_one_block_form_can_read(L, n, what):
+    """Small batches share eight blocks only where the matrices are aligned for 16-byte copies and the residual rows for pairs; rows at
+    any float, any stride and matrices aligned to 8 bytes (the head's to 4) are taken at every batch size, with the same bits."""
+    import torch
+    gen = torch.Generator(device="cuda").manual_seed(n)
+    rn = lambda *s: torch.randn(*s, device="cuda", generator=gen)  # noqa: E731
+
+    def moved(t, floats):
+        flat = torch.zeros(t.numel() + 4, device="cuda")
+        flat[floats:floats + t.numel()] = t.flatten()
+        return flat[floats:floats + t.numel()].view(t.shape)
+
+    shapes = {"wo_t": (384, 384), "ffn_norm_w": (384,), "up_t": (384, 1920), "down_t": (960, 384), "final_norm_w": (384,),
+              "head_w0_t": (384, 128), "head_b0": (128,), "head_w2": (128,), "head_b2": (1,)}
+    w = {k: rn(*v) / 20 for k, v in shapes.items()}
+    nw, wqc, h, y = rn(384), rn(384, 576) / 20, rn(n, 384), rn(n, 384)
+
+    def run(w, wqc, h, ldh):
+        rw = binding.ReadoutWeights(**{k: v.data_ptr() for k, v in w.items()})
+        lg, x2, q = (torch.full(sh, 9.0, device="cuda") for sh in ((n,), (n, 384), (n, 576)))
+        ok(L.shvk_readout_qc(h.data_ptr(), ldh, nw.data_ptr(), wqc.data_ptr(), q.data_ptr(), n, stream_ptr()))
+        ok(L.shvk_readout_tail(y.data_ptr(), h.data_ptr(), ldh, C.byref(rw), x2.data_ptr(), lg.data_ptr(), n, stream_ptr()))
+        sync()
+        return lg, x2, q
+
+    want = run(w, wqc, h, 384)
+    w2, wqc2, h2, ldh = dict(w), wqc, h, 384
+    if what == "rows":
+        h2 = moved(h, 1)
+    elif what == "odd_stride":
+        h2, ldh = torch.zeros(n, 385, device="cuda"), 385
+        h2[:, :384] = h
+    elif what == "matrices":
+        w2 = {k: moved(v, 2) for k, v in w.items()}
+        wqc2 = moved(wqc, 2)
+    else:
+        w2["head_w0_t"] = moved(w["head_w0_t"], 1)
+    for got, ref in zip(run(w2, wqc2, h2, ldh), want):
+        assert torch.equal(got, ref)
+
+
 def test_store_tokens(L):
     import torch
     blocks = torch.arange(4 * 6144, device="cuda", dtype=torch.float32).reshape(4, 6144)
