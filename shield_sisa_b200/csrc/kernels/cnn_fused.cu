@@ -234,12 +234,17 @@ __global__ void __launch_bounds__(256, C::MINB) block_kernel(const BlockArgs a) 
             ox = i / (C::CE / 2) % C::GX * C::PX;
             oy = i / (C::CE / 2 * C::GX) * C::SR;
             const int col = ch * C::CE + cp * 2;
-            const bool live = C::CEXP % C::CE == 0 || col < C::CEXP;
+            if (C::CEXP % C::CE != 0 && col >= C::CEXP) {   // padding of the last chunk; its expanded values are NaN behind an infinite pixel
+#pragma unroll
+                for (int r = 0; r < C::SR; ++r)
+#pragma unroll
+                    for (int p = 0; p < C::PX; ++p) v[r][p] = make_float2(0.0f, 0.0f);
+                return;
+            }
             float2 w[C::KS * C::KS];
 #pragma unroll
-            for (int k = 0; k < C::KS * C::KS; ++k)
-                w[k] = live ? __ldg(reinterpret_cast<const float2*>(a.wd + k * C::CEXP + col)) : make_float2(0.0f, 0.0f);
-            const float2 bias = live ? __ldg(reinterpret_cast<const float2*>(a.bd + col)) : make_float2(0.0f, 0.0f);
+            for (int k = 0; k < C::KS * C::KS; ++k) w[k] = __ldg(reinterpret_cast<const float2*>(a.wd + k * C::CEXP + col));
+            const float2 bias = __ldg(reinterpret_cast<const float2*>(a.bd + col));
             depthwise_pair<C::KS, C::S, C::PX, C::SR, C::P, C::IW>(E + (oy * C::S * C::IW + ox * C::S) * C::P + cp * 2, w, v);
 #pragma unroll
             for (int r = 0; r < C::SR; ++r)

@@ -648,3 +648,35 @@ def test_gated_block_gives_the_bits_of_the_layers(L, block, dtype):
         a, f = _block_both_ways(L, block, dtype, F, seed=F)
         for name in ("out", "sums", "gate", "y"):
             assert torch.equal(f[name], a[name]), (F, name)
+
+
+@pytest.mark.parametrize("block", [2, 3, 7, 8, 9])
+def test_fused_block_keeps_infinities(L, block):
+    """A pixel beyond fp16's range rounds to infinity as an operand: with positive weights every output it reaches is infinite, in the
+    layers and in the fused block alike; the channels that only pad the last chunk (blocks 8 to 10) must not make it NaN."""
+    import torch
+    cin, k, cexp, cout, _se, stride = _BLOCKS[block - 1]
+    H, W = 90, 160
+    for _cin, kk, *_r, st in _BLOCKS[:block - 1]:
+        H, W = (H + 2 * ((kk - 1) // 2) - kk) // st + 1, (W + 2 * ((kk - 1) // 2) - kk) // st + 1
+    pad = (k - 1) // 2
+    Ho, Wo = (H + 2 * pad - k) // stride + 1, (W + 2 * pad - k) // stride + 1
+    act = 1 if block < 7 else 2
+    gen = torch.Generator(device="cuda").manual_seed(block)
+    rp = lambda *s: torch.rand(*s, device="cuda", generator=gen) * 0.05 + 0.01  # noqa: E731
+    zeros = lambda *s: torch.zeros(s, device="cuda")  # noqa: E731
+    x, we, be, wd, bd, wp, bp = rp(1, H, W, cin), rp(cexp, cin), rp(cexp), rp(k * k, cexp), rp(cexp), rp(cout, cexp), rp(cout)
+    x[0, 5, 7] = 1e5
+    res = x if stride == 1 and cin == cout else None
+    E, dw, y, out = zeros(1, H, W, cexp), zeros(1, Ho, Wo, cexp), zeros(1, Ho, Wo, cout), zeros(1, Ho, Wo, cout)
+    assert L.shvk_cnn_pointwise_h(_ptr(x), _ptr(we), _ptr(be), None, 1, None, _ptr(E), H * W, cexp, cin, act, 2, stream_ptr()) == 0
+    assert L.shvk_cnn_depthwise(_ptr(E), _ptr(wd), _ptr(bd), _ptr(dw), 1, H, W, cexp, k, stride, Ho, Wo, act, stream_ptr()) == 0
+    assert L.shvk_cnn_pointwise_h(_ptr(dw), _ptr(wp), _ptr(bp), None, 1, _ptr(res) if res is not None else None, _ptr(y), Ho * Wo, cout, cexp, 0,
+                                  2, stream_ptr()) == 0
+    cols, kp = C.c_int(), C.c_int()
+    L.shvk_cnn_block_padding(block, C.byref(cols), C.byref(kp))
+    p_we, p_wp = _pack(L, we.cpu().numpy(), 0, 2, cols.value), _pack(L, wp.cpu().numpy(), 0, 2, None, kp.value)
+    assert L.shvk_cnn_block(block, _ptr(x), _ptr(p_we), _ptr(be), _ptr(wd), _ptr(bd), _ptr(p_wp), _ptr(bp), _ptr(out), None, 1, 2, stream_ptr()) == 0
+    sync()
+    assert torch.isinf(y).any() and not torch.isnan(y).any()
+    assert torch.equal(out, y)
