@@ -990,7 +990,7 @@ size_t sb::se_gate_frame_bytes(int C, int CS) { return size_t(gate_rows_padded(C
 extern "C" int shvk_cnn_se_gate_sums(const float* sums, const float* w1, const float* b1, const float* w2, const float* b2, float* gate,
                                      int F, int tiles, int HW, int C, int CS, void* stream) {
     if (F <= 0) return 0;
-    if (!sums || tiles <= 0 || HW <= 0 || C <= 0 || CS <= 0 || (C & 3)) return int(cudaErrorInvalidValue);
+    if (!sums || !w1 || !b1 || !w2 || !b2 || !gate || tiles <= 0 || HW <= 0 || C <= 0 || CS <= 0 || (C & 3)) return int(cudaErrorInvalidValue);
     // Frames per cluster: one while that gives an SM three blocks or fewer (960 channels, one / four: 56 frames 18.7 / 27 us, 75 frames
     // 29.8 / 29.8, 112 frames 33 / 30), else four (a weight row serves four frames)
     const int sms = sb::device_sms(), G = 8LL * F <= 3 * sms ? 1 : 4;

@@ -48,3 +48,11 @@ def test_library_loads_and_reports_revision(built):
     L.shv_cuda_default_options(opt)
     assert (opt.max_frames, opt.max_windows, opt.max_host_tokens, opt.token_slots, opt.use_graphs, opt.max_delay_us) == \
         (640, 512, 2048, 0, 1, 0)
+
+
+def test_gate_from_sums_refuses_missing_arguments(built):
+    """A missing array is an invalid value on the host, not a launch."""
+    L = binding.load_library(True)
+    for missing in range(6):
+        arrays = [None if i == missing else 0x10000 for i in range(6)]
+        assert L.shvk_cnn_se_gate_sums(*arrays, 1, 1, 60, 960, 240, None) == 1          # cudaErrorInvalidValue
