@@ -746,7 +746,7 @@ def run_ours(args, rank: int, world: int, local_rank: int):
         print(json.dumps(dev_cycles, indent=1), file=sys.stderr)
     alg_bytes_clip = 45853824 if mode == "fp32" else MODEL_BYTES_16BIT
     stack_frac = B * alg_bytes_clip / (ms_step / 1000.0) / (pk["hbm_gbs"] * 1e9)
-    launches = eng.launches() * args.steps * world
+    launches = eng.launches(B) * args.steps * world
     eng.close()
     del eng
     torch.cuda.empty_cache()

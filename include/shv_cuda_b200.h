@@ -31,8 +31,10 @@ int shv_cuda_b200_upload_tokens(shv_cuda_model* m, const float* tokens, size_t n
  * differ from those of the unrounded embeddings by what fp16 rounding of the inputs costs).  Blocks; 0 or -1. */
 int shv_cuda_b200_classify_f16(shv_cuda_model* m, const uint16_t* tokens_f16, size_t b, float* logits);
 
-/* Number of kernels one GPU batch launches (for launch accounting in benchmarks). */
+/* Number of kernels one GPU batch launches (for launch accounting in benchmarks): a batch of max_windows windows, and one of
+ * `windows` windows (16-bit modes: small batches run their feed-forward blocks as two kernels each); 0 outside 1..max_windows. */
 int shv_cuda_b200_launches_per_batch(const shv_cuda_model* m);
+int shv_cuda_b200_launches_for(const shv_cuda_model* m, int windows);
 
 /* Test hook, experimental library only (-1 in the certificate-checked library): the next `batches` GPU batches of a
  * 16-bit model run with one launch starved of its input (kind 1: a tensor-core GEMM, 2: the scan), so that the kernel's
@@ -108,7 +110,8 @@ float* shvb_engine_logits(shvb_engine* e, int slot);                 /* device p
 /* Waits for `stream`, then copies the first n logits of `slot` to host memory. */
 int shvb_engine_read_logits(shvb_engine* e, int slot, float* host, int n, void* stream);
 int shvb_engine_window_bucket(const shvb_engine* e, int B);          /* size class a batch of B is padded to */
-int shvb_engine_launches(const shvb_engine* e);                      /* kernels per classify */
+int shvb_engine_launches(const shvb_engine* e);                      /* kernels per classify of max_windows windows */
+int shvb_engine_launches_for(const shvb_engine* e, int B);           /* kernels per classify of B windows; 0 outside 1..max_windows */
 int shvb_engine_status(const shvb_engine* e);                        /* nonzero: a kernel's bounded wait gave up */
 /* Test hook, as shv_cuda_b200_test_starve: the next `batches` classify calls starve one launch (16-bit modes). */
 int shvb_engine_test_starve(shvb_engine* e, int kind, int batches);

@@ -101,6 +101,7 @@ def load_library(experimental: bool = True) -> C.CDLL:
         "shv_cuda_b200_upload_tokens": (i32, [vp, vp, sz, vp]),
         "shv_cuda_b200_classify_f16": (i32, [vp, vp, sz, vp]),
         "shv_cuda_b200_launches_per_batch": (i32, [vp]),
+        "shv_cuda_b200_launches_for": (i32, [vp, i32]),
         "shv_cuda_b200_test_starve": (i32, [vp, i32, i32]),
         "shv_box_load": (vp, [C.c_char_p, C.c_char_p, C.POINTER(i32), i32, C.POINTER(Options), i32]),
         "shv_box_load_with": (vp, [C.POINTER(BoxOps), C.c_char_p, C.c_char_p, C.POINTER(i32), i32, C.POINTER(Options), i32]),
@@ -128,6 +129,7 @@ def load_library(experimental: bool = True) -> C.CDLL:
         "shvb_engine_read_logits": (i32, [vp, i32, vp, i32, vp]),
         "shvb_engine_window_bucket": (i32, [vp, i32]),
         "shvb_engine_launches": (i32, [vp]),
+        "shvb_engine_launches_for": (i32, [vp, i32]),
         "shvb_engine_status": (i32, [vp]),
         "shvb_engine_test_starve": (i32, [vp, i32, i32]),
         "shvb_engine_bytes": (sz, [vp, i32]),
@@ -294,8 +296,9 @@ class CudaModel:
     def weight_bytes(self):
         return self.L.shv_cuda_weight_bytes(self.m)
 
-    def launches_per_batch(self):
-        return self.L.shv_cuda_b200_launches_per_batch(self.m)
+    def launches_per_batch(self, windows=None):
+        """Kernels of one GPU batch of `windows` windows (default: of max_windows)."""
+        return self.L.shv_cuda_b200_launches_per_batch(self.m) if windows is None else self.L.shv_cuda_b200_launches_for(self.m, windows)
 
     def test_starve(self, kind, batches=1):
         """Test hook of the experimental library: the next GPU batches starve one launch (1 GEMM, 2 scan)."""
@@ -525,14 +528,15 @@ class EngineCore:
         return self._profile(self.L.shvb_engine_profile, slot, batch, stream)
 
     def profile_encode(self, slot, frames, stream=0):
-        """[(kernel name, ms)] of one eager encode, one entry per launch."""
+        """[(kernel name, ms)] of one eager encode, one entry per step (a map's pooled sums share one with what runs beside them)."""
         return self._profile(self.L.shvb_engine_profile_encode, slot, frames, stream)
 
     def window_bucket(self, batch):
         return self.L.shvb_engine_window_bucket(self.e, batch)
 
-    def launches(self):
-        return self.L.shvb_engine_launches(self.e)
+    def launches(self, windows=None):
+        """Kernels of one classify of `windows` windows (default: of max_windows)."""
+        return self.L.shvb_engine_launches(self.e) if windows is None else self.L.shvb_engine_launches_for(self.e, windows)
 
     def status(self):
         return self.L.shvb_engine_status(self.e)

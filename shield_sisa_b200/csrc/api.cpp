@@ -949,7 +949,8 @@ int shv_cuda_b200_upload_tokens(shv_cuda_model* m, const float* tokens, size_t n
     }
 }
 
-int shv_cuda_b200_launches_per_batch(const shv_cuda_model* m) { return m ? m->pipe->engine->launches_per_classify() : 0; }
+int shv_cuda_b200_launches_per_batch(const shv_cuda_model* m) { return m ? m->pipe->engine->launches_per_full_classify() : 0; }
+int shv_cuda_b200_launches_for(const shv_cuda_model* m, int windows) { return m ? m->pipe->engine->launches_per_classify(windows) : 0; }
 
 int shv_cuda_b200_test_starve(shv_cuda_model* m, int kind, int batches) {
 #ifdef SHV_CUDA_EXPERIMENTAL

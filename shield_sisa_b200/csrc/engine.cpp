@@ -222,9 +222,14 @@ public:
         starve_kind_ = kind;
         starve_batches_ = batches > 0 ? batches : 0;
     }
-    // 16-bit modes: 24 kernels (26 in a batch whose feed-forward blocks are two GEMMs each).  Exact tier: 23 (its feed-forward blocks are two GEMMs each) + a launch that splits the
-    // A operand of the five GEMMs that do not read a normalised row (three o-projections, two FFN down projections)
-    int launches_per_classify() const override { return prec_ == Precision::FP32 ? 28 : 24; }
+    // 16-bit modes: 24 kernels, 26 where the two feed-forward blocks are two GEMMs each.  Exact tier: 23 (its feed-forward blocks are
+    // two GEMMs each) + a launch that splits the A operand of the five GEMMs that do not read a normalised row (three
+    // o-projections, two FFN down projections)
+    int launches_per_classify(int B) const override {
+        if (B <= 0 || B > cfg_.max_windows) return 0;
+        if (prec_ == Precision::FP32) return 28;
+        return two_launch_ffn(window_bucket(B) * NTOK) ? 26 : 24;
+    }
 
     // One eager classify / encode with an event after every launch; returns (kernel name, milliseconds) per launch.
     std::vector<std::pair<std::string, float>> profile(int slot, int B, cudaStream_t s) override {

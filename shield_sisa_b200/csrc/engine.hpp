@@ -66,8 +66,9 @@ public:
     // bounded wait runs out, the kernel sets its status word and returns (kind 1: the tensor-core GEMM of the first
     // output projection, 2: the first scan).  Nothing faults or spins without bound; the batch's results are invalid.
     virtual void inject_wait_timeout(int kind, int batches) = 0;
-    // Kernels launched by one classify of B windows (for launch accounting in benchmarks).
-    virtual int launches_per_classify() const = 0;
+    // Kernels launched by one classify of B windows, padded to their size class (for launch accounting in benchmarks).
+    virtual int launches_per_classify(int B) const = 0;
+    int launches_per_full_classify() const { return launches_per_classify(cfg_.max_windows); }
     // One eager classify of B windows with a CUDA event after every launch: (kernel name, milliseconds) per launch,
     // in launch order.  Synchronises the stream.
     virtual std::vector<std::pair<std::string, float>> profile(int slot, int B, cudaStream_t s) = 0;

@@ -117,7 +117,8 @@ int shvb_engine_window_bucket(const shvb_engine* e, int B) {
     guard([&] { out = e ? e->eng->window_bucket(B) : -1; });
     return out;
 }
-int shvb_engine_launches(const shvb_engine* e) { return e ? e->eng->launches_per_classify() : 0; }
+int shvb_engine_launches(const shvb_engine* e) { return e ? e->eng->launches_per_full_classify() : 0; }
+int shvb_engine_launches_for(const shvb_engine* e, int B) { return e ? e->eng->launches_per_classify(B) : 0; }
 int shvb_engine_status(const shvb_engine* e) { return e ? e->eng->device_status() : -1; }
 int shvb_engine_test_starve(shvb_engine* e, int kind, int batches) {
     return guard([&] {

@@ -232,3 +232,20 @@ def test_full_size_batch_is_row_independent_and_within_tolerance(mode, weight_fi
     print(f"full-size {mode} logits: max|err|/max|ref| {err:.3e}, rms err {rms:.3e} over {len(want)} clips "
           f"(max|ref| {np.abs(want).max():.3f})")
     assert err <= LOWP_TOL
+
+
+@pytest.mark.parametrize("mode", ["fp32", "bf16", "fp16"])
+def test_launch_counts_are_those_of_the_launch_sequence(mode, weight_files):
+    """The stated kernel counts against the sequences' own records: batches on both sides of the lines where the feed-forward blocks
+    of the 16-bit modes change between one kernel and two, size classes included, and the encoder."""
+    path, _ = weight_files("W3", 1)
+    for graphs in (False, True):
+        eng = binding.EngineCore(path, mode, max_windows=130, max_frames=3, use_graphs=graphs)
+        for b in (1, 45, 48, 64, 128, 130):
+            assert eng.launches(b) == len(eng.profile(0, eng.window_bucket(b), stream_ptr())), (graphs, b)
+        assert eng.launches() == eng.launches(130) and eng.launches(131) == eng.launches(0) == 0
+        # one record may cover two kernels: a gate of the exact tier with its pooled sums, block 4 of the 16-bit modes with its own
+        assert eng.encode_launches() == len(eng.profile_encode(0, 3, stream_ptr())) + (8 if mode == "fp32" else 1) == (64 if mode == "fp32" else 34)
+        eng.close()
+    with binding.CudaModel(path, mode, max_windows=130) as m:
+        assert m.launches_per_batch() == m.launches_per_batch(130) and m.launches_per_batch(1) == (28 if mode == "fp32" else 26)
