@@ -680,3 +680,27 @@ def test_fused_block_keeps_infinities(L, block):
     sync()
     assert torch.isinf(y).any() and not torch.isnan(y).any()
     assert torch.equal(out, y)
+
+
+@pytest.mark.parametrize("mode", ["bf16", "fp16"])
+def test_fused_encode_frame_independence_and_graphs(mode, weight_files):
+    """16-bit modes: a frame's tokens are bitwise the same alone, in batches of every size at which a fused kernel changes its form
+    (shares of channels, frames to a cluster, split row kernels), in another order, and through a padded CUDA graph."""
+    from shield_sisa_b200 import binding, weights as W
+    path, _ = weight_files("W5", 3)
+    frames = W.synth_frames(300, 23)
+    eager = binding.EngineCore(path, mode, max_windows=1, max_frames=300, use_graphs=False)
+    graph = binding.EngineCore(path, mode, max_windows=1, max_frames=300, use_graphs=True)
+    full = _encode(eager, frames)
+    assert np.isfinite(full).all()
+    for n in (1, 4, 39, 57, 75, 111, 151):
+        assert np.array_equal(_encode(eager, frames[:n], slot=n % 2), full[:n])
+    for i in (38, 150, 299):
+        assert np.array_equal(_encode(eager, frames[i:i + 1])[0], full[i])
+    perm = np.random.default_rng(1).permutation(300)
+    assert np.array_equal(_encode(eager, frames[perm], slot=1), full[perm])
+    for n in (300, 75, 7):
+        assert np.array_equal(_encode(graph, frames[:n]), full[:n])
+        assert np.array_equal(_encode(graph, frames[perm[:n]]), full[perm[:n]])          # the captured graph on other crops
+    eager.close()
+    graph.close()
