@@ -415,15 +415,15 @@ constexpr int tail_smem_bytes(int tb) { return (2 * tb * XP + tb * HP) * int(siz
 struct ReadoutShape { int tb; bool split; };
 inline bool aligned_to(const void* p, uintptr_t bytes) { return (reinterpret_cast<uintptr_t>(p) & (bytes - 1)) == 0; }
 ReadoutShape readout_shape(int B, bool may_split) {
-    int dev = 0, sms = 148, clusters = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    const int sms = device_sms();
+    if ((B + 7) / 8 > sms / CL) may_split = false;     // no more clusters than that fit, whatever the answer below
+    int clusters = 0;
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = dim3(unsigned(sms / CL) * CL);
     cfg.blockDim = dim3(NTC);
     cfg.dynamicSmemBytes = tail_split_smem(8);
-    if (cudaFuncSetAttribute(readout_tail_split_kernel<8>, cudaFuncAttributeMaxDynamicSharedMemorySize, tail_split_smem(8)) != cudaSuccess ||
-        cudaOccupancyMaxActiveClusters(&clusters, readout_tail_split_kernel<8>, &cfg) != cudaSuccess) {
+    if (may_split && (cudaFuncSetAttribute(readout_tail_split_kernel<8>, cudaFuncAttributeMaxDynamicSharedMemorySize, tail_split_smem(8)) != cudaSuccess ||
+                      cudaOccupancyMaxActiveClusters(&clusters, readout_tail_split_kernel<8>, &cfg) != cudaSuccess)) {
         cudaGetLastError();
         clusters = 0;
     }
