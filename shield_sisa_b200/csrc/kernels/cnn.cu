@@ -745,13 +745,14 @@ extern "C" int shvk_cnn_pointwise(const float* A, const float* W, const float* b
     if (sb::pointwise_args_bad(A, W, b, gate, gate_rows, R, out, N, K)) return int(cudaErrorInvalidValue);
     cudaStream_t s = cudaStream_t(stream);
     // Layers of 24, 40, 72 or 80 output channels: one tile spans the row, so a pixel is read once instead of for every 16 or 32
-    // columns (75 frames: 24 -> 72 channels 55 -> 44 us; 40 channels 51 -> 35, 80 channels 36 -> 33), as long as that leaves
-    // about a block per SM (20 frames, 80 channels: 37 against 24 us).  Wide layers: 128 columns do more per shared-memory
-    // read, but a block alone on its SM waits for its loads; up to three 64 x 64 tiles per SM are faster (75 frames, 160 channels
-    // of 960: 123 -> 85 us; token projection 109 -> 49; 112 channels, 564 tiles: 85 against 64).
+    // columns (75 frames: 24 -> 72 channels 55 -> 44 us; 40 channels 51 -> 35, 80 channels, 141 blocks, 36 -> 33), as long as
+    // that leaves two blocks for three SMs (20 frames, 80 channels, 38 blocks: 37 against 24 us).  Wide layers: 128 columns
+    // do more per shared-memory read, but a block alone on its SM waits for its loads; up to three 64 x 64 tiles per SM are
+    // faster (75 frames, 160 channels of 960: 123 -> 85 us; token projection 109 -> 49; 112 channels, 564 tiles: 85 against 64).
     int bn = sb::pointwise_tile_width(N);
-    if ((N == 24 || N == 40 || N == 72 || N == 80) && sb::blocks_for(M, 128) >= 100) bn = N;
-    else if (bn == 128 && (long long)sb::blocks_for(M, 64) * ((N + 63) / 64) <= 3 * 148) bn = 64;
+    const int sms = sb::device_sms();
+    if ((N == 24 || N == 40 || N == 72 || N == 80) && 3LL * sb::blocks_for(M, 128) >= 2 * sms) bn = N;
+    else if (bn == 128 && (long long)sb::blocks_for(M, 64) * ((N + 63) / 64) <= 3 * sms) bn = 64;
     const unsigned gy = unsigned((N + bn - 1) / bn);
     const bool deep = K >= 256;
 #define SHVK_POINTWISE(BM_, BN_, TM_, TN_, KS_, PACK_)                                                                           \
@@ -797,7 +798,7 @@ extern "C" int shvk_cnn_pointwise_tf32(const float* A, const float* W, const flo
         // wide layers: 64-column tiles (80 registers, three blocks per SM; the 128 x 128 tile needs 128 registers and
         // measured 5 % slower over the encoder); 128 rows per block, 64 when that leaves less than two waves of blocks
         const unsigned gy64 = unsigned((N + 63) / 64);
-        if ((long long)sb::blocks_for(M, 128) * gy64 >= 2LL * 3 * 148)
+        if ((long long)sb::blocks_for(M, 128) * gy64 >= 2LL * 3 * sb::device_sms())
             sb::pointwise_tf32_kernel<128, 64, 4, 2><<<sb::blocks_for(M, 128) * gy64, 256, 0, s>>>(A, W, b, gate, gate_rows, R, out, M, N, K, act, int(gy64));
         else
             sb::pointwise_tf32_kernel<64, 64, 4, 2><<<sb::blocks_for(M, 64) * gy64, 256, 0, s>>>(A, W, b, gate, gate_rows, R, out, M, N, K, act, int(gy64));
@@ -827,7 +828,7 @@ int launch_pointwise_h(const float* A, const float* W, const float* b, const flo
         const unsigned gy = unsigned((N + bn - 1) / bn);
         if (bn == 128) {
             const unsigned gy64 = unsigned((N + 63) / 64);
-            if ((long long)blocks_for(M, 128) * gy64 >= 2LL * 3 * 148) SB_PH(128, 64, 4, 2, gy64);
+            if ((long long)blocks_for(M, 128) * gy64 >= 2LL * 3 * device_sms()) SB_PH(128, 64, 4, 2, gy64);
             else SB_PH(64, 64, 4, 2, gy64);
         } else if (bn == 64) SB_PH(64, 64, 4, 2, gy);
         else if (bn == 32) SB_PH(128, 32, 8, 1, gy);

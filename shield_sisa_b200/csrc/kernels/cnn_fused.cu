@@ -844,7 +844,7 @@ int launch_block(const BlockArgs& args, int F, cudaStream_t s) {
     dim3 grid(unsigned(F) * C::TILES, 1);
     if (C::SE) {
         // a block redoes the tile's input for its share of the channels: as few shares as give the GPU four blocks per SM
-        const int want = int((4LL * 148 + grid.x - 1) / grid.x);
+        const int want = int((4LL * device_sms() + grid.x - 1) / grid.x);
         const int groups = want < 1 ? 1 : want > C::CHUNKS ? C::CHUNKS : want;
         a.chunks_per_group = (C::CHUNKS + groups - 1) / groups;
         grid.y = unsigned((C::CHUNKS + a.chunks_per_group - 1) / a.chunks_per_group);
@@ -1017,7 +1017,7 @@ int launch_rows_gate(const float* A, const uint4* W, const float* b, const float
     // Few rows: a warp's chain of k steps is all the time there is, so its loads run ahead and the n tiles go to other blocks.  us,
     // whole / split: 160 channels of 960: 4 frames 41 / 15, 40 frames 64 / 18, 160 frames 64 / 43, 320 frames 75 / 87; 112 channels
     // of 480: 4 frames 23 / 10, 40 frames 33 / 24, 80 frames 33 / 39 (300 row blocks).
-    const bool few = gx <= 160;
+    const bool few = 12LL * gx <= 13 * device_sms();     // about a row block per SM
     auto go = [&](auto kernel, unsigned gy) {
         kernel<<<dim3(gx, gy), 128, 0, s>>>(A, W, b, gate, gate_rows, R, out, M, N, K);
         return int(cudaGetLastError());
@@ -1067,7 +1067,8 @@ extern "C" int shvk_cnn_token_proj(const void* pooled, const void* W, float* tok
     const uint4* w = static_cast<const uint4*>(W);
     cudaStream_t s = cudaStream_t(stream);
     const unsigned gx = sb::blocks_of(rows, 64);
-    const bool few = gx <= 80;          // as in launch_rows_gate: 4 frames 26 / 9 us, 40 frames 55 / 12, 320 frames 51 / 37
+    // as in launch_rows_gate, up to a row block for about two SMs: 4 frames 26 / 9 us, 40 frames 55 / 12, 320 frames (80 blocks) 51 / 37
+    const bool few = 11LL * gx <= 6 * sb::device_sms();
     auto go = [&](auto kernel, unsigned gy) {
         kernel<<<dim3(gx, gy), 128, 0, s>>>(A, w, tokens, rows, 384, 960);
         return int(cudaGetLastError());

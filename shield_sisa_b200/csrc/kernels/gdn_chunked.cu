@@ -488,9 +488,7 @@ int launch_chunked(const void* q, const void* k, const void* v, const float* g, 
     const int prep_smem = 4 * int(sizeof(PrepWarp<DK>));
     cudaError_t e = cudaFuncSetAttribute(gdn_chunked_prep_kernel<DK>, cudaFuncAttributeMaxDynamicSharedMemorySize, prep_smem);
     if (e != cudaSuccess) return int(e);
-    int dev = 0, sms = 148;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    const int sms = device_sms();
     // one block a warp while that is a single wave of warps (576 blocks of the wider keys: 9.4 us for both kernels against 11.0)
     const int per = blocks <= 16ll * sms ? 1 : 2;
     gdn_chunked_prep_kernel<DK><<<unsigned((blocks + 4 * per - 1) / (4 * per)), 128, prep_smem, s>>>(
