@@ -1,6 +1,6 @@
 /*
  * shv_cnn_kernels.h -- thin C launch layer over the sm_100a frame-encoder kernels of the SHIELD-V engine
- * (MobileNetV3-Large features on 320x180 crops, 4x4 pooling; the 960 -> 384 token projection is shvk_gemm_f32).
+ * (MobileNetV3-Large features on 320x180 crops, 4x4 pooling; the 960 -> 384 token projection as one more 1x1 layer).
  *
  * Same conventions as shv_seq_kernels.h: every pointer is a device pointer, `stream` is a cudaStream_t passed as
  * void*, every function only enqueues work and returns a cudaError_t value (0 = success).  Activations are float32 in

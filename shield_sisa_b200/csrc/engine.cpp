@@ -19,7 +19,7 @@
 // encode (F frames, reference run_encode engine/cuda/engine.cu:338-403): stem -> 15 inverted-residual blocks
 //   (expand 1x1 | depthwise | squeeze-excite gate | project 1x1 with the gate applied to its input rows, + residual)
 //   -> 1x1 160 -> 960 -> 4x4 pooling -> 960 -> 384 token projection into slot.d_tokens.  float32 NHWC storage in every
-//   mode.  fp32 mode: a launch per layer (64).  bf16 / fp16 modes (33 launches): stem and block 1 in one kernel, expand +
+//   mode.  fp32 mode: a launch per layer (64).  bf16 / fp16 modes (34 launches): stem and block 1 in one kernel, expand +
 //   depthwise (+ project, where no gate stands between) of a block in one kernel, gate, project behind the gate, last
 //   convolution + pooling in one kernel; the 1x1 convolutions round their operands to the mode's type and multiply on the
 //   tensor cores.
@@ -153,12 +153,11 @@ struct CnnBlockDev {
     int tiles = 0;                                    // 16-bit modes: pooled sums per frame (squeeze-excite blocks)
 };
 
-// One all-row GEMM of the launch sequence: its argument block for the planned maximum row count and, in the 16-bit
-// modes, the tensor-core plan (TMA maps) made once for these buffers.
+// One all-row GEMM of the launch sequence: its argument block for the planned maximum row count and the tensor-core plan
+// (TMA maps) made once for these buffers.
 struct Site {
     shvk_gemm_args args{};
     alignas(64) unsigned char plan[512];
-    bool planned = false;
     const float* split_src = nullptr;    // exact tier: the fp32 A operand, split into args.A = [lo | hi] before every launch
 };
 
@@ -566,10 +565,8 @@ private:
         }
         make_site(sisa_in_, SN, D, xn_, s_w_all_, P_, SLD, SHVK_F32);
         sisa_in_.args.bias = s_b_all_;
-        for (Site* st : {&oproj_[0], &oproj_[1], &up_[0], &up_[1], &down_[0], &down_[1]}) {
+        for (Site* st : {&oproj_[0], &oproj_[1], &up_[0], &up_[1], &down_[0], &down_[1]})
             launch_ok(shvk_gemm_tc_plan(&st->args, dt_, st->plan), "tensor-core GEMM plan");
-            st->planned = true;
-        }
         if (prec_ == Precision::FP32) {
             launch_ok(shvk_gemm_tc_plan(&sisa_in_.args, dt_, sisa_in_.plan), "tensor-core GEMM plan");
         } else {
@@ -582,12 +579,8 @@ private:
             sisa_in_.args.C = sg_; sisa_in_.args.ldc = SG_LD;
             launch_ok(shvk_gemm_tc_plan_split16(&sisa_in_.args, dt_, SB_COLS, s16_, SB_COLS, sisa_in_.plan), "tensor-core GEMM plan");
         }
-        sisa_in_.planned = true;
         if (prec_ == Precision::FP32) {
-            for (Site* st : {&in_[0], &in_[1]}) {
-                launch_ok(shvk_gemm_tc_plan(&st->args, dt_, st->plan), "tensor-core GEMM plan");
-                st->planned = true;
-            }
+            for (Site* st : {&in_[0], &in_[1]}) launch_ok(shvk_gemm_tc_plan(&st->args, dt_, st->plan), "tensor-core GEMM plan");
             return;
         }
         // the chunk-blocked operand tiles of the in-projection live where the fp32 projection of the exact tier would
@@ -601,17 +594,11 @@ private:
                                            gdn_[i].a_log, gdn_[i].dt_bias, P_, dt_, inproj_plan_[i]), "in-projection plan");
     }
     void rows_gemm(const Site& st, int rows, cudaStream_t s) {
-        if (st.planned) {
-            if (st.split_src) {
-                launch_ok(shvk_split_tf32(st.split_src, st.args.K, st.args.K, rows, a2_, 2 * st.args.K, 0, s), "operand split");
-                mark("split_tf32", s);
-            }
-            launch_ok(shvk_gemm_tc_rows(st.plan, rows, s), "tensor-core GEMM");
-        } else {
-            shvk_gemm_args a = st.args;
-            a.M = rows;
-            launch_ok(shvk_gemm_f32(&a, s), "fp32 GEMM");
+        if (st.split_src) {
+            launch_ok(shvk_split_tf32(st.split_src, st.args.K, st.args.K, rows, a2_, 2 * st.args.K, 0, s), "operand split");
+            mark("split_tf32", s);
         }
+        launch_ok(shvk_gemm_tc_rows(st.plan, rows, s), "tensor-core GEMM");
     }
     // ---------------------------------------------------------------- debug dumps
     void dump(const char* name, const void* dev, size_t n, int dtype, cudaStream_t s) {
@@ -680,14 +667,15 @@ private:
         dump("tokens", sl.d_tokens, size_t(16) * D, SHVK_F32, s);
     }
     // bf16 / fp16 modes: block outputs alternate between X and E (a block's tiles read each other's halos, so it cannot run
-    // in place); the projection behind a gate writes where its residual is
+    // in place).  Two maps of the debug dumps stay inside fused kernels, the stem's and the last one's: a dump computes them
+    // again with the layer kernels, whose bits the fused ones give (tests/test_gpu_encoder.py).
     void run_encode_fused(int slot, int F, cudaStream_t s) {
         const Slot& sl = slots_[size_t(slot)];
         const CnnBlockDev& d0 = blk_[0];
         launch_ok(shvk_cnn_stem_block(sl.d_frames, lut_, cnn_.stem_w.data(), cnn_.stem_b.data(), d0.dw_w, d0.dw_b, d0.proj_p, d0.proj_b, cx_,
                                       F, dt_, s), "stem and block 1");
         mark("cnn.stem_block", s);
-        if (!dump_dir_.empty()) {                        // the stem's own map, which the fused kernel keeps to itself
+        if (!dump_dir_.empty()) {
             launch_ok(shvk_cnn_stem(sl.d_frames, lut_, stem_w_, stem_b_, ce_, 1, s), "stem");
             dump("cnn_stem_f0", ce_, size_t(16) * 90 * 160, SHVK_F32, s);
             dump("cnn_block01_f0", cx_, size_t(16) * 90 * 160, SHVK_F32, s);

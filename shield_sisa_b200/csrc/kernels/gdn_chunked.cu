@@ -10,18 +10,18 @@
 //     R = K S0,  U = T2 (V - diag(e) R),  O = M U + diag(scale e) Q S0,  S' = e_16 S0 + K^T diag(exp(c_16 - c_j)) U.
 // T2 and M do not depend on the state, only R, U, O and S' do.  Two kernels, chunk-parallel where the algebra allows:
 //
-//   prep   one warp per block, all B x H x T/16 blocks at once: the two Gram products on mma.sync, the decay masks, the
-//          16 x 16 triangular inverse (forward substitution over 16 lanes), T2 and M as bf16 tiles and the decays'
-//          exponentials into a workspace of 1,152 bytes per block
-//   scan   one CTA per (batch, head), or two or four with a share of the value columns each, walks the blocks with the state resident: per block only the chain R -> U -> O and
-//          the state update remain, every operand fragment read straight out of the staged K, Q, V, T2, M tiles with
-//          ldmatrix (tiles arrive by cp.async into a ring of three or four slots, XOR-swizzled so the fragment reads are
-//          conflict-free), one CTA barrier per block, the previous block's output rows written while the next block's
-//          products run
+//   prep   one warp per two blocks (per block while that is a single wave of warps), all B x H x T/16 blocks at once: the two
+//          Gram products on mma.sync, the decay masks, the 16 x 16 triangular inverse (forward substitution over 16 lanes, both
+//          blocks at once), T2 and M as bf16 tiles and the decays' exponentials into a workspace of 1,152 bytes per block
+//   scan   one CTA per (batch, head), or two or four with a share of the value columns each, walks the blocks with the state
+//          resident: per block only the chain R -> U -> O and the state update remain, every operand fragment read straight
+//          out of the staged K, Q, V, T2, M tiles with ldmatrix (tiles arrive by cp.async into a ring of three or four slots,
+//          two or three blocks ahead, XOR-swizzled so the fragment reads are conflict-free), one CTA barrier per block, the
+//          previous block's output rows written while the next block's products run
 //
 // The value dimension (128) is the MMA row dimension and is split over the warps of the scan CTA: four warps of 32
 // columns for DK = 64, eight warps of 16 columns for DK = 128, so that a warp's slice of S^T is 64 fp32 registers per lane
-// in both cases; the hand-over between the products of a block stays in registers (the accumulator layout of one is the
+// in both cases (a sequence shared by CTAs: four or two warps of 16 columns each); the hand-over between the products of a block stays in registers (the accumulator layout of one is the
 // A-operand layout of the next).  Operands are bf16, the state and all accumulation fp32.  A caller's chunk size (e.g.
 // 64) only groups these 16-token blocks: the result does not depend on it.
 //
@@ -228,7 +228,7 @@ gdn_chunked_prep_kernel(const __nv_bfloat16* __restrict__ Q, const __nv_bfloat16
 template <int DK> struct ScanStage {                      // one block's operands as they lie in shared memory
     __align__(16) uint8_t k[CB * DK * 2], q[CB * DK * 2];  // [token][key] bf16, swizzled rows of DK * 2 bytes
     __align__(16) uint8_t v[2][CB * 128];                  // [token][value] bf16 as two halves of 64 values (128-byte rows)
-    __align__(16) uint8_t w[WS_BLOCK];                     // T2 | M | c of the block
+    __align__(16) uint8_t w[WS_BLOCK];                     // the block's workspace: T2 | M | exp(c_i) | exp(c_16 - c_i)
 };
 
 // MI row tiles of 16 values per warp, NWARP warps: NWARP * 16 * MI values per CTA, blockIdx.y says which of the 128.
@@ -264,7 +264,6 @@ gdn_chunked_scan_kernel(const __nv_bfloat16* __restrict__ Q, const __nv_bfloat16
 #pragma unroll
             for (int e = 0; e < 4; ++e) S[mi][nj][e] = 0.0f;
 
-    // asynchronous copies of block `c` into ring slot c % NSLOT; every thread issues its share and commits one group
     // the thread's first element of the next block to fetch, and of the next block of output rows; its i-th copy is KROWS (VROWS)
     // token rows further on
     constexpr int KROWS = NTHR / VPR, VROWS = NTHR / V8;
@@ -288,6 +287,7 @@ gdn_chunked_scan_kernel(const __nv_bfloat16* __restrict__ Q, const __nv_bfloat16
         for (int i = 0; i < VI; ++i) { vdst[i] = v_dst(i); asm volatile("" : "+r"(vdst[i])); }
     }
     const long long kstep = KROWS * tok_stride_k;
+    // asynchronous copies of block `c` into ring slot c % NSLOT; every thread issues its share and commits one group
     auto issue = [&](int c) {
         if (c < NB) {
             ScanStage<DK>& st = sm.st[c % NSLOT];

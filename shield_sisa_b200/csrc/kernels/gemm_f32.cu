@@ -1,6 +1,7 @@
 // IEEE fp32 GEMM on CUDA cores: C = epilogue(A * W^T), A [M,K], W [N,K], both K-contiguous.
 //
-// The exact tier and the last-row projections (which stay fp32 in every mode) run here.  Each output element is one
+// The plain form of a GEMM, which the tests hold the tensor-core kernels against; the launch sequences use those and, for the
+// readout row and the exact tier's 1x1 layers, kernels of their own.  Each output element is one
 // thread's fma chain over k = 0..K-1 in order, K is never split, and the tile shape is fixed, so a row of C is bitwise
 // independent of M and of the other rows in the batch (the row-independence contract of engine/include/shv_cuda.h:31-34
 // and the k-order rule of engine/cuda/gemm.cuh:5-10).
