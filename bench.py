@@ -215,6 +215,25 @@ def encoder_work():
     return nbytes, flops
 
 
+def encoder_crossing_bytes(mode):
+    """HBM bytes per frame that the encoder's launches really read and write (each map once per launch that touches it, halos and
+    weights left out).  fp32 mode: the layer-boundary model itself.  16-bit modes: expanded maps stay on the SM; a gated block
+    writes its depthwise map and the projection reads it, block 4's map is read once more for its pooled sums."""
+    if mode == "fp32":
+        return encoder_work()[0]
+    nbytes = 172800 + 14400 * 16 * 4                               # crop -> stem and block 1
+    h, w = 90, 160
+    for i, (cin, k, cexp, cout, se, stride) in enumerate(_ENC_BLOCKS):
+        pad = (k - 1) // 2
+        ho, wo = (h + 2 * pad - k) // stride + 1, (w + 2 * pad - k) // stride + 1
+        if i > 0:
+            nbytes += h * w * cin * 4 + ho * wo * cout * 4
+            if se:                                                 # the projection is a launch of its own: map, residual
+                nbytes += ho * wo * (cexp * (3 if i == 3 else 2) + (cout if stride == 1 and cin == cout else 0)) * 4
+        h, w = ho, wo
+    return nbytes + 60 * 160 * 4 + 2 * 16 * 960 * 2 + 16 * 384 * 4      # last convolution and pooling, token projection
+
+
 def encoder_leg(binding, torch, wpath, mode, local_rank, frames=512, steps=10, warmup=3):
     """Frames/s of Engine::encode on crops resident in HBM (CUDA events on the launching stream, graphs on)."""
     eng = binding.EngineCore(wpath, mode, device=local_rank, max_windows=1, max_frames=frames, use_graphs=True)
@@ -240,10 +259,14 @@ def encoder_leg(binding, torch, wpath, mode, local_rank, frames=512, steps=10, w
     for name, t in eng.profile_encode(0, frames, stream):
         kinds[name] = kinds.get(name, 0.0) + t
     nbytes, flops = encoder_work()
+    crossing = encoder_crossing_bytes(mode)
     pk, pk_src = peaks()
     out = {"frames_per_s": frames / (ms / 1000.0), "frames": frames, "ms_per_encode": ms, "launches": eng.encode_launches(),
            "dtype": "f32 storage; 1x1 convolutions fp32 fma (fp32 mode) or bf16 / fp16 mma with f32 accumulation (16-bit modes)", "ms_by_kernel": kinds, "algorithmic_bytes_per_frame": nbytes, "flops_per_frame": flops,
-           "hbm_frac": frames * nbytes / (ms / 1000.0) / (pk["hbm_gbs"] * 1e9), "peak_source": pk_src,
+           "crossing_bytes_per_frame": crossing, "hbm_frac": frames * crossing / (ms / 1000.0) / (pk["hbm_gbs"] * 1e9),
+           "layer_model_frac": frames * nbytes / (ms / 1000.0) / (pk["hbm_gbs"] * 1e9), "peak_source": pk_src,
+           "removed_boundary": None if mode == "fp32" else "expanded maps: the layer model (algorithmic_bytes_per_frame) counts them "
+                               "written and read, the fused blocks keep them on the SM; hbm_frac is of the bytes that cross",
            "note": "frame encoder (MobileNetV3-Large, 320x180 crops -> 16 x 384 tokens), float32 NHWC storage in every "
                    "mode; crops resident in HBM; not part of `value`"}
     eng.close()

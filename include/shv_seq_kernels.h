@@ -57,7 +57,7 @@ typedef struct shvk_gemm_args {
     const float* R; long long ldr; float r_div;
     int swiglu;
 } shvk_gemm_args;
-/* IEEE fp32 FMA chain on CUDA cores, k in order (exact tier and the fp32-only last-row projections). A, W fp32. */
+/* IEEE fp32 FMA chain on CUDA cores, k in order; the plain form that tests compare with. A, W fp32. */
 int shvk_gemm_f32(const shvk_gemm_args* g, void* stream);
 /* tcgen05 tensor-core GEMM, A and W in ab_dtype (bf16 or fp16), fp32 accumulation in tensor memory, operands
  * staged by TMA.  Needs K % 64 == 0, 16-byte aligned operands and pitches.  shvk_gemm_tc_plan encodes the two TMA
