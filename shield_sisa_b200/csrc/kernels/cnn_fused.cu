@@ -985,7 +985,10 @@ extern "C" int shvk_cnn_stem_block(const uint8_t* frames, const float* lut, cons
     return dtype == sb::DT_BF16 ? go(sb::stem_block_kernel<__nv_bfloat16>) : go(sb::stem_block_kernel<__half>);
 }
 
-size_t sb::se_gate_frame_bytes(int C, int CS) { return size_t(gate_rows_padded(C) + gate_rows_padded(CS)) * sizeof(float); }
+size_t sb::se_gate_frame_bytes(int C, int CS) {
+    if (C > 1 << 20 || CS > 1 << 20) return ~size_t(0) / 8;             // nothing that fits, and nothing that overflows
+    return size_t(gate_rows_padded(C) + gate_rows_padded(CS)) * sizeof(float);
+}
 
 extern "C" int shvk_cnn_se_gate_sums(const float* sums, const float* w1, const float* b1, const float* w2, const float* b2, float* gate,
                                      int F, int tiles, int HW, int C, int CS, void* stream) {
