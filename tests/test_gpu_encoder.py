@@ -390,8 +390,8 @@ def test_row_kernels_split_by_channels_give_the_same_rows(L, N, K, dtype):
 @pytest.mark.parametrize("block", [2, 3, 4, 5, 7, 8, 9, 11, 12, 13, 14])
 def test_fused_block_matches_layers(L, block, dtype):
     """One fused block (expand + depthwise + project or pooled sums, gate, gated project) against the layer kernels on the same
-    input.  Both round the 1x1 operands to the same type; the fused Hardswish differs in the last bit of a float32, so an operand
-    can round the other way: an ulp of the 16-bit type (at most 2^-7 or 2^-10 relative) on isolated terms of a K-term sum."""
+    input, within what operands that round the other way would cost: an ulp of the 16-bit type (at most 2^-7 or 2^-10 relative) on
+    isolated terms of a K-term sum.  (That they do not, bit for bit, is tested further down.)"""
     import torch
     cin, k, cexp, cout, se, stride = _BLOCKS[block - 1]
     H, W = 90, 160
