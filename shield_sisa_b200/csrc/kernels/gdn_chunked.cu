@@ -13,7 +13,8 @@
 //   prep   one warp per two blocks (per block while that is a single wave of warps), all B x H x T/16 blocks at once: the two
 //          Gram products on mma.sync, the decay masks, the 16 x 16 triangular inverse (forward substitution over 16 lanes, both
 //          blocks at once), T2 and M as bf16 tiles and the decays' exponentials into a workspace of 1,152 bytes per block
-//   scan   one CTA per (batch, head), or two or four with a share of the value columns each, walks the blocks with the state
+//   scan   one CTA per (batch, head), or two or four with a share of the value columns each where sequences are few (with warps of
+//          their own for the state and for the outputs: gdn_chunked_chain_kernel), walks the blocks with the state
 //          resident: per block only the chain R -> U -> O and the state update remain, every operand fragment read straight
 //          out of the staged K, Q, V, T2, M tiles with ldmatrix (tiles arrive by cp.async into a ring of three or four slots,
 //          two or three blocks ahead, XOR-swizzled so the fragment reads are conflict-free), one CTA barrier per block, the
@@ -21,7 +22,7 @@
 //
 // The value dimension (128) is the MMA row dimension and is split over the warps of the scan CTA: four warps of 32
 // columns for DK = 64, eight warps of 16 columns for DK = 128, so that a warp's slice of S^T is 64 fp32 registers per lane
-// in both cases (a sequence shared by CTAs: four or two warps of 16 columns each); the hand-over between the products of a block stays in registers (the accumulator layout of one is the
+// in both cases (a sequence shared by two CTAs: four warps of 16 columns each); the hand-over between the products of a block stays in registers (the accumulator layout of one is the
 // A-operand layout of the next).  Operands are bf16, the state and all accumulation fp32.  A caller's chunk size (e.g.
 // 64) only groups these 16-token blocks: the result does not depend on it.
 //
@@ -469,12 +470,236 @@ gdn_chunked_scan_kernel(const __nv_bfloat16* __restrict__ Q, const __nv_bfloat16
     store_rows(NB - 1);
 }
 
+// ---------------------------------------------------------------------------------------------------- scan of few sequences
+// Few sequences leave the GPU to the latency of one: then a block's time is what one warp does for it, one instruction after the
+// other.  So each 16 value columns get two warps.  The chain warp holds the state and runs R -> U -> state update alone; it hands the
+// state and U, as the 16-bit fragments its own products used, through shared memory to the output warp, which computes Q S0 and M U a
+// block behind, writes the rows, and brings in the blocks to come.  The same products and roundings as in the whole form, in the same
+// order: the same bits.  NP pairs of warps per CTA, 16 NP of the 128 value columns (blockIdx.y says which).
+//
+// The hand-overs are named barriers (arrive on one side, sync on the other), two of each kind by the parity of the block:
+//   FULL   the block's operands have landed (output warps -> chain warps)
+//   HAND   state and U of the block are in shared memory, its operands are read (chain warps -> output warps)
+//   TAKEN  the output warps have them in registers (-> chain warps, which write that buffer again two blocks later)
+// and OUT among the output warps alone: all are through with a block, its ring slot may be filled again.
+template <int DK, int NP> struct ChainSmem {
+    static constexpr int NSLOT = 4;
+    ScanStage<DK> st[NSLOT];
+    uint4 sa[2][NP][DK / 16][32];                          // [parity][pair][k step][lane]: state, A fragments
+    uint4 ua[2][NP][32];                                   // U
+};
+enum { BAR_OUT = 1, BAR_FULL = 2, BAR_HAND = 4, BAR_TAKEN = 6 };   // the latter three + parity; 0 is __syncthreads
+template <int N> __device__ __forceinline__ void bar_arrive(int id) { asm volatile("bar.arrive %0, %1;" ::"r"(id), "n"(N) : "memory"); }
+template <int N> __device__ __forceinline__ void bar_wait(int id) { asm volatile("bar.sync %0, %1;" ::"r"(id), "n"(N) : "memory"); }
+
+template <int DK, typename TO, int NP>
+__global__ void __launch_bounds__(NP * 64, 2)
+gdn_chunked_chain_kernel(const __nv_bfloat16* __restrict__ Q, const __nv_bfloat16* __restrict__ K, const __nv_bfloat16* __restrict__ V,
+                         const uint8_t* __restrict__ ws, TO* __restrict__ O, int T, int H, int NB, float scale) {
+    constexpr int NTHR = NP * 64, NOUT = NP * 32, KSTEP = DK / 16, NJ = DK / 8, ROWB = DK * 2, NSLOT = ChainSmem<DK, NP>::NSLOT;
+    extern __shared__ __align__(128) uint8_t chain_smem_raw[];
+    ChainSmem<DK, NP>& sm = *reinterpret_cast<ChainSmem<DK, NP>*>((reinterpret_cast<uintptr_t>(chain_smem_raw) + 127) & ~uintptr_t(127));
+    const int bh = blockIdx.x, bidx = bh / H, head = bh % H;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int g = lane >> 2, t = lane & 3, lm = lane >> 3, lr = lane & 7;
+    const int pair = warp % NP, dvb = (blockIdx.y * NP + pair) * 16;       // the pair's first value column
+    if (warp < NP) {
+        // ------------------------------------------------------------------------------------------- chain
+        float S[NJ][4];
+#pragma unroll
+        for (int nj = 0; nj < NJ; ++nj)
+#pragma unroll
+            for (int e = 0; e < 4; ++e) S[nj][e] = 0.0f;
+        for (int c = 0; c < NB; ++c) {
+            const ScanStage<DK>& st = sm.st[c % NSLOT];
+            uint32_t sa[KSTEP][4];
+            if (c >= 2) bar_wait<NTHR>(BAR_TAKEN + (c & 1));
+#pragma unroll
+            for (int p = 0; p < KSTEP; ++p) {
+                sa[p][0] = cpack(S[2 * p][0], S[2 * p][1]);
+                sa[p][1] = cpack(S[2 * p][2], S[2 * p][3]);
+                sa[p][2] = cpack(S[2 * p + 1][0], S[2 * p + 1][1]);
+                sa[p][3] = cpack(S[2 * p + 1][2], S[2 * p + 1][3]);
+                sm.sa[c & 1][pair][p][lane] = make_uint4(sa[p][0], sa[p][1], sa[p][2], sa[p][3]);
+            }
+            bar_wait<NTHR>(BAR_FULL + (c & 1));
+            const uint32_t k_s = smem_u32(st.k);
+            const float* eg = reinterpret_cast<const float*>(st.w + WS_EG);
+            const float* dj = reinterpret_cast<const float*>(st.w + WS_DJ);
+            float R[2][4];
+#pragma unroll
+            for (int ni = 0; ni < 2; ++ni)
+#pragma unroll
+                for (int e = 0; e < 4; ++e) R[ni][e] = 0.0f;
+#pragma unroll
+            for (int p = 0; p < KSTEP; ++p) {
+                uint32_t bk[4];
+                ldsm4(k_s + tile_off<ROWB>((lm >> 1) * 8 + lr, 2 * p + (lm & 1)), bk);
+#pragma unroll
+                for (int ni = 0; ni < 2; ++ni) cmma(R[ni], sa[p], bk[2 * ni], bk[2 * ni + 1]);
+            }
+            uint32_t vv[4], bt[4], kf[KSTEP][4];
+            ldsm4t(smem_u32(st.v[dvb >> 6]) + tile_off<128>((lm >> 1) * 8 + lr, ((dvb & 63) >> 3) + (lm & 1)), vv);
+            ldsm4(smem_u32(st.w + WS_T2) + uint32_t(((lm >> 1) * 8 + lr) * 32 + (lm & 1) * 16), bt);
+#pragma unroll
+            for (int q = 0; q < KSTEP; ++q) ldsm4t(k_s + tile_off<ROWB>((lm & 1) * 8 + lr, 2 * q + (lm >> 1)), kf[q]);
+            float2 ner[2], dj2[2];
+#pragma unroll
+            for (int ni = 0; ni < 2; ++ni) {
+                const float2 e = *reinterpret_cast<const float2*>(eg + 8 * ni + 2 * t);
+                ner[ni] = make_float2(-e.x, -e.y);
+                dj2[ni] = *reinterpret_cast<const float2*>(dj + 8 * ni + 2 * t);
+            }
+            const float2 elast = make_float2(eg[CB - 1], eg[CB - 1]);
+#pragma unroll
+            for (int nj = 0; nj < NJ; ++nj)
+#pragma unroll
+                for (int e = 0; e < 4; e += 2) {
+                    const float2 v = mul2(make_float2(S[nj][e], S[nj][e + 1]), elast);
+                    S[nj][e] = v.x; S[nj][e + 1] = v.y;
+                }
+            uint32_t va[4];
+#pragma unroll
+            for (int h = 0; h < 4; ++h) {
+                const float2 d = fma2(ner[h >> 1], make_float2(R[h >> 1][2 * (h & 1)], R[h >> 1][2 * (h & 1) + 1]), make_float2(bf_lo(vv[h]), bf_hi(vv[h])));
+                va[h] = cpack(d.x, d.y);
+            }
+            float U[2][4];
+#pragma unroll
+            for (int ni = 0; ni < 2; ++ni) {
+#pragma unroll
+                for (int e = 0; e < 4; ++e) U[ni][e] = 0.0f;
+                cmma(U[ni], va, bt[2 * ni], bt[2 * ni + 1]);
+            }
+            uint32_t da[4];
+#pragma unroll
+            for (int ni = 0; ni < 2; ++ni) {
+                const float2 d0 = mul2(make_float2(U[ni][0], U[ni][1]), dj2[ni]), d1 = mul2(make_float2(U[ni][2], U[ni][3]), dj2[ni]);
+                da[2 * ni] = cpack(d0.x, d0.y);
+                da[2 * ni + 1] = cpack(d1.x, d1.y);
+            }
+#pragma unroll
+            for (int nj = 0; nj < NJ; ++nj) cmma(S[nj], da, kf[nj >> 1][2 * (nj & 1)], kf[nj >> 1][2 * (nj & 1) + 1]);
+            sm.ua[c & 1][pair][lane] = make_uint4(cpack(U[0][0], U[0][1]), cpack(U[0][2], U[0][3]), cpack(U[1][0], U[1][1]), cpack(U[1][2], U[1][3]));
+            bar_arrive<NTHR>(BAR_HAND + (c & 1));
+        }
+        return;
+    }
+    // ----------------------------------------------------------------------------------------------- output
+    constexpr int VPR = DK / 8, V8 = NP * 2, KI = CB * VPR / NOUT, KROWS = NOUT / VPR, VROWS = NOUT / V8;
+    static_assert(CB * VPR % NOUT == 0 && VROWS == CB, "whole rounds of copies, one vector of V a thread");
+    const int tid = threadIdx.x - NP * 32, v16 = blockIdx.y * V8 + tid % V8;
+    const long long tok_stride_k = (long long)H * DK, tok_stride_v = (long long)H * CDV;
+    const __nv_bfloat16* kp = K + ((long long)bidx * T * H + head) * DK + (tid / VPR) * tok_stride_k + tid % VPR * 8;
+    const __nv_bfloat16* qp = Q + ((long long)bidx * T * H + head) * DK + (tid / VPR) * tok_stride_k + tid % VPR * 8;
+    const __nv_bfloat16* vp = V + ((long long)bidx * T * H + head) * CDV + (tid / V8) * tok_stride_v + v16 * 8;
+    const uint8_t* wp = ws + (long long)bh * NB * WS_BLOCK;
+    TO* op = O + ((long long)bidx * T * H + head) * CDV + dvb;
+    uint32_t kdst[KI];
+#pragma unroll
+    for (int i = 0; i < KI; ++i) kdst[i] = tile_off<ROWB>(tid / VPR + i * KROWS, tid % VPR);
+    const uint32_t vdst = uint32_t(v16 >> 3) * (CB * 128) + tile_off<128>(tid / V8, v16 & 7);
+    auto issue = [&](int c) {
+        if (c < NB) {
+            ScanStage<DK>& st = sm.st[c % NSLOT];
+            const int left = T - c * CB;
+            const uint32_t sk = smem_u32(st.k), sq = smem_u32(st.q);
+#pragma unroll
+            for (int i = 0; i < KI; ++i) {
+                const int n = tid / VPR + i * KROWS < left ? 16 : 0;
+                cp_async16(sk + kdst[i], n ? static_cast<const void*>(kp + i * KROWS * tok_stride_k) : wp, n);
+                cp_async16(sq + kdst[i], n ? static_cast<const void*>(qp + i * KROWS * tok_stride_k) : wp, n);
+            }
+            const int n = tid / V8 < left ? 16 : 0;
+            cp_async16(smem_u32(st.v[0]) + vdst, n ? static_cast<const void*>(vp) : wp, n);
+            for (int v = tid; v < WS_BLOCK / 16; v += NOUT) cp_async16(smem_u32(st.w) + v * 16, wp + v * 16, 16);
+            kp += CB * tok_stride_k;
+            qp += CB * tok_stride_k;
+            vp += CB * tok_stride_v;
+            wp += WS_BLOCK;
+        }
+        cp_commit();                                       // an empty group past the end keeps the group count in step
+    };
+#pragma unroll
+    for (int c = 0; c < NSLOT; ++c) issue(c);
+    cp_wait<NSLOT - 1>();
+    bar_arrive<NTHR>(BAR_FULL);
+    for (int c = 0; c < NB; ++c) {
+        if (c + 1 < NB) {
+            cp_wait<NSLOT - 2>();                          // blocks up to c + 1
+            bar_arrive<NTHR>(BAR_FULL + ((c + 1) & 1));
+        }
+        bar_wait<NTHR>(BAR_HAND + (c & 1));
+        uint4 sa[KSTEP];
+#pragma unroll
+        for (int p = 0; p < KSTEP; ++p) sa[p] = sm.sa[c & 1][pair][p][lane];
+        const uint4 ua = sm.ua[c & 1][pair][lane];
+        const ScanStage<DK>& st = sm.st[c % NSLOT];
+        const uint32_t q_s = smem_u32(st.q);
+        uint32_t am[4];
+        ldsm4(smem_u32(st.w + WS_M) + uint32_t(((lm & 1) * 8 + lr) * 32 + (lm >> 1) * 16), am);
+        const float* eg = reinterpret_cast<const float*>(st.w + WS_EG);
+        const float eqs[2] = {eg[g] * scale, eg[g + 8] * scale};
+        float QS[2][4], Oa[2][4];
+#pragma unroll
+        for (int nt = 0; nt < 2; ++nt)
+#pragma unroll
+            for (int e = 0; e < 4; ++e) { QS[nt][e] = 0.0f; Oa[nt][e] = 0.0f; }
+        // Q as the operand A [token][key]; the state's registers are B fragments [key][value] of values 0-7 (0, 2) and 8-15 (1, 3)
+#pragma unroll
+        for (int p = 0; p < KSTEP; ++p) {
+            uint32_t qf[4];
+            ldsm4(q_s + tile_off<ROWB>((lm & 1) * 8 + lr, 2 * p + (lm >> 1)), qf);
+            cmma(QS[0], qf, sa[p].x, sa[p].z);
+            cmma(QS[1], qf, sa[p].y, sa[p].w);
+        }
+        cmma(Oa[0], am, ua.x, ua.z);
+        cmma(Oa[1], am, ua.y, ua.w);
+        if (c + 2 < NB) bar_arrive<NTHR>(BAR_TAKEN + (c & 1));
+        bar_wait<NOUT>(BAR_OUT);
+        issue(c + NSLOT);
+        // rows straight from the accumulators [token][value].  float32: 8 bytes a lane, a whole 32-byte sector per token and n tile;
+        // bf16: the lanes of a pair trade halves, so that a token's 32 bytes leave in one instruction
+        const int left = T - c * CB;
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            const float2 e2 = make_float2(eqs[h], eqs[h]);
+            float2 o[2];
+#pragma unroll
+            for (int nt = 0; nt < 2; ++nt) o[nt] = fma2(e2, make_float2(QS[nt][2 * h], QS[nt][2 * h + 1]), make_float2(Oa[nt][2 * h], Oa[nt][2 * h + 1]));
+            TO* const row = op + (g + 8 * h) * tok_stride_v;
+            if constexpr (sizeof(TO) == 2) {
+                const uint32_t w0 = cpack(o[0].x, o[0].y), w1 = cpack(o[1].x, o[1].y);
+                const bool odd = (t & 1) != 0;
+                const uint32_t got = __shfl_xor_sync(0xffffffffu, odd ? w0 : w1, 1);
+                if (g + 8 * h < left) *reinterpret_cast<uint2*>(row + (odd ? 6 + 2 * t : 2 * t)) = odd ? make_uint2(got, w1) : make_uint2(w0, got);
+            } else if (g + 8 * h < left) {
+#pragma unroll
+                for (int nt = 0; nt < 2; ++nt) *reinterpret_cast<float2*>(row + 8 * nt + 2 * t) = o[nt];
+            }
+        }
+        op += CB * tok_stride_v;
+    }
+    cp_wait<0>();
+}
+
 template <int DK, typename TO, int MI, int NWARP, int NSLOT>
 int launch_scan(const void* q, const void* k, const void* v, const void* ws, void* o, int B, int T, int H, int NB, float scale, cudaStream_t s) {
     const int smem = NSLOT * int(sizeof(ScanStage<DK>)) + 2 * CB * OT_PITCH * 4 + 128;
     const cudaError_t e = cudaFuncSetAttribute(gdn_chunked_scan_kernel<DK, TO, MI, NWARP, NSLOT>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     if (e != cudaSuccess) return int(e);
     gdn_chunked_scan_kernel<DK, TO, MI, NWARP, NSLOT><<<dim3(unsigned(B) * unsigned(H), CDV / (16 * MI * NWARP)), NWARP * 32, smem, s>>>(
+        static_cast<const __nv_bfloat16*>(q), static_cast<const __nv_bfloat16*>(k), static_cast<const __nv_bfloat16*>(v),
+        static_cast<const uint8_t*>(ws), static_cast<TO*>(o), T, H, NB, scale);
+    return int(cudaGetLastError());
+}
+
+template <int DK, typename TO, int NP>
+int launch_chain(const void* q, const void* k, const void* v, const void* ws, void* o, int B, int T, int H, int NB, float scale, cudaStream_t s) {
+    const int smem = int(sizeof(ChainSmem<DK, NP>)) + 128;
+    const cudaError_t e = cudaFuncSetAttribute(gdn_chunked_chain_kernel<DK, TO, NP>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    if (e != cudaSuccess) return int(e);
+    gdn_chunked_chain_kernel<DK, TO, NP><<<dim3(unsigned(B) * unsigned(H), CDV / (16 * NP)), NP * 64, smem, s>>>(
         static_cast<const __nv_bfloat16*>(q), static_cast<const __nv_bfloat16*>(k), static_cast<const __nv_bfloat16*>(v),
         static_cast<const uint8_t*>(ws), static_cast<TO*>(o), T, H, NB, scale);
     return int(cudaGetLastError());
@@ -495,11 +720,15 @@ int launch_chunked(const void* q, const void* k, const void* v, const float* g, 
         static_cast<const __nv_bfloat16*>(q), static_cast<const __nv_bfloat16*>(k), g, beta, static_cast<uint8_t*>(ws), T, H, NB, blocks, per, scale);
     e = cudaGetLastError();
     if (e != cudaSuccess) return int(e);
-    // The value columns of a sequence are independent: while sequences are too few to give every SM one, a sequence's columns
-    // are split over two CTAs or, with the wider keys, four, whose warps then have a scheduler each to themselves.  Both kernels, us,
-    // whole / 2 / 4: DK 64, 1,024 tokens: 72 sequences 59 / 39 / 43, 144 66 / 58 / 63; 18 sequences of 1,021 56 / 35 / 38; DK 128:
-    // 18 sequences of 1,021 84 / 52 / 47; of 1,024: 36 85 / 54 / 48, 72 89 / 58 / 56, 144 106 / 90 / 113; 288 of 2,048 343 / 348 / 395.
-    if (DK == 128 && 2 * seqs <= sms) return launch_scan<DK, TO, 1, 2, 4>(q, k, v, ws, o, B, T, H, NB, scale, s);
+    // The value columns of a sequence are independent: while sequences are too few to give every SM one, a sequence's columns are
+    // split over CTAs.  While those are at most one an SM (four a sequence, then two), the chain form: its output warps have a
+    // scheduler to themselves; beyond, two CTAs of the whole form, and from one sequence an SM on one.  Both kernels, 1,021
+    // tokens, us, whole form split in two (DK 128 to 74 sequences: four) / chain form on four CTAs / on two: DK 64: 6 sequences of 700
+    // 29.4 / 25.3 / 25.3, 18 40.5 / 33 / 35.5, 36 41.6 / 34 / 37, 48 41.7 / 42.6 / 37.7, 72 43.5 / 44 / 39.4, 96 61 / 59 / 63, 120 63 / 71 / 66;
+    // DK 128: 6 of 700 37.5 / 29.4 / 37.5, 18 52 / 41.5 / 54, 36 54 / 44 / 56, 48 60 / 62 / 57.7, 72 63 / 65 / 61, 96 86 / 90 / 101.
+    // Whole form in one CTA / two: DK 64, 1,024 tokens, 144 sequences 66 / 58; DK 128, 144 106 / 90, 288 of 2,048 343 / 348.
+    if (4 * seqs <= sms) return launch_chain<DK, TO, 2>(q, k, v, ws, o, B, T, H, NB, scale, s);
+    if (2 * seqs <= sms) return launch_chain<DK, TO, 4>(q, k, v, ws, o, B, T, H, NB, scale, s);
     if (seqs <= sms) return launch_scan<DK, TO, 1, 4, 4>(q, k, v, ws, o, B, T, H, NB, scale, s);
     // ring slots of a whole sequence, 3 / 4: 64 x 2,048, DK 64 248 / 254 us; 48 x 2,048, DK 128 314 / 309
     return launch_scan<DK, TO, DK == 64 ? 2 : 1, DK == 64 ? 4 : 8, DK == 64 ? 3 : 4>(q, k, v, ws, o, B, T, H, NB, scale, s);

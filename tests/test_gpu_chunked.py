@@ -83,6 +83,20 @@ def test_sequences_are_bitwise_the_same_however_they_are_split(L, dk, out_bf16):
             np.testing.assert_array_equal(got[i], alone[i % 3])
 
 
+@pytest.mark.parametrize("t", [1, 16, 17, 48, 79, 130])          # 1, 1, 2, 3, 5 and 9 blocks: fewer than the ring holds, odd and even
+@pytest.mark.parametrize("dk", [64, 128])
+def test_few_sequences_give_the_bits_of_many(L, dk, t):
+    """The form with separate warps for state and outputs (up to 74 sequences on 148 SMs, four CTAs a sequence up to 37, then two) against
+    the whole form: the same bits, in both output types, next to sequences of another batch entry and head."""
+    q, k, v, gg, beta = delta_inputs(1, t, 3, dk, 128, seed=t)
+    for out_bf16 in (False, True):
+        want, _ = run_chunked(L, *(np.repeat(x, 67, 0) for x in (q, k, v, gg, beta)), out_bf16=out_bf16)     # 201 sequences
+        assert np.isfinite(want).all()
+        for n in (1, 12, 13, 24, 25):                              # 3, 36, 39, 72, 75 sequences
+            got, _ = run_chunked(L, *(np.repeat(x, n, 0) for x in (q, k, v, gg, beta)), out_bf16=out_bf16)
+            np.testing.assert_array_equal(got, want[:n])
+
+
 def test_rejects_unsupported_shapes(L):
     import torch
     x = torch.zeros(4096, device="cuda")
