@@ -668,6 +668,107 @@ rows_gate_kernel(const float* __restrict__ A, const uint4* __restrict__ W, const
     }
 }
 
+// The same for many rows.  A warp still owns 16 rows and all n tiles, the sums are the same in the same order, but what a step reads comes
+// through a ring of shared memory, RowsTile::STAGES stages of two k tiles: the rows of A as they are (float32, a warp reads only its
+// own) and the weight fragments, once for all warps of the block.
+template <int NT> struct RowsTile {
+    static constexpr int NP = (NT + 1) / 2, STAGES = 4, W_BYTES = 2 * NP * 512;
+    static constexpr int stage_bytes(int warps) { return warps * 16 * 128 + W_BYTES; }
+};
+__device__ __forceinline__ void copy16(uint32_t dst, const void* src, bool in) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(in ? 16 : 0) : "memory");
+}
+template <int NT, typename HT>
+__global__ void __launch_bounds__(256, 2)
+rows_gate_tile_kernel(const float* __restrict__ A, const uint4* __restrict__ W, const float* __restrict__ bias, const float* __restrict__ gate,
+                      int gate_rows, const float* R, float* out, int M, int N, int K) {
+    using L = RowsTile<NT>;
+    constexpr int NP = L::NP, STAGES = L::STAGES;
+    extern __shared__ __align__(128) uint8_t smem[];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, t = lane & 3, rows = blockDim.x >> 1;
+    const int mb = blockIdx.x * rows, m0 = mb + warp * 16, kt = (K + 15) / 16, ns = (kt + 1) / 2;
+    const uint32_t sb = smem_addr(smem), stage_bytes = uint32_t(rows * 128 + L::W_BYTES);
+    // 16-byte piece c of row r of a stage lies at piece c ^ 4 (r & 1): the lanes of two rows read all 32 banks at once
+    const int cr = tid >> 3, cc = tid & 7, cstep = blockDim.x >> 3;
+    const float* const gsrc = A + cc * 4;
+    auto issue = [&](int s) {
+        if (s < ns) {
+            const uint32_t sa = sb + uint32_t(s % STAGES) * stage_bytes;
+            const bool in = s * 32 + cc * 4 < K;
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                const int r = cr + i * cstep;
+                copy16(sa + uint32_t(r * 128 + ((cc ^ ((r & 1) << 2)) << 4)), in ? gsrc + (long long)min(mb + r, M - 1) * K + s * 32 : A, in);
+            }
+            const uint32_t sw = sa + uint32_t(rows * 128);
+            const uint4* const ws = W + (long long)s * (2 * NP * 32);
+            const int have = min(2, kt - 2 * s) * NP * 32;
+            for (int i = tid; i < have; i += blockDim.x) copy16(sw + uint32_t(i * 16), ws + i, true);
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    const int ra = min(m0 + g, M - 1), rb = min(m0 + g + 8, M - 1);
+    const float* const ga = gate + (long long)(ra / gate_rows) * K + t * 4;
+    const float* const gb = gate + (long long)(rb / gate_rows) * K + t * 4;
+    const float4 zero = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    auto gates = [&](float4 (&v)[2], int k) {
+        const bool in = k * 16 + t * 4 < K;
+        v[0] = in ? __ldg(reinterpret_cast<const float4*>(ga + k * 16)) : zero;
+        v[1] = in ? __ldg(reinterpret_cast<const float4*>(gb + k * 16)) : zero;
+    };
+    float acc[NT][4];
+#pragma unroll
+    for (int n = 0; n < NT; ++n)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) acc[n][e] = 0.0f;
+#pragma unroll
+    for (int s = 0; s < STAGES - 1; ++s) issue(s);
+    float4 gv[2];
+    gates(gv, 0);
+    const uint32_t arow = uint32_t((warp * 16 + g) * 128);
+    for (int s = 0; s < ns; ++s) {
+        asm volatile("cp.async.wait_group %0;" ::"n"(STAGES - 2) : "memory");
+        __syncthreads();                                  // stage s has landed, stage s - 1 is read
+        issue(s + STAGES - 1);
+        const uint8_t* const st = smem + (s % STAGES) * stage_bytes;
+        const uint4* const ws = reinterpret_cast<const uint4*>(st + rows * 128) + lane;
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            const int k = 2 * s + h;
+            if (k >= kt) break;
+            const uint32_t piece = uint32_t(((h * 4 + t) ^ ((g & 1) << 2)) << 4);
+            const float4 va = *reinterpret_cast<const float4*>(st + arow + piece), vb = *reinterpret_cast<const float4*>(st + arow + 8 * 128 + piece);
+            const uint32_t af[4] = {Half<HT>::pack(va.x * gv[0].x, va.y * gv[0].y), Half<HT>::pack(vb.x * gv[1].x, vb.y * gv[1].y),
+                                    Half<HT>::pack(va.z * gv[0].z, va.w * gv[0].w), Half<HT>::pack(vb.z * gv[1].z, vb.w * gv[1].w)};
+            gates(gv, k + 1);
+#pragma unroll
+            for (int n = 0; n < NP; ++n) {
+                const uint4 b = ws[(h * NP + n) * 32];
+                Half<HT>::mma(acc[2 * n], af, b.x, b.y);
+                if (2 * n + 1 < NT) Half<HT>::mma(acc[2 * n + 1 < NT ? 2 * n + 1 : 0], af, b.z, b.w);
+            }
+        }
+    }
+#pragma unroll
+    for (int n = 0; n < NT; ++n) {
+        const int col = n * 8 + 2 * t;
+        const float2 bv = __ldg(reinterpret_cast<const float2*>(bias + col));
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            const int m = m0 + g + h * 8;
+            if (m >= M) continue;
+            float2 v = make_float2(acc[n][2 * h] + bv.x, acc[n][2 * h + 1] + bv.y);
+            const long long at = (long long)m * N + col;
+            if (R) {
+                const float2 r = *reinterpret_cast<const float2*>(R + at);
+                v.x += r.x;
+                v.y += r.y;
+            }
+            *reinterpret_cast<float2*>(out + at) = v;
+        }
+    }
+}
+
 // The same with A already in the mode's 16-bit type [M][K], K a multiple of 32, no bias (the token projection).  A lane loads 16
 // bytes, eight values of k; the first of two mma must have the lower sixteen of their 32 k, as in the layer kernel (which k share an
 // mma shows in the rounding, their order in it does not), so lanes t and t + 2 exchange 8 bytes: 4 frames
@@ -1025,10 +1126,26 @@ int launch_rows_gate(const float* A, const uint4* W, const float* b, const float
         kernel<<<dim3(gx, gy), 128, 0, s>>>(A, W, b, gate, gate_rows, R, out, M, N, K);
         return int(cudaGetLastError());
     };
+    // Rows of a block, 16 a warp: what leaves the busiest SM the fewest rows
+    auto tiled = [&](auto kernel, auto layout) {
+        int warps = 8;
+        long long least = 1LL << 62;
+        for (int w = 8; w >= 4; --w) {
+            const long long rows = ((blocks_of(M, w * 16) + device_sms() - 1) / device_sms()) * (long long)w;
+            if (rows < least) { least = rows; warps = w; }
+        }
+        const int smem = decltype(layout)::STAGES * decltype(layout)::stage_bytes(warps);
+        const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, decltype(layout)::STAGES * decltype(layout)::stage_bytes(8));
+        if (e != cudaSuccess) return int(e);
+        kernel<<<blocks_of(M, warps * 16), warps * 32, smem, s>>>(A, W, b, gate, gate_rows, R, out, M, N, K);
+        return int(cudaGetLastError());
+    };
+    // 40 channels of 72: three stages are too few for the ring to help (256 / 640 frames, direct / ring: 26.5 / 28.6, 61.4 / 61.3);
+    // of 120: 67.5 / 57.4, 141 / 120; 112 of 480: 73.7 / 51, 170 / 118; 160 of 960: 69.6 / 48, 154 / 108
     switch (N) {
-    case 40: return few ? go(rows_gate_kernel<5, 4, HT>, 1) : go(rows_gate_kernel<5, 0, HT>, 1);
-    case 112: return few ? go(rows_gate_kernel<2, 6, HT>, 7) : go(rows_gate_kernel<14, 0, HT>, 1);
-    case 160: return few ? go(rows_gate_kernel<4, 6, HT>, 5) : go(rows_gate_kernel<20, 0, HT>, 1);
+    case 40: return few ? go(rows_gate_kernel<5, 4, HT>, 1) : K > 96 ? tiled(rows_gate_tile_kernel<5, HT>, RowsTile<5>()) : go(rows_gate_kernel<5, 0, HT>, 1);
+    case 112: return few ? go(rows_gate_kernel<2, 6, HT>, 7) : tiled(rows_gate_tile_kernel<14, HT>, RowsTile<14>());
+    case 160: return few ? go(rows_gate_kernel<4, 6, HT>, 5) : tiled(rows_gate_tile_kernel<20, HT>, RowsTile<20>());
     default: return int(cudaErrorInvalidValue);
     }
 }

@@ -387,6 +387,33 @@ def test_row_kernels_split_by_channels_give_the_same_rows(L, N, K, dtype):
 
 
 @pytest.mark.parametrize("dtype", [1, 2])
+@pytest.mark.parametrize("N,K", [(40, 120), (112, 100), (112, 672), (160, 36), (160, 960)])
+def test_row_kernel_tiles_give_the_same_rows(L, N, K, dtype):
+    """The gated projection of many rows reads through a ring of shared memory, in blocks of four to eight warps by the row count: the
+    bits of the form for few rows, with an odd number of k tiles and a ragged last one, frames of 60 rows and of 7, with and
+    without a residual, nothing written past the rows."""
+    import torch
+    st = torch.cuda.current_stream().cuda_stream
+    rng = np.random.default_rng(N * K)
+    big, part = 148 * 128 + 64 * 148 + 5, 9000                 # `part` rows are few
+    P = _pack(L, (rng.standard_normal((N, K)) / 16).astype(np.float32), 1, dtype, k_pad=(K + 15) // 16 * 16)
+    A, R, b = torch.randn(big, K, device="cuda"), torch.randn(big, N, device="cuda"), torch.randn(N, device="cuda")
+    for gate_rows, res in ((60, True), (7, False)):
+        G = torch.rand((big + gate_rows - 1) // gate_rows, K, device="cuda")
+        call = lambda a, g, r, out, m: L.shvk_cnn_rows_gate(a.data_ptr(), P.data_ptr(), b.data_ptr(), g.data_ptr(), gate_rows,  # noqa: E731
+                                                            r.data_ptr() if res else None, out.data_ptr(), m, N, K, dtype, st)
+        want = torch.empty(big, N, device="cuda")
+        step = part // (gate_rows * 4) * gate_rows * 4          # whole frames, 16-byte aligned
+        for m0 in range(0, big, step):
+            assert call(A[m0:], G[m0 // gate_rows:], R[m0:], want[m0:], min(step, big - m0)) == 0
+        for m in (big, 148 * 112, 148 * 96 + 1, 148 * 80 - 3, 148 * 144, 10321):
+            out = torch.full((big, N), 9.0, device="cuda")
+            assert call(A, G, R, out, m) == 0
+            torch.cuda.synchronize()
+            assert torch.equal(out[:m], want[:m]) and (out[m:] == 9.0).all()
+
+
+@pytest.mark.parametrize("dtype", [1, 2])
 @pytest.mark.parametrize("block", [2, 3, 4, 5, 7, 8, 9, 11, 12, 13, 14])
 def test_fused_block_matches_layers(L, block, dtype):
     """One fused block (expand + depthwise + project or pooled sums, gate, gated project) against the layer kernels on the same
