@@ -100,13 +100,13 @@ __device__ __forceinline__ void depthwise_pair(const float* e, const float2 (&w)
 
 // ---------------------------------------------------------------------------------------------------- inverted residual
 // CIN -> CEXP (1x1, activation) -> depthwise KS x KS, stride S, activation -> COUT (1x1, + residual); COUT = 0: stop after
-// the depthwise map (squeeze-excite blocks).  TH x TW output pixels per block of 256 threads, CE expanded channels at a time.
+// the depthwise map (squeeze-excite blocks).  TH x TW output pixels per block of THREADS threads, CE expanded channels at a time.
 template <int CIN_, int CEXP_, int COUT_, int KS_, int S_, int HI_, int WI_, int TH_, int TW_, int CE_, int PX_, int SR_, int NSPLIT_,
-          bool HS_, bool RES_, int MINB_>
+          bool HS_, bool RES_, bool AHEAD_, int MINB_, int THREADS_ = 256>
 struct Block {
     static constexpr int CIN = CIN_, CEXP = CEXP_, COUT = COUT_, KS = KS_, S = S_, HI = HI_, WI = WI_, TH = TH_, TW = TW_, CE = CE_;
-    static constexpr int PX = PX_, SR = SR_, NSPLIT = NSPLIT_, MINB = MINB_;
-    static constexpr bool HS = HS_, RES = RES_, SE = COUT_ == 0;
+    static constexpr int PX = PX_, SR = SR_, NSPLIT = NSPLIT_, MINB = MINB_, THREADS = THREADS_, WARPS = THREADS_ / 32;
+    static constexpr bool HS = HS_, RES = RES_, SE = COUT_ == 0, AHEAD = AHEAD_;
     static constexpr int PAD = (KS - 1) / 2, HO = (HI + 2 * PAD - KS) / S + 1, WO = (WI + 2 * PAD - KS) / S + 1;
     static constexpr int TY = (HO + TH - 1) / TH, TX = (WO + TW - 1) / TW, TILES = TY * TX;
     static constexpr int IH = (TH - 1) * S + KS, IW = (TW - 1) * S + KS;
@@ -118,8 +118,9 @@ struct Block {
     static constexpr int CHUNKS = (CEXP + CE - 1) / CE;
     static constexpr int OPX = TH * TW, OMT = (OPX + 15) / 16, ONT = cmax(COUT / 8, 1), CK = up(CE, 16), DP = CK + 8;
     static constexpr int KFILL = cmax((CK - CE) / 2, 1);                       // k padding of a chunk, in pairs
-    static constexpr int UNITS = OMT * ONT, UPW = SE ? 1 : (UNITS + 7) / 8;
+    static constexpr int UNITS = OMT * ONT, UPW = SE ? 1 : (UNITS + WARPS - 1) / WARPS;
     static constexpr int STRIPS = TH / SR, GX = TW / PX, ITEMS = CE / 2 * GX * STRIPS;
+    static constexpr bool EARLY = !SE && ITEMS <= THREADS;   // a thread has one item, its channels are known before the chunk is
     // squeeze-excite: the pooled sums are taken over groups of 64 pixels in row order, as se_partial_kernel takes them.  A tile that
     // consists of whole groups sums them itself (POOL)
     static constexpr int GROUP = 64, GROUPS = (HO * WO + GROUP - 1) / GROUP, TGROUPS = (TH * TW + GROUP - 1) / GROUP;
@@ -128,10 +129,11 @@ struct Block {
     static constexpr int E_BYTES = up(IH * IW * P * 4, 16), X_BYTES = up(MROWS * XP * 2, 16), T_BYTES = up(MROWS * 2, 16);
     static constexpr int D_BYTES = SE ? 0 : up(OMT * 16 * DP * 2, 16);
     static constexpr int SMEM = E_BYTES + X_BYTES + T_BYTES + D_BYTES;
-    static_assert(CE % 8 == 0 && NT % NSPLIT == 0 && 8 % NSPLIT == 0 && TW % PX == 0 && TH % SR == 0, "tile shape");
+    static_assert(CE % 8 == 0 && NT % NSPLIT == 0 && WARPS % NSPLIT == 0 && TW % PX == 0 && TH % SR == 0, "tile shape");
     static_assert(SE ? CEXP % CE == 0 : CK == CE || CHUNKS == 1, "channel chunks");
     static_assert(SE || COUT % 8 == 0, "output channels");
-    static_assert(!SE || ITEMS <= 256, "a thread keeps its outputs until the tile's map is consumed");
+    static_assert(!SE || ITEMS <= THREADS, "a thread keeps its outputs until the tile's map is consumed");
+    static_assert(VPX * VW < 65536, "pixel numbers");
     static_assert(!POOL || (TW % RUN == 0 && GROUP % RUN == 0), "groups");
 };
 
@@ -149,7 +151,7 @@ struct BlockArgs {
 };
 
 template <class C, typename HT>
-__global__ void __launch_bounds__(256, C::MINB) block_kernel(const BlockArgs a) {
+__global__ void __launch_bounds__(C::THREADS, C::MINB) block_kernel(const BlockArgs a) {
     extern __shared__ __align__(16) uint8_t smem[];
     float* const E = reinterpret_cast<float*>(smem);
     uint16_t* const X = reinterpret_cast<uint16_t*>(smem + C::E_BYTES);
@@ -165,23 +167,50 @@ __global__ void __launch_bounds__(256, C::MINB) block_kernel(const BlockArgs a) 
     const int first = C::SE ? blockIdx.y * a.chunks_per_group : 0;
     const int last = C::SE ? min(first + a.chunks_per_group, C::CHUNKS) : C::CHUNKS;
 
-    // input pixels of the tile, rounded to 16 bits; channels past CIN and the halo outside the image are zero
-    constexpr int Q4 = C::KP / 4;
-    for (int i = tid; i < nv * Q4; i += 256) {
-        const int r = i / Q4, q = i % Q4, vy = r / vw, vx = r - vy * vw;
-        uint2 v = make_uint2(0u, 0u);
-        if (C::CIN % 16 == 0 || q * 4 < C::CIN) {
-            const float4 p = *reinterpret_cast<const float4*>(img + ((vy0 + vy) * C::WI + vx0 + vx) * C::CIN + q * 4);
-            v = make_uint2(Half<HT>::pack(p.x, p.y), Half<HT>::pack(p.z, p.w));
+    // Input pixels of the tile, rounded to 16 bits; channels past CIN and the halo outside the image are zero.  Eight loads of a thread
+    // fly together: one at a time, a tile waited for 9 to 20 round trips to L2, a third of the time of blocks 2 to 4.
+    constexpr int Q4 = C::KP / 4, FLY = 8;
+    const uint32_t per_row = (65536u + vw - 1) / vw;     // r / vw = r * per_row >> 16, exact while r * vw < 65536
+    for (int i0 = tid; i0 < nv * Q4; i0 += FLY * C::THREADS) {
+        float4 p[FLY];
+        int at[FLY];
+#pragma unroll
+        for (int j = 0; j < FLY; ++j) {
+            const int i = i0 + j * C::THREADS, r = i / Q4, q = i % Q4, vy = int(uint32_t(r) * per_row >> 16), vx = r - vy * vw;
+            p[j] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+            at[j] = r * C::XP + q * 4;
+            if (i < nv * Q4) {
+                if (C::CIN % 16 == 0 || q * 4 < C::CIN)
+                    p[j] = __ldg(reinterpret_cast<const float4*>(img + ((vy0 + vy) * C::WI + vx0 + vx) * C::CIN + q * 4));
+                if (q == 0) pos[r] = uint16_t((vy0 - iy0 + vy) * C::IW + (vx0 - ix0 + vx));
+            }
         }
-        *reinterpret_cast<uint2*>(X + r * C::XP + q * 4) = v;
-        if (q == 0) pos[r] = uint16_t((vy0 - iy0 + vy) * C::IW + (vx0 - ix0 + vx));
+#pragma unroll
+        for (int j = 0; j < FLY; ++j)
+            if (i0 + j * C::THREADS < nv * Q4)
+                *reinterpret_cast<uint2*>(X + at[j]) = make_uint2(Half<HT>::pack(p[j].x, p[j].y), Half<HT>::pack(p[j].z, p[j].w));
     }
     if (nv < C::IH * C::IW)
-        for (int i = tid; i < C::E_BYTES / 16; i += 256) reinterpret_cast<uint4*>(E)[i] = make_uint4(0u, 0u, 0u, 0u);
+        for (int i = tid; i < C::E_BYTES / 16; i += C::THREADS) reinterpret_cast<uint4*>(E)[i] = make_uint4(0u, 0u, 0u, 0u);
     if (!C::SE && C::CK != C::CE)                    // projection k padding of a single chunk
-        for (int i = tid; i < C::OMT * 16 * C::KFILL; i += 256)
+        for (int i = tid; i < C::OMT * 16 * C::KFILL; i += C::THREADS)
             reinterpret_cast<uint32_t*>(D)[i / C::KFILL * (C::DP / 2) + C::CE / 2 + i % C::KFILL] = 0u;
+    // Expand weights and biases of this warp's n tiles of a chunk.  AHEAD: asked for a phase early, before the barrier that ends the
+    // previous chunk's filter, where the registers allow (blocks 7 / 8 / 11 / 12 / 13, 640 frames: 203 / 140 / 207 / 308 / 241 us without,
+    // 195 / 132 / 195 / 290 / 229 with; blocks 4, 5 and 14 spill or gain nothing)
+    const int ns = warp % C::NSPLIT;
+    uint2 b[C::NW][C::KT];
+    float2 bias[C::NW];
+    auto load_expand = [&](int ch) {
+#pragma unroll
+        for (int n = 0; n < C::NW; ++n) {
+            const int nt = ch * C::NT + ns * C::NW + n, col = nt * 8 + 2 * t;
+#pragma unroll
+            for (int k = 0; k < C::KT; ++k) b[n][k] = __ldg(a.we + (nt * C::KT + k) * 32 + lane);
+            bias[n] = C::CEXP % C::CE == 0 || col < C::CEXP ? __ldg(reinterpret_cast<const float2*>(a.be + col)) : make_float2(0.0f, 0.0f);
+        }
+    };
+    if (C::AHEAD) load_expand(first);
     float pacc[C::UPW][4];
 #pragma unroll
     for (int u = 0; u < C::UPW; ++u)
@@ -189,21 +218,13 @@ __global__ void __launch_bounds__(256, C::MINB) block_kernel(const BlockArgs a) 
         for (int e = 0; e < 4; ++e) pacc[u][e] = 0.0f;
     __syncthreads();
 
-    const int ns = warp % C::NSPLIT, mtiles = (nv + 15) >> 4;
+    const int mtiles = (nv + 15) >> 4;
     const uint32_t xrow = smem_addr(X) + uint32_t(((lane & 15) * C::XP + (lane >> 4) * 8) * 2);
     for (int ch = first; ch < last; ++ch) {
-        // ---- expand: this warp's n tiles of the chunk for every (8 / NSPLIT)-th group of 16 input pixels
+        // ---- expand: this warp's n tiles of the chunk for every (WARPS / NSPLIT)-th group of 16 input pixels
         {
-            uint2 b[C::NW][C::KT];
-            float2 bias[C::NW];
-#pragma unroll
-            for (int n = 0; n < C::NW; ++n) {
-                const int nt = ch * C::NT + ns * C::NW + n, col = nt * 8 + 2 * t;
-#pragma unroll
-                for (int k = 0; k < C::KT; ++k) b[n][k] = __ldg(a.we + (nt * C::KT + k) * 32 + lane);
-                bias[n] = C::CEXP % C::CE == 0 || col < C::CEXP ? __ldg(reinterpret_cast<const float2*>(a.be + col)) : make_float2(0.0f, 0.0f);
-            }
-            for (int mt = warp / C::NSPLIT; mt < mtiles; mt += 8 / C::NSPLIT) {
+            if (!C::AHEAD) load_expand(ch);
+            for (int mt = warp / C::NSPLIT; mt < mtiles; mt += C::WARPS / C::NSPLIT) {
                 float c[C::NW][4];
 #pragma unroll
                 for (int n = 0; n < C::NW; ++n)
@@ -227,6 +248,15 @@ __global__ void __launch_bounds__(256, C::MINB) block_kernel(const BlockArgs a) 
                 }
             }
         }
+        float2 w0[C::KS * C::KS], bias0;                     // depthwise weights, asked for before the barrier
+        if constexpr (C::EARLY) {
+            const int col = ch * C::CE + tid % (C::CE / 2) * 2;
+            if (C::CEXP % C::CE == 0 || col < C::CEXP) {
+#pragma unroll
+                for (int k = 0; k < C::KS * C::KS; ++k) w0[k] = __ldg(reinterpret_cast<const float2*>(a.wd + k * C::CEXP + col));
+                bias0 = __ldg(reinterpret_cast<const float2*>(a.bd + col));
+            }
+        }
         __syncthreads();
         // ---- depthwise
         auto depthwise = [&](int i, float2 (&v)[C::SR][C::PX], int& oy, int& ox, int& cp) {
@@ -241,10 +271,16 @@ __global__ void __launch_bounds__(256, C::MINB) block_kernel(const BlockArgs a) 
                     for (int p = 0; p < C::PX; ++p) v[r][p] = make_float2(0.0f, 0.0f);
                 return;
             }
-            float2 w[C::KS * C::KS];
+            float2 w[C::KS * C::KS], bias;
+            if constexpr (C::EARLY) {
 #pragma unroll
-            for (int k = 0; k < C::KS * C::KS; ++k) w[k] = __ldg(reinterpret_cast<const float2*>(a.wd + k * C::CEXP + col));
-            const float2 bias = __ldg(reinterpret_cast<const float2*>(a.bd + col));
+                for (int k = 0; k < C::KS * C::KS; ++k) w[k] = w0[k];
+                bias = bias0;
+            } else {
+#pragma unroll
+                for (int k = 0; k < C::KS * C::KS; ++k) w[k] = __ldg(reinterpret_cast<const float2*>(a.wd + k * C::CEXP + col));
+                bias = __ldg(reinterpret_cast<const float2*>(a.bd + col));
+            }
             depthwise_pair<C::KS, C::S, C::PX, C::SR, C::P, C::IW>(E + (oy * C::S * C::IW + ox * C::S) * C::P + cp * 2, w, v);
 #pragma unroll
             for (int r = 0; r < C::SR; ++r)
@@ -254,7 +290,7 @@ __global__ void __launch_bounds__(256, C::MINB) block_kernel(const BlockArgs a) 
         float2 v[C::SR][C::PX];
         int oy, ox, cp;
         if constexpr (C::SE) {
-            const bool mine = C::ITEMS == 256 || tid < C::ITEMS;
+            const bool mine = C::ITEMS == C::THREADS || tid < C::ITEMS;
             auto inside = [&](int r, int p) { return (C::HO % C::TH == 0 || oy0 + oy + r < C::HO) && (C::WO % C::TW == 0 || ox0 + ox + p < C::WO); };
             if (mine) {
                 depthwise(tid, v, oy, ox, cp);
@@ -265,6 +301,7 @@ __global__ void __launch_bounds__(256, C::MINB) block_kernel(const BlockArgs a) 
                         if (inside(r, p))
                             *reinterpret_cast<float2*>(a.out + ((long long)(f * C::HO + oy0 + oy + r) * C::WO + ox0 + ox + p) * C::CEXP + ch * C::CE + cp * 2) = v[r][p];
             }
+            if (C::AHEAD && ch + 1 < last) load_expand(ch + 1);
             __syncthreads();                             // the expanded chunk is consumed
             if constexpr (C::POOL) {
                 // the outputs take the places of expanded pixels of the image (the next chunk writes those again, the halo stays zero)
@@ -280,7 +317,7 @@ __global__ void __launch_bounds__(256, C::MINB) block_kernel(const BlockArgs a) 
                 // threads, which rounds otherwise, 235 / 195 / 268 / 218 / 158; block 4, whose tiles cut the groups, is read again
                 // (332 -> 364).
                 const int n = C::HO % C::TH == 0 ? C::TH * C::TW : min(C::TH, C::HO - oy0) * C::TW;
-                for (int i = tid; i < C::CE * C::TGROUPS; i += 256) {
+                for (int i = tid; i < C::CE * C::TGROUPS; i += C::THREADS) {
                     const int c = i % C::CE, s = C::TGROUPS == 1 ? 0 : i / C::CE;
                     float part[8];
 #pragma unroll
@@ -301,7 +338,7 @@ __global__ void __launch_bounds__(256, C::MINB) block_kernel(const BlockArgs a) 
                 __syncthreads();
             }
         } else {
-            for (int i = tid; i < C::ITEMS; i += 256) {
+            for (int i = tid; i < C::ITEMS; i += C::THREADS) {
                 depthwise(i, v, oy, ox, cp);
 #pragma unroll
                 for (int r = 0; r < C::SR; ++r)
@@ -309,6 +346,7 @@ __global__ void __launch_bounds__(256, C::MINB) block_kernel(const BlockArgs a) 
                     for (int p = 0; p < C::PX; ++p)
                         reinterpret_cast<uint32_t*>(D)[((oy + r) * C::TW + ox + p) * (C::DP / 2) + cp] = Half<HT>::pack(v[r][p].x, v[r][p].y);
             }
+            if (C::AHEAD && ch + 1 < last) load_expand(ch + 1);
             __syncthreads();
             // ---- projection: this chunk's k range into the accumulators of the warp's (pixel group, n tile) units
             const uint32_t drow = smem_addr(D) + uint32_t(((lane & 15) * C::DP + (lane >> 4) * 8) * 2);
@@ -317,8 +355,8 @@ __global__ void __launch_bounds__(256, C::MINB) block_kernel(const BlockArgs a) 
             for (int k = 0; k < KC; ++k)
 #pragma unroll
                 for (int u = 0; u < C::UPW; ++u) {
-                    const int unit = warp + u * 8;
-                    if (C::UNITS % 8 != 0 && unit >= C::UNITS) break;
+                    const int unit = warp + u * C::WARPS;
+                    if (C::UNITS % C::WARPS != 0 && unit >= C::UNITS) break;
                     uint32_t af[4];
                     ldmatrix_x4(af, drow + uint32_t(((unit % C::OMT) * 16 * C::DP + k * 16) * 2));
                     const uint2 b = __ldg(a.wp + ((unit / C::OMT) * KALL + ch * KC + k) * 32 + lane);
@@ -329,8 +367,8 @@ __global__ void __launch_bounds__(256, C::MINB) block_kernel(const BlockArgs a) 
     if constexpr (C::SE) return;
 #pragma unroll
     for (int u = 0; u < C::UPW; ++u) {
-        const int unit = warp + u * 8;
-        if (C::UNITS % 8 != 0 && unit >= C::UNITS) break;
+        const int unit = warp + u * C::WARPS;
+        if (C::UNITS % C::WARPS != 0 && unit >= C::UNITS) break;
         const int n = unit / C::OMT * 8 + 2 * t;
         const float2 bias = __ldg(reinterpret_cast<const float2*>(a.bp + n));
 #pragma unroll
@@ -920,18 +958,18 @@ last_pool_kernel(const float* __restrict__ x, const uint2* __restrict__ w, const
     }
 }
 
-//                CIN CEXP COUT K  S  HI  WI  TH  TW  CE PX SR NS  HS     RES   blocks/SM
-using B2 = Block<16, 64, 24, 3, 2, 90, 160, 9, 8, 32, 2, 3, 1, false, false, 3>;
-using B3 = Block<24, 72, 24, 3, 1, 45, 80, 9, 16, 72, 4, 3, 1, false, true, 2>;
-using B4 = Block<24, 72, 0, 5, 2, 45, 80, 12, 10, 24, 2, 3, 1, false, false, 2>;
-using B5 = Block<40, 120, 0, 5, 1, 23, 40, 8, 40, 24, 4, 4, 1, false, false, 2>;
-using B7 = Block<40, 240, 80, 3, 2, 23, 40, 6, 10, 48, 2, 3, 1, true, false, 2>;
-using B8 = Block<80, 200, 80, 3, 1, 12, 20, 6, 20, 32, 4, 3, 2, true, true, 2>;
-using B9 = Block<80, 184, 80, 3, 1, 12, 20, 6, 20, 32, 4, 3, 2, true, true, 2>;
-using B11 = Block<80, 480, 0, 3, 1, 12, 20, 12, 20, 32, 4, 4, 2, true, false, 2>;
-using B12 = Block<112, 672, 0, 3, 1, 12, 20, 12, 20, 32, 4, 4, 2, true, false, 2>;
-using B13 = Block<112, 672, 0, 5, 2, 12, 20, 6, 10, 32, 2, 2, 2, true, false, 2>;
-using B14 = Block<160, 960, 0, 5, 1, 6, 10, 6, 10, 64, 5, 3, 4, true, false, 2>;
+//                CIN CEXP COUT K  S  HI  WI  TH  TW  CE PX SR NS  HS     RES    AHEAD  blocks/SM
+using B2 = Block<16, 64, 24, 3, 2, 90, 160, 9, 8, 32, 2, 3, 1, false, false, true, 3>;
+using B3 = Block<24, 72, 24, 3, 1, 45, 80, 9, 16, 72, 4, 3, 3, false, true, true, 2, 384>;
+using B4 = Block<24, 72, 0, 5, 2, 45, 80, 6, 10, 24, 2, 3, 1, false, false, false, 3>;
+using B5 = Block<40, 120, 0, 5, 1, 23, 40, 8, 40, 24, 4, 4, 1, false, false, false, 2>;
+using B7 = Block<40, 240, 80, 3, 2, 23, 40, 6, 10, 48, 2, 3, 1, true, false, true, 2>;
+using B8 = Block<80, 200, 80, 3, 1, 12, 20, 6, 20, 32, 4, 3, 2, true, true, true, 2>;
+using B9 = Block<80, 184, 80, 3, 1, 12, 20, 6, 20, 32, 4, 3, 2, true, true, true, 2>;
+using B11 = Block<80, 480, 0, 3, 1, 12, 20, 12, 20, 32, 4, 4, 2, true, false, true, 2>;
+using B12 = Block<112, 672, 0, 3, 1, 12, 20, 12, 20, 32, 4, 4, 2, true, false, true, 2>;
+using B13 = Block<112, 672, 0, 5, 2, 12, 20, 6, 10, 32, 2, 2, 2, true, false, true, 2>;
+using B14 = Block<160, 960, 0, 5, 1, 6, 10, 6, 10, 64, 5, 3, 4, true, false, false, 2>;
 
 inline unsigned blocks_of(long long n, int per) { return unsigned((n + per - 1) / per); }
 inline bool unaligned(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) != 0; }
@@ -950,7 +988,7 @@ int launch_block(const BlockArgs& args, int F, cudaStream_t s) {
         a.chunks_per_group = (C::CHUNKS + groups - 1) / groups;
         grid.y = unsigned((C::CHUNKS + a.chunks_per_group - 1) / a.chunks_per_group);
     }
-    block_kernel<C, HT><<<grid, 256, C::SMEM, s>>>(a);
+    block_kernel<C, HT><<<grid, C::THREADS, C::SMEM, s>>>(a);
     e = cudaGetLastError();
     if (e != cudaSuccess || !C::SE || C::POOL) return int(e);
     return se_partial_sums(a.out, a.sums, F, C::HO * C::WO, C::CEXP, s);
