@@ -389,16 +389,19 @@ __global__ void __launch_bounds__(C::THREADS, C::MINB) block_kernel(const BlockA
 
 // ---------------------------------------------------------------------------------------------------- stem + first block
 // uint8 crop -> normalisation -> 3x3/2 convolution 3 -> 16, Hardswish -> depthwise 3x3, ReLU -> 1x1 16 -> 16, + the stem's
-// output.  A block takes 10 x 32 output pixels: the 25 x 69 input pixels are looked up once into float32, the stem runs one
-// thread per pixel with its filter as kernel parameters (an FMA takes one operand from the constant bank, so a tap costs no
-// load), and its map stays in shared memory.
+// output.  A block takes 10 x 32 output pixels: the 25 x 69 input pixels are looked up once into float32, the stem runs two
+// pixels a thread with its filter as kernel parameters (an FMA takes one operand from the constant bank, so a tap costs no
+// load; from shared memory it takes 670 us instead of 558), and its map stays in shared memory.  It is bound by issue: crops come
+// as words (a byte at a time the index arithmetic was a third of it), four words a store, all loads of a thread in flight, four
+// blocks an SM (three: 595).  640 crops 724 -> 558 us.
 struct StemParams {
     float w[27 * 16];          // ((ky * 3 + kx) * 3 + ci) * 16 + co
     float b[16];
 };
 struct Stem {
     static constexpr int H = 90, W = 160, IMH = 180, IMW = 320, TH = 10, TW = 32, TILES = (H / TH) * (W / TW);
-    static constexpr int SH = TH + 2, SW = TW + 2, UH = 2 * SH + 1, UW = 2 * SW + 1, UP = UW * 3 + 1;   // stem map and input tile
+    static constexpr int SH = TH + 2, SW = TW + 2, UH = 2 * SH + 1, UW = 2 * SW + 1;   // stem map and input tile
+    static constexpr int ULEAD = 3, UWORDS = (ULEAD + UW * 3 + 3) / 4, UP = UWORDS * 4;   // a tile row: whole words of the crop's row, the first ULEAD bytes unused
     static constexpr int P = 20, DP = 24, PX = 2, SR = 5;
     static constexpr int OMT = TH * TW / 16;
     static constexpr int S_BYTES = SH * SW * P * 4, U_BYTES = up(UH * UP * 4, 16), D_BYTES = TH * TW * DP * 2;
@@ -406,7 +409,7 @@ struct Stem {
 };
 
 template <typename HT>
-__global__ void __launch_bounds__(256, 3)
+__global__ void __launch_bounds__(256, 4)
 stem_block_kernel(const uint8_t* __restrict__ frames, const float* __restrict__ lut, const __grid_constant__ StemParams sp,
                   const float* __restrict__ wd, const float* __restrict__ bd, const uint2* __restrict__ wp,
                   const float* __restrict__ bp, float* __restrict__ out) {
@@ -419,35 +422,82 @@ stem_block_kernel(const uint8_t* __restrict__ frames, const float* __restrict__ 
     const int f = blockIdx.x / Stem::TILES, tile = blockIdx.x % Stem::TILES;
     const int oy0 = tile / (Stem::W / Stem::TW) * Stem::TH, ox0 = tile % (Stem::W / Stem::TW) * Stem::TW;
     const uint8_t* const img = frames + (long long)f * (Stem::IMH * Stem::IMW * 3);
-    for (int i = tid; i < 768; i += 256) L[i] = lut[i];
-    __syncthreads();
-    // stem pixel (sy, sx) of the tile is map pixel (oy0 - 1 + sy, ox0 - 1 + sx); its taps start at crop pixel 2 (.) - 1
+    // stem pixel (sy, sx) of the tile is map pixel (oy0 - 1 + sy, ox0 - 1 + sx); its taps start at crop pixel 2 (.) - 1.  A thread's
+    // words of the tile are all asked for before the first is looked up
     const int uy0 = 2 * (oy0 - 1) - 1, ux0 = 2 * (ox0 - 1) - 1;
-    for (int i = tid; i < Stem::UH * Stem::UW * 3; i += 256) {
-        const int r = i / (Stem::UW * 3), c = i % (Stem::UW * 3), y = uy0 + r, x3 = ux0 * 3 + c;
-        float v = 0.0f;
-        if (y >= 0 && y < Stem::IMH && x3 >= 0 && x3 < Stem::IMW * 3) v = L[(c % 3) * 256 + img[y * (Stem::IMW * 3) + x3]];
-        U[r * Stem::UP + c] = v;
+    const bool words = (reinterpret_cast<uintptr_t>(frames) & 3) == 0;       // a crop's rows and a tile's first column are whole words then
+    constexpr int WORDS = Stem::UH * Stem::UWORDS, EACH = (WORDS + 255) / 256;
+    uint32_t raw[EACH];
+    auto word_at = [&](int i, int& x3, int& y) {
+        y = uy0 + i / Stem::UWORDS;
+        x3 = ux0 * 3 - Stem::ULEAD + 4 * (i % Stem::UWORDS);
+        return i < WORDS && y >= 0 && y < Stem::IMH && x3 >= 0 && x3 < Stem::IMW * 3;
+    };
+#pragma unroll
+    for (int j = 0; j < EACH; ++j) {
+        int x3, y;
+        raw[j] = 0;
+        if (word_at(tid + j * 256, x3, y)) {
+            const uint8_t* const at = img + y * (Stem::IMW * 3) + x3;
+            raw[j] = words ? __ldg(reinterpret_cast<const uint32_t*>(at)) : at[0] | at[1] << 8 | at[2] << 16 | uint32_t(at[3]) << 24;
+        }
+    }
+    for (int i = tid; i < 768; i += 256) L[i] = __ldg(lut + i);
+    __syncthreads();
+#pragma unroll
+    for (int j = 0; j < EACH; ++j) {
+        const int i = tid + j * 256, w = i % Stem::UWORDS;
+        if (EACH * 256 != WORDS && i >= WORDS) break;
+        int x3, y;
+        float4 v = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        if (word_at(i, x3, y)) {
+            const uint32_t q = raw[j];
+            const float* const l0 = L + w % 3 * 256;                          // byte k of the word has colour (w + k) % 3
+            const float* const l1 = L + (w + 1) % 3 * 256;
+            const float* const l2 = L + (w + 2) % 3 * 256;
+            v = make_float4(l0[q & 255], l1[q >> 8 & 255], l2[q >> 16 & 255], l0[q >> 24]);
+        }
+        *reinterpret_cast<float4*>(U + i / Stem::UWORDS * Stem::UP + 4 * w) = v;
     }
     __syncthreads();
-    for (int i = tid; i < Stem::SH * Stem::SW; i += 256) {
-        const int sy = i / Stem::SW, sx = i % Stem::SW, y = oy0 - 1 + sy, x = ox0 - 1 + sx;
-        float acc[16];
+    // two pixels of a row a thread: a weight pair serves both
+    for (int i2 = tid; i2 < Stem::SH * Stem::SW / 2; i2 += 256) {
+        const int sy = i2 / (Stem::SW / 2), sx = i2 % (Stem::SW / 2) * 2;
+        float2 acc[2][8];
 #pragma unroll
-        for (int c = 0; c < 16; ++c) acc[c] = 0.0f;
-        const float* const u = U + 2 * sy * Stem::UP + 6 * sx;
+        for (int p = 0; p < 2; ++p)
 #pragma unroll
-        for (int k = 0; k < 27; ++k) {
-            const float v = u[(k / 9) * Stem::UP + k % 9];
+            for (int c = 0; c < 8; ++c) acc[p][c] = make_float2(0.0f, 0.0f);
+        const float* const u = U + 2 * sy * Stem::UP + Stem::ULEAD + 6 * sx;
 #pragma unroll
-            for (int c = 0; c < 16; ++c) acc[c] = fmaf(sp.w[k * 16 + c], v, acc[c]);
+        for (int ky = 0; ky < 3; ++ky) {
+            float x[15];                                                      // the row's values of both pixels; all but the first in pairs
+            x[0] = u[ky * Stem::UP];
+#pragma unroll
+            for (int j = 1; j < 15; j += 2) {
+                const float2 q = *reinterpret_cast<const float2*>(u + ky * Stem::UP + j);
+                x[j] = q.x;
+                x[j + 1] = q.y;
+            }
+#pragma unroll
+            for (int k = 0; k < 9; ++k)
+#pragma unroll
+                for (int c = 0; c < 8; ++c) {
+                    const float2 w = make_float2(sp.w[(ky * 9 + k) * 16 + 2 * c], sp.w[(ky * 9 + k) * 16 + 2 * c + 1]);
+#pragma unroll
+                    for (int p = 0; p < 2; ++p) acc[p][c] = fma2(w, make_float2(x[k + 6 * p], x[k + 6 * p]), acc[p][c]);
+                }
         }
-        const bool in = y >= 0 && y < Stem::H && x >= 0 && x < Stem::W;       // the depthwise filter sees zeros outside the map
 #pragma unroll
-        for (int q = 0; q < 4; ++q) {
-            const float2 lo = hswish2(make_float2(acc[4 * q] + sp.b[4 * q], acc[4 * q + 1] + sp.b[4 * q + 1]));
-            const float2 hi = hswish2(make_float2(acc[4 * q + 2] + sp.b[4 * q + 2], acc[4 * q + 3] + sp.b[4 * q + 3]));
-            *reinterpret_cast<float4*>(M + i * Stem::P + q * 4) = in ? make_float4(lo.x, lo.y, hi.x, hi.y) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        for (int p = 0; p < 2; ++p) {
+            const int y = oy0 - 1 + sy, x = ox0 - 1 + sx + p;
+            const bool in = y >= 0 && y < Stem::H && x >= 0 && x < Stem::W;       // the depthwise filter sees zeros outside the map
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+                const float2 lo = hswish2(add2(acc[p][2 * q], make_float2(sp.b[4 * q], sp.b[4 * q + 1])));
+                const float2 hi = hswish2(add2(acc[p][2 * q + 1], make_float2(sp.b[4 * q + 2], sp.b[4 * q + 3])));
+                *reinterpret_cast<float4*>(M + (sy * Stem::SW + sx + p) * Stem::P + q * 4) = in ? make_float4(lo.x, lo.y, hi.x, hi.y) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+            }
         }
     }
     __syncthreads();

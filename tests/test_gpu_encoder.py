@@ -616,6 +616,25 @@ def test_fused_ends_give_the_bits_of_the_layers(L, dtype):
     assert torch.equal(low, pooled.to(tdt))
 
 
+def test_stem_block_takes_crops_at_any_address(L):
+    """Crops are read in words where their address allows, in bytes where it does not: the same map."""
+    import torch
+    frames = torch.randint(0, 256, (2, 180, 320, 3), device="cuda", dtype=torch.uint8)
+    lut, wd, bd, bp = (torch.randn(*n, device="cuda") for n in ((3, 256), (9, 16), (16,), (16,)))
+    ws, bs = np.random.default_rng(1).standard_normal((27, 16)).astype(np.float32), np.zeros(16, np.float32)
+    p_wp = _pack(L, np.random.default_rng(2).standard_normal((16, 16)).astype(np.float32), 0, 1)
+    outs = []
+    for shift in range(4):
+        moved = torch.zeros(frames.numel() + 4, device="cuda", dtype=torch.uint8)
+        moved[shift:shift + frames.numel()] = frames.reshape(-1)
+        out = torch.empty(2, 90, 160, 16, device="cuda")
+        assert L.shvk_cnn_stem_block(moved.data_ptr() + shift, _ptr(lut), ws.ctypes.data, bs.ctypes.data, _ptr(wd), _ptr(bd), _ptr(p_wp), _ptr(bp),
+                                     _ptr(out), 2, 1, stream_ptr()) == 0
+        sync()
+        outs.append(out)
+    assert all(torch.equal(o, outs[0]) for o in outs[1:])
+
+
 @pytest.mark.parametrize("dtype", [1, 2])
 @pytest.mark.parametrize("rows", [16, 80, 77, 5136])
 def test_token_projection_gives_the_bits_of_the_layer(L, rows, dtype):
