@@ -117,6 +117,7 @@ struct Block {
     static constexpr int P = CE % 16 == 8 ? CE : CE + 8;                     // fp32 pitch = 8 mod 16 words: expand's stores miss each other's banks
     static constexpr int CHUNKS = (CEXP + CE - 1) / CE;
     static constexpr int OPX = TH * TW, OMT = (OPX + 15) / 16, ONT = cmax(COUT / 8, 1), CK = up(CE, 16), DP = CK + 8;
+    static constexpr int KPAD = SE ? CEXP : up(CEXP, 64);                      // k of the projection weights as they are packed, for any CE
     static constexpr int KFILL = cmax((CK - CE) / 2, 1);                       // k padding of a chunk, in pairs
     static constexpr int UNITS = OMT * ONT, UPW = SE ? 1 : (UNITS + WARPS - 1) / WARPS;
     static constexpr int STRIPS = TH / SR, GX = TW / PX, ITEMS = CE / 2 * GX * STRIPS;
@@ -131,7 +132,7 @@ struct Block {
     static constexpr int SMEM = E_BYTES + X_BYTES + T_BYTES + D_BYTES;
     static_assert(CE % 8 == 0 && NT % NSPLIT == 0 && WARPS % NSPLIT == 0 && TW % PX == 0 && TH % SR == 0, "tile shape");
     static_assert(SE ? CEXP % CE == 0 : CK == CE || CHUNKS == 1, "channel chunks");
-    static_assert(SE || COUT % 8 == 0, "output channels");
+    static_assert(SE || (COUT % 8 == 0 && CHUNKS * CK <= KPAD), "output channels");
     static_assert(!SE || ITEMS <= THREADS, "a thread keeps its outputs until the tile's map is consumed");
     static_assert(VPX * VW < 65536, "pixel numbers");
     static_assert(!POOL || (TW % RUN == 0 && GROUP % RUN == 0), "groups");
@@ -350,7 +351,7 @@ __global__ void __launch_bounds__(C::THREADS, C::MINB) block_kernel(const BlockA
             __syncthreads();
             // ---- projection: this chunk's k range into the accumulators of the warp's (pixel group, n tile) units
             const uint32_t drow = smem_addr(D) + uint32_t(((lane & 15) * C::DP + (lane >> 4) * 8) * 2);
-            constexpr int KC = C::CK / 16, KALL = C::CHUNKS * KC;
+            constexpr int KC = C::CK / 16, KALL = C::KPAD / 16;
 #pragma unroll
             for (int k = 0; k < KC; ++k)
 #pragma unroll
@@ -1015,6 +1016,12 @@ using B4 = Block<24, 72, 0, 5, 2, 45, 80, 6, 10, 24, 2, 3, 1, false, false, fals
 using B5 = Block<40, 120, 0, 5, 1, 23, 40, 8, 40, 24, 4, 4, 1, false, false, false, 2>;
 using B7 = Block<40, 240, 80, 3, 2, 23, 40, 6, 10, 48, 2, 3, 1, true, false, true, 2>;
 using B8 = Block<80, 200, 80, 3, 1, 12, 20, 6, 20, 32, 4, 3, 2, true, true, true, 2>;
+// few frames: smaller tiles, so that more SMs work, and for the fewest more channels at a time, so that fewer phases stand in a row
+using B7F = Block<40, 240, 80, 3, 2, 23, 40, 3, 10, 80, 2, 3, 2, true, false, true, 2>;
+using B8F = Block<80, 200, 80, 3, 1, 12, 20, 6, 10, 32, 2, 3, 2, true, true, true, 2>;
+using B8S = Block<80, 200, 80, 3, 1, 12, 20, 3, 10, 64, 2, 3, 2, true, true, true, 2>;
+using B9F = Block<80, 184, 80, 3, 1, 12, 20, 6, 10, 32, 2, 3, 2, true, true, true, 2>;
+using B9S = Block<80, 184, 80, 3, 1, 12, 20, 3, 10, 64, 2, 3, 4, true, true, true, 2>;
 using B9 = Block<80, 184, 80, 3, 1, 12, 20, 6, 20, 32, 4, 3, 2, true, true, true, 2>;
 using B11 = Block<80, 480, 0, 3, 1, 12, 20, 12, 20, 32, 4, 4, 2, true, false, true, 2>;
 using B12 = Block<112, 672, 0, 3, 1, 12, 20, 12, 20, 32, 4, 4, 2, true, false, true, 2>;
@@ -1032,9 +1039,17 @@ int launch_block(const BlockArgs& args, int F, cudaStream_t s) {
     BlockArgs a = args;
     dim3 grid(unsigned(F) * C::TILES, 1);
     if (C::SE) {
-        // a block redoes the tile's input for its share of the channels: as few shares as give the GPU four blocks per SM
-        const int want = int((4LL * device_sms() + grid.x - 1) / grid.x);
-        const int groups = want < 1 ? 1 : want > C::CHUNKS ? C::CHUNKS : want;
+        // A block redoes the tile's input for its share of the channels, which costs about as much as three quarters of a chunk.  As many shares
+        // as make the busiest SM's time least: n blocks there take n / 2 pairs, which share the SM at 1.25 times the time of one,
+        // and the odd one.  us, one share / as the rule has it / 3 / 7: block 12, 48 frames 84 / 31 / 35 / 37, 96 frames 85 / 47 / 47 / 55, 256
+        // frames 117 / 117 / 127 / 131, 640 frames 304 / 280 / 283 / 346.
+        int groups = 1;
+        float least = 1e30f;
+        for (int g = 1; g <= C::CHUNKS; ++g) {
+            const long long n = (grid.x * (long long)g + device_sms() - 1) / device_sms();
+            const float t = ((C::CHUNKS + g - 1) / g + 0.75f) * (1.25f * float(n / 2) + float(n % 2));
+            if (t < least * 0.999f) { least = t; groups = g; }
+        }
         a.chunks_per_group = (C::CHUNKS + groups - 1) / groups;
         grid.y = unsigned((C::CHUNKS + a.chunks_per_group - 1) / a.chunks_per_group);
     }
@@ -1044,6 +1059,7 @@ int launch_block(const BlockArgs& args, int F, cudaStream_t s) {
     return se_partial_sums(a.out, a.sums, F, C::HO * C::WO, C::CEXP, s);
 }
 
+inline bool one_wave(long long blocks, int per_sm) { return blocks <= (long long)per_sm * device_sms(); }
 template <typename HT>
 int dispatch_block(int block, const BlockArgs& a, int F, cudaStream_t s) {
     switch (block) {
@@ -1051,9 +1067,16 @@ int dispatch_block(int block, const BlockArgs& a, int F, cudaStream_t s) {
     case 3: return launch_block<B3, HT>(a, F, s);
     case 4: return launch_block<B4, HT>(a, F, s);
     case 5: case 6: return launch_block<B5, HT>(a, F, s);
-    case 7: return launch_block<B7, HT>(a, F, s);
-    case 8: return launch_block<B8, HT>(a, F, s);
-    case 9: case 10: return launch_block<B9, HT>(a, F, s);
+    // Whole blocks of the deeper maps have two to four tiles a frame, too few to fill the GPU with few frames.  us, large tiles / F / S:
+    // block 7: 12 frames 20.2 / 16.1, 24 20.4 / 18, 40 27.9 / 26.2, 64 28.4 / 31.2; block 8: 12 26.2 / 17 / 14, 24 26 / 17.9 / 18,
+    // 40 26.3 / 22.1 / 25.9, 64 26.1 / 22.1 / 30.5, 96 32.6 / 37.3.  The lines: two blocks an SM, and for S one.
+    case 7: return one_wave(B7F::TILES * F, 2) ? launch_block<B7F, HT>(a, F, s) : launch_block<B7, HT>(a, F, s);
+    case 8:
+        return one_wave(B8S::TILES * F, 1) ? launch_block<B8S, HT>(a, F, s)
+             : one_wave(B8F::TILES * F, 2) ? launch_block<B8F, HT>(a, F, s) : launch_block<B8, HT>(a, F, s);
+    case 9: case 10:
+        return one_wave(B9S::TILES * F, 1) ? launch_block<B9S, HT>(a, F, s)
+             : one_wave(B9F::TILES * F, 2) ? launch_block<B9F, HT>(a, F, s) : launch_block<B9, HT>(a, F, s);
     case 11: return launch_block<B11, HT>(a, F, s);
     case 12: return launch_block<B12, HT>(a, F, s);
     case 13: return launch_block<B13, HT>(a, F, s);
@@ -1074,7 +1097,7 @@ int block_groups(int block) {
 }
 // expanded channels a block walks (a multiple of its chunk), and the k range of its projection
 void block_padding(int block, int* cols, int* k) {
-#define SB_PAD(B) do { *cols = B::CHUNKS * B::CE; *k = B::SE ? B::CEXP : B::CHUNKS * B::CK; } while (0)
+#define SB_PAD(B) do { *cols = *k = B::KPAD; } while (0)
     *cols = *k = 0;
     switch (block) {
     case 2: SB_PAD(B2); break;

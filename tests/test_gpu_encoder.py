@@ -587,6 +587,16 @@ def test_fused_block_gives_the_bits_of_the_layers(L, block, dtype):
     assert torch.equal(f["out"], a["out"])
 
 
+@pytest.mark.parametrize("block,frames", [(7, (37, 38)), (8, (18, 19, 74, 75)), (9, (18, 19, 74, 75))])
+def test_whole_block_gives_the_bits_of_the_layers_on_every_tile(L, block, frames):
+    """The deeper whole blocks take smaller tiles of a map for few frames: both sides of the lines (on 148 SMs)."""
+    import torch
+    for F in frames:
+        for dtype in (1, 2):
+            a, f = _block_both_ways(L, block, dtype, F, seed=F)
+            assert torch.equal(f["out"], a["out"]), (F, dtype)
+
+
 @pytest.mark.parametrize("dtype", [1, 2])
 def test_fused_ends_give_the_bits_of_the_layers(L, dtype):
     """Stem + block 1, and last convolution + pooling (rounded to the 16-bit type, as the token projection rounds its operand)."""
