@@ -608,8 +608,18 @@ se_gate_cluster_kernel(const float* __restrict__ sums, const float* __restrict__
     for (int i = tid; i < G * C; i += 256) {
         const int fr = i / C, c = i - fr * C;
         float s = 0.0f;
-        if (fr < nf)
-            for (int k = 0; k < tiles; ++k) s += sums[((long long)(f0 + fr) * tiles + k) * C + c];
+        if (fr < nf) {
+            const float* const p = sums + (long long)(f0 + fr) * tiles * C + c;
+            int k = 0;
+            for (; k + 4 < tiles; k += 5) {                          // five loads fly together: the wide early maps have 15 groups
+                float v[5];
+#pragma unroll
+                for (int e = 0; e < 5; ++e) v[e] = __ldg(p + (k + e) * C);
+#pragma unroll
+                for (int e = 0; e < 5; ++e) s += v[e];
+            }
+            for (; k < tiles; ++k) s += __ldg(p + k * C);
+        }
         pooled[c * G + fr] = s / hw;
     }
     for (int i = G * C + tid; i < G * CP; i += 256) pooled[i] = 0.0f;
@@ -1214,13 +1224,14 @@ extern "C" int shvk_cnn_se_gate_sums(const float* sums, const float* w1, const f
     const unsigned grid = sb::blocks_of(F, G) * 8;
     cudaStream_t s = cudaStream_t(stream);
     // Four outputs of a warp at a time up to two blocks an SM (960 channels, four / one: 75 frames 29.7 / 33.6 us, 130 frames 31.7 / 36.6);
-    // beyond, other clusters hide the loads and the narrow maps pay for the registers (120 channels, 300 frames 14.1 / 11.4)
+    // beyond, other clusters hide the loads and the narrow maps pay for the registers (120 channels, 300 frames 14.1 / 11.4), so two:
+    // a frame's values are read from shared memory once for both (640 frames, two / one: 960 channels 100 / 114 us, 480 55 / 60)
     auto go = [&](auto kernel) {
         kernel<<<grid, 256, smem, s>>>(sums, w1, b1, w2, b2, gate, F, tiles, float(HW), C, CS);
         return int(cudaGetLastError());
     };
     if (G == 1) return go(sb::se_gate_cluster_kernel<1, 4>);
-    return grid <= 2u * sms ? go(sb::se_gate_cluster_kernel<4, 4>) : go(sb::se_gate_cluster_kernel<4, 1>);
+    return grid <= 2u * sms ? go(sb::se_gate_cluster_kernel<4, 4>) : go(sb::se_gate_cluster_kernel<4, 2>);
 }
 
 namespace sb {
