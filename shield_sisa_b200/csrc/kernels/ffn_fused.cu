@@ -117,7 +117,7 @@ ffn_fused_kernel(const __grid_constant__ FfnMaps maps, const FfnParams p, int* _
     volatile int* abortp = &abort_flag;
 
     if (warp == 0) {
-        if (lane == 0) {                                             // ---- weight tiles, in the order the MMA thread consumes them
+        if (elect_one()) {                                             // ---- weight tiles, in the order the MMA thread consumes them
             int stage = 0;
             uint32_t phase = 0;
             bool ok = true;
@@ -146,7 +146,7 @@ ffn_fused_kernel(const __grid_constant__ FfnMaps maps, const FfnParams p, int* _
             if (!ok && !*abortp) { *abortp = 1; atomicCAS(status, 0, 1); }
         }
     } else if (warp == 2) {
-        if (lane == 0) {                                             // ---- the row block's xn rows, once per block
+        if (elect_one()) {                                             // ---- the row block's xn rows, once per block
             uint32_t n = 0;
             bool ok = true;
             for (int mt = blockIdx.x; ok && mt < p.m_tiles; mt += gridDim.x, ++n) {
@@ -157,7 +157,7 @@ ffn_fused_kernel(const __grid_constant__ FfnMaps maps, const FfnParams p, int* _
             if (!ok && !*abortp) { *abortp = 1; atomicCAS(status, 0, 4); }
         }
     } else if (warp == 1) {
-        if (lane == 0) {                                             // ---- MMA issue
+        if (elect_one()) {                                             // ---- MMA issue
             int stage = 0;
             uint32_t phase = 0, n = 0, slab = 0;                     // slab: slabs started by this CTA so far
             uint32_t hpar = 0;                                       // bit b: parity of the down products issued from hidden-layer buffer b

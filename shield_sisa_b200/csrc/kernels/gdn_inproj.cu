@@ -344,7 +344,7 @@ gdn_inproj_kernel(const __grid_constant__ InprojMaps maps, const InprojParams p,
     int m0, m1;
 
     if (warp == 0) {
-        if (lane == 0) {                                         // ---- W' tiles: 19 x 6 k-blocks per item through the ring
+        if (elect_one()) {                                         // ---- W' tiles: 19 x 6 k-blocks per item through the ring
             int stage = 0;
             uint32_t phase = 0;
             bool ok = true;
@@ -369,7 +369,7 @@ gdn_inproj_kernel(const __grid_constant__ InprojMaps maps, const InprojParams p,
             if (!ok && !*abortp) { *abortp = 1; atomicCAS(status, 0, 1); }
         }
     } else if (warp == 2) {
-        if (lane == 0) {                                         // ---- the item's xn rows, once per item
+        if (elect_one()) {                                         // ---- the item's xn rows, once per item
             uint32_t n = 0;
             bool ok = true;
             for (long long u = u0; u < u1; u += m1 - m0 + hop, ++n) {
@@ -382,7 +382,7 @@ gdn_inproj_kernel(const __grid_constant__ InprojMaps maps, const InprojParams p,
             if (!ok && !*abortp) { *abortp = 1; atomicCAS(status, 0, 4); }
         }
     } else if (warp == 1) {
-        if (lane == 0) {                                         // ---- MMA issue
+        if (elect_one()) {                                         // ---- MMA issue
             int stage = 0, acc = 0;
             uint32_t phase = 0, acc_phase = 0, n = 0;
             bool ok = true;

@@ -237,7 +237,7 @@ gemm_tc_kernel(const __grid_constant__ TcMaps maps, const TcParams p) {
     const uint32_t stage_tx = uint32_t(A_BYTES + p.BN * ROW_BYTES);
 
     if (warp == 0) {
-        if (lane == 0) {
+        if (elect_one()) {
             int stage = 0;
             uint32_t phase = 0;
             bool ok = true;
@@ -271,7 +271,7 @@ gemm_tc_kernel(const __grid_constant__ TcMaps maps, const TcParams p) {
             if (!ok && !*abortp) { *abortp = 1; atomicCAS(&g_tc_status, 0, 1); }
         }
     } else if (warp == 1) {
-        if (lane == 0) {
+        if (elect_one()) {
             int stage = 0, acc = 0;
             uint32_t phase = 0, acc_phase = 0;
             bool ok = true;
