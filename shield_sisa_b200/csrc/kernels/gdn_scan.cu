@@ -151,7 +151,7 @@ gdn_scan_kernel(const __grid_constant__ ScanMaps maps, const float* __restrict__
         ChunkBuf& b = sm.buf[chunk & 1];
         // every thread is done with the other buffer (post of chunk - 1 ended at the barrier closing the last
         // iteration): refill it while this chunk is processed
-        if (tid == 0 && chunk + 1 < NCHUNK) {
+        if (warp == 0 && chunk + 1 < NCHUNK && elect_one()) {
             tma::fence_proxy_async();
             issue(chunk + 1);
         }

@@ -12,15 +12,6 @@ namespace tc {
 
 __device__ __forceinline__ uint32_t smem_u32(const void* p) { return uint32_t(__cvta_generic_to_shared(p)); }
 
-// One lane of a converged warp, always the same.  The roles that issue copies and MMAs branch on this and not on lane == 0: those
-// instructions take their operands from uniform registers, and behind a branch that the compiler cannot see to be one thread's each
-// of them is wrapped in code for several: a k-block of two TMA loads took its thread 511 cycles to issue (393 behind elect), one of
-// four MMAs and a commit 575 (403), more than the tensor core needs for it.
-__device__ __forceinline__ bool elect_one() {
-    uint32_t one;
-    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(one));
-    return one != 0;
-}
 __device__ __forceinline__ void mbar_init(uint32_t bar, uint32_t count) {
     asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count) : "memory");
 }
