@@ -743,7 +743,7 @@ def run_ours(args, rank: int, world: int, local_rank: int):
             f_in, f_sc = L.shvk_dev_inproj_cycles, L.shvk_dev_scan_cycles
         except AttributeError:
             raise SystemExit("--dev-cycles needs the development build: python -m shield_sisa_b200.build --dev-probes")
-        b_in, b_sc = (C.c_ulonglong * 88)(), (C.c_ulonglong * 32)()
+        b_in, b_sc = (C.c_ulonglong * 152)(), (C.c_ulonglong * 32)()
         for f, b in ((f_in, b_in), (f_sc, b_sc)):
             f.argtypes, f.restype = [C.c_void_p], C.c_int
             f(b)                                          # discard what the steps above accumulated
@@ -762,8 +762,7 @@ def run_ours(args, rank: int, world: int, local_rank: int):
             "gdn_inproj": {
                 "w_producer": shares(b_in, 0, [(0, "wait_free_stage")], 7),
                 "mma_thread": shares(b_in, 1, [(0, "wait_drained_accumulator"), (1, "wait_weight_stage"), (2, "wait_token_tile")], 7),
-                **{f"epilogue_warp_{w}": shares(b_in, w, [(0, "wait_full_accumulator"), (1, "first_tmem_load"),
-                                                          (2, "later_tmem_loads"), (3, "tile_total")], 7) for w in range(3, 11)}},
+                **{f"epilogue_warp_{w}": shares(b_in, w, [(0, "wait_full_accumulator"), (3, "tile_total")], 7) for w in range(3, 19)}},
             "gdn_scan_t": {f"warp_{w}": shares(b_sc, w, [(0, "until_block_landed"), (1, "deferred_norm"), (2, "r_and_qs"), (3, "u_and_o"),
                                                          (4, "state_update"), (5, "sum_of_squares"), (6, "barrier")]) for w in range(4)}}
         print(json.dumps(dev_cycles, indent=1), file=sys.stderr)

@@ -20,11 +20,11 @@
 // operand traffic out of L2 is 4.0 MB per clip (whole items) instead of 8.6 MB with both operands streamed (which alone took
 // 2.0 ms per launch at 4096 clips, more than the products).  Neighbouring CTAs take the two tiles of one clip.
 //
-// Roles (352 threads): warp 0 streams W' tiles (TMA, 128-byte swizzle, no multicast), warp 2 loads the xn tile of the
+// Roles (608 threads): warp 0 streams W' tiles (TMA, 128-byte swizzle, no multicast), warp 2 loads the xn tile of the
 // next item as soon as the last product of the current one has read it, warp 1 issues tcgen05.mma (M 128, N 176,
-// K 16) into one of two accumulators and owns tensor memory, warps 3-10 are the epilogue: two warps per lane quadrant,
-// one for the first six chunks of the accumulator and one for the other five (it reads its three history columns
-// from the neighbour's range).  K is walked in order and never split; a token's column depends on no other token of
+// K 16) into one of two accumulators and owns tensor memory, warps 3-18 are the epilogue: four warps per lane quadrant,
+// with three chunks of the accumulator each (two or one for the last; a warp reads its three history columns from its
+// neighbour's range).  K is walked in order and never split; a token's column depends on no other token of
 // the batch, so clips stay independent bitwise.
 //
 // Every mbarrier wait is bounded (status word of the tensor-core GEMM, shvk_gemm_tc_status).
@@ -52,8 +52,9 @@ constexpr int W_STAGE_BYTES = TILE_M * TILE_K * 2, W_STAGES = 5;
 constexpr int XN_KB_BYTES = NT * TILE_K * 2, XN_BYTES = KBLOCKS * XN_KB_BYTES;
 constexpr int BAR_BYTES = 256;
 constexpr int SMEM_BYTES = XN_BYTES + W_STAGES * W_STAGE_BYTES + BAR_BYTES + 1024;
-constexpr int NTHREADS = 352;
+constexpr int EPI_WARPS = 16, EPI_SHARES = EPI_WARPS / 4, NTHREADS = 96 + 32 * EPI_WARPS;   // emit_tile says why sixteen
 constexpr uint32_t SPIN_LIMIT = 1u << 22;
+static_assert((EPI_SHARES - 1) * ((NT / 16 - 1 + EPI_SHARES - 1) / EPI_SHARES) < NT / 16 - 1, "every epilogue warp has a chunk");
 static_assert(TT_STRIDE + NT == pt::TOK_PAD && TT_STRIDE % pt::CHUNK == 0 && NT % pt::CHUNK == 0, "token tiles cover the padded clip in whole chunks");
 static_assert(XN_KB_BYTES % 1024 == 0 && W_STAGE_BYTES % 1024 == 0, "swizzled tiles need 1024-byte alignment");
 static_assert((2 * W_STAGES + 6) * 8 <= BAR_BYTES && SMEM_BYTES <= 232448, "shared memory budget");
@@ -74,24 +75,23 @@ struct InprojParams {
     int probe;       // timing probes of a development build (-DSHVK_DEV_PROBES, SHVK_INPROJ_PROBE): 1 no global stores,
                      // 2 no activation arithmetic, 4 no tensor-memory loads, 8 no MMA.  Constant 0 in the shipped libraries.
 };
-// The probe bits travel in the kernel parameters (constant bank) and, to the tile functions, in bits 8+ of `flags`: a
-// word in global memory would add a load in front of every tile and change the timings it is meant to explain.
+// The probe bits travel in the kernel parameters (constant bank): a word in global memory would add a load in front of every
+// tile and change the timings it is meant to explain.
 // Cycle counters of the same builds: lane 0 of every warp adds clock64() differences to eight slots in shared memory
 // (W producer: 0 wait for a free stage.  MMA thread: 0 wait for a drained accumulator, 1 for a weight stage, 2 for the
-// token tile.  Epilogue warps: 0 wait for a full accumulator, 1 first tensor-memory load of a tile, 2 the later ones,
-// 3 the whole tile.  All: 7 the role's loop.)  CTA 5 adds its totals to g_prof, read and cleared by
+// token tile.  Epilogue warps: 0 wait for a full accumulator, 3 the whole tile.  All: 7 the role's loop.)  CTA 5 adds its totals to g_prof, read and cleared by
 // shvk_dev_inproj_cycles.
 #ifdef SHVK_DEV_PROBES
-__device__ unsigned long long g_prof[11][8];
+__device__ unsigned long long g_prof[NTHREADS / 32][8];
 #define PROF_T() clock64()
 #define PROF_ADD(slot, dt) do { if ((threadIdx.x & 31) == 0) prof_s[(threadIdx.x >> 5) * 8 + (slot)] += (unsigned long long)(dt); } while (0)
 #define INPROJ_PROBE(bit) (probe_bits & (bit))
-#define INPROJ_TILE_FLAGS(f) ((f) | (p.probe << 8))
+#define INPROJ_PROBE_BITS p.probe
 #else
 #define PROF_T() 0ll
 #define PROF_ADD(slot, dt) do { } while (0)
 #define INPROJ_PROBE(bit) 0
-#define INPROJ_TILE_FLAGS(f) (f)
+#define INPROJ_PROBE_BITS 0
 #endif
 
 // x * sigmoid(x) = 0.5 x (1 + tanh(x / 2)) with the hardware tanh: absolute error ~5e-4 |x|, below the bf16 rounding
@@ -121,132 +121,130 @@ __device__ __forceinline__ void stg256(void* p, const uint32_t (&w)[8]) {
                  ::"l"(p), "r"(w[0]), "r"(w[1]), "r"(w[2]), "r"(w[3]), "r"(w[4]), "r"(w[5]), "r"(w[6]), "r"(w[7]) : "memory");
 }
 
-// What an epilogue does with its channel: q, k (conv + SiLU, stored in the mode's operand type: KIND_CONV_BF16 or
-// KIND_CONV_F16), v (conv + SiLU, fp16), output gate (SiLU, fp16), a | b (log decay and beta, fp32).
-enum : int { KIND_CONV_BF16 = 0, KIND_CONV_F16 = 1, KIND_SILU = 2, KIND_GATES = 3 };
-
+// What an epilogue does with its channel: q, k (conv + SiLU, stored in the mode's operand type), v (conv + SiLU, fp16), output gate
+// (SiLU, fp16); and, in functions of their own, a | b (log decay and beta, fp32).
 struct ChanConst {            // what the epilogue thread knows about its channel
     float4 w;                 // conv taps: tap j multiplies x[t - 3 + j]
     float bias;
-    float rate, dtb;          // KIND_GATES, decay rows: -exp(A_log), dt_bias
-    bool is_beta, active;     // KIND_GATES: beta row; lane has a channel at all
+    float rate, dtb;          // a | b, decay rows: -exp(A_log), dt_bias
+    bool is_beta, active;     // a | b: beta row; lane has a channel at all
     int half0;                // byte offset (0 or 16) of tokens 0-7 within the channel's 32-byte row of a chunk block
     int probe;                // probe bits of a development build, else 0
 };
 
-// Sixteen accumulator columns = one chunk of 16 tokens of one channel: activation, packing, and the channel's 32-byte
-// (KIND_GATES: 64-byte) row of the chunk block at `row`.  nvalid: how many of the 16 token slots lie inside the clip
-// (16 everywhere except in the clip's last chunk); the others are written as zeros.  x1, x2, x3: raw projections of the
-// three tokens before this chunk (conv kinds), updated to the chunk's last three.
-template <int KIND>
-__device__ __forceinline__ void emit_chunk(const uint32_t (&in)[16], uint8_t* row, const ChanConst& cc, int nvalid,
+// One chunk of a | b: sixteen accumulator columns into the channel's 64 bytes of the chunk block at `row`.  nvalid: how many of the 16
+// token slots lie inside the clip (16 everywhere except in the clip's last chunk); the others are written as zeros.
+__device__ __forceinline__ void emit_gates(const uint32_t (&in)[16], uint8_t* row, const ChanConst& cc, int nvalid) {
+    uint32_t v[16];
+#pragma unroll
+    for (int j = 0; j < 16; ++j) {
+        // beta rows: 1 / (1 + exp(-raw)); decay rows: rate * softplus(raw + dt_bias).  Both from one exponential and
+        // without a branch: the rows of the two kinds sit in one warp, and a divergent branch per token would run
+        // the sixteen tokens one after the other.
+        const float raw = __uint_as_float(in[j]);
+        const float ax = cc.is_beta ? -raw : raw + cc.dtb;
+        const float e1 = 1.0f + __expf(ax);
+        const float sp = cc.rate * (ax > 15.0f ? ax : __logf(e1));
+        const float o = cc.is_beta ? __fdividef(1.0f, e1) : sp;
+        v[j] = __float_as_uint(o);
+    }
+    if (nvalid < 16) {
+#pragma unroll
+        for (int j = 0; j < 16; ++j) v[j] = j < nvalid ? v[j] : 0u;
+    }
+    if (cc.active) {
+#pragma unroll
+        for (int q = 0; q < 4; ++q) stg128(row + 16 * q, v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3]);
+    }
+}
+
+// One chunk of q, k, v or the output gate: activation, packing, and the channel's 32-byte row of the chunk block at `row`.  conv and
+// f16 are the tile's, so their branches are the warp's.  x1, x2, x3: raw projections of the three tokens before this chunk,
+// updated to the chunk's last three.
+__device__ __forceinline__ void emit_chunk(uint32_t (&in)[16], uint8_t* row, const ChanConst& cc, bool conv, bool f16, int nvalid,
                                            float& x1, float& x2, float& x3) {
     [[maybe_unused]] const int probe_bits = cc.probe;
-    if (KIND == KIND_GATES) {
-        uint32_t v[16];
+    if (conv) {
+        const float l1 = __uint_as_float(in[15]), l2 = __uint_as_float(in[14]), l3 = __uint_as_float(in[13]);
 #pragma unroll
-        for (int j = 0; j < 16; ++j) {
-            // beta rows: 1 / (1 + exp(-raw)); decay rows: rate * softplus(raw + dt_bias).  Both from one exponential and
-            // without a branch: the rows of the two kinds sit in one warp, and a divergent branch per token would run
-            // the sixteen tokens one after the other.
-            const float raw = __uint_as_float(in[j]);
-            const float ax = cc.is_beta ? -raw : raw + cc.dtb;
-            const float e1 = 1.0f + __expf(ax);
-            const float sp = cc.rate * (ax > 15.0f ? ax : __logf(e1));
-            const float o = cc.is_beta ? __fdividef(1.0f, e1) : sp;
-            v[j] = __float_as_uint(o);
+        for (int j = 15; j >= 0; --j) {                              // from the end: the tokens before a token are raw still
+            const float p1 = j >= 1 ? __uint_as_float(in[j >= 1 ? j - 1 : 0]) : x1;
+            const float p2 = j >= 2 ? __uint_as_float(in[j >= 2 ? j - 2 : 0]) : j == 1 ? x1 : x2;
+            const float p3 = j >= 3 ? __uint_as_float(in[j >= 3 ? j - 3 : 0]) : j == 2 ? x1 : j == 1 ? x2 : x3;
+            float a = fmaf(cc.w.x, p3, cc.bias);
+            a = fmaf(cc.w.y, p2, a);
+            a = fmaf(cc.w.z, p1, a);
+            in[j] = __float_as_uint(fmaf(cc.w.w, __uint_as_float(in[j]), a));
         }
-        if (nvalid < 16) {
+        x1 = l1; x2 = l2; x3 = l3;
+    }
+    if (!INPROJ_PROBE(2)) {
 #pragma unroll
-            for (int j = 0; j < 16; ++j) v[j] = j < nvalid ? v[j] : 0u;
-        }
-        if (cc.active) {
+        for (int j = 0; j < 16; ++j) in[j] = __float_as_uint(silu_tanh(__uint_as_float(in[j])));
+    }
+    uint32_t o[8];
+    if (f16) {
 #pragma unroll
-            for (int q = 0; q < 4; ++q) stg128(row + 16 * q, v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3]);
-        }
+        for (int i = 0; i < 8; ++i) o[i] = pack_f16(__uint_as_float(in[2 * i]), __uint_as_float(in[2 * i + 1]));
     } else {
-        uint32_t o[8];
 #pragma unroll
-        for (int j = 0; j < 16; j += 2) {
-            float y[2];
+        for (int i = 0; i < 8; ++i) o[i] = pack_bf16(__uint_as_float(in[2 * i]), __uint_as_float(in[2 * i + 1]));
+    }
+    if (nvalid < 16) {                                               // the clip's last chunk: zero the token slots past its end
 #pragma unroll
-            for (int e = 0; e < 2; ++e) {
-                const float raw = __uint_as_float(in[j + e]);
-                float a = raw;
-                if (KIND == KIND_CONV_BF16 || KIND == KIND_CONV_F16) {
-                    a = fmaf(cc.w.x, x3, cc.bias);
-                    a = fmaf(cc.w.y, x2, a);
-                    a = fmaf(cc.w.z, x1, a);
-                    a = fmaf(cc.w.w, raw, a);
-                    x3 = x2; x2 = x1; x1 = raw;
-                }
-                y[e] = INPROJ_PROBE(2) ? raw : silu_tanh(a);
-            }
-            o[j >> 1] = KIND == KIND_CONV_BF16 ? pack_bf16(y[0], y[1]) : pack_f16(y[0], y[1]);
+        for (int i = 0; i < 8; ++i) o[i] = (2 * i < nvalid ? (o[i] & 0x0000ffffu) : 0u) | (2 * i + 1 < nvalid ? (o[i] & 0xffff0000u) : 0u);
+    }
+    // the two 16-byte halves of the row trade places in rows 4-7 of every eight, so that the scan's ldmatrix reads
+    // (eight rows of one half at a time) fall into eight different bank groups
+    if (!INPROJ_PROBE(1)) {
+        uint32_t w[8];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            w[i] = cc.half0 ? o[i + 4] : o[i];
+            w[i + 4] = cc.half0 ? o[i] : o[i + 4];
         }
-        if (nvalid < 16) {                                        // the clip's last chunk: zero the token slots past its end
-#pragma unroll
-            for (int i = 0; i < 8; ++i) o[i] = (2 * i < nvalid ? (o[i] & 0x0000ffffu) : 0u) | (2 * i + 1 < nvalid ? (o[i] & 0xffff0000u) : 0u);
-        }
-        // the two 16-byte halves of the row trade places in rows 4-7 of every eight, so that the scan's ldmatrix reads
-        // (eight rows of one half at a time) fall into eight different bank groups
-        if (!INPROJ_PROBE(1)) {
-            uint32_t w[8];
-#pragma unroll
-            for (int i = 0; i < 4; ++i) {
-                w[i] = cc.half0 ? o[i + 4] : o[i];
-                w[i + 4] = cc.half0 ? o[i] : o[i + 4];
-            }
-            stg256(row, w);
-        } else if (o[0] == 0x12345678u && o[7] == 0x9abcdef0u) {
-            stg128(row, o[0], o[1], o[2], o[3]);          // keeps the arithmetic alive
-        }
+        stg256(row, w);
+    } else if (o[0] == 0x12345678u && o[7] == 0x9abcdef0u) {
+        stg128(row, o[0], o[1], o[2], o[3]);                         // keeps the arithmetic alive
     }
 }
 
 // One token tile of one channel: ncols accumulator columns (a multiple of 16) starting at tensor-memory address taddr,
 // tokens tok0 .. tok0 + ncols - 1 of the clip, written to this channel's rows of the chunk blocks starting at dst (chunk
-// tok0 / 16).  x1, x2, x3: raw projections of tokens tok0 - 1, - 2, - 3 (conv kinds).  A real loop over pairs of chunks,
-// not unrolled over the tile: the body then stays resident in the instruction cache (fully unrolled, the eight epilogue
-// warps spent more cycles waiting for instructions than issuing them).
-template <int KIND>
-__device__ __noinline__ void emit_tile(uint32_t taddr, uint8_t* dst, float4 cw, float bias, float rate, float dtb, int flags,
-                                       int tok0, int ncols, bool has_hist, [[maybe_unused]] unsigned long long* prof_s) {
-    // the channel constants travel as scalars (registers), not as a struct behind a pointer (local memory)
-    ChanConst cc;
-    cc.w = cw; cc.bias = bias; cc.rate = rate; cc.dtb = dtb;
-    cc.is_beta = flags & 1; cc.active = flags & 2; cc.half0 = flags & 16; cc.probe = flags >> 8;
-    [[maybe_unused]] const int probe_bits = cc.probe;
-    uint32_t ra[16], rb[16];
+// tok0 / 16).
+//
+// ONE piece of code for q, k, v and the gate, a chunk to an iteration.  Channel tiles come as q | k, v, gate, q | k, ...: with a
+// function per kind, two chunks to an iteration, every tile started with code that the instruction cache next to the scheduler had
+// lost and ran it at most three times; a warp spent 750 cycles on a chunk of some 190 instructions, and more warps made it worse:
+// 336, 449 and 585 us per launch at 512 windows (bf16) with 8, 12 and 16 epilogue warps.  With this code they take 331, 307 and 297
+// (20: 305), and 2900, 2616 and 2488 us at 4096 windows (20: 2619).  A tensor-memory load is waited for 80 cycles at most, so
+// nothing is fetched ahead.  What remains at sixteen: without conv, activation and stores a launch still takes 217 us, the chain of
+// accumulator, drain and hand-over, with 146 us of products (2112 cycles a tile) under it.
+__device__ __forceinline__ void emit_tile(uint32_t taddr, uint8_t* dst, const ChanConst& cc, bool conv, bool f16, int tok0, int ncols, bool has_hist) {
+    uint32_t in[16];
     float x1 = 0.0f, x2 = 0.0f, x3 = 0.0f;
-#ifdef SHVK_DEV_PROBES
-    if (INPROJ_PROBE(4)) {
-#pragma unroll
-        for (int i = 0; i < 16; ++i) { ra[i] = 0x3f000000u + i; rb[i] = 0x3f100000u + i; }
-#pragma unroll 1
-        for (int c = 0; c < ncols; c += 32) {
-            emit_chunk<KIND>(ra, dst + (long long)(c >> 4) * pt::BLOCK_BYTES, cc, kTok - (tok0 + c), x1, x2, x3);
-            if (c + 16 >= ncols) break;
-            emit_chunk<KIND>(rb, dst + (long long)((c >> 4) + 1) * pt::BLOCK_BYTES, cc, kTok - (tok0 + c + 16), x1, x2, x3);
-        }
-        return;
+    if (has_hist && conv) {                                          // the three tokens before this warp's range
+        uint32_t h[4];
+        tc_ld4(taddr - 4u, h);
+        tc_wait_ld();
+        x1 = __uint_as_float(h[3]); x2 = __uint_as_float(h[2]); x3 = __uint_as_float(h[1]);
     }
-#endif
-    // The 16 columns before this warp's range hold its convolution history (their last three tokens).  They come with
-    // the first chunk in ONE 32-column load: a tensor-memory load takes the better part of a microsecond to return while
-    // the MMA pipe is busy, and a separate history load would put that wait in front of every tile.
-    if (has_hist) tc_ld16x2(taddr - 16u, rb, ra);
-    else tc_ld16(taddr, ra);
 #pragma unroll 1
-    for (int c = 0; c < ncols; c += 32) {
-        { [[maybe_unused]] const long long ta = PROF_T(); tc_wait_ld(); PROF_ADD(c == 0 ? 1 : 2, PROF_T() - ta); }
-        if (c == 0 && has_hist) { x1 = __uint_as_float(rb[15]); x2 = __uint_as_float(rb[14]); x3 = __uint_as_float(rb[13]); }
-        if (c + 16 < ncols) tc_ld16(taddr + uint32_t(c + 16), rb);
-        emit_chunk<KIND>(ra, dst + (long long)(c >> 4) * pt::BLOCK_BYTES, cc, kTok - (tok0 + c), x1, x2, x3);
-        if (c + 16 >= ncols) break;
-        { [[maybe_unused]] const long long ta = PROF_T(); tc_wait_ld(); PROF_ADD(2, PROF_T() - ta); }
-        if (c + 32 < ncols) tc_ld16(taddr + uint32_t(c + 32), ra);
-        emit_chunk<KIND>(rb, dst + (long long)((c >> 4) + 1) * pt::BLOCK_BYTES, cc, kTok - (tok0 + c + 16), x1, x2, x3);
+    for (int c = 0; c < ncols; c += 16) {
+        tc_ld16(taddr + uint32_t(c), in);
+        tc_wait_ld();
+        emit_chunk(in, dst + (long long)(c >> 4) * pt::BLOCK_BYTES, cc, conv, f16, kTok - (tok0 + c), x1, x2, x3);
+    }
+}
+__device__ __noinline__ void emit_tile_gates(uint32_t taddr, uint8_t* dst, float rate, float dtb, int flags, int tok0, int ncols) {
+    ChanConst cc{};
+    cc.rate = rate; cc.dtb = dtb; cc.is_beta = flags & 1; cc.active = flags & 2;
+    uint32_t in[16];
+#pragma unroll 1
+    for (int c = 0; c < ncols; c += 16) {
+        tc_ld16(taddr + uint32_t(c), in);
+        tc_wait_ld();
+        emit_gates(in, dst + (long long)(c >> 4) * pt::BLOCK_BYTES, cc, kTok - (tok0 + c));
     }
 }
 
@@ -297,11 +295,9 @@ gdn_inproj_kernel(const __grid_constant__ InprojMaps maps, const InprojParams p,
     __shared__ uint32_t tmem_base_slot;
     __shared__ int abort_flag;
 #ifdef SHVK_DEV_PROBES
-    __shared__ unsigned long long prof_arr[11 * 8];
+    __shared__ unsigned long long prof_arr[NTHREADS / 32 * 8];
     unsigned long long* prof_s = prof_arr;
-    if (threadIdx.x < 88) prof_arr[threadIdx.x] = 0;
-#else
-    unsigned long long* prof_s = nullptr;
+    if (threadIdx.x < NTHREADS / 32 * 8) prof_arr[threadIdx.x] = 0;
 #endif
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     auto wfull_bar = [&](int s) { return bars + 8u * s; };
@@ -313,7 +309,7 @@ gdn_inproj_kernel(const __grid_constant__ InprojMaps maps, const InprojParams p,
     if (threadIdx.x == 0) {
         abort_flag = 0;
         for (int s = 0; s < W_STAGES; ++s) { mbar_init(wfull_bar(s), 1); mbar_init(wempty_bar(s), 1); }
-        for (int a = 0; a < 2; ++a) { mbar_init(accf_bar(a), 1); mbar_init(acce_bar(a), 8); }
+        for (int a = 0; a < 2; ++a) { mbar_init(accf_bar(a), 1); mbar_init(acce_bar(a), EPI_WARPS); }
         mbar_init(xfull_bar, 1);
         mbar_init(xempty_bar, 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -420,7 +416,7 @@ gdn_inproj_kernel(const __grid_constant__ InprojMaps maps, const InprojParams p,
         }
     } else {
         // ------------------------------------------------------------------------------------------ epilogue
-        const int ew = warp - 3, quad = warp & 3, half = ew >> 2;    // half 0: the accumulator's first chunks, half 1: the rest
+        const int ew = warp - 3, quad = warp & 3, share = ew >> 2;
         const int r = quad * 32 + lane;                              // channel row within the tile
         const uint32_t tlane = tmem_base + (uint32_t(quad * 32) << 16);
         int acc = 0;
@@ -431,8 +427,9 @@ gdn_inproj_kernel(const __grid_constant__ InprojMaps maps, const InprojParams p,
             const int clip = int(item >> 1), tt = int(item & 1);
             // this warp's columns of the accumulator: [col0, col0 + ncols), written from chunk `chunk0` on; its three
             // history tokens are the columns just before col0 (none at the start of the clip)
-            const int col0 = half ? 96 : (tt ? 16 : 0);
-            const int ncols = half ? 80 : (tt ? 80 : 96);
+            const int first = tt ? 1 : 0, total = NT / 16 - first, per = (total + EPI_SHARES - 1) / EPI_SHARES;
+            const int cb = share * per, ce = min(cb + per, total);
+            const int col0 = (first + cb) * 16, ncols = (ce - cb) * 16;
             const int tok0 = tt * TT_STRIDE + col0, chunk0 = tok0 >> 4;
             const bool has_hist = col0 > 0;
             ChanSite cur = chan_site(p, m0, r);
@@ -446,10 +443,13 @@ gdn_inproj_kernel(const __grid_constant__ InprojMaps maps, const InprojParams p,
                 const uint32_t tacc = tlane + uint32_t(acc * 256);
                 uint8_t* dst = p.pt + ((long long)clip * kHeads + cur.head) * pt::HEAD_BYTES + cur.section + (long long)chunk0 * pt::BLOCK_BYTES;
                 const int type = m % 3;
-                if (m == M_TILES - 1) { if (quad == 0) emit_tile<KIND_GATES>(tacc + col0, dst, cur.w, cur.bias, cur.rate, cur.dtb, INPROJ_TILE_FLAGS(cur.flags), tok0, ncols, false, prof_s); }
-                else if (type == 2) emit_tile<KIND_SILU>(tacc + col0, dst, cur.w, cur.bias, cur.rate, cur.dtb, INPROJ_TILE_FLAGS(cur.flags), tok0, ncols, false, prof_s);
-                else if (type == 1 || p.qk_f16) emit_tile<KIND_CONV_F16>(tacc + col0, dst, cur.w, cur.bias, cur.rate, cur.dtb, INPROJ_TILE_FLAGS(cur.flags), tok0, ncols, has_hist, prof_s);
-                else emit_tile<KIND_CONV_BF16>(tacc + col0, dst, cur.w, cur.bias, cur.rate, cur.dtb, INPROJ_TILE_FLAGS(cur.flags), tok0, ncols, has_hist, prof_s);
+                if (m == M_TILES - 1) {
+                    if (quad == 0) emit_tile_gates(tacc + col0, dst, cur.rate, cur.dtb, cur.flags, tok0, ncols);
+                } else {
+                    ChanConst cc{};
+                    cc.w = cur.w; cc.bias = cur.bias; cc.half0 = cur.flags & 16; cc.probe = INPROJ_PROBE_BITS;
+                    emit_tile(tacc + col0, dst, cc, type != 2, type != 0 || p.qk_f16, tok0, ncols, has_hist);
+                }
                 PROF_ADD(3, PROF_T() - tp1);
                 tc_fence_before();
                 __syncwarp();
@@ -464,7 +464,7 @@ gdn_inproj_kernel(const __grid_constant__ InprojMaps maps, const InprojParams p,
     PROF_ADD(7, PROF_T() - tk0);
     __syncthreads();
 #ifdef SHVK_DEV_PROBES
-    if (threadIdx.x < 88 && blockIdx.x == 5) atomicAdd(&g_prof[threadIdx.x >> 3][threadIdx.x & 7], prof_arr[threadIdx.x]);
+    if (threadIdx.x < NTHREADS / 32 * 8 && blockIdx.x == 5) atomicAdd(&g_prof[threadIdx.x >> 3][threadIdx.x & 7], prof_arr[threadIdx.x]);
 #endif
     if (abort_flag) {
         // A role gave up: copies already issued may still land in this CTA's shared memory.  Give them time (bounded)
@@ -593,9 +593,9 @@ static int inproj_launch(const void* host_plan, int B, void* stream, int starve,
 }
 
 #ifdef SHVK_DEV_PROBES
-// Development builds only: the in-projection's cycle counters [11 warps][8 slots], read and cleared (synchronises the device).
+// Development builds only: the in-projection's cycle counters [19 warps][8 slots], read and cleared (synchronises the device).
 extern "C" __attribute__((visibility("default"))) int shvk_dev_inproj_cycles(unsigned long long* out) {
-    unsigned long long zero[88] = {0};
+    unsigned long long zero[sb::NTHREADS / 32 * 8] = {0};
     cudaDeviceSynchronize();
     cudaMemcpyFromSymbol(out, sb::g_prof, sizeof(zero));
     cudaMemcpyToSymbol(sb::g_prof, zero, sizeof(zero));
