@@ -266,16 +266,18 @@ private:
     void *xn_ = nullptr, *on_ = nullptr, *hid_ = nullptr;
     float* a2_ = nullptr;
     // 16-bit modes: whether the feed-forward blocks run as two GEMMs.  The fused kernel gives every 128 rows one SM, which takes
-    // 42 us for them however few there are; the two GEMMs spread a row block's columns over the SMs (the same sums in the
-    // same order) but move the hidden layer through L2: 12 us + 0.32 us per row block.  us per block, fused / two GEMMs: 1
-    // window 41 / 14, 8 42 / 19, 20 42 / 26, 40 44 / 42, 48 44 / 43, 56 44 / 46, 64 82 / 57, 80 83 / 69, 96 85 / 86,
-    // 112 85 / 98, 128 129 / 114.  Beyond FFN_TWO_ROWS the hidden layer would not stay in L2.
+    // 39-42 us for them however few there are, and 36 us more for every further round over the SMs; the two GEMMs spread a row
+    // block's columns over the SMs (the same sums in the same order) but move the hidden layer through L2: 19 us + 0.30 us per
+    // row block.  us per block, fused / two GEMMs: 1 window 39 / 24, 8 39 / 28, 20 41 / 37, 32 41 / 48, 48 43 / 57, 59 44 / 61,
+    // 64 74 / 70, 80 75 / 79, 96 79 / 95, 128 114 / 117.  us per classify, fused / two GEMMs: 20 windows 367 / 351, 28
+    // 417 / 406, 32 438 / 441, 40 473 / 491, 64 675 / 669, 80 793 / 797, 128 1233 / 1263.  Beyond FFN_TWO_ROWS the hidden
+    // layer would not stay in L2.
     static constexpr int FFN_TWO_ROWS = 128 * NTOK;
     bool two_launch_ffn(int rows) const {
         if (size_t(rows) > hid_rows_) return false;
         if (prec_ == Precision::FP32) return true;
         const int blocks = (rows + 127) / 128;
-        return 12 + 0.32 * blocks < 42.0 * ((blocks + sms_ - 1) / sms_);
+        return 19 + 0.30 * blocks < 6 + 36.0 * ((blocks + sms_ - 1) / sms_);
     }
     int sms_ = 148;
     size_t hid_rows_ = 0;                               // rows hid_ holds
