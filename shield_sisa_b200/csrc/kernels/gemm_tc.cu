@@ -64,7 +64,7 @@ __device__ int g_tc_status = 0;   // 0 ok; else 1 + role of the wait that gave u
 struct TcParams {
     int M, N, K, BN, n_tiles, m_tiles;
     const float* bias;
-    float r_div;
+    float r_div, r_inv;      // r_inv: 1 / r_div rounded, or 0 where the residual divides
     uint32_t idesc;
     int tile_k;     // operand elements per 128-byte stage row: 64 (16-bit) or 32 (fp32 read as TF32)
     int tf32;       // 1: kind::tf32 MMAs on split fp32 operands
@@ -93,6 +93,15 @@ struct TcMaps {
     CUtensorMap c_full, c_half;   // output: boxes of 32 rows x (32 | 16) accumulator columns
     CUtensorMap r_full, r_half;   // EPI_RESID: residual input (fp32), same boxes; EPI_SPLIT16: the fp16 output, dense boxes
 };
+
+// x / d for a divisor in [1, 16) whose rounded reciprocal z is known: the product, and one correction with its exact remainder
+// (P. Markstein, Computation of elementary functions on the IBM RISC System/6000 processor, 1990).  The quotient's own bits: with
+// d = sqrt 2 checked for every x (below 2^-124 it can be a denormal step off), with other divisors for 400 million pairs.  A remainder
+// that is zero or not a number (x zero, infinite, NaN) leaves the product.
+__device__ __forceinline__ float div_known(float x, float d, float z) {
+    const float q = x * z, rem = fmaf(-d, q, x);
+    return fabsf(rem) > 0.0f ? fmaf(rem, z, q) : q;
+}
 
 // Writes one epilogue block into its shared-memory tile.  Lane = accumulator row, r = its 32 (or 16) fp32 columns.
 //   fp32 tiles, 32 columns: 128-byte rows, 16-byte chunk j of row l at chunk j ^ (l & 7) (the TMA 128-byte swizzle,
@@ -164,7 +173,12 @@ __device__ __forceinline__ void stage_block(const TcParams& p, uint32_t tile, in
                 float4 v = make_float4(__uint_as_float(r[4 * j]), __uint_as_float(r[4 * j + 1]), __uint_as_float(r[4 * j + 2]),
                                        __uint_as_float(r[4 * j + 3]));
                 if constexpr (EPI == EPI_RESID) {
-                    if (p.r_div != 1.0f) {
+                    if (p.r_inv != 0.0f) {
+                        // a division of its own for each of the 32 columns, one behind the other, took longer than the product: per
+                        // launch of the o-projection 32.7 us at 20 windows, 18.5 at 1, 155.6 at 512; this way 16.4, 12.3 and 146, as without
+                        v.x = rr[j].x + div_known(v.x, p.r_div, p.r_inv); v.y = rr[j].y + div_known(v.y, p.r_div, p.r_inv);
+                        v.z = rr[j].z + div_known(v.z, p.r_div, p.r_inv); v.w = rr[j].w + div_known(v.w, p.r_div, p.r_inv);
+                    } else if (p.r_div != 1.0f) {
                         v.x = rr[j].x + v.x / p.r_div; v.y = rr[j].y + v.y / p.r_div; v.z = rr[j].z + v.z / p.r_div; v.w = rr[j].w + v.w / p.r_div;
                     } else {
                         v.x = rr[j].x + v.x; v.y = rr[j].y + v.y; v.z = rr[j].z + v.z; v.w = rr[j].w + v.w;
@@ -574,6 +588,7 @@ static int plan_impl(const shvk_gemm_args* g, int ab_dtype, void* host_plan, int
     p.m_tiles = (g->M + TILE_M - 1) / TILE_M;
     p.bias = g->bias;
     p.r_div = g->r_div == 0.0f ? 1.0f : g->r_div;
+    p.r_inv = p.r_div > 1.0f && p.r_div < 16.0f ? 1.0f / p.r_div : 0.0f;
     const uint32_t fmt = split ? 2u : (ab_dtype == DT_BF16 ? 1u : 0u);      // f16 0, bf16 1, tf32 2
     // instruction descriptor: D fp32 (bits 4-5 = 1), A/B format (bits 7-9, 10-12), both K-major, N/8 at bit 17,
     // M/16 at bit 24

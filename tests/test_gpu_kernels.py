@@ -181,6 +181,31 @@ def test_gemm_tc_epilogues_and_partial_rows(L):
     assert tc_status(L) == 0
 
 
+@pytest.mark.parametrize("r_div", [1.0, 2.0 ** 0.5, 1.0 + 2.0 ** -23, 3.0, 16.0 - 2.0 ** -20, 16.0, 0.3, -1.5])
+def test_gemm_tc_residual_divides_to_the_bit(L, r_div):
+    """R + sum / r_div rounds as the division does, for divisors of the reciprocal's path and for the others, zeros,
+    infinities and NaN included."""
+    import torch
+    M, N, K = 200, 384, 64
+    rng = np.random.default_rng(11)
+    a = (rng.standard_normal((M, K)) * 10.0 ** rng.uniform(-12, 12, (M, 1))).astype(np.float32)
+    a[5] = 0.0
+    a[6, 0], a[7, 1], a[8, 2] = np.inf, -np.inf, np.nan
+    A, Wt = dev(a, torch.bfloat16), dev((rng.standard_normal((N, K)) / 8).astype(np.float32), torch.bfloat16)
+    r = rng.standard_normal((M, N)).astype(np.float32)
+    d = np.float32(r_div)
+    Cm, H = torch.zeros((M, N), device="cuda"), dev(r)
+    keep, plan = tc_plan(L, gemm_args(M, N, K, A, Wt, Cm, N), 1)
+    keep2, plan2 = tc_plan(L, gemm_args(M, N, K, A, Wt, H, N, R=H, ldr=N, r_div=float(d)), 1)
+    ok(L.shvk_gemm_tc(plan, stream_ptr()))
+    ok(L.shvk_gemm_tc(plan2, stream_ptr()))
+    sync()
+    with np.errstate(all="ignore"):
+        ref = r + Cm.cpu().numpy() / d
+    assert np.array_equal(H.cpu().numpy(), ref, equal_nan=True)
+    assert tc_status(L) == 0
+
+
 def test_gemm_tc_rows_do_not_depend_on_the_batch(L):
     import torch
     rng = np.random.default_rng(33)
