@@ -24,16 +24,12 @@ size_t se_gate_frame_bytes(int C, int CS);       // shared memory of a frame in 
 int se_partial_sums(const float* x, float* partial, int F, int HW, int C, cudaStream_t s);   // cnn.cu
 namespace {
 
-// x * relu6(x + 3) / 6 of a pair, each step rounded as cnn.cu rounds it.  The quotient is a product and an FMA with 1/6 in two
-// parts (Brisebarre, Muller, Raina, "Accelerating correctly rounded floating-point division when the divisor is known in
-// advance", 2004); with the high part rounded down it is the IEEE quotient of every float32 of at least 1.25 x 2^-122 (tried
-// for all of them), infinity too.  Encoding 640 crops bf16 takes 6.09 ms; with x * saturate(x / 6 + 1/2), which rounds otherwise
-// (1e-7 absolute near -3), 5.99.
+// x * relu6(x + 3) / 6 of a pair, each step rounded as cnn.cu rounds it (div6).  Encoding 640 crops bf16 takes 6.09 ms; with
+// x * saturate(x / 6 + 1/2), which rounds otherwise (1e-7 absolute near -3), 5.99.
 __device__ __forceinline__ float2 hswish2(float2 x) {
-    constexpr float HI = 0x1.555554p-3f, LO = 0x1.555556p-27f;
     const float2 s = add2(x, make_float2(3.0f, 3.0f));
     const float2 p = mul2(x, make_float2(fminf(fmaxf(s.x, 0.0f), 6.0f), fminf(fmaxf(s.y, 0.0f), 6.0f)));
-    return fma2(p, make_float2(HI, HI), mul2(p, make_float2(LO, LO)));
+    return fma2(p, make_float2(SIXTH_HI, SIXTH_HI), mul2(p, make_float2(SIXTH_LO, SIXTH_LO)));
 }
 template <bool HS> __device__ __forceinline__ float2 act2(float2 x) { return HS ? hswish2(x) : make_float2(fmaxf(x.x, 0.0f), fmaxf(x.y, 0.0f)); }
 
@@ -665,7 +661,7 @@ se_gate_cluster_kernel(const float* __restrict__ sums, const float* __restrict__
             if (lane == 0)
 #pragma unroll
                 for (int fr = 0; fr < G; ++fr)
-                    if (fr < nf) gate[(long long)(f0 + fr) * C + c] = fminf(fmaxf(acc[u][fr] + b2[c] + 3.0f, 0.0f), 6.0f) / 6.0f;
+                    if (fr < nf) gate[(long long)(f0 + fr) * C + c] = div6(fminf(fmaxf(acc[u][fr] + b2[c] + 3.0f, 0.0f), 6.0f));
         }
     }
 }

@@ -94,15 +94,6 @@ struct TcMaps {
     CUtensorMap r_full, r_half;   // EPI_RESID: residual input (fp32), same boxes; EPI_SPLIT16: the fp16 output, dense boxes
 };
 
-// x / d for a divisor in [1, 16) whose rounded reciprocal z is known: the product, and one correction with its exact remainder
-// (P. Markstein, Computation of elementary functions on the IBM RISC System/6000 processor, 1990).  The quotient's own bits: with
-// d = sqrt 2 checked for every x (below 2^-124 it can be a denormal step off), with other divisors for 400 million pairs.  A remainder
-// that is zero or not a number (x zero, infinite, NaN) leaves the product.
-__device__ __forceinline__ float div_known(float x, float d, float z) {
-    const float q = x * z, rem = fmaf(-d, q, x);
-    return fabsf(rem) > 0.0f ? fmaf(rem, z, q) : q;
-}
-
 // Writes one epilogue block into its shared-memory tile.  Lane = accumulator row, r = its 32 (or 16) fp32 columns.
 //   fp32 tiles, 32 columns: 128-byte rows, 16-byte chunk j of row l at chunk j ^ (l & 7) (the TMA 128-byte swizzle,
 //                           which also makes these stores bank-conflict free); 16 columns: dense 64-byte rows
