@@ -248,7 +248,10 @@ template <int COLS, int TB> struct Share {
 // acc[c][e] += sum over a chunk's k of X[c][k] W[k][pair]; k ascending
 template <int COLS, int KC, int TPC>
 __device__ __forceinline__ void chunk_product(const float* w, const float* x, int xp, float (&acc)[TPC][2]) {
-#pragma unroll 4
+    // 32 (40) k in flight, a chunk in whole groups: with 16 a classify of one window takes 211 us instead of 209; with the next
+    // group's operands asked for ahead, through a second set of registers, 215
+    constexpr int UNROLL = KC % 120 ? 8 : 10;
+#pragma unroll UNROLL
     for (int k = 0; k < KC; k += 4) {
         float2 v[4];
 #pragma unroll
