@@ -35,8 +35,8 @@ template <> struct Row8<false> {
     }
 };
 template <> struct Row8<true> {
-    static __device__ __forceinline__ void load(const void* base, int i, float (&v)[8]) {
-        const uint4 u = static_cast<const uint4*>(base)[i];
+    static __device__ __forceinline__ void load(const void* base, int i, float (&v)[8]) { widen(static_cast<const uint4*>(base)[i], v); }
+    static __device__ __forceinline__ void widen(const uint4 u, float (&v)[8]) {
         const __half2* h = reinterpret_cast<const __half2*>(&u);
 #pragma unroll
         for (int e = 0; e < 4; ++e) {
@@ -66,8 +66,8 @@ template <> struct Row4<false> {
     }
 };
 template <> struct Row4<true> {
-    static __device__ __forceinline__ void load(const void* base, int i, float (&v)[4]) {
-        const uint2 u = static_cast<const uint2*>(base)[i];
+    static __device__ __forceinline__ void load(const void* base, int i, float (&v)[4]) { widen(static_cast<const uint2*>(base)[i], v); }
+    static __device__ __forceinline__ void widen(const uint2 u, float (&v)[4]) {
         const __half2* h = reinterpret_cast<const __half2*>(&u);
         const float2 f0 = __half22float2(h[0]), f1 = __half22float2(h[1]);
         v[0] = f0.x; v[1] = f0.y; v[2] = f1.x; v[3] = f1.y;
@@ -77,9 +77,14 @@ template <> struct Row4<true> {
 // Four CTAs of 192 threads per SM: the phases of one CTA alternate between loads and scans, and more resident CTAs keep
 // HBM busy through the scans.  B = 4096, 16-bit rows: a thread per token with sincosf and a value sum of one column per
 // thread 1.18 ms (256 threads x 4 CTAs; 352 x 3 1.16, 352 x 2 1.45, 192 x 5 1.10); hardware sin / cos and 16-byte value
-// reads 0.98 ms; eight threads per token in the score phase as well 0.73 ms (four, five and six CTAs per SM the same).
-template <bool H16>
-__global__ void __launch_bounds__(NT, 4)
+// reads 0.98 ms; eight threads per token in the score phase as well 0.76 ms (four, five and six CTAs per SM the same); with four
+// rounds of the scores and seven of the value sum in flight instead of two and four, 0.73 (512 windows: 114 -> 104 us).
+// FEW: as long as every (clip, head) has an SM to itself nothing else hides its loads, so a thread asks for all its pieces of K, B
+// and V before it does anything (188 registers, one CTA per SM); the arithmetic is the same.  us per classify, 16-bit, without /
+// with: 1 window 209.1 / 204.6, 20 311.0 / 302.9, 24 330.2 / 321.4; beyond, one at a time on an SM, 28 365.3 / 364.4, 48
+// 461.9 / 461.7, 96 857 / 864.
+template <bool H16, bool FEW>
+__global__ void __launch_bounds__(NT, FEW ? 1 : 4)
 sisa_attn_kernel(const void* __restrict__ Skvb, const float* __restrict__ Sgate, const float* __restrict__ QC,
                  const float* __restrict__ lambda_raw, float* __restrict__ Y) {
     using KV = typename std::conditional<H16, __half, float>::type;
@@ -97,6 +102,20 @@ sisa_attn_kernel(const void* __restrict__ Skvb, const float* __restrict__ Sgate,
     __shared__ float red[NT / 32];
     __shared__ float ypart[NT / 32][kDK];
 
+    constexpr int ROUNDS = (kTok + VSLOTS - 1) / VSLOTS;
+    [[maybe_unused]] uint4 krow[ROUNDS], vrow[ROUNDS];
+    [[maybe_unused]] uint2 brow[ROUNDS];
+    if constexpr (FEW) {                       // this thread's pieces of K, B and V of all its tokens: nothing they wait for
+#pragma unroll
+        for (int i = 0; i < ROUNDS; ++i) {
+            const int t = i * VSLOTS + (tid >> 3);
+            const bool in = t < kTok;
+            const KV* row = S0 + (long long)(in ? t : 0) * LDK;
+            krow[i] = __ldg(reinterpret_cast<const uint4*>(row + kSK + head * kDK) + (tid & 7));
+            brow[i] = __ldg(reinterpret_cast<const uint2*>(row + kSB + head * kState) + (tid & 7));
+            vrow[i] = __ldg(reinterpret_cast<const uint4*>(row + kSV + head * kDK) + (tid & 7));
+        }
+    }
     // per-token terms: theta[16] of this head is one 64-byte run, alpha and forget are single floats
     for (int tk = tid; tk < kTok; tk += NT) {
         const float* row = SG0 + (long long)tk * LDG + G0;
@@ -161,14 +180,19 @@ sisa_attn_kernel(const void* __restrict__ Skvb, const float* __restrict__ Sgate,
         for (int e = 0; e < 8; ++e) q8[e] = sq[8 * part + e];
 #pragma unroll
         for (int e = 0; e < 4; ++e) c4[e] = sc[4 * part + e];
-#pragma unroll 2
-        for (int t0 = 0; t0 < kTok; t0 += VSLOTS) {
-            const int t = t0 + slot;
+#pragma unroll(FEW ? ROUNDS : 4)
+        for (int i = 0; i < ROUNDS; ++i) {
+            const int t = i * VSLOTS + slot;
             float content = 0.0f, ssm = 0.0f;
             if (t < kTok) {
                 float kk[8], bb[4];
-                Row8<H16>::load(S0 + (long long)t * LDK + kSK + head * kDK, part, kk);
-                Row4<H16>::load(S0 + (long long)t * LDK + kSB + head * kState, part, bb);
+                if constexpr (FEW) {
+                    Row8<true>::widen(krow[i], kk);
+                    Row4<true>::widen(brow[i], bb);
+                } else {
+                    Row8<H16>::load(S0 + (long long)t * LDK + kSK + head * kDK, part, kk);
+                    Row4<H16>::load(S0 + (long long)t * LDK + kSB + head * kState, part, bb);
+                }
 #pragma unroll
                 for (int e = 0; e < 8; ++e) content = fmaf(q8[e], kk[e], content);
 #pragma unroll
@@ -218,10 +242,13 @@ sisa_attn_kernel(const void* __restrict__ Skvb, const float* __restrict__ Sgate,
     float y[8];
 #pragma unroll
     for (int e = 0; e < 8; ++e) y[e] = 0.0f;
-#pragma unroll 4
-    for (int t = slot; t < kTok; t += VSLOTS) {
+#pragma unroll(FEW ? ROUNDS : 7)
+    for (int i = 0; i < ROUNDS; ++i) {
+        const int t = i * VSLOTS + slot;
+        if (t >= kTok) break;
         float vv[8];
-        Row8<H16>::load(S0 + (long long)t * LDK + kSV + head * kDK, part, vv);
+        if constexpr (FEW) Row8<true>::widen(vrow[i], vv);
+        else Row8<H16>::load(S0 + (long long)t * LDK + kSV + head * kDK, part, vv);
         const float pt = score[t] * inv;
 #pragma unroll
         for (int e = 0; e < 8; ++e) y[e] = fmaf(pt, vv[e], y[e]);
@@ -249,7 +276,7 @@ sisa_attn_kernel(const void* __restrict__ Skvb, const float* __restrict__ Sgate,
 
 extern "C" int shvk_sisa_attn(const float* S, const float* QC, const float* lambda_raw, float* Y, int B, void* stream) {
     if (B <= 0) return 0;
-    sb::sisa_attn_kernel<false><<<unsigned(B) * sb::kHeads, sb::NT, 0, cudaStream_t(stream)>>>(S, S, QC, lambda_raw, Y);
+    sb::sisa_attn_kernel<false, false><<<unsigned(B) * sb::kHeads, sb::NT, 0, cudaStream_t(stream)>>>(S, S, QC, lambda_raw, Y);
     return int(cudaGetLastError());
 }
 
@@ -257,6 +284,7 @@ extern "C" int shvk_sisa_attn_h16(const void* S16, const float* SG, const float*
                                   void* stream) {
     if (B <= 0) return 0;
     if (!S16 || !SG || ((reinterpret_cast<uintptr_t>(S16) | reinterpret_cast<uintptr_t>(SG)) & 15)) return int(cudaErrorInvalidValue);
-    sb::sisa_attn_kernel<true><<<unsigned(B) * sb::kHeads, sb::NT, 0, cudaStream_t(stream)>>>(S16, SG, QC, lambda_raw, Y);
+    if (B <= sb::device_sms() / sb::kHeads) sb::sisa_attn_kernel<true, true><<<unsigned(B) * sb::kHeads, sb::NT, 0, cudaStream_t(stream)>>>(S16, SG, QC, lambda_raw, Y);
+    else sb::sisa_attn_kernel<true, false><<<unsigned(B) * sb::kHeads, sb::NT, 0, cudaStream_t(stream)>>>(S16, SG, QC, lambda_raw, Y);
     return int(cudaGetLastError());
 }

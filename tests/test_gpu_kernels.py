@@ -870,6 +870,22 @@ def test_sisa_attention_matches_oracle(L, weight_files):
     assert rel_err(Y16.cpu().numpy(), tr["sisa.attn_y_last"]) < 2e-3           # fp16 rounding of K, V, B only
 
 
+@pytest.mark.parametrize("B", [1, 24, 25])
+def test_sisa_attn_of_few_clips_has_the_bits_of_many(L, B):
+    """Up to a (clip, head) per SM the rows of K, B and V are all asked for first; the results do not change."""
+    import torch
+    rng = np.random.default_rng(7)
+    many = 60
+    s16 = dev(rng.standard_normal((many * 321, 960)).astype(np.float16))
+    sg = dev((rng.standard_normal((many * 321, 112)) * 0.3).astype(np.float32))
+    qc, lam = dev(rng.standard_normal((many, 576)).astype(np.float32)), dev(rng.standard_normal(6).astype(np.float32))
+    Y, Yb = torch.zeros((many, 384), device="cuda"), torch.full((many, 384), 7.0, device="cuda")
+    ok(L.shvk_sisa_attn_h16(s16.data_ptr(), sg.data_ptr(), qc.data_ptr(), lam.data_ptr(), Y.data_ptr(), many, stream_ptr()))
+    ok(L.shvk_sisa_attn_h16(s16.data_ptr(), sg.data_ptr(), qc.data_ptr(), lam.data_ptr(), Yb.data_ptr(), B, stream_ptr()))
+    sync()
+    assert torch.isfinite(Y).all() and torch.equal(Y[:B], Yb[:B]) and (Yb[B:] == 7.0).all()
+
+
 def test_gemm_tc_split16_epilogue(L):
     """SISA projection shape: columns below 960 leave as fp16 rows, the rest as fp32 (+ bias) rows of pitch 112."""
     import torch
