@@ -18,7 +18,7 @@
 // chunk's tiles (the block's last 1,280 bytes).  The 16 x 16 triangular inverse is a forward substitution in fp32, one
 // column per lane.
 //
-// gdn_scan_t_kernel: one CTA (four warps) owns one (clip, head) and walks its 21 chunk blocks.  A block (q^T, k^T, v^T,
+// gdn_scan_t_kernel: one CTA (four warps, and with few clips a fifth that loads) owns one (clip, head) and walks its 21 chunk blocks.  A block (q^T, k^T, v^T,
 // gate^T tiles, log decays, betas, and what the preparation added: 13,696 contiguous bytes) arrives by ONE bulk copy into
 // a three-slot ring, two chunks ahead.  Nothing is converted or re-laid-out: every operand fragment of the chunk's
 // products comes straight out of the landed tiles with ldmatrix (transposing where the product wants tokens along the
@@ -294,8 +294,12 @@ __device__ unsigned long long g_scan_cycles[4][8];
 #define SCAN_TICK(slot) do { } while (0)
 #endif
 
-template <typename T>
-__global__ void __launch_bounds__(128, 3)
+// LOADER: asking for a block (proxy fence, expected bytes, copy) costs the warp that does it some 290 of a chunk's 2,000 cycles, and the
+// others wait for it at the barrier.  As long as two CTAs per SM hold the batch a fifth warp does it: us per classify, fp16,
+// without / with: 1 window 204.8 / 200.8, 24 321.5 / 317.3, 48 461.9 / 456.9.  With three CTAs per SM the others' work hides it, and
+// five warps leave too few registers for three: 56 windows 517 / 552.
+template <typename T, bool LOADER>
+__global__ void __launch_bounds__(LOADER ? 160 : 128, LOADER ? 2 : 3)
 gdn_scan_t_kernel(const uint8_t* __restrict__ ptb, const float* __restrict__ o_norm_w, T* __restrict__ on, int* __restrict__ status,
                   uint32_t wait_polls, int starve) {
     extern __shared__ uint8_t scan_t_smem_raw[];
@@ -368,9 +372,23 @@ gdn_scan_t_kernel(const uint8_t* __restrict__ ptb, const float* __restrict__ o_n
     unsigned ticks[8] = {0, 0, 0, 0, 0, 0, 0, 0};
     unsigned tick0 = unsigned(clock());
 #endif
+    if constexpr (LOADER) {
+        if (warp == 4) {                                  // the fifth warp asks for the blocks, behind the same barriers
+            for (int chunk = 0; chunk < NCHUNK; ++chunk) {
+                if (chunk + 2 < NCHUNK && elect_one()) {
+                    tma::fence_proxy_async();
+                    issue(chunk + 2);
+                }
+                __syncwarp();
+                if (!tma::mbar_wait_bounded(bars0 + 8u * uint32_t(chunk % NSLOT), uint32_t(chunk / NSLOT) & 1u, wait_polls)) return;
+                __syncthreads();
+            }
+            return;
+        }
+    }
     for (int chunk = 0; chunk < NCHUNK; ++chunk) {
         Block& b = sm.blk[chunk % NSLOT];
-        if (tid == 0 && chunk + 2 < NCHUNK) {
+        if (!LOADER && tid == 0 && chunk + 2 < NCHUNK) {
             // ring slot (chunk + 2) % 3 was last read by chunk - 1, which ended at the previous barrier
             tma::fence_proxy_async();
             issue(chunk + 2);
@@ -543,11 +561,13 @@ gdn_scan_t_kernel(const uint8_t* __restrict__ ptb, const float* __restrict__ o_n
 
 template <typename T>
 int launch(const void* ptb, const float* o_norm_w, void* on, int B, uint32_t polls, int starve, cudaStream_t stream) {
-    const cudaError_t e = cudaFuncSetAttribute(gdn_scan_t_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES);
+    const bool loader = (long long)B * kHeads <= 2ll * device_sms();
+    const auto kernel = loader ? gdn_scan_t_kernel<T, true> : gdn_scan_t_kernel<T, false>;
+    const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES);
     if (e != cudaSuccess) return int(e);
     int* status = gdn_scan_t_status_word();
     if (!status) return int(cudaErrorInvalidSymbol);
-    gdn_scan_t_kernel<T><<<unsigned(B) * kHeads, 128, SMEM_BYTES, stream>>>(static_cast<const uint8_t*>(ptb), o_norm_w,
+    kernel<<<unsigned(B) * kHeads, loader ? 160 : 128, SMEM_BYTES, stream>>>(static_cast<const uint8_t*>(ptb), o_norm_w,
                                                                             static_cast<T*>(on), status, polls, starve);
     return int(cudaGetLastError());
 }

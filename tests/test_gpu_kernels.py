@@ -683,6 +683,31 @@ def test_gdn_inproj_tiles_match_oracle(L, weight_files, recipe, stage, B, mode):
     assert (dec[:, :, 321:] == 0).all() and (beta[:, :, 321:] == 0).all()
 
 
+def test_gdn_scan_of_few_clips_has_the_bits_of_many(L, weight_files):
+    """With two CTAs per SM or fewer a fifth warp loads the blocks; the results do not change, and both forms give up."""
+    import torch
+    _, w0 = weight_files("W3", 1)
+    w = rounded_mixer_weights(w0, "gdn_a")
+    many = 2 * torch.cuda.get_device_properties(0).multi_processor_count // 6 + 1
+    pt, keep = run_inproj(L, w, "gdn_a", bf16_round(np.random.default_rng(3).standard_normal((many, 321, 384))), many)
+    ow = dev((1.0 + 0.1 * np.random.default_rng(1).standard_normal(128)).astype(np.float32))
+    out = {}
+    for B in (many, many - 1, 1):
+        out[B] = torch.full((many * 321, 768), 9.0, device="cuda", dtype=torch.bfloat16)
+        ok(L.shvk_gdn_scan_t(pt.data_ptr(), ow.data_ptr(), out[B].data_ptr(), 1, B, stream_ptr()))
+    sync()
+    for B in (many - 1, 1):
+        assert torch.equal(out[B][:B * 321], out[many][:B * 321]) and (out[B][B * 321:] == 9.0).all()
+    for B in (many, many - 1):
+        on, st = torch.full((many * 321, 768), 5.0, device="cuda", dtype=torch.bfloat16), C.c_int(-1)
+        ok(L.shvk_gdn_scan_t_starved(pt.data_ptr(), ow.data_ptr(), on.data_ptr(), 1, B, 1024, stream_ptr()))
+        sync()
+        ok(L.shvk_gdn_scan_status(C.byref(st)))
+        ok(L.shvk_status_clear_async(stream_ptr()))
+        sync()
+        assert st.value != 0 and (on == 5.0).all()
+
+
 @pytest.mark.parametrize("recipe,stage,B", [("W3", "gdn_a", 2), ("W3", "gdn_b", 1), ("W1", "gdn_a", 3)])
 def test_gdn_inproj_scan_matches_oracle(L, weight_files, recipe, stage, B):
     """In-projection + scan of the 16-bit modes against the oracle's gated delta-rule output."""
