@@ -270,9 +270,9 @@ private:
     // block's columns over the SMs (the same sums in the same order) but move the hidden layer through L2: 19 us + 0.30 us per
     // row block.  us per block, fused / two GEMMs: 1 window 39 / 24, 8 39 / 28, 20 41 / 37, 32 41 / 48, 48 43 / 57, 59 44 / 61,
     // 64 74 / 70, 80 75 / 79, 96 79 / 95, 128 114 / 117.  us per classify, fused / two GEMMs: 20 windows 367 / 351, 28
-    // 417 / 406, 32 438 / 441, 40 473 / 491, 64 675 / 669, 80 793 / 797, 128 1233 / 1263.  Beyond FFN_TWO_ROWS the hidden
-    // layer would not stay in L2.
-    static constexpr int FFN_TWO_ROWS = 128 * NTOK;
+    // 417 / 406, 32 438 / 441, 40 473 / 491, 64 675 / 669, 80 793 / 797, 120 1223 / 1241, 128 1233 / 1263.  Beyond FFN_TWO_ROWS
+    // (two rounds) the fused kernel is the faster one throughout.
+    static constexpr int FFN_TWO_ROWS = 80 * NTOK;
     bool two_launch_ffn(int rows) const {
         if (size_t(rows) > hid_rows_) return false;
         if (prec_ == Precision::FP32) return true;

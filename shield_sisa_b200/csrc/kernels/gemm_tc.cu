@@ -486,7 +486,7 @@ int choose_bn(int n) {
 // row block.  While the plan's width gives no more than two tiles per SM, what counts is the longest chain of one SM: tiles
 // per SM times (k steps, and filling the ring and draining the last accumulator: about 600 + 8 bn cycles), and a narrower
 // tile spreads a short problem over more SMs.  o-projection (N 384, K 768), us per launch at the plan's width / this one: 1
-// window 25 / 17, 8 26 / 17, 32 34 / 29, from 64 on the same.
+// window 25 / 17, 8 26 / 17, 32 34 / 29, from 64 on the same (both with 6 us or more of divisions in the epilogue, since gone).
 // A column's sum does not depend on the width of its tile.  EPI_SPLIT16 needs multiples of 32.
 int launch_bn(const TcParams& p, int epi, int sms) {
     if ((long long)p.m_tiles * p.n_tiles > 2ll * sms) return p.BN;
