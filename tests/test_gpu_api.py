@@ -2,6 +2,7 @@
 device token slots, pinned buffers, and failure reporting with the failure injected on the host."""
 import os
 import threading
+import time
 
 import numpy as np
 import pytest
@@ -65,6 +66,51 @@ def test_many_jobs_coalesce_and_keep_order(model):
     got = np.concatenate(outs)
     np.testing.assert_array_equal(got.view(np.uint32), want.view(np.uint32))
     assert max(sizes) <= 16 and sum(1 for s in sizes if s > 1) > 0      # at least some jobs shared a batch
+
+
+def test_a_callback_does_not_hold_back_jobs_behind_it(model):
+    """While a callback runs, the batches behind it go on and so do jobs submitted meanwhile, small ones too, as long as lanes
+    are free: none of them waits for the callback to return."""
+    tok = W.synth_tokens(1, 23)
+    want = model.classify(tok)
+    entered, release = threading.Event(), threading.Event()
+
+    def cb(job, status, user):
+        entered.set()
+        release.wait(10)
+
+    outs = [np.zeros(1, np.float32) for _ in range(4)]
+    jobs = [model.submit(1, outs[0], window_tokens=blocks_of(tok), callback=cb)]
+    assert entered.wait(10)
+    for o in outs[1:]:                                                   # three more: the four lanes are taken then
+        jobs.append(model.submit(1, o, window_tokens=blocks_of(tok)))
+        time.sleep(0.1)                                      # its GPU work ends meanwhile, and nothing is queued
+    release.set()
+    for job, _ in jobs:
+        assert job and model.job_wait(job) == 0
+        assert model.job_timing(job)[1]["queue_ms"] < 50.0
+        model.job_free(job)
+    np.testing.assert_array_equal(np.concatenate(outs).view(np.uint32), np.repeat(want, 4).view(np.uint32))
+
+
+def test_small_jobs_behind_two_batches_share_the_third(weight_files):
+    """With one batch on the GPU and one queued, single windows wait for the first to end and then run as one batch."""
+    path, _ = weight_files("W3", 1)
+    tok = W.synth_tokens(1, 23)
+    slots = np.arange(20, dtype=np.int32)
+    with binding.CudaModel(path, "fp32", max_windows=512, max_host_tokens=20, token_slots=20) as m:
+        m.upload_tokens(tok[0], slots)
+        sizes, outs, jobs = (512, 512) + 8 * (1,), [], []                # 512 windows keep the GPU busy for tens of milliseconds
+        for n in sizes:
+            outs.append(np.zeros(n, np.float32))
+            jobs.append(m.submit(n, outs[-1], window_slots=np.tile(slots, n)))
+        seen = []
+        for job, _ in jobs:
+            assert job and m.job_wait(job) == 0
+            seen.append(m.job_timing(job)[1]["batch_windows"])
+            m.job_free(job)
+    assert seen == [512, 512] + 8 * [8]
+    assert len({o.tobytes() for o in outs[2:]}) == 1 and (np.concatenate(outs) == outs[2][0]).all()
 
 
 def test_request_validation(model):
