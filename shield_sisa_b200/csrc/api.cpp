@@ -105,6 +105,7 @@ struct shv_cuda_job {
     std::vector<Entry> entries;             // n_windows * 20
     std::vector<Span> spans;                // the job's host blocks in entry order (or in upload order)
     int n_host = 0;
+    size_t host_bytes = 0;                  // of the spans
     std::vector<int32_t> host_slot;         // upload job: destination slot of every host block (empty otherwise)
     float* logits_out = nullptr;
     shv_cuda_callback callback = nullptr;
@@ -261,6 +262,7 @@ public:
             pending_.push_back(j);
             pending_windows_ += j->n_windows;
             pending_blocks_ += j->n_host;
+            pending_bytes_ += j->host_bytes;
             pending_crops_ += j->n_crops;
         }
         work_.notify_all();
@@ -294,6 +296,7 @@ private:
     std::condition_variable work_;           // pending job, freed lane, launched batch, shutdown
     std::deque<shv_cuda_job*> pending_;
     long pending_windows_ = 0, pending_blocks_ = 0, pending_crops_ = 0;   // what the jobs in `pending_` hold
+    size_t pending_bytes_ = 0;               // of the host blocks
     std::deque<Lane*> idle_;
     std::deque<Flight> flying_;
     int unfinished_ = 0;                     // batches of `flying_` whose GPU work the finisher has not seen end
@@ -343,6 +346,7 @@ private:
             pending_.pop_front();
             pending_windows_ -= j->n_windows;
             pending_blocks_ -= j->n_host;
+            pending_bytes_ -= j->host_bytes;
             pending_crops_ -= j->n_crops;
             out.push_back(j);
             windows += j->n_windows;
@@ -359,9 +363,15 @@ private:
     // requests and took the GPU as long as 30 more.  Median, 10th and 90th percentile of 50: 7.52 (7.43 to 7.62) -> 6.77 ms (6.68 to
     // 6.84), 10 participants 2.75 (2.73 to 2.78) -> 1.94 (1.92 to 1.95).)  How long a callback takes is the caller's affair, and while
     // one runs nobody sees the batches behind it end: no job waits then.
+    //
+    // A batch's worth of host tokens is that of 36 windows where kernels are as fast as their upload: a window's 491,520 bytes take the
+    // copy engine 9 us, the 16-bit kernels 10 in a batch of 50, and a wait leaves the copy engine idle.  Thousand windows/s, bf16,
+    // windows a call x callers, no waiting / up to 256 windows: 4 x 4 17.0 / 22.1, 20 x 4 61 / 67, 32 x 4 74.6 / 75.1, 40 x 4 85 / 80,
+    // 50 x 4 90 / 82, 100 x 4 98 / 86, 250 x 4 106 / 93; up to 48: 32 x 4 76.9, 40 x 4 83.  The exact tier takes 40 us a window.
     bool worth_a_lane() const {
+        const int token_windows = mode == "fp32" ? upload_windows() : std::min(upload_windows(), 36);
         return unfinished_ < 2 || calling_back_ || pending_windows_ >= upload_windows() || pending_crops_ >= upload_crops() ||
-               pending_blocks_ >= long(upload_windows()) * kWin;
+               pending_bytes_ >= size_t(token_windows) * kWin * kTokBytes || pending_blocks_ >= std::max(block_cap(), 1);
     }
 
     // ------------------------------------------------------------------------------------------ feeder
@@ -597,6 +607,7 @@ void group_spans(shv_cuda_job& j, const std::vector<const float*>& blocks, bool 
         size_t end = at + 1;
         while (end < blocks.size() && blocks[end] == blocks[end - 1] + step) ++end;
         j.spans.push_back(Span{blocks[at], int(end - at), is_pinned(blocks[at], (end - at) * block_bytes), half});
+        j.host_bytes += (end - at) * block_bytes;
         at = end;
     }
     j.n_host = int(blocks.size());

@@ -113,6 +113,32 @@ def test_small_jobs_behind_two_batches_share_the_third(weight_files):
     assert len({o.tobytes() for o in outs[2:]}) == 1 and (np.concatenate(outs) == outs[2][0]).all()
 
 
+def test_host_tokens_behind_two_batches_are_uploaded_at_once(weight_files):
+    """Host tokens of 36 windows or more do not wait where the kernels are no slower than the upload (the 16-bit modes): the job
+    gets a batch of its own, and single windows that follow it share the next."""
+    path, _ = weight_files("W3", 1)
+    tok = W.synth_tokens(1, 23)
+    slots = np.arange(20, dtype=np.int32)
+    with binding.CudaModel(path, "bf16", max_windows=2048, max_host_tokens=40 * 20, token_slots=20) as m:
+        m.upload_tokens(tok[0], slots)
+        sizes = (2048, 2048, 36) + 8 * (1,)                              # 2,048 windows keep the GPU busy for some 16 ms
+        outs = [np.zeros(n, np.float32) for n in sizes]
+        host = blocks_of(tok) * 36
+        reqs = [binding.build_request(n, o, **({"window_tokens": host} if n == 36 else {"window_slots": np.tile(slots, n)}))
+                for n, o in zip(sizes, outs)]
+        jobs = []
+        for n, (req, _) in zip(sizes, reqs):
+            jobs.append(m.L.shv_cuda_submit(m.m, binding.C.byref(req)))
+            time.sleep(0.002 if n == 36 else 0)
+        seen = []
+        for job in jobs:
+            assert job and m.job_wait(job) == 0
+            seen.append(m.job_timing(job)[1]["batch_windows"])
+            m.job_free(job)
+    assert seen == [2048, 2048, 36] + 8 * [8]
+    assert (np.concatenate(outs) == outs[2][0]).all()
+
+
 def test_request_validation(model):
     L = model.L
     tok = W.synth_tokens(1, 23)
