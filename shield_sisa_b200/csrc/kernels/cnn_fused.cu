@@ -1051,8 +1051,9 @@ int launch_block(const BlockArgs& args, int F, cudaStream_t s) {
         // frames 117 / 117 / 127 / 131, 640 frames 304 / 280 / 283 / 346.
         int groups = 1;
         float least = 1e30f;
+        const int sms = device_sms();
         for (int g = 1; g <= C::CHUNKS; ++g) {
-            const long long n = (grid.x * (long long)g + device_sms() - 1) / device_sms();
+            const long long n = (grid.x * (long long)g + sms - 1) / sms;
             const float t = ((C::CHUNKS + g - 1) / g + 0.75f) * (1.25f * float(n / 2) + float(n % 2));
             if (t < least * 0.999f) { least = t; groups = g; }
         }
@@ -1239,7 +1240,8 @@ int launch_rows_gate(const float* A, const uint4* W, const float* b, const float
     // Few rows: a warp's chain of k steps is all the time there is, so its loads run ahead and the n tiles go to other blocks.  us,
     // whole / split: 160 channels of 960: 4 frames 41 / 15, 40 frames 64 / 18, 160 frames 64 / 43, 320 frames 75 / 87; 112 channels
     // of 480: 4 frames 23 / 10, 40 frames 33 / 24, 80 frames 33 / 39 (300 row blocks).
-    const bool few = 12LL * gx <= 13 * device_sms();     // about a row block per SM
+    const int sms = device_sms();
+    const bool few = 12LL * gx <= 13 * sms;     // about a row block per SM
     auto go = [&](auto kernel, unsigned gy) {
         kernel<<<dim3(gx, gy), 128, 0, s>>>(A, W, b, gate, gate_rows, R, out, M, N, K);
         return int(cudaGetLastError());
@@ -1249,7 +1251,7 @@ int launch_rows_gate(const float* A, const uint4* W, const float* b, const float
         int warps = 8;
         long long least = 1LL << 62;
         for (int w = 8; w >= 4; --w) {
-            const long long rows = ((blocks_of(M, w * 16) + device_sms() - 1) / device_sms()) * (long long)w;
+            const long long rows = ((blocks_of(M, w * 16) + sms - 1) / sms) * (long long)w;
             if (rows < least) { least = rows; warps = w; }
         }
         const int smem = decltype(layout)::STAGES * decltype(layout)::stage_bytes(warps);
