@@ -73,7 +73,7 @@ struct InprojParams {
     int starve;      // test launch only: the producer withholds the first weight tile of its first work item
     int qk_f16;      // q^T / k^T tiles in fp16 (fp16 mode) instead of bf16
     int probe;       // timing probes of a development build (-DSHVK_DEV_PROBES, SHVK_INPROJ_PROBE): 1 no global stores,
-                     // 2 no activation arithmetic, 4 no tensor-memory loads, 8 no MMA.  Constant 0 in the shipped libraries.
+                     // 2 no activation arithmetic, 8 no MMA.  Constant 0 in the shipped libraries.
 };
 // The probe bits travel in the kernel parameters (constant bank): a word in global memory would add a load in front of every
 // tile and change the timings it is meant to explain.
