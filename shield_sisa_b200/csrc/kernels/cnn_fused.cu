@@ -779,7 +779,7 @@ rows_gate_tile_kernel(const float* __restrict__ A, const uint4* __restrict__ W, 
                       int gate_rows, const float* R, float* out, int M, int N, int K) {
     using L = RowsTile<NT>;
     constexpr int NP = L::NP, STAGES = L::STAGES;
-    extern __shared__ __align__(128) uint8_t smem[];
+    extern __shared__ __align__(16) uint8_t smem[];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, t = lane & 3, rows = blockDim.x >> 1;
     const int mb = blockIdx.x * rows, m0 = mb + warp * 16, kt = (K + 15) / 16, ns = (kt + 1) / 2;
     const uint32_t sb = smem_addr(smem), stage_bytes = uint32_t(rows * 128 + L::W_BYTES);
