@@ -84,19 +84,20 @@ __device__ __forceinline__ void cluster_sync() {
 }
 
 // x / d for a divisor in [1, 16) whose rounded reciprocal z is known: the product, and one correction with its exact remainder
-// (P. Markstein, Computation of elementary functions on the IBM RISC System/6000 processor, 1990).  The quotient's own bits, for
-// d = sqrt 2 checked for every x on the CPU: below 2^-105, where the remainder is no longer exact, it can be one step off.  A
-// remainder that is zero or not a number (x zero, infinite, NaN) leaves the product.
-__device__ __forceinline__ float div_known(float x, float d, float z) {
+// (P. Markstein, Computation of elementary functions on the IBM RISC System/6000 processor, 1990).  The quotient's own bits for
+// every x of at least 2^-102 (for d = sqrt 2, tried with all of them, 2^-105; for other d with all mantissas): far below, where the
+// remainder is no longer exact, it can be one step off.  A remainder that is zero or not a number (x zero, infinite, NaN) leaves the
+// product.
+__host__ __device__ __forceinline__ float div_known(float x, float d, float z) {
     const float q = x * z, rem = fmaf(-d, q, x);
     return fabsf(rem) > 0.0f ? fmaf(rem, z, q) : q;
 }
 
 // x / 6 as a product and an FMA with 1/6 in two parts (Brisebarre, Muller, Raina, "Accelerating correctly rounded floating-point
 // division when the divisor is known in advance", 2004); with the high part rounded down it is the IEEE quotient of every float32
-// of at least 1.25 x 2^-122 (tried for all of them), infinity too.
+// above 1.25 x 2^-122 (tried for all of them), infinity too, and at most one step off below.
 constexpr float SIXTH_HI = 0x1.555554p-3f, SIXTH_LO = 0x1.555556p-27f;
-__device__ __forceinline__ float div6(float x) { return fmaf(x, SIXTH_HI, x * SIXTH_LO); }
+__host__ __device__ __forceinline__ float div6(float x) { return fmaf(x, SIXTH_HI, x * SIXTH_LO); }
 
 // Four consecutive outputs in storage type T (16, 8 or 8 bytes, address aligned accordingly).
 template <typename T> __device__ __forceinline__ void store_quad(T* p, float a, float b, float c, float d);
