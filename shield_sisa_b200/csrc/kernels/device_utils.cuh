@@ -36,10 +36,9 @@ __device__ __forceinline__ float warp_max(float v) {
     return v;
 }
 
-// One lane of a converged warp, always the same.  The roles that issue copies and MMAs branch on this and not on lane == 0: those
-// instructions take their operands from uniform registers, and behind a branch that the compiler cannot see to be one thread's each
-// of them is wrapped in code for several: a k-block of two TMA loads took its thread 511 cycles to issue (393 behind elect), one of
-// four MMAs and a commit 575 (403), more than the tensor core needs for it.
+// One lane of a converged warp, always the same.  The roles that issue copies and MMAs branch on this and not on lane == 0: measured,
+// a k-block of two TMA loads took its thread 511 cycles to issue behind lane == 0 (393 behind elect), one of four MMAs and a commit
+// 575 (403), more than the tensor core needs for it.
 __device__ __forceinline__ bool elect_one() {
     uint32_t one;
     asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(one));
