@@ -484,18 +484,22 @@ int choose_bn(int n) {
 
 // Accumulator width of one launch.  With tiles for every SM many times over it is the plan's: what counts is the time of a
 // row block.  While the plan's width gives no more than two tiles per SM, what counts is the longest chain of one SM: tiles
-// per SM times (k steps, and filling the ring and draining the last accumulator: about 600 + 8 bn cycles), and a narrower
-// tile spreads a short problem over more SMs.  o-projection (N 384, K 768), us per launch at the plan's width / this one: 1
-// window 25 / 17, 8 26 / 17, 32 34 / 29, from 64 on the same (both with 6 us or more of divisions in the epilogue, since gone).
+// per SM times the time of one, which goes with the operand rows that it brings in (128 + bn), and a narrower tile spreads a
+// short problem over more SMs.  us per launch, operands in L2, at the plan's width / this one, 1, 8, 14, 20, 32 windows: o-projection
+// 11.2 / 7.4, 11.3 / 7.8, 11.6 / 9.4, 11.7 / 11.7, 16.1 / 14.3; SISA projection 7.6 / 5.7, 8.0 / 7.2, 10.6 / 9.4, then the same;
+// feed-forward up 7.8 / 5.5, 10.4 / 8.7, then the same; down 13.2 / 10.0, 12.2 / 8.7, 12.5 / 10.2, 12.7 / 12.7, 18.3 / 15.8; from 45
+// windows on all the same.  Of every width, at eighteen window counts, for these shapes and the exact tier's five, the rule's is within
+// 0.7 % of the best on average.  (Counting the k steps' tensor time, where that is longer, and 600 + 8 bn cycles for the ends took 96
+// columns for the o-projection of 40 to 44 windows: 17 us instead of 16, exact tier 80 instead of 65.)
 // A column's sum does not depend on the width of its tile.  EPI_SPLIT16 needs multiples of 32.
 int launch_bn(const TcParams& p, int epi, int sms) {
     if ((long long)p.m_tiles * p.n_tiles > 2ll * sms) return p.BN;
-    const int step = epi == EPI_SPLIT16 ? 32 : 16, nk = p.K / p.tile_k;
+    const int step = epi == EPI_SPLIT16 ? 32 : 16;
     int best = p.BN;
     long long best_cost = -1;
     for (int bn = p.BN; bn >= 64; bn -= step) {
         const long long tiles = (long long)p.m_tiles * ((p.N + bn - 1) / bn), waves = (tiles + sms - 1) / sms;
-        const long long cost = waves * (nk * (2 * bn > 128 + bn ? 2 * bn : 128 + bn) + 600 + 8 * bn);
+        const long long cost = waves * (TILE_M + bn);
         if (best_cost < 0 || cost < best_cost) { best_cost = cost; best = bn; }
     }
     return best;
