@@ -481,8 +481,8 @@ def gdn_scan_float64(P, cw, cb, a_log, dt_bias, ow):
 @pytest.mark.parametrize("shift", [-12.0, -2.0, 2.0, 30.0, "mixed", "none"])
 def test_gdn_scan_at_every_strength_of_decay(L, shift):
     """The scan keeps the state divided by its decay within a chunk: decays of almost 1, of a few percent a token (the scale falls below its
-    line inside a chunk), of exactly 0, any mix of them, and none at all.  A float32 recurrence of 321 tokens stays within a few
-    hundred roundings (6e-8 each) of float64; measured 1.7e-7 to 4.1e-7, with the state decayed at every token instead 1.7e-7 to 5.1e-7."""
+    line inside a chunk), of exactly 0, any mix of them, and none at all.  Measured 1.7e-7 to 4.1e-7 from float64 (a rounding is 6e-8),
+    with the state decayed at every token instead 1.7e-7 to 5.1e-7; the bound is four times the larger."""
     import torch
     rng = np.random.default_rng(5)
     B = 2
@@ -500,7 +500,7 @@ def test_gdn_scan_at_every_strength_of_decay(L, shift):
     ref, got = gdn_scan_float64(P, cw, cb, a_log, dt, ow), on.cpu().numpy()
     err = float(np.linalg.norm(got - ref) / np.linalg.norm(ref))
     print(f"gdn_scan, decay {shift}: rel {err:.3e}")
-    assert np.isfinite(got).all() and err < 2e-5
+    assert np.isfinite(got).all() and err < 2e-6
 
 
 @pytest.mark.parametrize("recipe,stage,B", [("W3", "gdn_a", 2), ("W3", "gdn_b", 1), ("W1", "gdn_a", 3)])
