@@ -80,8 +80,7 @@ template <int ROWB> __device__ __forceinline__ uint32_t tile_off(int row, int ch
 // fetched meanwhile), then both triangular inverses at once, a half-warp each, rows of L read 128 bits at a time.  The
 // kernel is bound by issue and shared-memory latency, not by its 250 MB (64 x 2,048 tokens, 6 heads); with one block a warp
 // everywhere both kernels take 259 us there against 248.
-// (declared with a minimum of CTAs per SM: without one the assembler keeps the kernel at 40-48 registers by moving loads
-// next to their uses)
+// (declared with a minimum of CTAs per SM: without one the kernel gets 40-48 registers)
 constexpr int LF_PITCH = CB + 4, LF_SLOT = CB * LF_PITCH + 16;    // floats; the two slots start 16 banks apart
 template <int DK> struct PrepWarp {
     __align__(16) uint8_t k[CB * DK * 2], q[CB * DK * 2];

@@ -34,9 +34,9 @@ __device__ __forceinline__ void dot_columns(const float* __restrict__ X, int xp,
     const float* wp = Wt + n0;
     // The weights of D steps of four k are loaded before the first of them is used, so that D x 4 loads are in flight per
     // thread (with few clips per CTA the kernel is bound by the latency of exactly these loads).  This needs the registers
-    // for them: the kernels are declared with a minimum number of CTAs per SM, because without one the assembler keeps the
-    // register count low for occupancy by moving every load next to its use, which runs the steps one L2 round trip
-    // after the other (B = 512: 0.27 ms for the tail kernel against 0.14 ms).
+    // for them: the kernels are declared with a minimum number of CTAs per SM, because without one they get 32 to 37
+    // registers (-Xptxas -v) and the steps run one L2 round trip after the other (B = 512: 0.27 ms for the tail kernel against
+    // 0.14 ms).
     constexpr int D = TB >= 8 ? 4 : 8;
     static_assert(K % (4 * D) == 0, "the k loop walks whole groups of steps");
 #pragma unroll 1
